@@ -124,8 +124,8 @@ int32_t tmc_ctx_profile_read(tmc_ctx* ctx, int32_t max, char* names, double* ms,
  * setting gives identical meshes; the settings trade the latency of small calls against the
  * throughput of large ones.  Defaults follow the device's SM count; tmc_ctx_autotune measures. */
 enum {
-  TMC_TUNE_GROUP_LANES = 1,          /* lanes the DMC projection pass may fill with a group of lanes
-                                        per vertex (small meshes); 0 = one thread per vertex */
+  TMC_TUNE_GROUP_LANES = 1,          /* kept and read back, no effect: the DMC projection shares
+                                        its samples among the lanes of each warp at every size */
   TMC_TUNE_WARP_LIST_MAX = 2,        /* DMC float64-fallback lists up to this length run one warp
                                         per vertex (0 = one thread per vertex, retries by warp) */
   TMC_TUNE_VERTEX_BLOCKS_PER_SM = 3, /* grid cap of the per-vertex DMC passes, 1..64 */

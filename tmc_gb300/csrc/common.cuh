@@ -60,6 +60,8 @@ struct Grid {
   float org_hi[3], org_lo[3], sp_hi[3], sp_lo[3];
   float inv2_hi[3], inv2_lo[3];  // 1 / (2 * spacing)
   float iso_f;
+  float iso_lo;   // the isovalue's remainder: (iso_f, iso_lo) as ffx::ff_from_double makes it
+  bool iso_exact; // the isovalue is the float iso_f
   Div32 div_cx, div_cy;  // division by nx - 1 and ny - 1 (cell index -> i, j, k); set_divisors()
   // fused generation (single-volume launches): the classification evaluates the field from `gen` at
   // the float32 spacing gd instead of reading f, and writes each point once to gen_out (== f), which
@@ -338,7 +340,7 @@ __host__ __device__ __forceinline__ int64_t ceil_div(int64_t a, int64_t b) { ret
 // measures candidates on the caller's own volumes.
 struct Tuning {
   int sms = 1;
-  int64_t group_lanes = 0;        // lanes the projection pass may fill with lane groups (0: one thread per vertex)
+  int64_t group_lanes = 0;        // TMC_TUNE_GROUP_LANES (no effect)
   int64_t warp_list_max = 0;      // float64 fallback lists up to this length run one warp per vertex
   int vertex_blocks_per_sm = 32;  // grid cap of the per-vertex passes (rounded to whole waves)
   int emit_blocks_per_sm = 8;     // grid cap of the TMC emission kernel

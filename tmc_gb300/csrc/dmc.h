@@ -17,10 +17,6 @@ struct DmcVertexOut {
   float* vuvw;
 };
 
-namespace repr {
-struct ProjRecord;
-}
-
 struct DmcScratch {
   uint32_t* rec;                  // per listed cell (slot)
   int32_t* voff;                  // per listed cell (slot)
@@ -29,11 +25,11 @@ struct DmcScratch {
   unsigned long long* tile_sums;  // per scan tile
   unsigned long long* totals;     // [0] = (vertices << 32) | quads
   unsigned long long* stats;      // 8 counters
-  // two-pass vertices (per vertex): projection records, projected points, the one-pass list
-  repr::ProjRecord* proj;
+  // per vertex: the projected points, the one-pass list, the points that lack a coordinate
   float4* vp;
   uint32_t* fb_list;
-  unsigned* fb_count;             // [0] fb_list entries, [1] tail_list entries
+  uint32_t* w_list;
+  unsigned* fb_count;             // entries of [0] fb_list, [1] tail_list, [2] w_list
   uint32_t* tail_list;            // vertices without a valid 7x7 sample (26x26 retry)
   // listed cells (common.cuh): rec, voff and qoff hold one entry per listed cell at its slot
   CellMask* mask;                 // per 32 cells of the space
@@ -42,7 +38,6 @@ struct DmcScratch {
   uint8_t* vrank;                 // per vertex: rank among its cell's vertices (vwork: the cell's slot)
   unsigned* amb_n;                // listed cells with an ambiguous case (their slots wait in qoff)
 };
-constexpr size_t kProjRecordBytes = 144;  // sizeof(repr::ProjRecord)
 
 // Each launcher returns the number of kernels it launched.
 // Per-cell scratch is indexed in the cell space (space.n cells, padding included).

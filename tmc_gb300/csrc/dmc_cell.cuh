@@ -12,9 +12,13 @@ namespace tmc {
 //   bits 3-4   nQ: crossed interior edges among the cell's edges 0, 3, 8 (quads it owns)
 //   bits 5-28  for each edge e, 2 bits: rank of the used contour holding e
 //   bit  29    ambiguous case
+//   bit  30    some contour is used and some is not: the ranks do not say which edges belong to which
 __device__ __forceinline__ int rec_nv(uint32_t r) { return r & 7; }
 __device__ __forceinline__ int rec_nq(uint32_t r) { return (r >> 3) & 3; }
 __device__ __forceinline__ int rec_rank(uint32_t r, int e) { return (r >> (5 + 2 * e)) & 3; }
+
+__device__ __forceinline__ uint32_t rec_map(uint32_t r) { return (r >> 5) & 0xFFFFFFu; }  // all edges' ranks
+__device__ __forceinline__ bool rec_unused(uint32_t r) { return (r >> 30) & 1; }
 
 __device__ __forceinline__ bool edge_interior(const Grid& g, int i, int j, int k, int e) {
   const int off = edge_off(e), ax = edge_axis(e);
@@ -82,6 +86,7 @@ __device__ __forceinline__ uint32_t record_from_contours(const Grid& g, int i, i
   nq += ((em >> 0) & 1) && (inner || edge_interior(g, i, j, k, 0));
   nq += ((em >> 3) & 1) && (inner || edge_interior(g, i, j, k, 3));
   nq += ((em >> 8) & 1) && (inner || edge_interior(g, i, j, k, 8));
+  if (nv != 0 && nv != ncnt) rec |= 1u << 30;
   rec |= (uint32_t)nv | ((uint32_t)nq << 3);
   return rec;
 }

@@ -15,8 +15,7 @@
 //   dmc_classify_kernel  case, contours, per-cell record (counts + edge->vertex rank map) and
 //                        per-tile sums for the scan
 //   dmc_offsets_kernel   in-tile scan -> per-cell vertex / quad offsets
-//   dmc_vertex_setup_kernel, dmc_project_kernel (dmc_project_group_kernel for small meshes),
-//   dmc_vertex_finish_kernel
+//   dmc_vertex_point_kernel, dmc_vertex_w_kernel, dmc_vertex_finish_kernel
 //                        vertex representatives (cpp_dmc representative/projection) in float32
 //                        and float-float, normals, positions
 //   dmc_vertex_kernel    the vertices those leave, with every float64 fallback
@@ -32,8 +31,6 @@
 #include "scan.cuh"
 
 namespace tmc {
-
-static_assert(sizeof(repr::ProjRecord) == kProjRecordBytes, "record size");
 
 __constant__ uint64_t c_case_contour[256] = TMC_CASE_CONTOUR_INIT;
 
@@ -585,139 +582,178 @@ __global__ void __launch_bounds__(kVertexThreads) dmc_vertex_warp_kernel(CellSpa
   flush_stats(st, stats);
 }
 
-// Two-pass vertices, pass 1: contour, plane, sample coordinates, mean point -> one record per
-// vertex.  Only the vertex's own contour is evaluated: its edge points are summed and boxed as they
-// are computed (no point array, nothing in local memory).  Contours with neighbour-contour
-// exclusion go to the one-pass kernel's list.
-__global__ void __launch_bounds__(kVertexThreads, 5) dmc_vertex_setup_kernel(CellSpace space, const uint16_t* cellof, const uint8_t* vrank,
-                                                                              const uint32_t* vwork, int64_t nv,
-                                                                              repr::ProjRecord* recs, uint32_t* list,
-                                                                              unsigned* count,
-                                                                              unsigned long long* stats) {
-  __shared__ uint64_t cc[256];
-  for (int c = threadIdx.x; c < 256; c += blockDim.x) cc[c] = c_case_contour[c];
-  __syncthreads();
-  GridCache G;
-  int f64 = 0;
-  for (int64_t vidx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; vidx < nv;
-       vidx += (int64_t)gridDim.x * blockDim.x) {
+// Crossed edges of every MC case, two bits per edge (dmc_repr.cuh's edge sets)
+struct CaseEdges {
+  uint32_t m[256];
+};
+constexpr CaseEdges make_case_edges() {
+  CaseEdges t{};
+  for (int c = 0; c < 256; c++)
+    for (int e = 0; e < 12; e++) {
+      const int a = (int)((TMC_PK_EDGE_V0 >> (4 * e)) & 0xF), b = (int)((TMC_PK_EDGE_V1 >> (4 * e)) & 0xF);
+      t.m[c] |= (uint32_t)(((c >> a) ^ (c >> b)) & 1) << (2 * e);
+    }
+  return t;
+}
+__device__ const CaseEdges d_case_edges = make_case_edges();
+
+// Appends x to a list for the active lanes with `take` set: one atomic per warp.
+__device__ __forceinline__ void append(uint32_t* list, unsigned* count, bool take, uint32_t x) {
+  const unsigned am = __activemask(), bal = __ballot_sync(am, take);
+  if (!bal) return;
+  const int lane = threadIdx.x & 31, leader = __ffs(bal) - 1;
+  unsigned base = 0;
+  if (lane == leader) base = atomicAdd(count, (unsigned)__popc(bal));
+  base = __shfl_sync(am, base, leader);
+  if (take) list[base + __popc(bal & ((1u << lane) - 1u))] = x;
+}
+
+// The vertices' projected points, one lane per vertex.  The contour's edge set comes from the cell's
+// record and case, so no polygon is walked again; the frame of the search (repr::vertex_frame) sits
+// in shared memory, a column per lane, and nothing is written to memory but the point.
+// p (local coordinates) goes to vp, or w != 0 marks what is still open: 1 the one-pass kernels' list,
+// 4 + plane the missing coordinate of dmc_vertex_w_kernel's list.
+//
+// The number of samples a lane still has to bound after its first one varies (none for 70 % of the
+// vertices of the noise field, more than ten for 1 %): looping over its own, a lane would keep its
+// warp busy until the warp's largest number is reached (6 active lanes per instruction, measured).
+// So the warp lists all its lanes' samples and its lanes take them 32 at a time, whosever they are.
+// Bound by instruction issue (73 % active, 19 lanes per instruction, 68 registers, DRAM 210 MB).
+// 5.5 M vertices (320^3 noise field): 0.44 ms, 1.06 ms with the per-lane loops; the separate set-up
+// and projection kernels this replaces (a 144-byte record per vertex written and read in between,
+// nine samples bounded per vertex) took 1.15 + 0.85 ms.
+constexpr int kSampleWindow = 64;  // samples listed at a time
+template <bool kBatch>
+__global__ void __launch_bounds__(kVertexThreads) dmc_vertex_point_kernel(CellSpace space, const uint16_t* cellof,
+                                                                          const uint8_t* ccase, const uint32_t* rec,
+                                                                          const uint8_t* vrank, const uint32_t* vwork,
+                                                                          int64_t nv, float4* vp, uint32_t* list,
+                                                                          uint32_t* wlist, unsigned* count) {
+  constexpr int kWarps = kVertexThreads / 32;
+  constexpr unsigned kAll = 0xffffffffu;
+  __shared__ float frames[repr::kFrameFloats * kVertexThreads];
+  __shared__ uint16_t items[kWarps][kSampleWindow];
+  __shared__ repr::SampleBound bounds[kWarps][kSampleWindow];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  uint16_t* item = items[wid];
+  repr::SampleBound* bound = bounds[wid];
+  float* const warp_frames = frames + 32 * wid;
+  const repr::FrameCol F{warp_frames + lane, kVertexThreads};
+  const int64_t step = (int64_t)gridDim.x * kVertexThreads;
+  for (int64_t first = ((int64_t)blockIdx.x * kWarps + wid) * 32; first < nv; first += step) {  // warp-uniform
+    const int64_t vidx = first + lane;
+    const bool valid = vidx < nv;
+    int prj = -1;
+    ffx::ff iso{0, 0};
+    if (valid) {
+      const uint32_t slot = vwork[vidx];
+      const int rank = vrank[vidx];
+      const uint32_t r = rec[slot];
+      const uint32_t crossed = d_case_edges.m[__ldg(ccase + slot)];
+      const uint32_t vcell = slot_cell(cellof, slot);
+      const Grid& g = kBatch ? space.grids[__ldg(space.tile_vol + vcell / kScanTile)] : space.one;
+      int i, j, k;
+      cell_ijk(g, vcell - g.vbase, i, j, k);
+      float c[8];
+      load_corners(g, i, j, k, c);
+#pragma unroll
+      for (int q = 0; q < 8; q++) F[q] = c[q];
+      const uint32_t em = repr::edges_of_rank(rec_map(r), rank, crossed);
+      const int n = __popc(em);
+      // another contour of three edges excludes samples inside its box (one-pass kernels); in a cell
+      // with an unused contour some edges have no rank of their own
+      bool redo = rec_unused(r);
+      if (rec_nv(r) > 1 && n != 3)
+        for (int t = 0; t < rec_nv(r); t++)
+          redo = redo || (t != rank && __popc(repr::edges_of_rank(rec_map(r), t, crossed)) == 3);
+      iso = ffx::ff{g.iso_f, g.iso_lo};
+      if (!redo) prj = repr::vertex_frame(F, em, n, g.iso, iso, g.iso_exact);
+    }
+    repr::SampleSet S;
+    uint64_t need = 0, seen = 0;
+    int q0 = 0;
+    bool ring = false;
+    if (prj >= 0) {
+      q0 = repr::seed_sample(F);
+      seen = 1ull << q0;
+      S.add(repr::sample_bound(F, q0), q0);
+      // the seed not surely valid: its neighbours before everything else
+      ring = !(S.m < INFINITY);
+      need = (ring ? repr::ring_of(q0) : repr::samples_within(F, S.m)) & ~seen;
+    }
+    for (;;) {
+      const int c = __popcll(need);
+      int upto = c;  // inclusive scan of the lanes' numbers
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(kAll, upto, o);
+        if (lane >= o) upto += y;
+      }
+      const int from = upto - c, total = __shfl_sync(kAll, upto, 31);
+      for (int w = 0; w < total; w += kSampleWindow) {
+        const int end = min(w + kSampleWindow, total);
+        __syncwarp();  // the frames are written, the previous window's bounds are read
+        if (from < end && upto > w) {
+          uint64_t m = need;
+          for (int k = from; k < min(upto, end); k++, m &= m - 1)
+            if (k >= w) item[k - w] = (uint16_t)(lane << 6 | (__ffsll((long long)m) - 1));
+        }
+        __syncwarp();
+        for (int k = w + lane; k < end; k += 32) {
+          const int x = item[k - w];
+          bound[k - w] = repr::sample_bound(repr::FrameCol{warp_frames + (x >> 6), kVertexThreads}, x & 63);
+        }
+        __syncwarp();
+        for (int k = max(from, w); k < min(upto, end); k++) S.add(bound[k - w], item[k - w] & 63);
+      }
+      if (!__any_sync(kAll, ring)) break;
+      seen |= need;
+      need = ring ? repr::samples_within(F, S.m) & ~seen : 0ull;
+      ring = false;
+    }
+    float p[3] = {0, 0, 0};
+    int what = repr::kRedo;
+    if (prj >= 0 && S.decided()) what = repr::sample_point(F, S.q1, prj, iso, p);
+    __syncwarp();  // the frames are read
+    if (valid) {
+      append(list, count, what == repr::kRedo, (uint32_t)vidx);
+      append(wlist, count + 2, what == repr::kW64, (uint32_t)vidx);
+      vp[vidx] =
+          make_float4(p[0], p[1], p[2], what == repr::kFound ? 0.0f : (what == repr::kRedo ? 1.0f : 4.0f + prj));
+    }
+  }
+}
+
+// The points whose last coordinate needs float64 (mostly bilinear values exactly on a float midpoint,
+// where a box spans the whole cell and the sample coordinates are eighths), listed by
+// dmc_vertex_point_kernel: a few per cent of the vertices, so that there nearly every warp would
+// wait for the float64 pipe; here every lane has one.
+__global__ void __launch_bounds__(kVertexThreads) dmc_vertex_w_kernel(CellSpace space, const uint16_t* cellof,
+                                                                      const uint32_t* vwork, const uint32_t* wlist,
+                                                                      const unsigned* count, float4* vp,
+                                                                      unsigned long long* stats) {
+  const unsigned n = count[2];
+  for (unsigned a = blockIdx.x * blockDim.x + threadIdx.x; a < n; a += gridDim.x * blockDim.x) {
+    const uint32_t vidx = wlist[a];
     const uint32_t vcell = slot_cell(cellof, vwork[vidx]);
-    const int rank = vrank[vidx];
-    G.load(space, vcell);
-    const Grid& g = G.g;
+    const Grid& g = space.grids ? space.grids[__ldg(space.tile_vol + vcell / kScanTile)] : space.one;
     int i, j, k;
     cell_ijk(g, vcell - g.vbase, i, j, k);
     float u[8];
     load_corners(g, i, j, k, u);
-    const uint64_t c = dmc_polygon(mc_case(u, g.iso_up), u, g.iso, cc);
-    // the rank-th used contour (one with an interior edge), as vertex_contour selects it
-    const int ncnt = cnt_count(c);
-    int flat = 0, seen = 0, tsel = -1, tstart = 0;
-    for (int t = 0; t < ncnt && tsel < 0; t++) {
-      const int sz = cnt_size(c, t);
-      bool used = false;
-      for (int q = 0; q < sz; q++) used = used || edge_interior(g, i, j, k, cnt_edge(c, flat + q));
-      if (used) {
-        if (seen == rank) {
-          tsel = t;
-          tstart = flat;
-        }
-        seen++;
-      }
-      flat += sz;
-    }
-    repr::ProjRecord& R = recs[vidx];  // written in place: no copy in local memory
-    bool ok = tsel >= 0;              // cannot fail: counted
-    if (ok) {
-      const int n = cnt_size(c, tsel);
-      repr::ContourAcc A;
-      repr::contour_acc(u, g.iso, G.iso_ff, c, tstart, n, A);
-      int f64c = 0;
-      ok = repr::projection_record_acc(u, g.iso, c, tsel, tstart, n, A, R, f64c);
-      if (ok) f64 += f64c;  // contours redone by the one-pass kernel are counted there
-    }
-    if (!ok) {
-      R.prj = -1;
-      list[atomicAdd(count, 1u)] = (uint32_t)vidx;
-    }
+    const float4 q = vp[vidx];
+    float p[3] = {q.x, q.y, q.z};
+    const int prj = (int)q.w - 4;
+    const float w = repr::vertex_w_f64(u, g.iso, p, prj);
+#pragma unroll
+    for (int d = 0; d < 3; d++)
+      if (d == 2 - prj) p[d] = w;
+    vp[vidx] = make_float4(p[0], p[1], p[2], 0.0f);
   }
-  if (f64) atomicAdd(stats + 7, (unsigned long long)f64);
+  if (blockIdx.x == 0 && threadIdx.x == 0 && n) atomicAdd(stats + 7, 3ull * n);
 }
 
-// Two-pass vertices, pass 2: the projection from the record.  p (local coordinates) goes to vp;
-// vertices that need float64 go to the one-pass kernel's list (vp.w = 1 marks them).
-__global__ void __launch_bounds__(kVertexThreads) dmc_project_kernel(const repr::ProjRecord* recs, int64_t nv,
-                                                                     float4* vp, uint32_t* list, unsigned* count,
-                                                                     unsigned long long* stats) {
-  __shared__ float sample_lb[49 * kVertexThreads];
-  int f64 = 0;
-  for (int64_t vidx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; vidx < nv;
-       vidx += (int64_t)gridDim.x * blockDim.x) {
-    const repr::ProjRecord& R = recs[vidx];
-    if (R.prj < 0) {  // already listed by the set-up pass
-      vp[vidx] = make_float4(0, 0, 0, 1);
-      continue;
-    }
-    float p[3] = {0, 0, 0};
-    int f = 0;
-    const int r = repr::projection_from_record(R, p, sample_lb + threadIdx.x, kVertexThreads, f);
-    if (r != 0) list[atomicAdd(count, 1u)] = (uint32_t)vidx;  // redone (and counted) by the one-pass kernel
-    else f64 += f;
-    vp[vidx] = make_float4(p[0], p[1], p[2], r != 0 ? 1.0f : 0.0f);
-  }
-  if (f64) atomicAdd(stats + 7, (unsigned long long)f64);
-}
-
-// Two-pass vertices, pass 2 for small meshes: G lanes per record (G a power of two, 2..32) split
-// its 49 samples, so that a call's latency is that of ~49/G exact samples instead of one thread's
-// serial projection.  Same outputs and lists as dmc_project_kernel.
-__global__ void __launch_bounds__(kVertexThreads) dmc_project_group_kernel(const repr::ProjRecord* recs, int64_t nv,
-                                                                           int G, float4* vp, uint32_t* list,
-                                                                           unsigned* count,
-                                                                           unsigned long long* stats) {
-  const int lane = threadIdx.x & 31;
-  const int gl = lane & (G - 1);
-  const int64_t per_warp = 32 / G;
-  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  int f64 = 0;
-  // base is the same on every lane of a warp, so all lanes reach the shuffles
-  for (int64_t base = warp * per_warp; base < nv; base += nwarps * per_warp) {
-    const int64_t vidx = base + lane / G;
-    const bool valid = vidx < nv;
-    const repr::ProjRecord& R = recs[valid ? vidx : base];
-    const bool listed = R.prj < 0;  // already listed by the set-up pass (same for the whole group)
-    repr::LaneBest b = repr::lane_none();
-    bool unc = false;
-    repr::ProjCtx P;
-    if (valid && !listed) {
-      repr::ctx_from_record(R, P);
-      b = repr::record_lane(P, R, gl, G, f64, unc);
-    }
-    for (int o = G >> 1; o > 0; o >>= 1) {
-      repr::LaneBest x;
-      x.d = __shfl_xor_sync(0xffffffffu, b.d, o);
-      x.w = __shfl_xor_sync(0xffffffffu, b.w, o);
-      x.q = __shfl_xor_sync(0xffffffffu, b.q, o);
-      unc = __shfl_xor_sync(0xffffffffu, (int)unc, o) != 0 || unc;
-      if (repr::lane_better(x, b)) b = x;
-    }
-    if (!valid || gl != 0) continue;
-    if (listed) {
-      vp[vidx] = make_float4(0, 0, 0, 1);
-    } else if (unc || b.q == repr::kNoSample) {
-      list[atomicAdd(count, 1u)] = (uint32_t)vidx;  // redone (and counted) by the one-pass kernels
-      vp[vidx] = make_float4(0, 0, 0, 1);
-    } else {
-      float p[3];
-      repr::lane_point(P, R.us, R.vs, 7, b, p);
-      vp[vidx] = make_float4(p[0], p[1], p[2], 0.0f);
-    }
-  }
-  if (f64) atomicAdd(stats + 7, (unsigned long long)f64);
-}
-
-// Two-pass vertices, pass 3: positions, normals and local coordinates of the projected vertices.
+// Positions, normals and local coordinates of the projected vertices.
 template <bool kFF>
 __global__ void __launch_bounds__(kVertexThreads, 4) dmc_vertex_finish_kernel(CellSpace space, const uint16_t* cellof,
                                                                             const uint32_t* vwork,
@@ -907,8 +943,9 @@ int dmc_front_emit(const CellSpace& space, DmcScratch& s, DmcVertexOut vo, int64
         s.mask, s.rec, s.tile_sums, tiles, s.voff, s.qoff, s.vwork, s.vrank);
   }
   // per-vertex grids: whole waves of each kernel's resident blocks
-  static const int r_setup = resident_blocks(dmc_vertex_setup_kernel, kVertexThreads);
-  static const int r_project = resident_blocks(dmc_project_kernel, kVertexThreads);
+  static const int r_point = resident_blocks(dmc_vertex_point_kernel<false>, kVertexThreads);
+  static const int r_point_batch = resident_blocks(dmc_vertex_point_kernel<true>, kVertexThreads);
+  static const int r_w = resident_blocks(dmc_vertex_w_kernel, kVertexThreads);
   static const int r_finish = resident_blocks(dmc_vertex_finish_kernel<true>, kVertexThreads);
   static const int r_finish32 = resident_blocks(dmc_vertex_finish_kernel<false>, kVertexThreads);
   static const int r_quad = resident_blocks(dmc_quad_kernel<false>, kQuadThreads);
@@ -917,21 +954,17 @@ int dmc_front_emit(const CellSpace& space, DmcScratch& s, DmcVertexOut vo, int64
     return (unsigned)wave_grid(resident, sms, tu.vertex_blocks_per_sm, nv, kVertexThreads);
   };
   {
-    Stage t(prof, "dmc_vertex_setup", st);
-    cudaMemsetAsync(s.fb_count, 0, 2 * sizeof(unsigned), st);
-    dmc_vertex_setup_kernel<<<vgrid(r_setup), kVertexThreads, 0, st>>>(space, s.cellof, s.vrank, s.vwork, nv, s.proj, s.fb_list,
-                                                                       s.fb_count, s.stats);
-  }
-  {
-    Stage t(prof, "dmc_project", st);
-    // lanes per record: as many as the tuning's lane budget allows (small meshes), else one thread
-    int G = 1;
-    while (G < 32 && nv * G * 2 <= tu.group_lanes) G *= 2;
-    if (G >= 4)
-      dmc_project_group_kernel<<<(unsigned)std::max<int64_t>(1, ceil_div(nv * G, kVertexThreads)), kVertexThreads, 0,
-                                 st>>>(s.proj, nv, G, s.vp, s.fb_list, s.fb_count, s.stats);
+    Stage t(prof, "dmc_vertex_point", st);
+    cudaMemsetAsync(s.fb_count, 0, 3 * sizeof(unsigned), st);
+    if (space.grids)
+      dmc_vertex_point_kernel<true><<<vgrid(r_point_batch), kVertexThreads, 0, st>>>(
+          space, s.cellof, s.ccase, s.rec, s.vrank, s.vwork, nv, s.vp, s.fb_list, s.w_list, s.fb_count);
     else
-      dmc_project_kernel<<<vgrid(r_project), kVertexThreads, 0, st>>>(s.proj, nv, s.vp, s.fb_list, s.fb_count, s.stats);
+      dmc_vertex_point_kernel<false><<<vgrid(r_point), kVertexThreads, 0, st>>>(
+          space, s.cellof, s.ccase, s.rec, s.vrank, s.vwork, nv, s.vp, s.fb_list, s.w_list, s.fb_count);
+    // the list's length is only known on the device: one wave, sized for a tenth of the vertices
+    dmc_vertex_w_kernel<<<(unsigned)wave_grid(r_w, sms, 1, ceil_div(nv, 10), kVertexThreads), kVertexThreads, 0, st>>>(
+        space, s.cellof, s.vwork, s.w_list, s.fb_count, s.vp, s.stats);
   }
   {
     Stage t(prof, "dmc_vertex_finish", st);

@@ -859,10 +859,9 @@ TMC_HD void representative_fast(const float u[8], double iso, uint64_t c, int t,
 }
 
 // ---------------------------------------------------------------------------------------------
-// two-pass form: a set-up pass writes one ProjRecord per vertex, a projection pass reads it.  Each
-// pass is a small kernel (registers, instruction cache); contours that need anything beyond the
-// float32 / float-float path (the neighbour-contour exclusion, a float64 sample, the 26x26 tail) are
-// left to the one-pass kernel.
+// two-pass form: a set-up writes one ProjRecord per vertex, a projection reads it; contours that need
+// anything beyond the float32 / float-float path are refused.  Host code: the CPU checks compare its
+// 3x3 search with the other forms (the kernels use the one-step form below).
 // ---------------------------------------------------------------------------------------------
 struct alignas(16) ProjRecord {
   float fp[8];        // corner values permuted to the projection frame
@@ -956,6 +955,348 @@ TMC_HD int projection_from_record(const ProjRecord& R, float p_out[3], float* bu
     p_out[P.W] = pt[2];
   }
   return r;
+}
+
+// ---------------------------------------------------------------------------------------------
+// one-step form: from a contour's edge set to the projected point, nothing written in between.
+//
+// What makes it cheap (counted on the noise, blob, periodic and saddle fields):
+//  * the contour is a set of edges.  Its mean point and box need no order and no points: a coordinate
+//    off the edge's axis is 0 or 1, so those are population counts and mask tests, and only the
+//    parameters themselves (at most four per axis) are summed and boxed.
+//  * the search starts from the one sample nearest to the mean point instead of the 3x3 around it:
+//    its distance already excludes nearly every other sample by the in-plane distance (1.85 float32
+//    evaluations per contour instead of 9.1 on noise, 1.2 on smooth fields, 5.3 on seeded saddles).
+//  * in more than 99.5 % of contours one sample is left whose validity is certain.  It is the
+//    reference's choice whatever its exact distance, so only its w needs its exact rounding.
+// Everything else (more than one candidate left, no certain sample, a neighbour contour that may
+// exclude samples, an uncertified box) returns kRedo: the one-pass kernels decide.
+// ---------------------------------------------------------------------------------------------
+// Edge sets with two bits per edge (bit 2e), the layout of the cell records' edge -> rank map.
+constexpr uint32_t spread_edges(uint32_t m) {
+  uint32_t r = 0;
+  for (int e = 0; e < 12; e++) r |= ((m >> e) & 1u) << (2 * e);
+  return r;
+}
+constexpr uint32_t kAllEdges = 0x555555u;
+// edges off axis d whose coordinate d is 1 / 0
+TMC_HD uint32_t edges_one(int d) {
+  constexpr uint32_t x = spread_edges(0x622), y = spread_edges(0xC44), z = spread_edges(0x0F0);
+  return d == 0 ? x : (d == 1 ? y : z);
+}
+TMC_HD uint32_t edges_zero(int d) {
+  constexpr uint32_t x = spread_edges(0x988), y = spread_edges(0x311), z = spread_edges(0x00F);
+  return d == 0 ? x : (d == 1 ? y : z);
+}
+
+TMC_HD int popc32(uint32_t x) {
+#ifdef __CUDA_ARCH__
+  return __popc(x);
+#else
+  return __builtin_popcount(x);
+#endif
+}
+TMC_HD int lowest_bit32(uint32_t x) {
+#ifdef __CUDA_ARCH__
+  return __ffs((int)x) - 1;
+#else
+  return __builtin_ctz(x);
+#endif
+}
+
+// the edges that carry rank r in a cell record's edge -> rank map (two bits per edge), among `crossed`
+TMC_HD uint32_t edges_of_rank(uint32_t map, int r, uint32_t crossed) {
+  const uint32_t x = map ^ ((uint32_t)r * kAllEdges);
+  return ~(x | (x >> 1)) & crossed;
+}
+
+enum { kFound = 0, kRedo = 1, kW64 = 2 };
+
+// The edge parameter as edge_param_fast finds it; false when it is not certified (the caller then
+// takes the float64 value).  exact_iso: the isovalue is a float, so a corner at it gives exactly 0.
+// Ranges: a denominator or numerator near the ends of the float range is left to float64.
+TMC_HD bool edge_param_certain(float f0, float f1, ff iso, bool exact_iso, float& l) {
+  ff t = ffx::two_sum(iso.hi, -f0);
+  t.lo += iso.lo;
+  const ff num = ffx::quick_two_sum(t.hi, t.lo);
+  const ff den = ffx::two_sum(f1, -f0);
+  const float ad = fabsf(den.hi);
+  if (!(ad > 0x1p-60f && ad < 0x1p120f)) return false;
+  if (num.hi == 0.0f && exact_iso) {
+    l = 0.0f;
+    return true;
+  }
+  if (!(fabsf(num.hi) > 0x1p-90f)) return false;
+  const float r = ffx::rcp_est(den.hi);
+  const ff q = ffx::ff_quot(num, den, r);
+  l = q.hi;
+  return ffx::ff_certain(q, fabsf(q.hi) * 0x1p-42f + fmaxf(fabsf(iso.hi), fabsf(f0)) * 0x1p-45f * fabsf(r));
+}
+
+// fl32(lo + i (hi - lo) / 8) as sample_coords: lo (8 - i) / 8 + hi i / 8 with both products' errors
+// kept, so that one addition rounds.  Exact (hence the reference's float) when both ends are 0 or
+// their exponents are at most 17 apart and away from underflow (sample_range_exact): every term is
+// then a multiple of ulp(lo) / 8 and the sum of the three small ones has at most 24 bits.
+TMC_HD float sample_at(float lo, float hi, int i) {
+  const float c = (float)i * 0.125f;
+  const ff a = ffx::two_prod(hi, c), b = ffx::two_prod(lo, 1.0f - c);
+  const ff s = ffx::two_sum(a.hi, b.hi);
+  return s.hi + (s.lo + (a.lo + b.lo));
+}
+TMC_HD bool sample_range_exact(float lo, float hi) {
+  const int eh = (int)(ffx::fbits(hi) >> 23), el = (int)(ffx::fbits(lo) >> 23);  // both >= 0
+  return (hi == 0.0f || eh > 64) && (lo == 0.0f || (el > 64 && eh - el <= 17));
+}
+
+// The reference's float of one face's bilinear value at (u, v), f the face's four corners and sabs
+// their largest magnitude; false when its rounding is not certified.  The weights are in [0, 1] and
+// sum to one, so each of the dozen float-float operations errs by at most 2^-46 sabs.
+TMC_HD bool bilinear_certain(float f0, float f1, float f2, float f3, float sabs, float u, float v, float& g) {
+  const float omu = 1 - u, omv = 1 - v;
+  const ff A = ffx::ff_add_abs(ffx::two_prod(omu, f0), ffx::two_prod(u, f1));
+  const ff B = ffx::ff_add_abs(ffx::two_prod(omu, f2), ffx::two_prod(u, f3));
+  ff a = ffx::two_prod(A.hi, omv), b = ffx::two_prod(B.hi, v);
+  a.lo = ffx::fma_rn(A.lo, omv, a.lo);
+  b.lo = ffx::fma_rn(B.lo, v, b.lo);
+  const ff G = ffx::ff_add_abs(a, b);
+  g = G.hi;
+  return sabs > 0x1p-80f && ffx::ff_certain(G, sabs * 0x1p-43f);
+}
+
+// One contour's search, as the lanes of a warp share it: the projection frame (corners permuted so
+// that the plane's axes come first), the box and the mean point in it.  Kept as a column of floats
+// (shared memory on the GPU, one column per lane) so that any lane can estimate any lane's samples.
+enum { kFp = 0, kUlo = 8, kUhi, kVlo, kVhi, kWlo, kWhi, kPu, kPv, kPw, kSabsLo, kSabsHi, kIso, kIsoErr, kFrameFloats };
+struct FrameCol {
+  float* p;
+  int stride;
+  TMC_HD float& operator[](int f) const { return p[f * stride]; }
+};
+
+// The frame of the contour with edge set `em` (n edges) of the cell whose corners are the first
+// eight floats of the column; returns its projection plane, or -1 when the one-pass kernels must
+// decide.
+TMC_HD int vertex_frame(const FrameCol& F, uint32_t em, int n, double iso, ff iso_ff, bool exact_iso) {
+  // edge parameters: sums and extremes per axis
+  float sh[3] = {0, 0, 0}, sl[3] = {0, 0, 0}, mn[3] = {1, 1, 1}, mx[3] = {0, 0, 0};
+  bool ok = true;
+#pragma unroll 1
+  for (uint32_t m = em; m; m &= m - 1) {
+    const int e = lowest_bit32(m) >> 1;
+    const int ax = e < 8 ? (e & 1) : 2;
+    const int v0 = nibr(EDGE_V0, e);
+    const float f0 = F[v0], f1 = F[v0 + (1 << ax)];
+    float l;
+    if (!edge_param_certain(f0, f1, iso_ff, exact_iso, l)) l = edge_param_f64(iso, f0, f1) + 0.0f;
+    ok = ok && l >= 0.0f && l <= 1.0f;  // not so for values at the ends of the float range
+    const ff t = ffx::two_sum(ax == 0 ? sh[0] : (ax == 1 ? sh[1] : sh[2]), l);
+#pragma unroll
+    for (int d = 0; d < 3; d++)
+      if (ax == d) {
+        sh[d] = t.hi;
+        sl[d] += t.lo;
+        mn[d] = fminf(mn[d], l);
+        mx[d] = fmaxf(mx[d], l);
+      }
+  }
+  if (!ok) return -1;
+  // mean point (the float within 2^-23 of the reference's float64 mean) and box
+  ff pm[3];
+  float box[3][2];
+  const float fn = (float)n, rn = ffx::rcp_est(fn);
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    ff t = ffx::two_sum((float)popc32(em & edges_one(d)), sh[d]);
+    t.lo += sl[d];
+    const float q1 = t.hi * rn;
+    pm[d] = ffx::quick_two_sum(q1, (ffx::fma_rn(-q1, fn, t.hi) + t.lo) * rn);
+    box[d][0] = (em & edges_zero(d)) ? 0.0f : mn[d];
+    box[d][1] = (em & edges_one(d)) ? 1.0f : mx[d];
+  }
+  float f[8];
+#pragma unroll
+  for (int q = 0; q < 8; q++) f[q] = F[q];
+  const int prj = n >= 6 ? plane_from_gradient_f(f, pm[0].hi, pm[1].hi, pm[2].hi) : plane_from_extent_box_ff(box);
+  if (prj < 0) return -1;
+  // the frame's axes: (A, B, W) = (x, y, z), (x, z, y) or (y, z, x)
+  if (prj != 0) {
+    const float x1 = f[1], x2 = f[2], x3 = f[3], x5 = f[5], x6 = f[6];
+    F[1] = prj == 1 ? x1 : x2;
+    F[2] = f[4];
+    F[3] = prj == 1 ? x5 : x6;
+    F[4] = prj == 1 ? x2 : x1;
+    F[5] = x3;
+    F[6] = prj == 1 ? x6 : x5;
+  }
+  const float lo4 = prj == 0 ? fmaxf(fabsf(f[1]), fabsf(f[2])) : fmaxf(fabsf(prj == 1 ? f[1] : f[2]), fabsf(f[4]));
+  const float hi4 = prj == 0 ? fmaxf(fabsf(f[5]), fabsf(f[6])) : fmaxf(fabsf(prj == 1 ? f[6] : f[5]), fabsf(f[3]));
+  F[kSabsLo] = fmaxf(fmaxf(fabsf(f[0]), lo4), fabsf(prj == 0 ? f[3] : (prj == 1 ? f[5] : f[6])));
+  F[kSabsHi] = fmaxf(fmaxf(fabsf(f[7]), hi4), fabsf(prj == 0 ? f[4] : (prj == 1 ? f[2] : f[1])));
+  F[kPu] = prj == 2 ? pm[1].hi : pm[0].hi;
+  F[kPv] = prj == 0 ? pm[1].hi : pm[2].hi;
+  F[kPw] = prj == 0 ? pm[2].hi : (prj == 1 ? pm[1].hi : pm[0].hi);
+  const float ulo = prj == 2 ? box[1][0] : box[0][0], uhi = prj == 2 ? box[1][1] : box[0][1];
+  const float vlo = prj == 0 ? box[1][0] : box[2][0], vhi = prj == 0 ? box[1][1] : box[2][1];
+  F[kUlo] = ulo;
+  F[kUhi] = uhi;
+  F[kVlo] = vlo;
+  F[kVhi] = vhi;
+  float wlo, whi;
+  w_window(prj == 0 ? box[2][0] : (prj == 1 ? box[1][0] : box[0][0]),
+           prj == 0 ? box[2][1] : (prj == 1 ? box[1][1] : box[0][1]), wlo, whi);
+  F[kWlo] = wlo;
+  F[kWhi] = whi;
+  F[kIso] = iso_ff.hi;
+  F[kIsoErr] = fabsf(iso_ff.lo) + fabsf(iso_ff.hi) * 0x1p-30f;
+  return sample_range_exact(ulo, uhi) && sample_range_exact(vlo, vhi) ? prj : -1;
+}
+
+// Sample q = 7 i + j of a frame in float32.  Lower and upper bounds of its distance as the reference
+// rounds it: lb = +inf when it is surely not valid, ub = +inf unless it surely is.
+struct SampleBound {
+  float lb, ub;
+};
+TMC_HD SampleBound sample_bound(const FrameCol& F, int q) {
+  const int i = q / 7, j = q - 7 * i;
+  const float u = sample_at(F[kUlo], F[kUhi], i + 1), v = sample_at(F[kVlo], F[kVhi], j + 1);
+  const float omu = 1 - u, omv = 1 - v;
+  const float A1 = ffx::fma_rn(u, F[1], omu * F[0]), B1 = ffx::fma_rn(u, F[3], omu * F[2]);
+  const float A2 = ffx::fma_rn(u, F[5], omu * F[4]), B2 = ffx::fma_rn(u, F[7], omu * F[6]);
+  const float g1 = ffx::fma_rn(v, B1, omv * A1), g2 = ffx::fma_rn(v, B2, omv * A2);
+  const float Eg1 = F[kSabsLo] * 0x1p-20f + fabsf(g1) * 0x1p-23f;
+  const float Eg2 = F[kSabsHi] * 0x1p-20f + fabsf(g2) * 0x1p-23f;
+  const float den = g2 - g1, ad = fabsf(den);
+  const float Eden = (Eg1 + Eg2 + ad * 0x1p-23f) * 1.0001f;
+  // w unknown (includes g1 == g2), or a denominator the reciprocal estimate does not serve
+  if (!(ad > 2 * Eden && ad > 0x1p-100f && ad < 0x1p120f)) return SampleBound{0.0f, INFINITY};
+  const float num = F[kIso] - g1;
+  const float Enum = Eg1 + F[kIsoErr] + fabsf(num) * 0x1p-23f;
+  const float w = num * ffx::rcp_est(den);  // within 2^-21
+  const float aw = fabsf(w);
+  const float Ew = ((Enum + aw * Eden) * ffx::rcp_est(ad - Eden) + aw * 0x1p-20f) * 1.0001f + 1e-30f;
+  const float wlo = F[kWlo], whi = F[kWhi];
+  if (w + Ew < wlo || w - Ew > whi) return SampleBound{INFINITY, INFINITY};
+  const float Ep = 0x1p-22f;
+  const float e0 = F[kPu] - u, e1 = F[kPv] - v, e2 = F[kPw] - w;
+  const float D = e0 * e0 + e1 * e1 + e2 * e2;
+  const float ED = (2 * (fabsf(e0) + fabsf(e1)) * Ep + 2 * fabsf(e2) * (Ew + Ep) + (Ew + Ep) * (Ew + Ep) +
+                    2 * Ep * Ep + D * 0x1p-20f) * 1.0001f + 1e-30f;
+  return SampleBound{fmaxf(D - ED, 0.0f), w - Ew >= wlo && w + Ew <= whi ? D + ED : INFINITY};
+}
+
+// The sample nearest to the mean point (a guess is enough: it is only where the search starts)
+TMC_HD int seed_sample(const FrameCol& F) {
+  const float du = (F[kUhi] - F[kUlo]) * 0.125f, dv = (F[kVhi] - F[kVlo]) * 0.125f;
+  const int i = du > 0 ? (int)fminf(fmaxf((F[kPu] - F[kUlo]) * ffx::rcp_est(du) + 0.5f, 1.0f), 7.0f) - 1 : 0;
+  const int j = dv > 0 ? (int)fminf(fmaxf((F[kPv] - F[kVlo]) * ffx::rcp_est(dv) + 0.5f, 1.0f), 7.0f) - 1 : 0;
+  return 7 * i + j;
+}
+// its neighbours in the 7x7 grid, itself included
+TMC_HD uint64_t ring_of(int q) {
+  const int i = q / 7, j = q - 7 * i;
+  const uint64_t row = (uint64_t)((7u << j) >> 1 & 0x7Fu);
+  return (row << (7 * i)) | (i > 0 ? row << (7 * i - 7) : 0ull) | (i < 6 ? row << (7 * i + 7) : 0ull);
+}
+// the samples whose in-plane distance, a lower bound of the distance whatever w is, is within m
+TMC_HD uint64_t samples_within(const FrameCol& F, float m) {
+  const float Ep = 0x1p-20f;  // the mean point's and the coordinates' roundings
+  const float pu = F[kPu], pv = F[kPv], ulo = F[kUlo], vlo = F[kVlo];
+  const float du = (F[kUhi] - ulo) * 0.125f, dv = (F[kVhi] - vlo) * 0.125f;
+  float e1s[7];
+#pragma unroll
+  for (int j = 0; j < 7; j++) {
+    const float e = fmaxf(fabsf(pv - (vlo + (float)(j + 1) * dv)) - Ep, 0.0f);
+    e1s[j] = e * e * (1.0f - 0x1p-19f);
+  }
+  uint64_t in = 0;
+#pragma unroll
+  for (int i = 0; i < 7; i++) {
+    const float e = fmaxf(fabsf(pu - (ulo + (float)(i + 1) * du)) - Ep, 0.0f);
+    const float room = m - e * e * (1.0f - 0x1p-19f);
+    unsigned row = 0;
+#pragma unroll
+    for (int j = 0; j < 7; j++) row |= (unsigned)(e1s[j] <= room) << j;
+    in |= (uint64_t)row << (7 * i);
+  }
+  return in;
+}
+
+// The samples seen so far: m the smallest upper bound, l1 (sample q1) and l2 the two smallest lower
+// bounds.  l2 > m: only q1 can have the smallest distance, and it is surely valid (the sample with
+// upper bound m has a lower bound within m, so it is q1).
+struct SampleSet {
+  float m = INFINITY, l1 = INFINITY, l2 = INFINITY;
+  int q1 = 0;
+  TMC_HD void add(SampleBound b, int q) {
+    m = fminf(m, b.ub);
+    l2 = fminf(l2, fmaxf(l1, b.lb));
+    if (b.lb < l1) {
+      l1 = b.lb;
+      q1 = q;
+    }
+  }
+  TMC_HD bool decided() const { return m < INFINITY && l2 > m; }
+};
+
+// The representative at sample q of a frame: p complete (kFound), or but for its coordinate W = 2 -
+// prj, whose rounding needs float64 (kW64, vertex_w_f64).  w = (iso - g1) / (g2 - g1) of the
+// reference's floats g1, g2.
+TMC_HD int sample_point(const FrameCol& F, int q, int prj, ff iso_ff, float p[3]) {
+  const int i = q / 7, j = q - 7 * i;
+  const float u = sample_at(F[kUlo], F[kUhi], i + 1), v = sample_at(F[kVlo], F[kVhi], j + 1);
+  float g1, g2;
+  bool ok = bilinear_certain(F[0], F[1], F[2], F[3], F[kSabsLo], u, v, g1);
+  ok = bilinear_certain(F[4], F[5], F[6], F[7], F[kSabsHi], u, v, g2) && ok;
+  const float den = g2 - g1, ad = fabsf(den);  // the reference subtracts the two floats
+  ff t = ffx::two_sum(iso_ff.hi, -g1);
+  t.lo += iso_ff.lo;
+  const ff num = ffx::quick_two_sum(t.hi, t.lo);
+  const float r = ffx::rcp_est(den);
+  const ff W = ffx::ff_quot(num, ffx::ff_from(den), r);
+  ok = ok && ad > 0x1p-60f && ad < 0x1p120f && fabsf(num.hi) > 0x1p-90f &&
+       ffx::ff_certain(W, fabsf(W.hi) * 0x1p-42f + fmaxf(fabsf(iso_ff.hi), fabsf(g1)) * 0x1p-45f * fabsf(r));
+  p[0] = prj == 2 ? W.hi : u;
+  p[1] = prj == 0 ? v : (prj == 1 ? W.hi : u);
+  p[2] = prj == 0 ? W.hi : v;
+  return ok ? kFound : kW64;
+}
+
+// The search on one thread (the order of the kernel's rounds; the CPU checks run it).
+TMC_HD int vertex_point(const FrameCol& F, uint32_t em, int n, double iso, ff iso_ff, bool exact_iso, float p[3],
+                        int& prj) {
+  prj = vertex_frame(F, em, n, iso, iso_ff, exact_iso);
+  if (prj < 0) return kRedo;
+  SampleSet S;
+  const int q0 = seed_sample(F);
+  S.add(sample_bound(F, q0), q0);
+  uint64_t seen = 1ull << q0;
+  for (int round = 0; round < 2; round++) {
+    const bool ring = round == 0 && !(S.m < INFINITY);
+    uint64_t need = (ring ? ring_of(q0) : samples_within(F, S.m)) & ~seen;
+    seen |= need;
+    for (; need; need &= need - 1) {
+      const int q = lowest_bit(need);
+      S.add(sample_bound(F, q), q);
+    }
+    if (!ring) break;
+  }
+  if (!S.decided()) return kRedo;
+  return sample_point(F, S.q1, prj, iso_ff, p);
+}
+
+// The missing coordinate of a kW64 point, as the reference computes it: float64 bilinear values of
+// the frame's two faces rounded to float, float64 quotient rounded to float.
+TMC_HD float vertex_w_f64(const float u[8], double iso, const float p[3], int prj) {
+  int A, B, W;
+  uint32_t perm;
+  plane(prj, A, B, W, perm);
+  float fp[8];
+#pragma unroll
+  for (int q = 0; q < 8; q++) fp[q] = corner_at(u, (perm >> (4 * q)) & 0xF);
+  const float su = prj == 2 ? p[1] : p[0], sv = prj == 0 ? p[1] : p[2];
+  const float g1 = bilinear_f64(fp[0], fp[1], fp[2], fp[3], su, sv);
+  const float g2 = bilinear_f64(fp[4], fp[5], fp[6], fp[7], su, sv);
+  return w_f64(iso, g1, g2);
 }
 
 // ---------------------------------------------------------------------------------------------

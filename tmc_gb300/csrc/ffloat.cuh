@@ -158,6 +158,43 @@ TMC_HD bool ff_round(ff x, float err, float& out) {
   return true;
 }
 
+// The same decision as two float additions: rounding is certain when hi swallows lo + err and
+// lo - err alike.  err is taken a quarter larger, which covers the rounding of lo +- err and a sum
+// that lands on a midpoint (ties go to even), as long as err >= 2^-45 |hi|.
+TMC_HD bool ff_certain(ff x, float err) {
+  const float e = err * 1.25f;
+  return std::isfinite(x.hi) && x.hi + (x.lo + e) == x.hi && x.hi + (x.lo - e) == x.hi;
+}
+
+// Reciprocal within an ulp or two (2^-22): one instruction on the GPU.  Only for normal x whose
+// reciprocal is normal too (callers check the range): subnormals are flushed.
+TMC_HD float rcp_est(float x) {
+#ifdef __CUDA_ARCH__
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+#else
+  return 1.0f / x;
+#endif
+}
+
+// num / den within 2^-43 of the quotient, from r = rcp_est(den.hi): the estimate, its remainder (the
+// leading difference is exact) and one correction.
+TMC_HD ff ff_quot(ff num, ff den, float r) {
+  const float q1 = num.hi * r;
+  const ff p = two_prod(q1, den.hi);
+  const float rem = fma_rn(-q1, den.lo, ((num.hi - p.hi) - p.lo) + num.lo);
+  return quick_two_sum(q1, rem * r);
+}
+
+// a + b with |error| <= 2^-46 (|a| + |b|): the low parts added once (no bound relative to a
+// cancelled sum, unlike ff_add)
+TMC_HD ff ff_add_abs(ff a, ff b) {
+  ff s = two_sum(a.hi, b.hi);
+  s.lo += a.lo + b.lo;
+  return quick_two_sum(s.hi, s.lo);
+}
+
 // smallest float >= x / largest float <= x, for a finite double x
 TMC_HD float f_ceil(double x) {
   float f = (float)x;

@@ -269,20 +269,20 @@ tmc::Grid make_grid(const tmc_volume* vol, const float* dev, double iso) {
     g.inv2_lo[d] = c.lo;
   }
   g.iso_f = (float)iso;
+  g.iso_lo = (float)(iso - (double)g.iso_f);
+  g.iso_exact = (double)g.iso_f == iso;
   g.set_divisors();
   return g;
 }
 
 void mesh_reset(tmc_mesh* m) { std::memset(m, 0, sizeof(*m)); }
 
-// per-vertex scratch of the two-pass vertex kernels
+// per-vertex scratch of the vertex kernels
 cudaError_t dmc_vertex_scratch(Allocs& al, tmc::DmcScratch& sc, int64_t nv) {
-  uint8_t* rec = nullptr;
-  cudaError_t e = al.get(&rec, nv * (int64_t)tmc::kProjRecordBytes);
-  sc.proj = reinterpret_cast<tmc::repr::ProjRecord*>(rec);
-  if (e == cudaSuccess) e = al.get(&sc.vp, nv);
+  cudaError_t e = al.get(&sc.vp, nv);
   if (e == cudaSuccess) e = al.get(&sc.fb_list, nv);
-  if (e == cudaSuccess) e = al.get(&sc.fb_count, 2);
+  if (e == cudaSuccess) e = al.get(&sc.w_list, nv);
+  if (e == cudaSuccess) e = al.get(&sc.fb_count, 3);
   if (e == cudaSuccess) e = al.get(&sc.tail_list, nv);
   return e;
 }
@@ -1285,7 +1285,6 @@ extern "C" tmc_status tmc_ctx_autotune(tmc_ctx* ctx, int32_t n, const tmc_reques
   };
   const bool host_field = n == 1 && !reqs[0].vol.on_device;
   std::vector<Axis> axes = {
-      {TMC_TUNE_GROUP_LANES, {0, sm * 12 * 32, sm * 24 * 32, sm * 48 * 32}},
       {TMC_TUNE_WARP_LIST_MAX, {0, sm * 8, sm * 32, sm * 128}},
       {TMC_TUNE_VERTEX_BLOCKS_PER_SM, {8, 16, 32}},
       {TMC_TUNE_EMIT_BLOCKS_PER_SM, {4, 8, 16}},
