@@ -820,14 +820,16 @@ tmc_status tmc_extract(tmc_ctx* ctx, const tmc_volume* vol, double iso, uint32_t
   const int64_t ncell = g.ncells();
   tmc::TmcScratch sc{};
   TMC_CUDA(ctx, al.get(&sc.rec, ncell));
-  TMC_CUDA(ctx, al.get(&sc.voff, ncell));
+  TMC_CUDA(ctx, al.get(&sc.rv, ncell));
   TMC_CUDA(ctx, al.get(&sc.toff, ncell));
   TMC_CUDA(ctx, al.get(&sc.cellof, ncell));
+  TMC_CUDA(ctx, al.get(&sc.ccase, ncell));
   const tmc::CellSpace space = tmc::single_space(g);
   TMC_CUDA(ctx, al.get(&sc.mask, tmc::tmc_tiles(space) * (tmc::kScanTile / 32)));
   TMC_CUDA(ctx, al.get(&sc.tile_sums, tmc::tmc_tiles(space)));
   TMC_CUDA(ctx, al.get(&sc.totals, 2));
-  TMC_CUDA(ctx, al.get(&sc.amb_n, 1));
+  TMC_CUDA(ctx, al.get(&sc.amb_n, 2));
+  TMC_CUDA(ctx, al.get(&sc.chunks, tmc::tmc_tiles(space) * (tmc::kScanTile / 32)));
   sc.stats = ctx->d_stats;
   TMC_CUDA(ctx, cudaMemsetAsync(sc.stats, 0, 8 * sizeof(unsigned long long), st));
   ctx->launches += tmc::tmc_classify(space, sc, st, &ctx->prof, gates.data(), (int)gates.size());
@@ -997,7 +999,6 @@ tmc_status batch_run(tmc_ctx* ctx, const std::vector<int>& idx, const tmc_reques
   tmc::CellMask* mask = nullptr;
   uint16_t* cellof = nullptr;
   TMC_CUDA(ctx, al.get(&rec, ncell));
-  TMC_CUDA(ctx, al.get(&voff, ncell));
   TMC_CUDA(ctx, al.get(&qoff, ncell));
   TMC_CUDA(ctx, al.get(&cellof, ncell));
   TMC_CUDA(ctx, al.get(&mask, tiles * (tmc::kScanTile / 32)));
@@ -1008,6 +1009,7 @@ tmc_status batch_run(tmc_ctx* ctx, const std::vector<int>& idx, const tmc_reques
   tmc::TmcScratch tsc{};
   int64_t n_amb_rec = 0;
   if (dmc) {
+    TMC_CUDA(ctx, al.get(&voff, ncell));
     dsc = tmc::DmcScratch{rec, voff, qoff, nullptr, tile_sums, totals, ctx->d_stats};
     dsc.mask = mask;
     dsc.cellof = cellof;
@@ -1015,10 +1017,13 @@ tmc_status batch_run(tmc_ctx* ctx, const std::vector<int>& idx, const tmc_reques
     TMC_CUDA(ctx, al.get(&dsc.ccase, ncell));
     ctx->launches += tmc::dmc_front_count(space, dsc, st, &ctx->prof);
   } else {
-    tsc = tmc::TmcScratch{rec, voff, qoff, tile_sums, totals, ctx->d_stats};
+    tsc = tmc::TmcScratch{rec, nullptr, qoff, tile_sums, totals, ctx->d_stats};
     tsc.mask = mask;
     tsc.cellof = cellof;
-    TMC_CUDA(ctx, al.get(&tsc.amb_n, 1));
+    TMC_CUDA(ctx, al.get(&tsc.rv, ncell));
+    TMC_CUDA(ctx, al.get(&tsc.ccase, ncell));
+    TMC_CUDA(ctx, al.get(&tsc.chunks, tiles * (tmc::kScanTile / 32)));
+    TMC_CUDA(ctx, al.get(&tsc.amb_n, 2));
     ctx->launches += tmc::tmc_classify(space, tsc, st, &ctx->prof);
     TMC_CUDA(ctx, tmc_ambiguous_records(ctx, al, tsc, n_amb_rec));
     ctx->launches += tmc::tmc_count(space, tsc, n_amb_rec, ctx->sms, st, &ctx->prof);

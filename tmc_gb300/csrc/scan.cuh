@@ -84,6 +84,50 @@ __device__ __forceinline__ void store8(int32_t* p, int64_t first, int64_t n, con
   }
 }
 
+// eight (a, b) pairs, as store8
+__device__ __forceinline__ void store8_pairs(uint2* p, int64_t first, int64_t n, const uint32_t a[8],
+                                             const uint32_t b[8]) {
+  uint2* q = p + first;
+  if (first + 8 <= n && ((uintptr_t)q & 15) == 0) {
+#pragma unroll
+    for (int s = 0; s < 8; s += 2) *reinterpret_cast<uint4*>(q + s) = make_uint4(a[s], b[s], a[s + 1], b[s + 1]);
+  } else {
+#pragma unroll
+    for (int s = 0; s < 8; s++)
+      if (first + s < n) q[s] = make_uint2(a[s], b[s]);
+  }
+}
+
+// The chunk list: every tile's listed slots in chunks of 32, each entry the chunk's first slot (a
+// multiple of 32) with its number of cells minus one in the low bits.  The emission kernels take
+// chunks from it instead of looking at every tile's 64 possible ones (a smooth field lists 60 of a
+// tile's 2048 cells: two chunks).  One warp per tile; the block reserves its warps' entries with one
+// atomic, so the list follows the tiles up to the order in which blocks run, which is about theirs:
+// the cells in flight stay within a narrow band that the L2 holds.  Every thread of the block calls it.
+template <int kWarps>
+__device__ __forceinline__ void list_chunks(int64_t tile, uint32_t listed, uint32_t* chunks, unsigned* nchunks) {
+  __shared__ unsigned at[kWarps];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const unsigned c = (listed + 31) / 32;
+  if (lane == 0) at[wid] = c;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned sum = 0;
+    for (int w = 0; w < kWarps; w++) sum += at[w];
+    unsigned base = sum ? atomicAdd(nchunks, sum) : 0u;
+    for (int w = 0; w < kWarps; w++) {
+      const unsigned x = at[w];
+      at[w] = base;
+      base += x;
+    }
+  }
+  __syncthreads();
+  for (unsigned q = lane; q < c; q += 32) {
+    const uint32_t left = listed - 32 * q;
+    chunks[at[wid] + q] = (uint32_t)(tile * kScanTile) + 32 * q + (left < 32 ? left - 1 : 31);
+  }
+}
+
 // In-tile offsets with one warp per tile: the tile's listed slots are walked 256 at a time, each
 // lane owning 8 consecutive slots (the blocked accessors above), scanned with warp shuffles and a
 // carry from one step to the next; no block barrier, and a tile's few listed slots (a few hundred

@@ -572,7 +572,7 @@ __device__ void load_amb_cell(const Grid& g, int i, int j, int k, const float u[
 // listed by slot (amb_list, warp-aggregated appends) for the float64 counting pass.
 template <bool kGen>
 __global__ void __launch_bounds__(kScanThreads, 6) tmc_classify_kernel(CellSpace space, int64_t tile0, uint32_t* rec,
-                                                                   uint16_t* cellof, CellMask* mask,
+                                                                   uint16_t* cellof, uint8_t* ccase, CellMask* mask,
                                                                    unsigned long long* tile_sums,
                                                                    unsigned long long* stats, uint32_t* amb_list,
                                                                    unsigned* amb_n) {
@@ -604,6 +604,7 @@ __global__ void __launch_bounds__(kScanThreads, 6) tmc_classify_kernel(CellSpace
     amb += listed;
     rec[slot] = r;
     cellof[slot] = (uint16_t)off;
+    ccase[slot] = (uint8_t)cs;
     local += ((unsigned long long)trec_nv(r) << 32) | (unsigned long long)trec_ntri(r);
     const unsigned am = __activemask();
     const unsigned bal = __ballot_sync(am, listed);
@@ -712,16 +713,20 @@ __global__ void __launch_bounds__(128) tmc_amb_count_kernel(CellSpace space, con
   if (sing) atomicAdd(stats + 5, sing);
 }
 
-// In-tile exclusive scan of the listed cells' records -> their vertex and triangle offsets (blocked
-// layout over the tile's slots).
+// In-tile exclusive scan of the listed cells' records -> per slot the record beside its vertex offset
+// (rv, what the emission needs of a neighbour in one load) and the triangle offset, and the tile's
+// chunks of 32 slots appended to the chunk list (common.cuh, list_chunks).
 __global__ void __launch_bounds__(32 * kOffsetWarps) tmc_offsets_kernel(const CellMask* mask, const uint32_t* rec,
                                                                        const unsigned long long* tile_off,
-                                                                       int64_t tiles, int32_t* voff, int32_t* toff) {
+                                                                       int64_t tiles, uint2* rv, int32_t* toff,
+                                                                       uint32_t* chunks, unsigned* nchunks) {
   const int lane = threadIdx.x & 31;
   const int64_t tile = (int64_t)blockIdx.x * kOffsetWarps + (threadIdx.x >> 5);
+  const uint32_t listed = tile < tiles ? tile_listed(mask, tile) : 0;
+  list_chunks<kOffsetWarps>(tile, listed, chunks, nchunks);
   if (tile >= tiles) return;  // the whole warp
   const int64_t base = tile * kScanTile;
-  const int64_t end = base + tile_listed(mask, tile);
+  const int64_t end = base + listed;
   unsigned long long carry = tile_off[tile];
   for (int64_t step = base; step < end; step += kOffsetStep) {  // warp-uniform
     const int64_t first = step + (int64_t)lane * kScanItems;
@@ -733,134 +738,196 @@ __global__ void __launch_bounds__(32 * kOffsetWarps) tmc_offsets_kernel(const Ce
     const unsigned long long inc = warp_inclusive_scan(sum);
     unsigned long long pre = carry + inc - sum;
     carry += __shfl_sync(0xffffffffu, inc, 31);
-    int32_t vo[kScanItems], to[kScanItems];
+    uint32_t vo[kScanItems];
+    int32_t to[kScanItems];
 #pragma unroll
     for (int s = 0; s < kScanItems; s++) {
-      vo[s] = (int32_t)(pre >> 32);
+      vo[s] = (uint32_t)(pre >> 32);
       to[s] = (int32_t)(pre & 0xffffffffull);
       pre += ((unsigned long long)trec_nv(r[s]) << 32) | trec_ntri(r[s]);
     }
-    store8(voff, first, end, vo);
+    store8_pairs(rv, first, end, r, vo);
     store8(toff, first, end, to);
   }
 }
 
-// corner value v of a cell's eight (selects, so that a run-time index keeps u in registers)
-__device__ __forceinline__ float pick8(const float u[8], int v) {
-  float r = u[0];
-#pragma unroll
-  for (int q = 1; q < 8; q++) r = (v == q) ? u[q] : r;
-  return r;
-}
-
-// edge vertex: interpolation as t_mc (mc/MarchingCubes.cpp:241-254), float64
-__device__ __forceinline__ void edge_vertex_f64(const Grid& g, int i, int j, int k, int e, const float u[8],
-                                                const TmcVertexOut& out, int32_t idx) {
-  const int v0 = edge_v0(e), v1 = edge_v1(e);
-  const double F0 = pick8(u, v0), F1 = pick8(u, v1);
-  const double l = (g.iso - F0) / (F1 - F0);
-  const int i0 = i + (v0 & 1), j0 = j + ((v0 >> 1) & 1), k0 = k + ((v0 >> 2) & 1);
-  const int i1 = i + (v1 & 1), j1 = j + ((v1 >> 1) & 1), k1 = k + ((v1 >> 2) & 1);
-  const double p0[3] = {g.ox + i0 * g.dx, g.oy + j0 * g.dy, g.oz + k0 * g.dz};
-  const double p1[3] = {g.ox + i1 * g.dx, g.oy + j1 * g.dy, g.oz + k1 * g.dz};
-  double n0[3], n1[3];
-  tmc_point_gradient(g, i0, j0, k0, n0);
-  tmc_point_gradient(g, i1, j1, k1, n1);
-  double ip[3], in[3];
-#pragma unroll
-  for (int d = 0; d < 3; d++) ip[d] = (1 - l) * p0[d] + l * p1[d];
-#pragma unroll
-  for (int d = 0; d < 3; d++) in[d] = (1 - l) * n0[d] + l * n1[d];
-  const double nl = sqrt(in[0] * in[0] + in[1] * in[1] + in[2] * in[2]);
-  const int64_t o = 3 * (int64_t)idx;
+// An edge vertex's two field values and the two ends' field differences along each axis, as pairs of
+// points: for the edge's own axis the ends share their values.  Borders: one-sided differences over
+// one spacing (UGrid::gradient, mc/MarchingCubes.cpp:1451-1509), bit d of `one` for the first end and
+// bit 4 + d for the second.
+struct EdgeStencil {
+  float f0, f1;
+  float hi[2][3], lo[2][3];  // end, axis
+  int one;
+};
+__device__ __forceinline__ void load_stencil(const Grid& g, const int p0[3], int ax, EdgeStencil& S) {
+  const int64_t sy = g.nx, sz = (int64_t)g.nx * g.ny;
+  const float* f = g.f + (int64_t)p0[2] * sz + (int64_t)p0[1] * sy + p0[0];
+  const int64_t sa = ax == 0 ? 1 : (ax == 1 ? sy : sz);
+  S.f0 = __ldg(f);
+  S.f1 = __ldg(f + sa);
+  S.one = 0;
 #pragma unroll
   for (int d = 0; d < 3; d++) {
-    out.v[o + d] = (float)ip[d];
-    out.n[o + d] = (float)(in[d] / nl);
-    if (out.v64) out.v64[o + d] = ip[d];
+    const int64_t sd = d == 0 ? 1 : (d == 1 ? sy : sz);
+    const int n = d == 0 ? g.nx : (d == 1 ? g.ny : g.nz);
+    const bool own = d == ax;
+    // first end: its neighbour before (after, on the edge's axis, is the second end)
+    const bool low = p0[d] == 0, high = p0[d] == n - 1;  // the upper border is never on the edge's axis
+    const float* l0 = low ? f : f - sd;
+    const float* h0 = own ? f + sd : (high ? f : f + sd);
+    S.lo[0][d] = __ldg(l0);
+    S.hi[0][d] = __ldg(h0);
+    S.one |= (int)(low || (!own && high)) << d;
+    // second end
+    const float* e = f + sa;
+    const bool last = own ? p0[d] + 1 == n - 1 : high;
+    S.lo[1][d] = __ldg(own ? f : (low ? e : e - sd));
+    S.hi[1][d] = __ldg(last ? e : e + sd);
+    S.one |= (int)(last || (!own && low)) << (4 + d);
   }
 }
 
-// edge vertex in float32 (positions within an ulp: the grid coordinate i + l is formed exactly as a
-// float pair); the float64 variant above is used when float64 positions are requested
-__device__ __forceinline__ void tmc_gradient_f(const Grid& g, int i, int j, int k, const float inv[3],
-                                               const float inv2[3], float out[3]) {
-  if (i == 0) out[0] = (g.at(i + 1, j, k) - g.at(i, j, k)) * inv[0];
-  else if (i == g.nx - 1) out[0] = (g.at(i, j, k) - g.at(i - 1, j, k)) * inv[0];
-  else out[0] = (g.at(i + 1, j, k) - g.at(i - 1, j, k)) * inv2[0];
-  if (j == 0) out[1] = (g.at(i, j + 1, k) - g.at(i, j, k)) * inv[1];
-  else if (j == g.ny - 1) out[1] = (g.at(i, j, k) - g.at(i, j - 1, k)) * inv[1];
-  else out[1] = (g.at(i, j + 1, k) - g.at(i, j - 1, k)) * inv2[1];
-  if (k == 0) out[2] = (g.at(i, j, k + 1) - g.at(i, j, k)) * inv[2];
-  else if (k == g.nz - 1) out[2] = (g.at(i, j, k) - g.at(i, j, k - 1)) * inv[2];
-  else out[2] = (g.at(i, j, k + 1) - g.at(i, j, k - 1)) * inv2[2];
+// A unit normal from the interpolated gradient in float-float: within 2^-30 of the float64 one where
+// the gradients cancel to no less than 2^-10 of their size; false below that.
+// kEach: every component within 2^-27 of itself (none cancels to below 2^-14 of its inputs), so that
+// its float32 rounding is the float64 normal's but for midpoints; else false.
+template <bool kEach>
+__device__ __forceinline__ bool edge_normal_ff(const Grid& g, const EdgeStencil& S, ffx::ff l, float out[3]) {
+  ffx::ff in[3];
+  float scale = 0;
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    const ffx::ff s{g.inv2_hi[d], g.inv2_lo[d]};
+    const float m0 = (S.one >> d) & 1 ? 2.0f : 1.0f, m1 = (S.one >> (4 + d)) & 1 ? 2.0f : 1.0f;
+    // differences in units of 1 / (2 spacing); doubling is exact
+    const ffx::ff a = ffx::two_sum(S.hi[0][d], -S.lo[0][d]), b = ffx::two_sum(S.hi[1][d], -S.lo[1][d]);
+    const ffx::ff a2{a.hi * m0, a.lo * m0}, b2{b.hi * m1, b.lo * m1};
+    in[d] = ffx::ff_mul(ffx::ff_add(a2, ffx::ff_mul(l, ffx::ff_sub(b2, a2))), s);
+    const float size = fmaxf(fabsf(a2.hi), fabsf(b2.hi)) * s.hi;
+    if (kEach && !(fabsf(in[d].hi) >= 0x1p-14f * size)) return false;
+    scale = fmaxf(scale, size);
+  }
+  const ffx::ff dot =
+      ffx::ff_add(ffx::ff_add(ffx::ff_mul(in[0], in[0]), ffx::ff_mul(in[1], in[1])), ffx::ff_mul(in[2], in[2]));
+  // out of range (or not finite), or cancelled: float64
+  if (!(dot.hi > 0x1p-80f && dot.hi < 0x1p80f) || !(scale <= 0x1p10f * sqrtf(dot.hi))) return false;
+  // 1/sqrt(dot): float estimate and one Newton step in float-float
+  const float r0 = rsqrtf(dot.hi);
+  const ffx::ff h = ffx::ff_mul_f(ffx::ff_mul_f(dot, r0), r0);
+  const ffx::ff r = ffx::ff_mul_f(ffx::ff_sub(ffx::ff_from(1.5f), ffx::ff_mul_f(h, 0.5f)), r0);
+#pragma unroll
+  for (int d = 0; d < 3; d++) out[d] = ffx::ff_mul(in[d], r).hi;
+  return true;
 }
 
-__device__ __forceinline__ void edge_vertex_f32(const Grid& g, int i, int j, int k, int e, const float u[8],
-                                                const TmcVertexOut& out, int32_t idx, const float inv[3],
-                                                const float inv2[3]) {
-  const int v0 = edge_v0(e), v1 = edge_v1(e), ax = edge_axis(e);
-  const float F0 = pick8(u, v0), F1 = pick8(u, v1);
-  const float l = (g.iso_f - F0) / (F1 - F0);
-  const int i0 = i + (v0 & 1), j0 = j + ((v0 >> 1) & 1), k0 = k + ((v0 >> 2) & 1);
-  const int i1 = i + (v1 & 1), j1 = j + ((v1 >> 1) & 1), k1 = k + ((v1 >> 2) & 1);
-  const int gi[3] = {i0, j0, k0};
-  const int64_t base = 3 * (int64_t)idx;
+struct Float3 {
+  float x[3];
+};
+// the reference's float64 normal, for the few edge vertices the float pairs do not serve
+__device__ __noinline__ Float3 edge_normal_f64(const Grid& g, const EdgeStencil S) {
+  const double f0 = S.f0, f1 = S.f1, l = (g.iso - f0) / (f1 - f0);
+  const double sp[3] = {g.dx, g.dy, g.dz};
+  double in[3];
+  for (int d = 0; d < 3; d++) {
+    const double n0 = ((double)S.hi[0][d] - (double)S.lo[0][d]) / ((S.one >> d) & 1 ? sp[d] : 2 * sp[d]);
+    const double n1 = ((double)S.hi[1][d] - (double)S.lo[1][d]) / ((S.one >> (4 + d)) & 1 ? sp[d] : 2 * sp[d]);
+    in[d] = (1 - l) * n0 + l * n1;
+  }
+  const double nl = sqrt(in[0] * in[0] + in[1] * in[1] + in[2] * in[2]);
+  Float3 r;
+  for (int d = 0; d < 3; d++) r.x[d] = (float)(in[d] / nl);
+  return r;
+}
+// the same from float pairs where they serve
+template <bool kEach>
+__device__ __noinline__ Float3 edge_normal_precise(const Grid& g, const EdgeStencil S) {
+  const ffx::ff num = ffx::ff_sub(ffx::ff{g.iso_f, g.iso_lo}, ffx::ff_from(S.f0));
+  const ffx::ff l = ffx::ff_div(num, ffx::two_sum(S.f1, -S.f0));
+  Float3 r;
+  if (edge_normal_ff<kEach>(g, S, l, r.x)) return r;
+  return edge_normal_f64(g, S);
+}
+
+// The vertex on local edge e of cell (i, j, k), written at index idx.
+// kF64: positions as t_mc (mc/MarchingCubes.cpp:241-254) in float64.  Otherwise positions within an
+// ulp (the grid coordinate i + l formed exactly as a float pair), and normals in float32, whose
+// interpolation errs by a few ulps of its inputs' size: where the gradients cancel to below 1/16 of
+// that it would exceed ~4e-6 of the unit normal, and the float pairs take over.
+template <bool kF64>
+__device__ __forceinline__ void edge_vertex(const Grid& g, int i, int j, int k, int e, const TmcVertexOut& out,
+                                            int64_t idx) {
+  const int v0 = edge_v0(e), ax = edge_axis(e);
+  const int p0[3] = {i + (v0 & 1), j + ((v0 >> 1) & 1), k + ((v0 >> 2) & 1)};
+  EdgeStencil S;
+  load_stencil(g, p0, ax, S);
+  const int64_t base = 3 * idx;
+  if (kF64) {
+    const double F0 = S.f0, F1 = S.f1;
+    const double l = (g.iso - F0) / (F1 - F0);
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      const double o = d == 0 ? g.ox : (d == 1 ? g.oy : g.oz), h = d == 0 ? g.dx : (d == 1 ? g.dy : g.dz);
+      const double a = o + p0[d] * h, b = d == ax ? o + (p0[d] + 1) * h : a;
+      const double x = (1 - l) * a + l * b;
+      out.v[base + d] = (float)x;
+      out.v64[base + d] = x;
+    }
+    const Float3 n = edge_normal_precise<true>(g, S);
+#pragma unroll
+    for (int d = 0; d < 3; d++) out.n[base + d] = n.x[d];
+    return;
+  }
+  const float l = (g.iso_f - S.f0) / (S.f1 - S.f0);
 #pragma unroll
   for (int d = 0; d < 3; d++) {
     // origin + (index + l) * spacing, with index + l exact as a float pair
-    const ffx::ff t = (d == ax) ? ffx::two_sum((float)gi[d], l) : ffx::ff_from((float)gi[d]);
+    const ffx::ff t = (d == ax) ? ffx::two_sum((float)p0[d], l) : ffx::ff_from((float)p0[d]);
     const ffx::ff x = ffx::ff_add(ffx::ff{g.org_hi[d], g.org_lo[d]}, ffx::ff_mul(t, ffx::ff{g.sp_hi[d], g.sp_lo[d]}));
     out.v[base + d] = x.hi + x.lo;
   }
-  float n0[3], n1[3];
-  tmc_gradient_f(g, i0, j0, k0, inv, inv2, n0);
-  tmc_gradient_f(g, i1, j1, k1, inv, inv2, n1);
   float in[3], scale = 0;
 #pragma unroll
   for (int d = 0; d < 3; d++) {
-    in[d] = fmaf(l, n1[d] - n0[d], n0[d]);
-    scale = fmaxf(scale, fmaxf(fabsf(n0[d]), fabsf(n1[d])));
+    const float s = g.inv2f[d];  // the border's 1/spacing is its double, exactly
+    const float n0 = (S.hi[0][d] - S.lo[0][d]) * ((S.one >> d) & 1 ? 2 * s : s);
+    const float n1 = (S.hi[1][d] - S.lo[1][d]) * ((S.one >> (4 + d)) & 1 ? 2 * s : s);
+    in[d] = fmaf(l, n1 - n0, n0);
+    scale = fmaxf(scale, fmaxf(fabsf(n0), fabsf(n1)));
   }
   const float dot = in[0] * in[0] + in[1] * in[1] + in[2] * in[2];
-  // The float32 interpolation errs by a few ulps of `scale`; where the gradients cancel to below
-  // 1/16 of it that would exceed ~4e-6 of the unit normal: the reference's float64 normal instead.
   if (scale <= 16.0f * sqrtf(dot)) {
     const float rn = rsqrtf(dot);
 #pragma unroll
     for (int d = 0; d < 3; d++) out.n[base + d] = in[d] * rn;
     return;
   }
-  double m0[3], m1[3];
-  tmc_point_gradient(g, i0, j0, k0, m0);
-  tmc_point_gradient(g, i1, j1, k1, m1);
-  const double F0d = F0, F1d = F1, ld = (g.iso - F0d) / (F1d - F0d);
-  double md[3];
+  const Float3 n = edge_normal_precise<false>(g, S);
 #pragma unroll
-  for (int d = 0; d < 3; d++) md[d] = (1 - ld) * m0[d] + ld * m1[d];
-  const double nl = sqrt(md[0] * md[0] + md[1] * md[1] + md[2] * md[2]);
-#pragma unroll
-  for (int d = 0; d < 3; d++) out.n[base + d] = (float)(md[d] / nl);
+  for (int d = 0; d < 3; d++) out.n[base + d] = n.x[d];
 }
 
-// Vertex index of each crossed edge of a cell, within the cell's volume (vfirst: the volume's first
-// vertex in the space-wide numbering; vbase: the cell's first vertex, space-wide).
+// Vertex index of crossed edge e of a cell, within the cell's volume, wherever its owner is (vfirst:
+// the volume's first vertex in the space-wide numbering; first: the cell's first vertex, space-wide).
+__device__ __forceinline__ int32_t border_vertex_id(const Grid& g, int i, int j, int k, int e, uint32_t own,
+                                                    int32_t first, int32_t vfirst, const CellMask* mask,
+                                                    const uint2* rv) {
+  if (own & (1u << e)) return first - vfirst + __popc(own & ((1u << e) - 1u));
+  int oi, oj, ok, oe = 0;
+  edge_owner(i, j, k, e, oi, oj, ok, oe);
+  const uint2 o = __ldg(rv + listed_slot(mask, (uint32_t)g.vcell(oi, oj, ok)));  // crossed edge: listed owner
+  return (int32_t)o.y - vfirst + __popc(trec_owned(o.x) & ((1u << oe) - 1u));
+}
+// The same for all crossed edges (em) of a cell.
 __device__ __forceinline__ void tmc_vertex_ids(const Grid& g, int i, int j, int k, uint32_t em, uint32_t own,
-                                               int32_t vbase, int32_t vfirst, const CellMask* mask,
-                                               const uint32_t* rec, const int32_t* voff, int32_t vid[12]) {
+                                               int32_t first, int32_t vfirst, const CellMask* mask, const uint2* rv,
+                                               int32_t vid[12]) {
 #pragma unroll
   for (int e = 0; e < 12; e++) vid[e] = -1;
   // crossed edges as a mask, lowest first: the lanes of a warp resolve their k-th edges together
   for (uint32_t m = em; m; m &= m - 1) {
     const int e = __ffs(m) - 1;
-    if (own & (1u << e)) {
-      vid[e] = vbase - vfirst + __popc(own & em & ((1u << e) - 1u));
-    } else {
-      int oi, oj, ok, oe = 0;
-      edge_owner(i, j, k, e, oi, oj, ok, oe);
-      const uint32_t os = listed_slot(mask, (uint32_t)g.vcell(oi, oj, ok));  // crossed edge: listed owner
-      vid[e] = voff[os] - vfirst + __popc(trec_owned(rec[os]) & ((1u << oe) - 1u));
-    }
+    vid[e] = border_vertex_id(g, i, j, k, e, own, first, vfirst, mask, rv);
   }
 }
 
@@ -868,8 +935,8 @@ __device__ __forceinline__ void tmc_vertex_ids(const Grid& g, int i, int j, int 
 // cell's vertex indices, and the inner vertices from the recorded parameters (float64 trilinear
 // position and normal).  A cell with more triangles than its record holds runs p_slice again.
 __global__ void __launch_bounds__(128) tmc_ambiguous_kernel(CellSpace space, const CellMask* mask,
-                                                            const uint16_t* cellof, const uint32_t* rec,
-                                                            const int32_t* voff, const int32_t* toff,
+                                                            const uint16_t* cellof, const uint2* rv,
+                                                            const int32_t* toff,
                                                             const unsigned long long* tile_off, TmcVertexOut out,
                                                             int32_t* tris, const AmbRec* recs, const unsigned* count) {
   const unsigned na = *count;
@@ -879,17 +946,17 @@ __global__ void __launch_bounds__(128) tmc_ambiguous_kernel(CellSpace space, con
     if ((info >> 18) & 1) continue;  // singular face: the reference emits nothing for the cell
     const uint32_t slot = R.slot;
     const int64_t vcell = slot_cell(cellof, slot);
-    const uint32_t r = rec[slot];
+    const uint2 r = rv[slot];
     const Grid g = space.grid_of_tile(vcell / kScanTile);
     const int32_t vfirst = (int32_t)(tile_off[g.vbase / kScanTile] >> 32);
     int i, j, k;
     tcell_ijk(g, vcell - g.vbase, i, j, k);
     const unsigned cs = info & 0xFF;
     const uint32_t em = case_edge_mask(cs);
-    const uint32_t own = trec_owned(r);
+    const uint32_t own = trec_owned(r.x);
     int32_t vid[12];
-    tmc_vertex_ids(g, i, j, k, em, own, voff[slot], vfirst, mask, rec, voff, vid);
-    const int32_t ibase = voff[slot] - vfirst + __popc(own);
+    tmc_vertex_ids(g, i, j, k, em, own, (int32_t)r.y, vfirst, mask, rv, vid);
+    const int32_t ibase = (int32_t)r.y - vfirst + __popc(own);
     // inner vertices are numbered within the volume: shift the outputs to its first vertex
     InnerOut io{out.v + 3 * (int64_t)vfirst, out.n + 3 * (int64_t)vfirst, out.v64 ? out.v64 + 3 * (int64_t)vfirst : nullptr};
     const int nt = (int)((info >> 8) & 63), ni = (int)((info >> 14) & 7);
@@ -948,99 +1015,145 @@ __global__ void __launch_bounds__(128) tmc_ambiguous_kernel(CellSpace space, con
   }
 }
 
-// One active cell: its owned edge vertices and (unambiguous case) its table triangles.
-template <bool kPos64>
-__device__ __forceinline__ void emit_cell(const Grid& g, int32_t vfirst, uint32_t slot, int64_t vcell,
-                                          const CellMask* mask, const uint32_t* rec, const int32_t* voff,
-                                          const int32_t* toff, const TmcVertexOut& out, int32_t* tris) {
-  const int64_t cell = vcell - g.vbase;
-  const uint32_t r = rec[slot];
-  int i, j, k;
-  tcell_ijk(g, cell, i, j, k);
-  float u[8];
-  tload_corners(g, i, j, k, u);
-  unsigned cs = 0;
+// The vertex indices on the crossed edges of an interior cell (no index 0), into its column of vid.
+// Nine of the edges belong to six neighbours; every neighbour that owns a crossed one is looked up
+// once, and the six look-ups (a mask word, then the record and offset in one load) are independent.
+__device__ __forceinline__ void interior_vertex_ids(int64_t vcell, int cx, int64_t cxy, uint32_t em, uint32_t own,
+                                                    int32_t first, int32_t vfirst, const CellMask* mask,
+                                                    const uint2* rv, int32_t* vid) {
+  // neighbour (0,-1,-1): its edge 6 is edge 0 here; (0,0,-1): 5, 6 are 1, 2; (-1,0,-1): 5 is 3;
+  // (0,-1,0): 6, 10 are 4, 9; (-1,0,0): 5, 10 are 7, 11; (-1,-1,0): 10 is 8
+  const int64_t off[6] = {-cxy - cx, -cxy, -cxy - 1, -(int64_t)cx, -1, -(int64_t)cx - 1};
+  constexpr int kEdge[6][2] = {{0, -1}, {1, 2}, {3, -1}, {4, 9}, {7, 11}, {8, -1}};
+  constexpr int kOwner[6][2] = {{6, -1}, {5, 6}, {5, -1}, {6, 10}, {5, 10}, {10, -1}};
+  uint32_t slot[6];
 #pragma unroll
-  for (int v = 0; v < 8; v++) cs |= (unsigned)(u[v] >= g.iso_up) << v;
-  const uint32_t em = case_edge_mask(cs);
-  const uint32_t own = trec_owned(r);
-  const int32_t vbase = voff[slot];
-  // owned edge vertices, in edge order (the crossed owned edges as a mask, lowest first)
-  int rank = 0;
-  for (uint32_t mo = em & own; mo; mo &= mo - 1, rank++) {
-    const int e = __ffs(mo) - 1;
-    if (kPos64 && out.v64 && (g.flags & kGridPos64)) edge_vertex_f64(g, i, j, k, e, u, out, vbase + rank);
-    else {
-      const float inv2[3] = {g.inv2f[0], g.inv2f[1], g.inv2f[2]};
-      const float inv[3] = {2 * inv2[0], 2 * inv2[1], 2 * inv2[2]};  // = fl(1/spacing): doubling is exact
-      edge_vertex_f32(g, i, j, k, e, u, out, vbase + rank, inv, inv2);
-    }
+  for (int q = 0; q < 6; q++) {
+    const uint32_t want = (1u << kEdge[q][0]) | (kEdge[q][1] >= 0 ? 1u << (kEdge[q][1] & 15) : 0u);
+    slot[q] = (em & want) ? listed_slot(mask, (uint32_t)(vcell + off[q])) : 0xffffffffu;
   }
-  // ambiguous: triangles and inner vertices from the cell's ambiguous-cell record (tmc_ambiguous_kernel)
-  if ((r >> 21) & 1) return;
-  int32_t vid[12];
-  tmc_vertex_ids(g, i, j, k, em, own, vbase, vfirst, mask, rec, voff, vid);
-  TriSink ts{tris + 3 * (int64_t)toff[slot], 0};
-  // unambiguous: table triangles with reversed winding (t_mc, mc/MarchingCubes.cpp:276-294)
-  const uint64_t tw = c_tmc_tris[cs];
-  const int nt = (int)(tw & 0xF);
-  for (int t = 0; t < nt; t++) {
-    const int e0 = (int)((tw >> (4 + 12 * t)) & 0xF), e1 = (int)((tw >> (8 + 12 * t)) & 0xF),
-              e2 = (int)((tw >> (12 + 12 * t)) & 0xF);
-    ts.put(vid[e2], vid[e1], vid[e0]);
-  }
+  uint2 o[6];
+#pragma unroll
+  for (int q = 0; q < 6; q++) o[q] = slot[q] != 0xffffffffu ? __ldg(rv + slot[q]) : make_uint2(0, 0);
+#pragma unroll
+  for (int q = 0; q < 6; q++)
+#pragma unroll
+    for (int t = 0; t < 2; t++)
+      if (kEdge[q][t] >= 0)  // columns of edges that are not crossed are never read
+        vid[32 * (kEdge[q][t] & 15)] =
+            (int32_t)o[q].y - vfirst + __popc(trec_owned(o[q].x) & ((1u << (kOwner[q][t] & 15)) - 1u));
+#pragma unroll
+  for (int e = 5; e <= 10; e = e == 6 ? 10 : e + 1) vid[32 * e] = first - vfirst + __popc(own & ((1u << e) - 1u));
 }
 
-// Each warp walks chunks of 32 consecutive slots of the listed cells, appends the cells with a
-// record to its own queue in shared memory (ballot + popcount), and processes the queue 32 cells at
-// a time, one per lane: all lanes busy, and no block barrier (warps never wait for one another).
+// One warp per chunk of 32 consecutive listed cells of one tile (the chunk list of the offsets pass).
+// A cell owns 0 to 12 vertices (1.06 on average on the 512^3 noise field, at most 3 away from the
+// lower borders) and 0 to 5 triangles: with a cell per lane the lanes of a warp run as long as the
+// largest, so the warp lists its vertices and then its triangles and takes them one per lane.
+// Outputs are contiguous across the lanes.  Each cell's vertex indices (interior_vertex_ids) go to
+// shared memory, a column per cell, where the triangle lanes pick them by edge.  Ambiguous cells'
+// triangles come from their records (tmc_ambiguous_kernel).
+// Bound by the latency of the field and neighbour loads (long_scoreboard, 58 % issue active, 24 lanes
+// per instruction); 64 registers for four blocks per SM (80 registers and three blocks: 4 % slower).
+// 512^3 noise field, 17.0 M vertices and 33.7 M triangles: 0.81 ms, 2.30 ms with a cell per lane;
+// float64 positions (190x151x171 blobs): 20 us, 116 us with every normal in float64.
 constexpr int kEmitThreads = 256;
+__device__ const uint64_t d_tmc_tris[256] = TMC_TRIANGLES_INIT;
 // kPos64: some volume of the launch wants float64 positions (the float64 edge-vertex path is
-// compiled only into that instantiation, which keeps the common one's code small)
+// compiled only into that instantiation)
 template <bool kBatch, bool kPos64>
 __global__ void __launch_bounds__(kEmitThreads, 4) tmc_emit_kernel(CellSpace space, const CellMask* mask,
-                                                                   const uint16_t* cellof, const uint32_t* rec,
-                                                                   const int32_t* voff, const int32_t* toff,
-                                                                   const unsigned long long* tile_off,
-                                                                   TmcVertexOut out, int32_t* tris) {
+                                                                const uint16_t* cellof, const uint8_t* ccase,
+                                                                const uint2* rv, const int32_t* toff,
+                                                                const unsigned long long* tile_off,
+                                                                const uint32_t* chunks, const unsigned* nchunks,
+                                                                TmcVertexOut out, int32_t* tris) {
   constexpr int kWarps = kEmitThreads / 32;
-  __shared__ uint32_t queue[kWarps][64];
+  constexpr unsigned kAll = 0xffffffffu;
+  __shared__ int32_t vids[kWarps][12 * 32];    // edge, cell
+  __shared__ uint16_t items[kWarps][12 * 32];  // cell << 4 | edge, or cell << 4 | triangle
+  __shared__ int4 cells[kWarps][32];           // i, j, k, first vertex minus its place in the list
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  uint32_t* Q = queue[wid];
-  const int64_t tiles = ceil_div(space.n, kScanTile), chunks = tiles * (kScanTile / 32);
-  int qn = 0;  // queued cells (the same on every lane)
-  for (int64_t chunk = (int64_t)blockIdx.x * kWarps + wid;; chunk += (int64_t)gridDim.x * kWarps) {
-    const bool more = chunk < chunks;
-    if (more) {
-      int64_t tile;
-      uint32_t first;
-      slot_chunk(chunk, tiles, tile, first);
-      const uint32_t slot = first + lane, r = slot & (kScanTile - 1);
-      const bool act = r < tile_listed(mask, tile) && rec[slot] != 0;
-      const unsigned bal = __ballot_sync(0xffffffffu, act);
-      if (act) Q[qn + __popc(bal & ((1u << lane) - 1u))] = slot;
-      qn += __popc(bal);
-      __syncwarp();
+  int32_t* vid = vids[wid];
+  uint16_t* item = items[wid];
+  int4* cell = cells[wid];
+  const unsigned n = *nchunks;
+  for (unsigned q = blockIdx.x * kWarps + wid; q < n; q += gridDim.x * kWarps) {
+    const uint32_t chunk = chunks[q], slot0 = chunk & ~31u, slot = slot0 + lane;
+    const bool in = (uint32_t)lane <= (chunk & 31u);  // the chunk's number of cells minus one
+    const int64_t tile = slot0 >> kTileShift;
+    const Grid& g = kBatch ? space.grids[__ldg(space.tile_vol + tile)] : space.one;
+    const int32_t vfirst = kBatch ? (int32_t)(__ldg(tile_off + g.vbase / kScanTile) >> 32) : 0;
+    uint2 r = make_uint2(0, 0);
+    unsigned cs = 0;
+    int64_t vcell = 0;
+    int i = 0, j = 0, k = 0;
+    if (in) {
+      r = __ldg(rv + slot);
+      cs = __ldg(ccase + slot);
+      vcell = slot_cell(cellof, slot);
+      tcell_ijk(g, vcell - g.vbase, i, j, k);
     }
-    while (qn >= 32 || (!more && qn > 0)) {
-      const int take = qn < 32 ? qn : 32;
-      if (lane < take) {
-        const uint32_t slot = Q[lane];
-        const uint32_t vcell = slot_cell(cellof, slot);
-        // the cell's volume: read in place (a batch's grid table, or the launch parameter)
-        const Grid& g = kBatch ? space.grids[__ldg(space.tile_vol + vcell / kScanTile)] : space.one;
-        const int32_t vfirst = kBatch ? (int32_t)(tile_off[g.vbase / kScanTile] >> 32) : 0;
-        emit_cell<kPos64>(g, vfirst, slot, vcell, mask, rec, voff, toff, out, tris);
+    const uint32_t own = trec_owned(r.x);
+    const bool amb = (r.x >> 21) & 1;
+    const int nt = amb ? 0 : trec_ntri(r.x);  // of the table, for an unambiguous case
+    // the vertices
+    int upto = __popc(own);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(kAll, upto, o);
+      if (lane >= o) upto += y;
+    }
+    int from = upto - __popc(own);
+    int total = __shfl_sync(kAll, upto, 31);
+    cell[lane] = make_int4(i, j, k, (int32_t)r.y - from);
+    for (uint32_t m = own; m; m &= m - 1) item[from++] = (uint16_t)(lane << 4 | (__ffs(m) - 1));
+    __syncwarp();
+    for (int t = lane; t < total; t += 32) {
+      const int x = item[t];
+      const int4 c = cell[x >> 4];
+      if (kPos64 && (!kBatch || (g.flags & kGridPos64))) edge_vertex<true>(g, c.x, c.y, c.z, x & 15, out, c.w + t);
+      else edge_vertex<false>(g, c.x, c.y, c.z, x & 15, out, c.w + t);
+    }
+    // the vertex indices of the cells with triangles
+    if (nt) {
+      const uint32_t em = case_edge_mask(cs);
+      if (i > 0 && j > 0 && k > 0) {
+        interior_vertex_ids(vcell, g.cx(), (int64_t)g.cx() * g.cy(), em, own, (int32_t)r.y, vfirst, mask, rv, vid + lane);
+      } else {
+        for (uint32_t m = em; m; m &= m - 1) {
+          const int e = __ffs(m) - 1;
+          vid[32 * e + lane] = border_vertex_id(g, i, j, k, e, own, (int32_t)r.y, vfirst, mask, rv);
+        }
       }
-      __syncwarp();
-      const int rest = qn - take;  // at most 31: move them to the front
-      const uint32_t x = lane < rest ? Q[take + lane] : 0u;
-      __syncwarp();
-      if (lane < rest) Q[lane] = x;
-      __syncwarp();
-      qn = rest;
     }
-    if (!more) break;
+    __syncwarp();  // the vertex list is read
+    // the triangles
+    upto = nt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(kAll, upto, o);
+      if (lane >= o) upto += y;
+    }
+    from = upto - nt;
+    total = __shfl_sync(kAll, upto, 31);
+    const int32_t to = nt ? __ldg(toff + slot) - from : 0;
+    for (int t = 0; t < nt; t++) item[from + t] = (uint16_t)(lane << 4 | t);
+    __syncwarp();
+    for (int t0 = 0; t0 < total; t0 += 32) {  // warp-uniform: the shuffles need every lane
+      const int t = t0 + lane, x = t < total ? item[t] : 0, o = x >> 4;
+      const unsigned ocs = __shfl_sync(kAll, cs, o);
+      const int32_t oto = __shfl_sync(kAll, to, o);
+      if (t < total) {
+        // reversed winding (t_mc, mc/MarchingCubes.cpp:276-294)
+        const unsigned tw = (unsigned)(__ldg(d_tmc_tris + ocs) >> (4 + 12 * (x & 15)));
+        int32_t* w = tris + 3 * ((int64_t)oto + t);
+        w[0] = vid[32 * ((tw >> 8) & 0xF) + o];
+        w[1] = vid[32 * ((tw >> 4) & 0xF) + o];
+        w[2] = vid[32 * (tw & 0xF) + o];
+      }
+    }
+    __syncwarp();  // vid, item and cell are read
   }
 }
 
@@ -1057,15 +1170,15 @@ int tmc_classify(const CellSpace& space, TmcScratch& s, cudaStream_t st, Prof* p
   int k = 0;
   {
     Stage t(prof, "tmc_classify", st);
-    cudaMemsetAsync(s.amb_n, 0, sizeof(unsigned), st);
+    cudaMemsetAsync(s.amb_n, 0, 2 * sizeof(unsigned), st);  // and the chunk counter behind it
     auto classify = [&](int64_t t0, int64_t t1) {
       if (t1 <= t0) return;
       if (space.one.gen)  // fused generation (single volumes)
         tmc_classify_kernel<true><<<(unsigned)(t1 - t0), kScanThreads, 0, st>>>(
-            space, t0, s.rec, s.cellof, s.mask, s.tile_sums, s.stats, amb_cells, s.amb_n);
+            space, t0, s.rec, s.cellof, s.ccase, s.mask, s.tile_sums, s.stats, amb_cells, s.amb_n);
       else
         tmc_classify_kernel<false><<<(unsigned)(t1 - t0), kScanThreads, 0, st>>>(
-            space, t0, s.rec, s.cellof, s.mask, s.tile_sums, s.stats, amb_cells, s.amb_n);
+            space, t0, s.rec, s.cellof, s.ccase, s.mask, s.tile_sums, s.stats, amb_cells, s.amb_n);
       k++;
     };
     if (ngates == 0) classify(0, tiles);
@@ -1100,7 +1213,8 @@ int tmc_count(const CellSpace& space, TmcScratch& s, int64_t n_amb, int sms, cud
   Stage t(prof, "tmc_scan", st);
   scan_tile_sums_kernel<<<1, 1024, 0, st>>>(s.tile_sums, tiles, s.totals);
   tmc_offsets_kernel<<<(unsigned)ceil_div(tiles, kOffsetWarps), 32 * kOffsetWarps, 0, st>>>(s.mask, s.rec, s.tile_sums,
-                                                                                           tiles, s.voff, s.toff);
+                                                                                           tiles, s.rv, s.toff,
+                                                                                           s.chunks, s.amb_n + 1);
   return k + 2;
 }
 
@@ -1109,18 +1223,19 @@ int tmc_emit(const CellSpace& space, TmcScratch& s, int64_t n_amb, TmcVertexOut 
   const int sms = tu.sms;
   {
     Stage t(prof, "tmc_emit", st);
-    const int64_t blocks = std::max<int64_t>(
-        1, std::min<int64_t>(ceil_div(space.n, 32 * (kEmitThreads / 32)), (int64_t)sms * tu.emit_blocks_per_sm));
-#define TMC_EMIT(B, P)                                                                                       \
-  tmc_emit_kernel<B, P><<<(unsigned)blocks, kEmitThreads, 0, st>>>(space, s.mask, s.cellof, s.rec, s.voff, s.toff, \
-                                                                  s.tile_sums, vo, tris)
+    // whole waves; the number of chunks is only known on the device
+#define TMC_EMIT(B, P)                                                                                          \
+  {                                                                                                             \
+    static const int res = resident_blocks(tmc_emit_kernel<B, P>, kEmitThreads);                                \
+    const int64_t blocks = wave_grid(res, sms, tu.emit_blocks_per_sm, ceil_div(space.n, 32), kEmitThreads / 32); \
+    tmc_emit_kernel<B, P><<<(unsigned)blocks, kEmitThreads, 0, st>>>(space, s.mask, s.cellof, s.ccase, s.rv, s.toff, \
+                                                                     s.tile_sums, s.chunks, s.amb_n + 1, vo, tris);  \
+  }
     const bool pos64 = vo.v64 != nullptr;
     if (space.grids) {
-      if (pos64) TMC_EMIT(true, true);
-      else TMC_EMIT(true, false);
+      if (pos64) TMC_EMIT(true, true) else TMC_EMIT(true, false)
     } else {
-      if (pos64) TMC_EMIT(false, true);
-      else TMC_EMIT(false, false);
+      if (pos64) TMC_EMIT(false, true) else TMC_EMIT(false, false)
     }
 #undef TMC_EMIT
   }
@@ -1128,7 +1243,7 @@ int tmc_emit(const CellSpace& space, TmcScratch& s, int64_t n_amb, TmcVertexOut 
   Stage t2(prof, "tmc_ambiguous", st);
   static const int r_amb = resident_blocks(tmc_ambiguous_kernel, 128);
   tmc_ambiguous_kernel<<<(unsigned)wave_grid(r_amb, sms, 8, n_amb, 128), 128, 0, st>>>(
-      space, s.mask, s.cellof, s.rec, s.voff, s.toff, s.tile_sums, vo, tris, reinterpret_cast<const AmbRec*>(s.amb_rec),
+      space, s.mask, s.cellof, s.rv, s.toff, s.tile_sums, vo, tris, reinterpret_cast<const AmbRec*>(s.amb_rec),
       s.amb_n);
   return 2;
 }

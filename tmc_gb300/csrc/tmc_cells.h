@@ -18,21 +18,23 @@ constexpr int kTmcAmbRecWords = 32;
 
 struct TmcScratch {
   uint32_t* rec;
-  int32_t* voff;
+  uint2* rv;            // record and vertex offset
   int32_t* toff;
   unsigned long long* tile_sums;
   unsigned long long* totals;
   unsigned long long* stats;
-  unsigned* amb_n;      // ambiguous cells listed by the classification
+  unsigned* amb_n;      // [0] ambiguous cells listed by the classification, [1] chunks
   uint32_t* amb_rec;    // kTmcAmbRecWords words per ambiguous cell: what the counting pass keeps of
                         // its p_slice for the emission pass (tmc_cells.cu, AmbRec)
   uint32_t* amb_sorted; // the ambiguous cells' slots sorted by MC case (one per ambiguous cell)
   uint8_t* amb_key;     // their cases, in list order (one per ambiguous cell)
   unsigned* amb_hist;   // 512: per-case counts, then scatter cursors
-  // listed cells (common.cuh): rec, voff and toff hold one entry per listed cell at its slot, the
+  // listed cells (common.cuh): rec, rv and toff hold one entry per listed cell at its slot, the
   // ambiguous-cell list holds slots
   CellMask* mask;       // per 32 cells of the space
   uint16_t* cellof;     // per slot: in-tile offset of the listed cell
+  uint8_t* ccase;       // per slot: its MC case
+  uint32_t* chunks;     // kScanTile / 32 per tile: the chunk list (scan.cuh)
 };
 
 // Per-cell scratch is indexed in the cell space; triangles hold vertex indices within their own
