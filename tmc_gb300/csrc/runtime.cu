@@ -126,7 +126,7 @@ cudaError_t tmc_ambiguous_records(tmc_ctx* ctx, Allocs& al, tmc::TmcScratch& sc,
   if ((e = al.get(&sc.amb_rec, na * tmc::kTmcAmbRecWords)) != cudaSuccess) return e;
   if ((e = al.get(&sc.amb_sorted, na)) != cudaSuccess) return e;
   if ((e = al.get(&sc.amb_key, na)) != cudaSuccess) return e;
-  return al.get(&sc.amb_hist, 512);
+  return al.get(&sc.amb_hist, 513);
 }
 
 float iso_up(double iso) {
@@ -837,10 +837,10 @@ tmc_status tmc_extract(tmc_ctx* ctx, const tmc_volume* vol, double iso, uint32_t
   int64_t n_amb = 0;
   TMC_CUDA(ctx, tmc_ambiguous_records(ctx, al, sc, n_amb));
   ctx->launches += tmc::tmc_count(space, sc, n_amb, ctx->sms, st, &ctx->prof);
-  TMC_CUDA(ctx, cudaMemcpyAsync(h, sc.totals, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-  TMC_CUDA(ctx, cudaMemcpyAsync(h + 1, sc.stats, 8 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+  TMC_CUDA(ctx, cudaMemcpyAsync(h, sc.totals, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
   TMC_CUDA(ctx, tmc::host_wait(st));
   const int64_t nv = (int64_t)(h[0] >> 32), nt = (int64_t)(h[0] & 0xffffffffull);
+  const int64_t n_overflow = (int64_t)h[1];
 
   MeshPriv* mp = new (std::nothrow) MeshPriv();
   if (!mp) return fail(ctx, TMC_ERR_OOM, "host allocation failed");
@@ -861,7 +861,7 @@ tmc_status tmc_extract(tmc_ctx* ctx, const tmc_volume* vol, double iso, uint32_t
   TMC_OWN(vo.n, 3 * nv);
   if (flags & TMC_OUT_POS_F64) TMC_OWN(vo.v64, 3 * nv);
   TMC_OWN(tris, 3 * nt);
-  ctx->launches += tmc::tmc_emit(space, sc, n_amb, vo, tris, ctx->tune, st, &ctx->prof);
+  ctx->launches += tmc::tmc_emit(space, sc, n_amb, n_overflow, vo, tris, ctx->tune, st, &ctx->prof);
   TMC_CUDA(ctx, cudaGetLastError());
   out->nr_v = nv;
   out->nr_t = nt;
@@ -1031,8 +1031,7 @@ tmc_status batch_run(tmc_ctx* ctx, const std::vector<int>& idx, const tmc_reques
   std::vector<unsigned long long> toff((size_t)tiles + 1);
   unsigned long long* h = (unsigned long long*)ctx->h_pinned;
   TMC_CUDA(ctx, cudaMemcpyAsync(toff.data(), tile_sums, tiles * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-  TMC_CUDA(ctx, cudaMemcpyAsync(h, totals, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-  TMC_CUDA(ctx, cudaMemcpyAsync(h + 1, ctx->d_stats, 8 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+  TMC_CUDA(ctx, cudaMemcpyAsync(h, totals, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
   TMC_CUDA(ctx, tmc::host_wait(st));
   toff[(size_t)tiles] = h[0];
   const int64_t NV = (int64_t)(h[0] >> 32), NF = (int64_t)(h[0] & 0xffffffffull);
@@ -1081,7 +1080,7 @@ tmc_status batch_run(tmc_ctx* ctx, const std::vector<int>& idx, const tmc_reques
   } else {
     TMC_CUDA(ctx, get_shared(&faces, 3 * NF));
     tmc::TmcVertexOut vo{v, nn, v64};
-    ctx->launches += tmc::tmc_emit(space, tsc, n_amb_rec, vo, faces, ctx->tune, st, &ctx->prof);
+    ctx->launches += tmc::tmc_emit(space, tsc, n_amb_rec, (int64_t)h[1], vo, faces, ctx->tune, st, &ctx->prof);
   }
   TMC_CUDA(ctx, cudaGetLastError());
 

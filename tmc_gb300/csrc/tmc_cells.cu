@@ -490,71 +490,96 @@ __device__ __forceinline__ void amb_geometry(const Grid& g, int i, int j, int k,
   }
 }
 
-// Corner positions alone (float64, as amb_geometry).
-__device__ __forceinline__ void amb_positions(const Grid& g, int i, int j, int k, double P[8][3]) {
-  const double x[2] = {g.ox + i * g.dx, g.ox + (i + 1) * g.dx};
-  const double y[2] = {g.oy + j * g.dy, g.oy + (j + 1) * g.dy};
-  const double z[2] = {g.oz + k * g.dz, g.oz + (k + 1) * g.dz};
+// One inner vertex of the emission: local parameters (u, v, w) of cell (i, j, k), written at index
+// `at` of the outputs.
+// The field difference along axis d at grid point p as the two values and whether it is one-sided
+// (UGrid::gradient, mc/MarchingCubes.cpp:1451-1509).
+__device__ __forceinline__ bool axis_pair(const Grid& g, const int p[3], int d, float& hi, float& lo) {
+  const int n = d == 0 ? g.nx : (d == 1 ? g.ny : g.nz);
+  int a[3] = {p[0], p[1], p[2]}, b[3] = {p[0], p[1], p[2]};
+  const bool low = p[d] == 0, high = p[d] == n - 1;
+  if (!high) a[d] += 1;
+  if (!low) b[d] -= 1;
+  hi = g.at(a[0], a[1], a[2]);
+  lo = g.at(b[0], b[1], b[2]);
+  return low || high;
+}
+
+// The reference's float64 arithmetic (:1073-1083 and :1283-1293), one axis after another.
+__device__ __noinline__ void inner_vertex_f64(const Grid& g, int i, int j, int k, double u, double v, double w,
+                                              const TmcVertexOut out, int64_t at) {
+  double ip[3], in[3];
 #pragma unroll
-  for (int q = 0; q < 8; q++) {
-    P[q][0] = x[q & 1];
-    P[q][1] = y[(q >> 1) & 1];
-    P[q][2] = z[(q >> 2) & 1];
+  for (int d = 0; d < 3; d++) {
+    const double o = d == 0 ? g.ox : (d == 1 ? g.oy : g.oz), h = d == 0 ? g.dx : (d == 1 ? g.dy : g.dz);
+    const int c0 = d == 0 ? i : (d == 1 ? j : k);
+    double P[8], N[8];
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      const int p[3] = {i + (q & 1), j + ((q >> 1) & 1), k + ((q >> 2) & 1)};
+      P[q] = o + (c0 + ((q >> d) & 1)) * h;
+      float hi, lo;
+      const bool one = axis_pair(g, p, d, hi, lo);
+      N[q] = ((double)hi - (double)lo) / (one ? h : 2 * h);
+    }
+    ip[d] = (1 - w) * ((1 - v) * (P[0] + u * (P[1] - P[0])) + v * (P[2] + u * (P[3] - P[2]))) +
+            w * ((1 - v) * (P[4] + u * (P[5] - P[4])) + v * (P[6] + u * (P[7] - P[6])));
+    in[d] = (1 - w) * ((1 - v) * (N[0] + u * (N[1] - N[0])) + v * (N[2] + u * (N[3] - N[2]))) +
+            w * ((1 - v) * (N[4] + u * (N[5] - N[4])) + v * (N[6] + u * (N[7] - N[6])));
+  }
+  const double factor = sqrt(in[0] * in[0] + in[1] * in[1] + in[2] * in[2]);
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    out.v[3 * at + d] = (float)ip[d];
+    out.n[3 * at + d] = (float)(in[d] / factor);
+    if (out.v64) out.v64[3 * at + d] = ip[d];
   }
 }
 
-// tmc_point_gradient in float-float: the exact float difference times 1/(2 spacing) (1/spacing on
-// the border), within ~2^-46 of the reference's float64 quotient.
-__device__ __forceinline__ ffx::ff grad_axis_ff(float hi_v, float lo_v, bool border, float s_hi, float s_lo) {
-  const float m = border ? 2.0f : 1.0f;  // 1/spacing = 2 * 1/(2 spacing), exactly
-  return ffx::ff_mul(ffx::two_sum(hi_v, -lo_v), ffx::ff{s_hi * m, s_lo * m});
-}
-__device__ __forceinline__ void tmc_gradient_ff(const Grid& g, int i, int j, int k, ffx::ff out[3]) {
-  const int i1 = i == g.nx - 1 ? i : i + 1, i0 = i == 0 ? 0 : i - 1;
-  const int j1 = j == g.ny - 1 ? j : j + 1, j0 = j == 0 ? 0 : j - 1;
-  const int k1 = k == g.nz - 1 ? k : k + 1, k0 = k == 0 ? 0 : k - 1;
-  out[0] = grad_axis_ff(g.at(i1, j, k), g.at(i0, j, k), i == 0 || i == g.nx - 1, g.inv2_hi[0], g.inv2_lo[0]);
-  out[1] = grad_axis_ff(g.at(i, j1, k), g.at(i, j0, k), j == 0 || j == g.ny - 1, g.inv2_hi[1], g.inv2_lo[1]);
-  out[2] = grad_axis_ff(g.at(i, j, k1), g.at(i, j, k0), k == 0 || k == g.nz - 1, g.inv2_hi[2], g.inv2_lo[2]);
-}
-
-// a + t (b - a), all float pairs
-__device__ __forceinline__ ffx::ff ff_lerp_ff(ffx::ff a, ffx::ff b, ffx::ff t) {
-  return ffx::ff_add(a, ffx::ff_mul(ffx::ff_sub(b, a), t));
-}
-
-// One inner vertex of the emission pass: the float64 position as inner_vertex forms it, the normal
-// from the float-float corner gradients N (trilinear at (u, v, w), normalised; within a few 2^-40 of
-// the reference's float64 normal).  Only the float32 rounding of the normal is output, so the float
-// pairs serve wherever the gradients do not cancel to below 2^-10 of their size; there it returns
-// false and the caller computes the normal in float64.
-__device__ __forceinline__ bool inner_vertex_ff(const double (*P)[3], const ffx::ff (*N)[3], float scale, double u,
-                                                double v, double w, const InnerOut& geo, int64_t index) {
-  double ip[3];
-  cell_trilinear3(P, u, v, w, ip);
+// The same for float32 outputs in float-float (within 2^-44 of the position's size; the normal within
+// 2^-30 of the float64 one), except where the gradients cancel to below 2^-10 of their size.
+__device__ __forceinline__ void inner_vertex_ff(const Grid& g, int i, int j, int k, double u, double v, double w,
+                                                const TmcVertexOut& out, int64_t at) {
   const ffx::ff U = ffx::ff_from_double(u), V = ffx::ff_from_double(v), W = ffx::ff_from_double(w);
+  auto lerp = [](ffx::ff a, ffx::ff b, ffx::ff t) {
+    return ffx::ff_add_abs(a, ffx::ff_mul(ffx::ff_add_abs(b, ffx::ff_neg(a)), t));
+  };
   ffx::ff in[3];
+  float scale = 0;
 #pragma unroll
   for (int d = 0; d < 3; d++) {
-    const ffx::ff a0 = ff_lerp_ff(N[0][d], N[1][d], U), a1 = ff_lerp_ff(N[2][d], N[3][d], U);
-    const ffx::ff a2 = ff_lerp_ff(N[4][d], N[5][d], U), a3 = ff_lerp_ff(N[6][d], N[7][d], U);
-    in[d] = ff_lerp_ff(ff_lerp_ff(a0, a1, V), ff_lerp_ff(a2, a3, V), W);
+    ffx::ff N[8];  // in units of 1 / (2 spacing)
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      const int p[3] = {i + (q & 1), j + ((q >> 1) & 1), k + ((q >> 2) & 1)};
+      float hi, lo;
+      const float m = axis_pair(g, p, d, hi, lo) ? 2.0f : 1.0f;
+      const ffx::ff x = ffx::two_sum(hi, -lo);
+      N[q] = ffx::ff{x.hi * m, x.lo * m};
+      scale = fmaxf(scale, fabsf(N[q].hi) * g.inv2_hi[d]);
+    }
+    const ffx::ff t = lerp(lerp(lerp(N[0], N[1], U), lerp(N[2], N[3], U), V),
+                           lerp(lerp(N[4], N[5], U), lerp(N[6], N[7], U), V), W);
+    in[d] = ffx::ff_mul(t, ffx::ff{g.inv2_hi[d], g.inv2_lo[d]});
   }
   const ffx::ff dot =
       ffx::ff_add(ffx::ff_add(ffx::ff_mul(in[0], in[0]), ffx::ff_mul(in[1], in[1])), ffx::ff_mul(in[2], in[2]));
-  if (!(dot.hi > 0.0f) || !(scale <= 0x1p10f * sqrtf(dot.hi))) return false;
+  if (!(dot.hi > 0x1p-80f && dot.hi < 0x1p80f) || !(scale <= 0x1p10f * sqrtf(dot.hi))) {
+    inner_vertex_f64(g, i, j, k, u, v, w, out, at);
+    return;
+  }
   // 1/sqrt(dot): float estimate and one Newton step in float-float
   const float r0 = rsqrtf(dot.hi);
   const ffx::ff h = ffx::ff_mul_f(ffx::ff_mul_f(dot, r0), r0);
   const ffx::ff r = ffx::ff_mul_f(ffx::ff_sub(ffx::ff_from(1.5f), ffx::ff_mul_f(h, 0.5f)), r0);
-  const int64_t o = 3 * index;
 #pragma unroll
-  for (int q = 0; q < 3; q++) {
-    geo.v[o + q] = (float)ip[q];
-    geo.n[o + q] = ffx::ff_mul(in[q], r).hi;
-    if (geo.v64) geo.v64[o + q] = ip[q];
+  for (int d = 0; d < 3; d++) {
+    const int c0 = d == 0 ? i : (d == 1 ? j : k);
+    const ffx::ff t = ffx::ff_add(ffx::ff_from((float)c0), d == 0 ? U : (d == 1 ? V : W));
+    const ffx::ff x = ffx::ff_add(ffx::ff{g.org_hi[d], g.org_lo[d]}, ffx::ff_mul(t, ffx::ff{g.sp_hi[d], g.sp_lo[d]}));
+    out.v[3 * at + d] = x.hi;
+    out.n[3 * at + d] = ffx::ff_mul(in[d], r).hi;
   }
-  return true;
 }
 
 __device__ void load_amb_cell(const Grid& g, int i, int j, int k, const float u[8], AmbCell& a, bool geometry) {
@@ -667,10 +692,35 @@ __global__ void tmc_amb_cursor_kernel(const unsigned* hist, unsigned* cursor) {
   cursor[threadIdx.x] = x[threadIdx.x] - hist[threadIdx.x];
 }
 
-__global__ void tmc_amb_sort_kernel(const uint32_t* list, const uint8_t* key, int64_t n, unsigned* cursor,
-                                    uint32_t* sorted) {
-  for (int64_t a = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; a < n; a += (int64_t)gridDim.x * blockDim.x)
-    sorted[atomicAdd(cursor + key[a], 1u)] = list[a];
+// A block ranks its cells per case in shared memory and takes each case's range with one atomic: the
+// per-case cursors are few and hot (one atomic per cell: 1.58 ms for the 11 M ambiguous cells of the
+// 1024x1024x64 saddle field, 0.31 ms for the 1.3 M of the 512^3 noise field; 0.08 and 0.02 ms so).
+constexpr int kSortItems = 8, kSortTile = 256 * kSortItems;
+__global__ void __launch_bounds__(256) tmc_amb_sort_kernel(const uint32_t* list, const uint8_t* key, int64_t n,
+                                                           unsigned* cursor, uint32_t* sorted) {
+  __shared__ unsigned h[256];
+  for (int64_t base = (int64_t)blockIdx.x * kSortTile; base < n; base += (int64_t)gridDim.x * kSortTile) {
+    h[threadIdx.x] = 0;
+    __syncthreads();
+    unsigned k[kSortItems], rank[kSortItems];
+#pragma unroll
+    for (int s = 0; s < kSortItems; s++) {
+      const int64_t a = base + s * 256 + threadIdx.x;
+      k[s] = a < n ? key[a] : 0u;
+      rank[s] = a < n ? atomicAdd(&h[k[s]], 1u) : 0u;
+    }
+    __syncthreads();
+    const unsigned c = h[threadIdx.x];
+    __syncthreads();
+    if (c) h[threadIdx.x] = atomicAdd(cursor + threadIdx.x, c);
+    __syncthreads();
+#pragma unroll
+    for (int s = 0; s < kSortItems; s++) {
+      const int64_t a = base + s * 256 + threadIdx.x;
+      if (a < n) sorted[h[k[s]] + rank[s]] = list[a];
+    }
+    __syncthreads();
+  }
 }
 
 // Ambiguous cells from the classification's list: p_slice in counting mode (float64); the counts go
@@ -680,7 +730,8 @@ __global__ void tmc_amb_sort_kernel(const uint32_t* list, const uint8_t* key, in
 __global__ void __launch_bounds__(128) tmc_amb_count_kernel(CellSpace space, const uint16_t* cellof, uint32_t* rec,
                                                             unsigned long long* tile_sums,
                                                             unsigned long long* stats, const uint32_t* list,
-                                                            const unsigned* count, AmbRec* recs) {
+                                                            const unsigned* count, AmbRec* recs,
+                                                            unsigned* overflow) {
   const unsigned na = *count;
   unsigned long long sing = 0;
   for (unsigned a = blockIdx.x * blockDim.x + threadIdx.x; a < na; a += gridDim.x * blockDim.x) {
@@ -708,6 +759,7 @@ __global__ void __launch_bounds__(128) tmc_amb_count_kernel(CellSpace space, con
     rec[slot] |= (uint32_t)ar.inner << 12 | (uint32_t)ts.n << 15 | (ar.error ? (1u << 22) : 0u);
     const unsigned long long add = ((unsigned long long)ar.inner << 32) | (unsigned long long)ts.n;
     if (add) atomicAdd(tile_sums + (slot >> kTileShift), add);
+    if (ts.n > kAmbRecTris) atomicAdd(overflow, 1u);
     sing += ar.error;
   }
   if (sing) atomicAdd(stats + 5, sing);
@@ -719,10 +771,14 @@ __global__ void __launch_bounds__(128) tmc_amb_count_kernel(CellSpace space, con
 __global__ void __launch_bounds__(32 * kOffsetWarps) tmc_offsets_kernel(const CellMask* mask, const uint32_t* rec,
                                                                        const unsigned long long* tile_off,
                                                                        int64_t tiles, uint2* rv, int32_t* toff,
-                                                                       uint32_t* chunks, unsigned* nchunks) {
+                                                                       uint32_t* chunks, unsigned* nchunks,
+                                                                       const unsigned* overflow,
+                                                                       unsigned long long* totals) {
   const int lane = threadIdx.x & 31;
   const int64_t tile = (int64_t)blockIdx.x * kOffsetWarps + (threadIdx.x >> 5);
   const uint32_t listed = tile < tiles ? tile_listed(mask, tile) : 0;
+  // read by the host with the totals: cells whose triangles overflow their records
+  if (blockIdx.x == 0 && threadIdx.x == 0) totals[1] = overflow ? *overflow : 0u;
   list_chunks<kOffsetWarps>(tile, listed, chunks, nchunks);
   if (tile >= tiles) return;  // the whole warp
   const int64_t base = tile * kScanTile;
@@ -931,90 +987,6 @@ __device__ __forceinline__ void tmc_vertex_ids(const Grid& g, int i, int j, int 
   }
 }
 
-// Ambiguous cells, one thread per record of the counting pass: the recorded triangles with the
-// cell's vertex indices, and the inner vertices from the recorded parameters (float64 trilinear
-// position and normal).  A cell with more triangles than its record holds runs p_slice again.
-__global__ void __launch_bounds__(128) tmc_ambiguous_kernel(CellSpace space, const CellMask* mask,
-                                                            const uint16_t* cellof, const uint2* rv,
-                                                            const int32_t* toff,
-                                                            const unsigned long long* tile_off, TmcVertexOut out,
-                                                            int32_t* tris, const AmbRec* recs, const unsigned* count) {
-  const unsigned na = *count;
-  for (unsigned a = blockIdx.x * blockDim.x + threadIdx.x; a < na; a += gridDim.x * blockDim.x) {
-    const AmbRec& R = recs[a];
-    const uint32_t info = R.info;
-    if ((info >> 18) & 1) continue;  // singular face: the reference emits nothing for the cell
-    const uint32_t slot = R.slot;
-    const int64_t vcell = slot_cell(cellof, slot);
-    const uint2 r = rv[slot];
-    const Grid g = space.grid_of_tile(vcell / kScanTile);
-    const int32_t vfirst = (int32_t)(tile_off[g.vbase / kScanTile] >> 32);
-    int i, j, k;
-    tcell_ijk(g, vcell - g.vbase, i, j, k);
-    const unsigned cs = info & 0xFF;
-    const uint32_t em = case_edge_mask(cs);
-    const uint32_t own = trec_owned(r.x);
-    int32_t vid[12];
-    tmc_vertex_ids(g, i, j, k, em, own, (int32_t)r.y, vfirst, mask, rv, vid);
-    const int32_t ibase = (int32_t)r.y - vfirst + __popc(own);
-    // inner vertices are numbered within the volume: shift the outputs to its first vertex
-    InnerOut io{out.v + 3 * (int64_t)vfirst, out.n + 3 * (int64_t)vfirst, out.v64 ? out.v64 + 3 * (int64_t)vfirst : nullptr};
-    const int nt = (int)((info >> 8) & 63), ni = (int)((info >> 14) & 7);
-    int32_t* t = tris + 3 * (int64_t)toff[slot];
-    if ((info >> 17) & 1) {
-      float u[8];
-      tload_corners(g, i, j, k, u);
-      AmbCell amb;
-      load_amb_cell(g, i, j, k, u, amb, ni > 0);
-      TriSink ts{t, nullptr, 0};
-      p_slice_dev(cs, amb.F, g.iso, vid, ibase, ts, amb.P, amb.N, &io, nullptr);
-      continue;
-    }
-    for (int q = 0; q < nt; q++) {
-      const unsigned code = R.tri[q];
-#pragma unroll
-      for (int c = 0; c < 3; c++) {
-        const int x = (int)((code >> (5 * c)) & 31u);
-        t[3 * q + c] = x < 12 ? vid[x] : ibase + (x - 12);
-      }
-    }
-    if (ni) {
-      // positions in float64 (the output's), normals (float32 outputs only) from float-float
-      // gradients; the float64 gradients for float64 outputs and where the gradients cancel
-      double P[8][3];
-      amb_positions(g, i, j, k, P);
-      ffx::ff N[8][3];
-      float scale = 0;
-#pragma unroll
-      for (int q = 0; q < 8; q++) {
-        tmc_gradient_ff(g, i + (q & 1), j + ((q >> 1) & 1), k + ((q >> 2) & 1), N[q]);
-        scale = fmaxf(scale, fmaxf(fabsf(N[q][0].hi), fmaxf(fabsf(N[q][1].hi), fabsf(N[q][2].hi))));
-      }
-      double uvw[6][3];
-      int nv = 1;
-      if (ni == 1) {
-        uvw[0][0] = R.prm[0];
-        uvw[0][1] = R.prm[1];
-        uvw[0][2] = R.prm[2];
-      } else {
-        const double ui[2] = {R.prm[0], R.prm[1]}, vi[2] = {R.prm[2], R.prm[3]}, wi[2] = {R.prm[4], R.prm[5]};
-        hex_corners(ui, vi, wi, uvw);
-        nv = 6;
-      }
-      for (int q = 0; q < nv; q++) {
-        // float64 outputs requested for this volume: the reference's float64 normal (and its
-        // float32 rounding), as its edge vertices have
-        if (!(g.flags & kGridPos64) &&
-            inner_vertex_ff(P, N, scale, uvw[q][0], uvw[q][1], uvw[q][2], io, (int64_t)ibase + q))
-          continue;
-        double Pd[8][3], Nd[8][3];
-        amb_geometry(g, i, j, k, Pd, Nd);
-        inner_vertex(Pd, Nd, uvw[q][0], uvw[q][1], uvw[q][2], io, (int64_t)ibase + q);
-      }
-    }
-  }
-}
-
 // The vertex indices on the crossed edges of an interior cell (no index 0), into its column of vid.
 // Nine of the edges belong to six neighbours; every neighbour that owns a crossed one is looked up
 // once, and the six look-ups (a mask word, then the record and offset in one load) are independent.
@@ -1044,6 +1016,149 @@ __device__ __forceinline__ void interior_vertex_ids(int64_t vcell, int cx, int64
             (int32_t)o[q].y - vfirst + __popc(trec_owned(o[q].x) & ((1u << (kOwner[q][t] & 15)) - 1u));
 #pragma unroll
   for (int e = 5; e <= 10; e = e == 6 ? 10 : e + 1) vid[32 * e] = first - vfirst + __popc(own & ((1u << e) - 1u));
+}
+
+// Ambiguous cells from the counting pass's records, 32 to a warp: the recorded triangles with the
+// cells' vertex indices, and the inner vertices from the recorded parameters, both taken one per lane
+// (a cell has 1 to 36 triangles and 0, 1 or 6 inner vertices; the lane's cell is found by a binary
+// search in the running counts).  Cells whose triangles overflow their records are left out
+// (tmc_ambiguous_again_kernel).  Float32 outputs take positions and normals from float pairs, one
+// axis after another (96 registers; 254 with float64 positions and all 24 gradients of a cell held
+// at once).  512^3 noise: 0.81 -> 0.41 ms; 1024x1024x64 saddles, 11 M ambiguous cells: 10.3 -> 3.2 ms.
+constexpr int kAmbThreads = 128;
+__device__ __forceinline__ int owner_of(const int32_t* upto, int t) {  // first cell with upto[cell] > t
+  int o = 0;
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1)
+    if (upto[o + s - 1] <= t) o += s;
+  return o;
+}
+__global__ void __launch_bounds__(kAmbThreads) tmc_ambiguous_kernel(CellSpace space, const CellMask* mask,
+                                                                    const uint16_t* cellof, const uint2* rv,
+                                                                    const int32_t* toff,
+                                                                    const unsigned long long* tile_off,
+                                                                    TmcVertexOut out, int32_t* tris,
+                                                                    const AmbRec* recs, const unsigned* count) {
+  constexpr int kWarps = kAmbThreads / 32;
+  constexpr unsigned kAll = 0xffffffffu;
+  __shared__ int32_t vids[kWarps][18 * 32];     // local code (edge, then inner vertex), cell
+  __shared__ int32_t tupto[kWarps][32], iupto[kWarps][32], tbase[kWarps][32];
+  __shared__ int4 cells[kWarps][32];            // i, j, k, volume
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  int32_t* vid = vids[wid];
+  const unsigned na = *count, step = gridDim.x * kAmbThreads;
+  for (unsigned a0 = (blockIdx.x * kWarps + wid) * 32; a0 < na; a0 += step) {
+    const unsigned a = a0 + lane;
+    const uint32_t info = a < na ? recs[a].info : 0u;
+    // a singular face: the reference emits nothing for the cell
+    const bool on = a < na && !((info >> 17) & 3);
+    int nt = 0, ni = 0, vol = 0;
+    int32_t vfirst = 0;
+    if (on) {
+      nt = (int)((info >> 8) & 63);
+      ni = (int)((info >> 14) & 7);
+      const uint32_t slot = recs[a].slot;
+      const int64_t vcell = slot_cell(cellof, slot);
+      const uint2 r = __ldg(rv + slot);
+      vol = space.grids ? __ldg(space.tile_vol + vcell / kScanTile) : 0;
+      const Grid& g = space.grids ? space.grids[vol] : space.one;
+      vfirst = (int32_t)(__ldg(tile_off + g.vbase / kScanTile) >> 32);
+      int i, j, k;
+      tcell_ijk(g, vcell - g.vbase, i, j, k);
+      const uint32_t em = case_edge_mask(info & 0xFF), own = trec_owned(r.x);
+      if (i > 0 && j > 0 && k > 0) {
+        interior_vertex_ids(vcell, g.cx(), (int64_t)g.cx() * g.cy(), em, own, (int32_t)r.y, vfirst, mask, rv, vid + lane);
+      } else {
+        for (uint32_t m = em; m; m &= m - 1) {
+          const int e = __ffs(m) - 1;
+          vid[32 * e + lane] = border_vertex_id(g, i, j, k, e, own, (int32_t)r.y, vfirst, mask, rv);
+        }
+      }
+      const int32_t ibase = (int32_t)r.y - vfirst + __popc(own);
+      for (int q = 0; q < ni; q++) vid[32 * (12 + q) + lane] = ibase + q;
+      cells[wid][lane] = make_int4(i, j, k, vol);
+    }
+    int tu = nt, iu = ni;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(kAll, tu, o), y = __shfl_up_sync(kAll, iu, o);
+      if (lane >= o) {
+        tu += x;
+        iu += y;
+      }
+    }
+    tupto[wid][lane] = tu;
+    iupto[wid][lane] = iu;
+    tbase[wid][lane] = nt ? __ldg(toff + recs[a].slot) - (tu - nt) : 0;
+    const int ttotal = __shfl_sync(kAll, tu, 31), itotal = __shfl_sync(kAll, iu, 31);
+    __syncwarp();
+    for (int t = lane; t < ttotal; t += 32) {
+      const int o = owner_of(tupto[wid], t);
+      const int q = t - (o ? tupto[wid][o - 1] : 0);
+      const unsigned code = recs[a0 + o].tri[q];
+      int32_t* w = tris + 3 * ((int64_t)tbase[wid][o] + t);
+      w[0] = vid[32 * (code & 31) + o];
+      w[1] = vid[32 * ((code >> 5) & 31) + o];
+      w[2] = vid[32 * ((code >> 10) & 31) + o];
+    }
+    for (int t = lane; t < itotal; t += 32) {
+      const int o = owner_of(iupto[wid], t);
+      const int from = o ? iupto[wid][o - 1] : 0, q = t - from;
+      const int4 c = cells[wid][o];
+      const Grid& g = space.grids ? space.grids[c.w] : space.one;
+      const double* prm = recs[a0 + o].prm;
+      double u = prm[0], v = prm[1], w = prm[2];
+      if (iupto[wid][o] - from > 1) {  // corner q of the inner hexagon (hex_corners)
+        u = prm[(0x1C >> q) & 1];
+        v = prm[2 + ((0x38 >> q) & 1)];
+        w = prm[4 + ((0x0E >> q) & 1)];
+      }
+      // vertices are numbered within the volume; the outputs start at its first one
+      const int64_t at = (int64_t)vid[32 * (12 + q) + o] + (int32_t)(__ldg(tile_off + g.vbase / kScanTile) >> 32);
+      // float64 outputs requested for this volume: the reference's float64 arithmetic
+      if (g.flags & kGridPos64) inner_vertex_f64(g, c.x, c.y, c.z, u, v, w, out, at);
+      else inner_vertex_ff(g, c.x, c.y, c.z, u, v, w, out, at);
+    }
+    __syncwarp();  // the columns are read
+  }
+}
+
+// The cells with more triangles than their records hold: p_slice again, one thread per record.  Launched
+// only when the counting pass found one.
+__global__ void __launch_bounds__(128) tmc_ambiguous_again_kernel(CellSpace space, const CellMask* mask,
+                                                            const uint16_t* cellof, const uint2* rv,
+                                                            const int32_t* toff,
+                                                            const unsigned long long* tile_off, TmcVertexOut out,
+                                                            int32_t* tris, const AmbRec* recs, const unsigned* count) {
+  const unsigned na = *count;
+  for (unsigned a = blockIdx.x * blockDim.x + threadIdx.x; a < na; a += gridDim.x * blockDim.x) {
+    const AmbRec& R = recs[a];
+    const uint32_t info = R.info;
+    if (((info >> 17) & 3) != 1) continue;
+    const uint32_t slot = R.slot;
+    const int64_t vcell = slot_cell(cellof, slot);
+    const uint2 r = rv[slot];
+    const Grid g = space.grid_of_tile(vcell / kScanTile);
+    const int32_t vfirst = (int32_t)(tile_off[g.vbase / kScanTile] >> 32);
+    int i, j, k;
+    tcell_ijk(g, vcell - g.vbase, i, j, k);
+    const unsigned cs = info & 0xFF;
+    const uint32_t em = case_edge_mask(cs);
+    const uint32_t own = trec_owned(r.x);
+    int32_t vid[12];
+    tmc_vertex_ids(g, i, j, k, em, own, (int32_t)r.y, vfirst, mask, rv, vid);
+    const int32_t ibase = (int32_t)r.y - vfirst + __popc(own);
+    // inner vertices are numbered within the volume: shift the outputs to its first vertex
+    InnerOut io{out.v + 3 * (int64_t)vfirst, out.n + 3 * (int64_t)vfirst, out.v64 ? out.v64 + 3 * (int64_t)vfirst : nullptr};
+    const int ni = (int)((info >> 14) & 7);
+    int32_t* t = tris + 3 * (int64_t)toff[slot];
+    float u[8];
+    tload_corners(g, i, j, k, u);
+    AmbCell amb;
+    load_amb_cell(g, i, j, k, u, amb, ni > 0);
+    TriSink ts{t, nullptr, 0};
+    p_slice_dev(cs, amb.F, g.iso, vid, ibase, ts, amb.P, amb.N, &io, nullptr);
+  }
 }
 
 // One warp per chunk of 32 consecutive listed cells of one tile (the chunk list of the offsets pass).
@@ -1201,25 +1316,29 @@ int tmc_count(const CellSpace& space, TmcScratch& s, int64_t n_amb, int sms, cud
     Stage ta(prof, "tmc_amb_count", st);
     // the list sorted by MC case (the records follow its order, so the emission pass is sorted too)
     const unsigned gs = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n_amb, 256), (int64_t)sms * 8));
-    cudaMemsetAsync(s.amb_hist, 0, 256 * sizeof(unsigned), st);
+    cudaMemsetAsync(s.amb_hist, 0, 513 * sizeof(unsigned), st);
     tmc_amb_key_kernel<<<gs, 256, 0, st>>>(space, s.cellof, amb_cells, n_amb, s.amb_key, s.amb_hist);
     tmc_amb_cursor_kernel<<<1, 256, 0, st>>>(s.amb_hist, s.amb_hist + 256);
-    tmc_amb_sort_kernel<<<gs, 256, 0, st>>>(amb_cells, s.amb_key, n_amb, s.amb_hist + 256, s.amb_sorted);
+    tmc_amb_sort_kernel<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n_amb, kSortTile), (int64_t)sms * 8)),
+                          256, 0, st>>>(amb_cells, s.amb_key, n_amb, s.amb_hist + 256, s.amb_sorted);
     static const int r_amb = resident_blocks(tmc_amb_count_kernel, 128);
     tmc_amb_count_kernel<<<(unsigned)wave_grid(r_amb, sms, 16, n_amb, 128), 128, 0, st>>>(
-        space, s.cellof, s.rec, s.tile_sums, s.stats, s.amb_sorted, s.amb_n, reinterpret_cast<AmbRec*>(s.amb_rec));
+        space, s.cellof, s.rec, s.tile_sums, s.stats, s.amb_sorted, s.amb_n, reinterpret_cast<AmbRec*>(s.amb_rec),
+        s.amb_hist + 512);
     k += 4;
   }
   Stage t(prof, "tmc_scan", st);
   scan_tile_sums_kernel<<<1, 1024, 0, st>>>(s.tile_sums, tiles, s.totals);
   tmc_offsets_kernel<<<(unsigned)ceil_div(tiles, kOffsetWarps), 32 * kOffsetWarps, 0, st>>>(s.mask, s.rec, s.tile_sums,
                                                                                            tiles, s.rv, s.toff,
-                                                                                           s.chunks, s.amb_n + 1);
+                                                                                           s.chunks, s.amb_n + 1,
+                                                                                           n_amb > 0 ? s.amb_hist + 512 : nullptr,
+                                                                                           s.totals);
   return k + 2;
 }
 
-int tmc_emit(const CellSpace& space, TmcScratch& s, int64_t n_amb, TmcVertexOut vo, int32_t* tris, const Tuning& tu,
-             cudaStream_t st, Prof* prof) {
+int tmc_emit(const CellSpace& space, TmcScratch& s, int64_t n_amb, int64_t n_overflow, TmcVertexOut vo, int32_t* tris,
+             const Tuning& tu, cudaStream_t st, Prof* prof) {
   const int sms = tu.sms;
   {
     Stage t(prof, "tmc_emit", st);
@@ -1241,11 +1360,15 @@ int tmc_emit(const CellSpace& space, TmcScratch& s, int64_t n_amb, TmcVertexOut 
   }
   if (n_amb == 0) return 1;
   Stage t2(prof, "tmc_ambiguous", st);
-  static const int r_amb = resident_blocks(tmc_ambiguous_kernel, 128);
-  tmc_ambiguous_kernel<<<(unsigned)wave_grid(r_amb, sms, 8, n_amb, 128), 128, 0, st>>>(
+  static const int r_amb = resident_blocks(tmc_ambiguous_kernel, kAmbThreads);
+  tmc_ambiguous_kernel<<<(unsigned)wave_grid(r_amb, sms, 8, n_amb, kAmbThreads), kAmbThreads, 0, st>>>(
       space, s.mask, s.cellof, s.rv, s.toff, s.tile_sums, vo, tris, reinterpret_cast<const AmbRec*>(s.amb_rec),
       s.amb_n);
-  return 2;
+  if (n_overflow == 0) return 2;
+  tmc_ambiguous_again_kernel<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n_amb, 128), (int64_t)sms * 2)),
+                               128, 0, st>>>(space, s.mask, s.cellof, s.rv, s.toff, s.tile_sums, vo, tris,
+                                             reinterpret_cast<const AmbRec*>(s.amb_rec), s.amb_n);
+  return 3;
 }
 
 }  // namespace tmc

@@ -28,7 +28,7 @@ struct TmcScratch {
                         // its p_slice for the emission pass (tmc_cells.cu, AmbRec)
   uint32_t* amb_sorted; // the ambiguous cells' slots sorted by MC case (one per ambiguous cell)
   uint8_t* amb_key;     // their cases, in list order (one per ambiguous cell)
-  unsigned* amb_hist;   // 512: per-case counts, then scatter cursors
+  unsigned* amb_hist;   // 513: per-case counts, scatter cursors, cells that overflow their records
   // listed cells (common.cuh): rec, rv and toff hold one entry per listed cell at its slot, the
   // ambiguous-cell list holds slots
   CellMask* mask;       // per 32 cells of the space
@@ -47,7 +47,8 @@ int tmc_classify(const CellSpace& space, TmcScratch& s, cudaStream_t st, Prof* p
 // The ambiguous cells' counts (p_slice, float64) into their records and s.amb_rec (n_amb records,
 // n_amb = *s.amb_n), then the vertex and triangle offsets.
 int tmc_count(const CellSpace& space, TmcScratch& s, int64_t n_amb, int sms, cudaStream_t st, Prof* prof = nullptr);
-int tmc_emit(const CellSpace& space, TmcScratch& s, int64_t n_amb, TmcVertexOut vo, int32_t* tris, const Tuning& tu,
-             cudaStream_t st, Prof* prof = nullptr);
+// totals[1] after it: cells with more triangles than their records hold (tmc_emit's n_overflow)
+int tmc_emit(const CellSpace& space, TmcScratch& s, int64_t n_amb, int64_t n_overflow, TmcVertexOut vo, int32_t* tris,
+             const Tuning& tu, cudaStream_t st, Prof* prof = nullptr);
 
 }  // namespace tmc
