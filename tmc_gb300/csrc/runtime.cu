@@ -126,7 +126,8 @@ cudaError_t tmc_ambiguous_records(tmc_ctx* ctx, Allocs& al, tmc::TmcScratch& sc,
   if ((e = al.get(&sc.amb_rec, na * tmc::kTmcAmbRecWords)) != cudaSuccess) return e;
   if ((e = al.get(&sc.amb_sorted, na)) != cudaSuccess) return e;
   if ((e = al.get(&sc.amb_key, na)) != cudaSuccess) return e;
-  return al.get(&sc.amb_hist, 513);
+  if ((e = al.get(&sc.amb_doubt, na)) != cudaSuccess) return e;
+  return al.get(&sc.amb_hist, 514);
 }
 
 float iso_up(double iso) {

@@ -154,7 +154,8 @@ struct TriSink {
 // p_slice again (32 words, 16-byte aligned):
 //   w[0]     slot of the cell
 //   w[1]     bits 0-7 MC case, 8-13 triangles, 14-16 inner vertices, 17 triangles beyond the record
-//            (emission runs p_slice again), 18 a singular face the reference cannot triangulate
+//            (emission runs p_slice again), 18 a singular face the reference cannot triangulate,
+//            19 the parameters are float pairs (hi, lo) in the float64 slots
 //   w[2..13] six float64 parameters of the inner vertices: (u, v, w) of the single inner vertex, or
 //            (u0, u1, v0, v1, w0, w1) of the six hexagon corners
 //   w[14..31] kAmbRecTris triangles as packed local codes (TriSink)
@@ -206,6 +207,45 @@ __device__ __forceinline__ void inner_vertex(const double (*P)[3], const double 
     geo.n[o + q] = (float)(in[q] / factor);
     if (geo.v64) geo.v64[o + q] = ip[q];
   }
+}
+
+// The triangles of contours without an inner vertex (:1128-1176).  vid(e): the vertex on edge e.
+template <typename Vid>
+__device__ __forceinline__ void slice_contours(uint64_t c, int cnt, const Vid& vid, TriSink& tri) {
+  int flat = 0;
+  for (int t = 0; t < cnt; t++) {
+    const int sz = cnt_size(c, t);
+    int e[6];
+    for (int q = 0; q < 6; q++) e[q] = (q < sz) ? vid[cnt_edge(c, flat + q)] : -1;
+    switch (sz) {
+      case 3: tri.put(e[0], e[1], e[2]); break;
+      case 4: tri.put(e[0], e[1], e[2]); tri.put(e[0], e[2], e[3]); break;
+      case 5: tri.put(e[0], e[1], e[2]); tri.put(e[0], e[2], e[3]); tri.put(e[0], e[3], e[4]); break;
+      case 6:
+        tri.put(e[0], e[1], e[3]); tri.put(e[1], e[2], e[3]); tri.put(e[0], e[3], e[4]); tri.put(e[0], e[4], e[5]);
+        break;
+      default: break;
+    }
+    flat += sz;
+  }
+}
+// The triangles around one inner vertex (:1262-1281): contours of three edges stay triangles, the
+// others fan around it; returns whether any does.
+template <typename Vid>
+__device__ __forceinline__ bool slice_fans(uint64_t c, int cnt, const Vid& vid, int32_t inner, TriSink& tri) {
+  bool used = false;
+  int flat = 0;
+  for (int t = 0; t < cnt; t++) {
+    const int sz = cnt_size(c, t);
+    if (sz == 3) {
+      tri.put(vid[cnt_edge(c, flat)], vid[cnt_edge(c, flat + 1)], vid[cnt_edge(c, flat + 2)]);
+    } else {
+      used = true;
+      for (int r = 0; r < sz; r++) tri.put(vid[cnt_edge(c, flat + r)], vid[cnt_edge(c, flat + (r + 1) % sz)], inner);
+    }
+    flat += sz;
+  }
+  return used;
 }
 
 __device__ AmbResult p_slice_dev(unsigned ic, const double F[8], double iso, const int32_t vid[12], int32_t ibase,
@@ -402,22 +442,7 @@ __device__ AmbResult p_slice_dev(unsigned ic, const double F[8], double iso, con
   const unsigned nr_w = ((q_sol & 0x18) == 0x18) + ((q_sol & 0x24) == 0x24);
   const unsigned nr_t = nr_u + nr_v + nr_w;
   if (nr_t == nr_u || nr_t == nr_v || nr_t == nr_w) {
-    int flat = 0;
-    for (int t = 0; t < cnt; t++) {
-      const int sz = cnt_size(c, t);
-      int e[6];
-      for (int q = 0; q < 6; q++) e[q] = (q < sz) ? vid[cnt_edge(c, flat + q)] : -1;
-      switch (sz) {
-        case 3: tri.put(e[0], e[1], e[2]); break;
-        case 4: tri.put(e[0], e[1], e[2]); tri.put(e[0], e[2], e[3]); break;
-        case 5: tri.put(e[0], e[1], e[2]); tri.put(e[0], e[2], e[3]); tri.put(e[0], e[3], e[4]); break;
-        case 6:
-          tri.put(e[0], e[1], e[3]); tri.put(e[1], e[2], e[3]); tri.put(e[0], e[3], e[4]); tri.put(e[0], e[4], e[5]);
-          break;
-        default: break;
-      }
-      flat += sz;
-    }
+    slice_contours(c, cnt, vid, tri);
     return res;
   }
   // saddle points: one inner vertex (:1178-1296)
@@ -450,18 +475,7 @@ __device__ AmbResult p_slice_dev(unsigned ic, const double F[8], double iso, con
       uc = fs00 * ui[0] + fs01 * ui[1]; vc = fs00 * vi[0] + fs01 * vi[1]; wc = fs00 * wi[0] + fs01 * wi[1];
     }
   }
-  bool pt_used = false;
-  int flat = 0;
-  for (int t = 0; t < cnt; t++) {
-    const int sz = cnt_size(c, t);
-    if (sz == 3) {
-      tri.put(vid[cnt_edge(c, flat)], vid[cnt_edge(c, flat + 1)], vid[cnt_edge(c, flat + 2)]);
-    } else {
-      pt_used = true;
-      for (int r = 0; r < sz; r++) tri.put(vid[cnt_edge(c, flat + r)], vid[cnt_edge(c, flat + (r + 1) % sz)], ibase);
-    }
-    flat += sz;
-  }
+  const bool pt_used = slice_fans(c, cnt, vid, ibase, tri);
   if (pt_used) {
     res.inner = 1;
     if (geo) inner_vertex(P, N, uc, vc, wc, *geo, ibase);
@@ -538,9 +552,8 @@ __device__ __noinline__ void inner_vertex_f64(const Grid& g, int i, int j, int k
 
 // The same for float32 outputs in float-float (within 2^-44 of the position's size; the normal within
 // 2^-30 of the float64 one), except where the gradients cancel to below 2^-10 of their size.
-__device__ __forceinline__ void inner_vertex_ff(const Grid& g, int i, int j, int k, double u, double v, double w,
-                                                const TmcVertexOut& out, int64_t at) {
-  const ffx::ff U = ffx::ff_from_double(u), V = ffx::ff_from_double(v), W = ffx::ff_from_double(w);
+__device__ __noinline__ void inner_vertex_ff(const Grid& g, int i, int j, int k, ffx::ff U, ffx::ff V, ffx::ff W,
+                                             const TmcVertexOut out, int64_t at) {
   auto lerp = [](ffx::ff a, ffx::ff b, ffx::ff t) {
     return ffx::ff_add_abs(a, ffx::ff_mul(ffx::ff_add_abs(b, ffx::ff_neg(a)), t));
   };
@@ -565,7 +578,7 @@ __device__ __forceinline__ void inner_vertex_ff(const Grid& g, int i, int j, int
   const ffx::ff dot =
       ffx::ff_add(ffx::ff_add(ffx::ff_mul(in[0], in[0]), ffx::ff_mul(in[1], in[1])), ffx::ff_mul(in[2], in[2]));
   if (!(dot.hi > 0x1p-80f && dot.hi < 0x1p80f) || !(scale <= 0x1p10f * sqrtf(dot.hi))) {
-    inner_vertex_f64(g, i, j, k, u, v, w, out, at);
+    inner_vertex_f64(g, i, j, k, ffx::ff_to_double(U), ffx::ff_to_double(V), ffx::ff_to_double(W), out, at);
     return;
   }
   // 1/sqrt(dot): float estimate and one Newton step in float-float
@@ -723,18 +736,244 @@ __global__ void __launch_bounds__(256) tmc_amb_sort_kernel(const uint32_t* list,
   }
 }
 
-// Ambiguous cells from the classification's list: p_slice in counting mode (float64); the counts go
+// ------------------------------------------------------------------------------------------
+// p_slice's decisions on the FP32 pipes: float pairs with error bounds
+// ------------------------------------------------------------------------------------------
+// The float64 pipe runs at 1/57 of the float32 rate, and p_slice needs some 250 float64 operations
+// per cell for a handful of decisions: which side of the isovalue each saddle face's decider lies on,
+// and which roots of the inner quadratic lie in (0, 1).  Here each is computed in float pairs with a
+// bound of its distance to the reference's float64 value (whose own roundings are some 2^-7 of it),
+// and taken when the bound leaves no doubt.  A cell with any doubt, a singular face, an inner hexagon,
+// or an inner vertex whose float64 position is an output, is left to the float64 kernel: 0.3 % of the
+// ambiguous cells of the 512^3 noise field, 21 % of the 1024x1024x64 field of near-singular saddles.
+// Both passes: 0.17 + 0.07 ms and 1.35 + 2.0 ms; 0.64 and 5.94 ms with every cell in float64.
+//
+// The corner values and the isovalue are scaled by the power of two that brings the largest into
+// [1, 2) (the parameters do not change), away from both ends of the float range.
+struct Root {
+  ffx::ff x;
+  float e;  // bound
+};
+// 1: x surely in (0, 1), 0: surely not, -1: in doubt
+__device__ __forceinline__ int in_unit(const Root& r) {
+  const float e = r.e * 1.01f, y = (1.0f - r.x.hi) - r.x.lo;
+  if (r.x.hi > e && y > e) return 1;
+  if (r.x.hi < -e || y < -e) return 0;
+  return -1;
+}
+// (iso - g1) / (g2 - g1) with g1 = f0 + u (f1 - f0), g2 = f2 + u (f3 - f2)
+__device__ __forceinline__ Root cross_root(float f0, float f1, float f2, float f3, ffx::ff iso, const Root& u) {
+  using namespace ffx;
+  const ff d0 = two_sum(f1, -f0), d1 = two_sum(f3, -f2);
+  const ff g1 = ff_add_abs(ff_from(f0), ff_mul(u.x, d0)), g2 = ff_add_abs(ff_from(f2), ff_mul(u.x, d1));
+  const ff num = ff_add_abs(iso, ff_neg(g1)), den = ff_add_abs(g2, ff_neg(g1));
+  const float step = (1.0f + 2.0f * fabsf(u.x.hi)) * 0x1p-42f;  // of each pair operation here
+  const float e1 = fabsf(d0.hi) * u.e + step, e2 = fabsf(d1.hi) * u.e + step;
+  const float en = e1 + step, ed = e1 + e2 + 2 * step, ad = fabsf(den.hi);
+  Root v;
+  if (!(ad > 4 * ed && ad > 0x1p-60f)) return Root{ff_from(0.0f), INFINITY};
+  v.x = ff_quot(num, den, rcp_est(den.hi));
+  v.e = ((en + fabsf(v.x.hi) * ed) * rcp_est(ad - ed) + fabsf(v.x.hi) * 0x1p-42f) * 1.01f;
+  return v;
+}
+
+// Contours and roots of one ambiguous cell with scaled corners f; false when in doubt.  The roots are
+// those of mc/MarchingCubes.cpp:715-795, q_sol its bit set (0 without real roots).
+__device__ __forceinline__ bool slice_decide(const float f[8], ffx::ff iso, unsigned cs, uint64_t& contours,
+                                             Root u[2], Root v[2], Root w[2], unsigned& q_sol) {
+  using namespace ffx;
+  uint64_t to = ~0ull;
+  bool ok = true;
+#pragma unroll
+  for (int q = 0; q < 6; q++) {
+    const uint32_t fv = face_v_pack(q);
+    const int fc = face_case(cs, fv);
+    int sep = 0;
+    if (fc == 6 || fc == 9) {
+      const float a = f[nib(fv, 0)], b = f[nib(fv, 1)], c = f[nib(fv, 2)], d = f[nib(fv, 3)];
+      const ff num = ff_add_abs(two_prod(a, d), ff_neg(two_prod(b, c)));
+      const ff den = ff_add_abs(two_sum(a, -b), two_sum(d, -c));
+      // decider > isovalue  <=>  num - iso den has den's sign; magnitudes 8 and 16
+      const ff t = ff_add_abs(num, ff_neg(ff_mul(iso, den)));
+      ok = ok && fabsf(t.hi) > 0x1p-38f && fabsf(den.hi) > 0x1p-24f;
+      sep = (t.hi > 0.0f) == (den.hi > 0.0f);
+    }
+    face_segments(fc, sep, face_e_pack(q), to);
+  }
+  if (!ok) return false;
+  contours = connect_contours(to, case_edge_mask(cs));
+  // a = d01 t1 - d45 t2, b = i0 t1 + d01 d64 - i4 t2 - d45 d20, c = i0 d64 - i4 d20, t1 = d76 + d45,
+  // t2 = d32 + d01, i = iso - f.  The d are exact; with T1, T2, I0, I4 the sums of the magnitudes that
+  // t1, t2, i0, i4 add up, each product errs by at most 2^-43.8 of the product of those (the pair sums
+  // by 2^-46, the pair product by 2^-45), their sums by 2^-45 more.
+  const ff d01 = two_sum(f[0], -f[1]), d45 = two_sum(f[4], -f[5]), d64 = two_sum(f[6], -f[4]), d20 = two_sum(f[2], -f[0]);
+  const ff d76 = two_sum(f[7], -f[6]), d32 = two_sum(f[3], -f[2]);
+  const ff t1 = ff_add_abs(d76, d45), t2 = ff_add_abs(d32, d01);
+  const ff i0 = ff_add_abs(iso, ff_from(-f[0])), i4 = ff_add_abs(iso, ff_from(-f[4]));
+  const ff a = ff_add_abs(ff_mul(d01, t1), ff_neg(ff_mul(d45, t2)));
+  const ff b = ff_add_abs(ff_add_abs(ff_mul(i0, t1), ff_mul(d01, d64)),
+                          ff_neg(ff_add_abs(ff_mul(i4, t2), ff_mul(d45, d20))));
+  const ff c = ff_add_abs(ff_mul(i0, d64), ff_neg(ff_mul(i4, d20)));
+  const float m01 = fabsf(d01.hi), m45 = fabsf(d45.hi), m64 = fabsf(d64.hi), m20 = fabsf(d20.hi);
+  const float T1 = fabsf(d76.hi) + m45, T2 = fabsf(d32.hi) + m01;
+  const float I0 = fabsf(iso.hi) + fabsf(f[0]), I4 = fabsf(iso.hi) + fabsf(f[4]);
+  const float Ea = (m01 * T1 + m45 * T2) * 0x1p-43f + 0x1p-80f;
+  const float Eb = (I0 * T1 + m01 * m64 + I4 * T2 + m45 * m20) * 0x1p-43f + 0x1p-80f;
+  const float Ec = (I0 * m64 + I4 * m20) * 0x1p-43f + 0x1p-80f;
+  const float aa = fabsf(a.hi), ab = fabsf(b.hi), ac = fabsf(c.hi);
+  const ff b2 = ff_mul(b, b), ac4 = ff_mul(ff{4 * a.hi, 4 * a.lo}, c);
+  const ff d = ff_add_abs(b2, ff_neg(ac4));
+  const float Ed = (2 * ab * Eb + 4 * (aa * Ec + ac * Ea) + (b2.hi + fabsf(ac4.hi)) * 0x1p-43f + 0x1p-70f) * 1.01f;
+  q_sol = 0;
+  if (d.hi < -Ed) return true;  // no real roots
+  if (!(d.hi > 2 * Ed && aa > 4 * Ea)) return false;
+  // s = sqrt(d): the rounded root and one Newton step
+  const float s0 = sqrtf(d.hi), rs = rcp_est(s0);
+  const ff p = two_prod(s0, s0);
+  const ff s = quick_two_sum(s0, (((d.hi - p.hi) - p.lo) + d.lo) * (0.5f * rs));
+  const float Es = Ed * rs + s0 * 0x1p-43f;
+  const ff a2{2 * a.hi, 2 * a.lo};
+  const float ra = rcp_est(a2.hi);
+#pragma unroll
+  for (int r = 0; r < 2; r++) {
+    const ff n = ff_add_abs(ff_neg(b), r == 0 ? ff_neg(s) : s);
+    u[r].x = ff_quot(n, a2, ra);
+    const float au = fabsf(u[r].x.hi);
+    u[r].e = ((Eb + Es + (ab + s0) * 0x1p-45f + au * (2 * Ea)) * rcp_est(2 * (aa - Ea)) + au * 0x1p-42f) * 1.01f;
+    v[r] = cross_root(f[0], f[1], f[2], f[3], iso, u[r]);
+    w[r] = cross_root(f[0], f[1], f[4], f[5], iso, u[r]);
+    const int x = in_unit(u[r]), y = in_unit(v[r]), z = in_unit(w[r]);
+    if (x < 0 || y < 0 || z < 0) return false;
+    q_sol |= (unsigned)x << r | (unsigned)y << (2 + r) | (unsigned)z << (4 + r);
+  }
+  return true;
+}
+
+struct IdentityVid {  // local codes: edges 0..11
+  __device__ __forceinline__ int operator[](int e) const { return e; }
+};
+
+// The inner vertex of a cell with saddle points (mc/MarchingCubes.cpp:1178-1261), from the certain
+// roots; false when a parameter is not known to 2^-28 (its bound; the value itself is some 2^-10 of that off).
+__device__ __forceinline__ bool slice_center(unsigned q_sol, const Root u[2], const Root v[2], const Root w[2],
+                                             ffx::ff out[3]) {
+  using namespace ffx;
+  const unsigned f00 = q_sol & 1, f01 = (q_sol >> 1) & 1, f10 = (q_sol >> 2) & 1, f11 = (q_sol >> 3) & 1,
+                 f20 = (q_sol >> 4) & 1, f21 = (q_sol >> 5) & 1;
+  const unsigned fc1 = f00 * f10 + f01 * f11, fc2 = f00 * f20 + f01 * f21, fc3 = f10 * f21 + f11 * f20;
+  const unsigned faces = fc1 + fc2 + fc3;
+  float e = 0;
+  // s0 x0 + s1 x1
+  auto pick = [&e](unsigned s0, const Root& x0, unsigned s1, const Root& x1) {
+    e = fmaxf(e, (s0 ? x0.e : 0.0f) + (s1 ? x1.e : 0.0f));
+    return ff_add_abs(s0 ? x0.x : ff_from(0.0f), s1 ? x1.x : ff_from(0.0f));
+  };
+  auto half = [](ff x, unsigned n) { return n == 2 ? ff{0.5f * x.hi, 0.5f * x.lo} : x; };
+  out[0] = out[1] = out[2] = ff_from(0.0f);
+  if (faces == 2) {
+    if (fc1 == 0) {
+      out[0] = pick(f00, u[0], f01, u[1]); out[1] = pick(f10, v[0], f11, v[1]); out[2] = pick(f10, w[1], f11, w[0]);
+    } else if (fc2 == 0) {
+      out[0] = pick(f00, u[0], f01, u[1]); out[1] = pick(f00, v[0], f01, v[1]); out[2] = pick(f00, w[1], f01, w[0]);
+    } else if (fc3 == 0) {
+      out[0] = pick(f10, u[0], f11, u[1]); out[1] = pick(f10, v[0], f11, v[1]); out[2] = pick(f10, w[0], f11, w[1]);
+    }
+  } else if (faces == 3) {
+    if (!(f00 + f01) || !(f10 + f11) || !(f20 + f21)) return false;
+    out[0] = half(pick(f00, u[0], f01, u[1]), f00 + f01);
+    out[1] = half(pick(f10, v[0], f11, v[1]), f10 + f11);
+    out[2] = half(pick(f20, w[0], f21, w[1]), f20 + f21);
+  } else if (faces == 4) {
+    if (f20 + f21 == 1) {
+      out[0] = pick(f20, u[0], f21, u[1]); out[1] = pick(f21, v[0], f20, v[1]); out[2] = pick(f20, w[0], f21, w[1]);
+    } else if (f10 + f11 == 1) {
+      out[0] = pick(f10, u[0], f11, u[1]); out[1] = pick(f10, v[0], f11, v[1]); out[2] = pick(f11, w[0], f10, w[1]);
+    } else if (f00 + f01 == 1) {
+      out[0] = pick(f00, u[0], f01, u[1]); out[1] = pick(f00, v[0], f01, v[1]); out[2] = pick(f00, w[0], f01, w[1]);
+    }
+  }
+  return e <= 0x1p-28f;
+}
+
+// Ambiguous cells from the case-sorted list, on the FP32 pipes: what tmc_amb_count_kernel writes for
+// them, or their place in the list appended to `doubt` for that kernel.
+__global__ void __launch_bounds__(128) tmc_amb_decide_kernel(CellSpace space, const uint16_t* cellof, uint32_t* rec,
+                                                             unsigned long long* tile_sums, const uint32_t* list,
+                                                             unsigned na, AmbRec* recs, uint32_t* doubt,
+                                                             unsigned* ndoubt) {
+  for (unsigned a = blockIdx.x * blockDim.x + threadIdx.x; a < na; a += gridDim.x * blockDim.x) {
+    const uint32_t slot = list[a];
+    const int64_t vcell = slot_cell(cellof, slot);
+    const Grid& g = space.grids ? space.grids[__ldg(space.tile_vol + vcell / kScanTile)] : space.one;
+    int i, j, k;
+    tcell_ijk(g, vcell - g.vbase, i, j, k);
+    float f[8];
+    tload_corners(g, i, j, k, f);
+    unsigned cs = 0;
+    float m = fabsf(g.iso_f);
+#pragma unroll
+    for (int v = 0; v < 8; v++) {
+      cs |= (unsigned)(f[v] >= g.iso_up) << v;
+      m = fmaxf(m, fabsf(f[v]));
+    }
+    const bool pos64 = (g.flags & kGridPos64) != 0;
+    // scale by 2^-e, e the exponent of the largest value (in two exact steps: e may be near the ends)
+    const int ex = (int)(ffx::fbits(m) >> 23) - 127;
+    bool ok = m > 0x1p-100f && m < 0x1p100f;
+    const float sc = ffx::bitsf((uint32_t)(127 - (ok ? ex : 0)) << 23);
+#pragma unroll
+    for (int v = 0; v < 8; v++) f[v] *= sc;
+    const ffx::ff iso{g.iso_f * sc, g.iso_lo * sc};
+    uint64_t c = 0;
+    Root u[2], v[2], w[2];
+    unsigned q_sol = 0;
+    ok = ok && slice_decide(f, iso, cs, c, u, v, w, q_sol) && __popc(q_sol) != 6;
+    if (ok) {
+      AmbRec& R = recs[a];
+      TriSink ts{nullptr, R.tri, 0};
+      const int cnt = cnt_count(c);
+      const unsigned nr_u = ((q_sol & 0x5) == 0x5) + ((q_sol & 0xA) == 0xA);
+      const unsigned nr_v = ((q_sol & 0x11) == 0x11) + ((q_sol & 0x22) == 0x22);
+      const unsigned nr_w = ((q_sol & 0x18) == 0x18) + ((q_sol & 0x24) == 0x24);
+      const unsigned nr_t = nr_u + nr_v + nr_w;
+      int inner = 0;
+      if (nr_t == nr_u || nr_t == nr_v || nr_t == nr_w) {
+        slice_contours(c, cnt, IdentityVid{}, ts);
+      } else {
+        ffx::ff x[3];
+        ok = !pos64 && slice_center(q_sol, u, v, w, x);
+        if (ok && slice_fans(c, cnt, IdentityVid{}, 12, ts)) {
+          inner = 1;
+          float2* prm = reinterpret_cast<float2*>(R.prm);
+#pragma unroll
+          for (int d = 0; d < 3; d++) prm[d] = make_float2(x[d].hi, x[d].lo);
+        }
+      }
+      if (ok) {
+        R.slot = slot;
+        R.info = cs | (uint32_t)ts.n << 8 | (uint32_t)inner << 14 | (1u << 19);
+        rec[slot] |= (uint32_t)inner << 12 | (uint32_t)ts.n << 15;
+        const unsigned long long add = ((unsigned long long)inner << 32) | (unsigned long long)ts.n;
+        if (add) atomicAdd(tile_sums + (slot >> kTileShift), add);
+      }
+    }
+    if (!ok) doubt[atomicAdd(ndoubt, 1u)] = a;
+  }
+}
+
+// Ambiguous cells in doubt (places in the case-sorted list): p_slice in counting mode (float64); the counts go
 // into the cell record and, atomically, into the cell's tile sum (one thread per listed cell, no
 // tile barrier to wait on).  The triangles (as local codes) and the inner vertices' parameters go
 // into the cell's ambiguous-cell record, which the emission pass reads instead of running p_slice.
 __global__ void __launch_bounds__(128) tmc_amb_count_kernel(CellSpace space, const uint16_t* cellof, uint32_t* rec,
                                                             unsigned long long* tile_sums,
                                                             unsigned long long* stats, const uint32_t* list,
-                                                            const unsigned* count, AmbRec* recs,
-                                                            unsigned* overflow) {
+                                                            const uint32_t* doubt, const unsigned* count,
+                                                            AmbRec* recs, unsigned* overflow) {
   const unsigned na = *count;
   unsigned long long sing = 0;
-  for (unsigned a = blockIdx.x * blockDim.x + threadIdx.x; a < na; a += gridDim.x * blockDim.x) {
+  for (unsigned x = blockIdx.x * blockDim.x + threadIdx.x; x < na; x += gridDim.x * blockDim.x) {
+    const unsigned a = doubt[x];
     const uint32_t slot = list[a];
     const int64_t vcell = slot_cell(cellof, slot);
     const Grid g = space.grid_of_tile(vcell / kScanTile);
@@ -1107,6 +1346,13 @@ __global__ void __launch_bounds__(kAmbThreads) tmc_ambiguous_kernel(CellSpace sp
       const int4 c = cells[wid][o];
       const Grid& g = space.grids ? space.grids[c.w] : space.one;
       const double* prm = recs[a0 + o].prm;
+      if ((recs[a0 + o].info >> 19) & 1) {  // float pairs: one inner vertex, float32 outputs
+        const float2* x = reinterpret_cast<const float2*>(prm);
+        const ffx::ff U{x[0].x, x[0].y}, V{x[1].x, x[1].y}, W{x[2].x, x[2].y};
+        inner_vertex_ff(g, c.x, c.y, c.z, U, V, W, out,
+                        (int64_t)vid[32 * 12 + o] + (int32_t)(__ldg(tile_off + g.vbase / kScanTile) >> 32));
+        continue;
+      }
       double u = prm[0], v = prm[1], w = prm[2];
       if (iupto[wid][o] - from > 1) {  // corner q of the inner hexagon (hex_corners)
         u = prm[(0x1C >> q) & 1];
@@ -1117,7 +1363,7 @@ __global__ void __launch_bounds__(kAmbThreads) tmc_ambiguous_kernel(CellSpace sp
       const int64_t at = (int64_t)vid[32 * (12 + q) + o] + (int32_t)(__ldg(tile_off + g.vbase / kScanTile) >> 32);
       // float64 outputs requested for this volume: the reference's float64 arithmetic
       if (g.flags & kGridPos64) inner_vertex_f64(g, c.x, c.y, c.z, u, v, w, out, at);
-      else inner_vertex_ff(g, c.x, c.y, c.z, u, v, w, out, at);
+      else inner_vertex_ff(g, c.x, c.y, c.z, ffx::ff_from_double(u), ffx::ff_from_double(v), ffx::ff_from_double(w), out, at);
     }
     __syncwarp();  // the columns are read
   }
@@ -1316,16 +1562,20 @@ int tmc_count(const CellSpace& space, TmcScratch& s, int64_t n_amb, int sms, cud
     Stage ta(prof, "tmc_amb_count", st);
     // the list sorted by MC case (the records follow its order, so the emission pass is sorted too)
     const unsigned gs = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n_amb, 256), (int64_t)sms * 8));
-    cudaMemsetAsync(s.amb_hist, 0, 513 * sizeof(unsigned), st);
+    cudaMemsetAsync(s.amb_hist, 0, 514 * sizeof(unsigned), st);
     tmc_amb_key_kernel<<<gs, 256, 0, st>>>(space, s.cellof, amb_cells, n_amb, s.amb_key, s.amb_hist);
     tmc_amb_cursor_kernel<<<1, 256, 0, st>>>(s.amb_hist, s.amb_hist + 256);
     tmc_amb_sort_kernel<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n_amb, kSortTile), (int64_t)sms * 8)),
                           256, 0, st>>>(amb_cells, s.amb_key, n_amb, s.amb_hist + 256, s.amb_sorted);
+    static const int r_decide = resident_blocks(tmc_amb_decide_kernel, 128);
+    tmc_amb_decide_kernel<<<(unsigned)wave_grid(r_decide, sms, 16, n_amb, 128), 128, 0, st>>>(
+        space, s.cellof, s.rec, s.tile_sums, s.amb_sorted, (unsigned)n_amb, reinterpret_cast<AmbRec*>(s.amb_rec),
+        s.amb_doubt, s.amb_hist + 513);
     static const int r_amb = resident_blocks(tmc_amb_count_kernel, 128);
-    tmc_amb_count_kernel<<<(unsigned)wave_grid(r_amb, sms, 16, n_amb, 128), 128, 0, st>>>(
-        space, s.cellof, s.rec, s.tile_sums, s.stats, s.amb_sorted, s.amb_n, reinterpret_cast<AmbRec*>(s.amb_rec),
-        s.amb_hist + 512);
-    k += 4;
+    tmc_amb_count_kernel<<<(unsigned)wave_grid(r_amb, sms, 4, n_amb, 128), 128, 0, st>>>(
+        space, s.cellof, s.rec, s.tile_sums, s.stats, s.amb_sorted, s.amb_doubt, s.amb_hist + 513,
+        reinterpret_cast<AmbRec*>(s.amb_rec), s.amb_hist + 512);
+    k += 5;
   }
   Stage t(prof, "tmc_scan", st);
   scan_tile_sums_kernel<<<1, 1024, 0, st>>>(s.tile_sums, tiles, s.totals);
