@@ -179,16 +179,6 @@ __global__ void __launch_bounds__(32 * kOffsetWarps) dmc_offsets_kernel(const Ce
 // estimateGradient at a grid point (cpp_dmc/UniformGrid.cpp:512-540): central differences with
 // the reference's border indexing ((i<0) ? 0 : (i>=max) ? max-i : i).
 __device__ __forceinline__ int grad_index(int i, int max) { return (i < 0) ? 0 : (i >= max) ? max - i : i; }
-// Central differences at a grid point, exact as float pairs (the reference's float64 difference
-// of two floats); the 1/(2*spacing) factor is applied after the interpolation.
-__device__ __forceinline__ void point_diff_ff(const Grid& g, int i, int j, int k, ffx::ff out[3]) {
-  const int i0 = grad_index(i - 1, g.nx), i1 = grad_index(i + 1, g.nx);
-  const int j0 = grad_index(j - 1, g.ny), j1 = grad_index(j + 1, g.ny);
-  const int k0 = grad_index(k - 1, g.nz), k1 = grad_index(k + 1, g.nz);
-  out[0] = ffx::two_sum(g.at(i1, j, k), -g.at(i0, j, k));
-  out[1] = ffx::two_sum(g.at(i, j1, k), -g.at(i, j0, k));
-  out[2] = ffx::two_sum(g.at(i, j, k1), -g.at(i, j, k0));
-}
 // a + t*(b - a) in float-float
 __device__ __forceinline__ ffx::ff ff_lerp(ffx::ff a, ffx::ff b, float t) {
   return ffx::ff_add(a, ffx::ff_mul_f(ffx::ff_sub(b, a), t));
@@ -199,7 +189,7 @@ struct Normal64 {
 };
 // The reference's float64 normal (UniformGrid::normal on estimateGradient values), for the rare
 // vertices whose gradients cancel so much that the float-float result would lose its margin.
-__device__ __noinline__ Normal64 normal_f64(const Grid g, int i, int j, int k, double pu, double pv, double pw,
+__device__ __noinline__ Normal64 normal_f64(const Grid& g, int i, int j, int k, double pu, double pv, double pw,
                                             int flip) {
   const double inv2d[3] = {1.0 / (2 * g.dx), 1.0 / (2 * g.dy), 1.0 / (2 * g.dz)};
   double G[8][3];
@@ -225,13 +215,73 @@ __device__ __noinline__ Normal64 normal_f64(const Grid g, int i, int j, int k, d
   for (int d = 0; d < 3; d++) r.n[d] = nv3[d] / s;
   return r;
 }
-__device__ __forceinline__ void point_gradient_f(const Grid& g, int i, int j, int k, float inv2d[3], float out[3]) {
-  const int i0 = grad_index(i - 1, g.nx), i1 = grad_index(i + 1, g.nx);
-  const int j0 = grad_index(j - 1, g.ny), j1 = grad_index(j + 1, g.ny);
-  const int k0 = grad_index(k - 1, g.nz), k1 = grad_index(k + 1, g.nz);
-  out[0] = (g.at(i1, j, k) - g.at(i0, j, k)) * inv2d[0];
-  out[1] = (g.at(i, j1, k) - g.at(i, j0, k)) * inv2d[1];
-  out[2] = (g.at(i, j, k1) - g.at(i, j, k0)) * inv2d[2];
+// The 32 field values behind the central differences at a cell's corners: the corners themselves and,
+// along each axis, the four values before and the four after them (one end of every difference is a
+// corner).  The reference's border indexing (grad_index): before index 0 comes point 0, after the last
+// point comes point 0.
+// One axis at a time: the corners stay, the axis's eight outer values are loaded when it is its turn.
+struct AxisLines {
+  float lo[4], hi[4];  // before and after, the four corner lines in corner order
+};
+__device__ __forceinline__ void load_axis(const Grid& g, int i, int j, int k, int d, AxisLines& S) {
+  const int64_t sy = g.nx, sz = (int64_t)g.nx * g.ny;
+  const float* f = g.f + (int64_t)k * sz + (int64_t)j * sy + i;
+  const int64_t st = d == 0 ? 1 : (d == 1 ? sy : sz);
+  const int at = d == 0 ? i : (d == 1 ? j : k), n = d == 0 ? g.nx : (d == 1 ? g.ny : g.nz);
+  const float* lo = at > 0 ? f - st : f;
+  const float* hi = at + 2 < n ? f + 2 * st : f - at * st;
+  const int64_t sa = d == 0 ? sy : 1, sb = d == 2 ? sy : sz;
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const int64_t o = (q & 1 ? sa : 0) + (q & 2 ? sb : 0);
+    S.lo[q] = __ldg(lo + o);
+    S.hi[q] = __ldg(hi + o);
+  }
+}
+// the two values of the difference along axis d at corner q
+__device__ __forceinline__ void corner_pair(const float c[8], const AxisLines& S, int d, int q, float& hi, float& lo) {
+  const int line = d == 0 ? q >> 1 : (d == 1 ? (q & 1) | (q >> 1 & 2) : q & 3);
+  const bool up = (q >> d) & 1;
+  hi = up ? S.hi[line] : c[q | 1 << d];
+  lo = up ? c[q & ~(1 << d)] : S.lo[line];
+}
+
+// The normal at local coordinates p from the corner differences, as float pairs normalised (within
+// 2^-30 of the reference's float64 normal); false where the gradients cancel to below 2^-10 of their
+// size (float64 there).
+__device__ __forceinline__ bool normal_ff(const Grid& g, int i, int j, int k, const float c[8], const float p[3],
+                                          int flip, ffx::ff out[3]) {
+  ffx::ff nv3[3];
+  float scale = 0;  // largest |difference| * 1/(2 spacing): the size of the interpolation's inputs
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    AxisLines S;
+    load_axis(g, i, j, k, d, S);
+    ffx::ff G[8];
+    float md = 0;
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      float hi, lo;
+      corner_pair(c, S, d, q, hi, lo);
+      G[q] = ffx::two_sum(hi, -lo);
+      md = fmaxf(md, fabsf(G[q].hi));
+    }
+    scale = fmaxf(scale, md * g.inv2_hi[d]);
+    const ffx::ff a0 = ff_lerp(G[0], G[1], p[0]), a1 = ff_lerp(G[2], G[3], p[0]);
+    const ffx::ff a2 = ff_lerp(G[4], G[5], p[0]), a3 = ff_lerp(G[6], G[7], p[0]);
+    const ffx::ff b0 = ff_lerp(a0, a1, p[1]), b1 = ff_lerp(a2, a3, p[1]);
+    const ffx::ff t = ffx::ff_mul(ff_lerp(b0, b1, p[2]), ffx::ff{g.inv2_hi[d], g.inv2_lo[d]});
+    nv3[d] = flip ? ffx::ff_neg(t) : t;
+  }
+  const ffx::ff dot =
+      ffx::ff_add(ffx::ff_add(ffx::ff_mul(nv3[0], nv3[0]), ffx::ff_mul(nv3[1], nv3[1])), ffx::ff_mul(nv3[2], nv3[2]));
+  // 1/sqrt(dot): float estimate and one Newton step in float-float
+  const float r0 = rsqrtf(dot.hi);
+  const ffx::ff h = ffx::ff_mul_f(ffx::ff_mul_f(dot, r0), r0);
+  const ffx::ff r = ffx::ff_mul_f(ffx::ff_sub(ffx::ff_from(1.5f), ffx::ff_mul_f(h, 0.5f)), r0);
+#pragma unroll
+  for (int d = 0; d < 3; d++) out[d] = ffx::ff_mul(nv3[d], r);
+  return dot.hi > 0x1p-80f && dot.hi < 0x1p80f && scale <= 0x1p10f * sqrtf(dot.hi);
 }
 
 constexpr int kVertexThreads = 128;
@@ -242,18 +292,12 @@ struct GridCache {
   int vol = -1;
   Grid g{};
   ffx::ff iso_ff{0, 0};
-  float inv2d[3] = {0, 0, 0};
-  ffx::ff inv2d_ff[3] = {{0, 0}, {0, 0}, {0, 0}};
   __device__ __forceinline__ void load(const CellSpace& space, uint32_t vcell) {
     const int v = space.grids ? __ldg(space.tile_vol + vcell / kScanTile) : 0;
     if (v == vol) return;
     vol = v;
     g = space.grids ? space.grids[v] : space.one;
     iso_ff = ffx::ff_from_double(g.iso);
-    for (int d = 0; d < 3; d++) {
-      inv2d[d] = (float)g.inv2[d];
-      inv2d_ff[d] = ffx::ff_from_double(g.inv2[d]);
-    }
   }
 };
 
@@ -310,115 +354,91 @@ __device__ __forceinline__ bool vertex_contour(const Grid& g, int i, int j, int 
 // Position, normal and local coordinates of vertex vidx at local coordinates p of cell (i, j, k).
 // p64: the float64 local coordinates when they are not the floats p (the reference's unrounded mean
 // point, for contours without any valid projection sample), else null.
-// kFF: the float-float normal path (float64 normals kept for the simplification) is compiled in
+// kFF: some volume keeps normals as float pairs (simplification); the float32 normals alone otherwise
+// Float64 (1/57 of the float32 rate) is kept to what it must decide: positions that are float64
+// outputs, float32 positions whose rounding the float pair does not certify, normals whose gradients
+// cancel to below 2^-10 of their size.  The gradients take 32 field loads (48 point by point), one
+// axis after another (109 registers).  16.6 M vertices with float64 positions and pair normals: 1.40
+// -> 1.09 ms; 7.6 M with float32 outputs: 0.49 -> 0.30 ms; 47 M of the saddle field, where many
+// gradients cancel to below 1/16 (float64 normals before): 15.4 -> 2.74 ms.
 template <bool kFF = true>
-__device__ __forceinline__ void vertex_outputs(const GridCache& G, int i, int j, int k, int64_t cell,
+__device__ __forceinline__ void vertex_outputs(const Grid& g, int i, int j, int k, int64_t cell,
                                                const float p[3], const double* p64, int64_t vidx,
                                                const DmcVertexOut& out, int flip, repr::Stats& st) {
-  const Grid& g = G.g;
   const int64_t o = 3 * vidx;
   // a simplified volume: its float32 positions and normals are written after the passes, from the
   // float64 positions and the float-pair normals kept here
   const bool keep64 = out.n64 && (g.flags & kGridNormal64);
   float2* n2 = reinterpret_cast<float2*>(out.n64);
   // position: UniformGrid::position (cpp_dmc/UniformGrid.h:300-305)
-  const double lx = p64 ? p64[0] : (double)p[0], ly = p64 ? p64[1] : (double)p[1], lz = p64 ? p64[2] : (double)p[2];
-  const double px = g.ox + (i + lx) * g.dx;
-  const double py = g.oy + (j + ly) * g.dy;
-  const double pz = g.oz + (k + lz) * g.dz;
-  if (!keep64) {
-    out.v[o] = (float)px;
-    out.v[o + 1] = (float)py;
-    out.v[o + 2] = (float)pz;
-  }
-  if (out.v64) {
-    out.v64[o] = px;
-    out.v64[o + 1] = py;
-    out.v64[o + 2] = pz;
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    const int c = d == 0 ? i : (d == 1 ? j : k);
+    const double og = d == 0 ? g.ox : (d == 1 ? g.oy : g.oz), sp = d == 0 ? g.dx : (d == 1 ? g.dy : g.dz);
+    if (!p64 && !out.v64) {
+      const ffx::ff t = ffx::ff_mul(ffx::two_sum((float)c, p[d]), ffx::ff{g.sp_hi[d], g.sp_lo[d]});
+      const ffx::ff x = ffx::ff_add_abs(ffx::ff{g.org_hi[d], g.org_lo[d]}, t);
+      out.v[o + d] = ffx::ff_certain(x, (fabsf(g.org_hi[d]) + fabsf(t.hi)) * 0x1p-43f) ? x.hi
+                                                                                       : (float)(og + (c + (double)p[d]) * sp);
+    } else {
+      const double x = og + (c + (p64 ? p64[d] : (double)p[d])) * sp;
+      if (!keep64) out.v[o + d] = (float)x;
+      if (out.v64) out.v64[o + d] = x;
+    }
   }
   // normal: trilinear interpolation of the 8 corner gradients, normalised (UniformGrid::normal,
   // cpp_dmc/UniformGrid.h:286-298).  When it is kept for the simplification merges it is computed
   // in float-float (relative error ~2^-40, far below the float32 output's 2^-24) on the FP32 pipes.
-  if (p64) {
-    // float64 local coordinates: the reference's float64 normal at them
-    const Normal64 nf = normal_f64(g, i, j, k, lx, ly, lz, flip);
-    for (int d = 0; d < 3; d++) {
-      if (keep64) {
-        const ffx::ff x = ffx::ff_from_double(nf.n[d]);
-        n2[o + d] = make_float2(x.hi, x.lo);
-      } else {
-        out.n[o + d] = (float)nf.n[d];
+  ffx::ff nf[3];
+  bool pairs = false;  // nf holds the normal
+  if (!p64) {
+    float c[8];
+    load_corners(g, i, j, k, c);
+    if (!(kFF && keep64)) {
+      float nv3[3];
+      const float sgn = flip ? -1.0f : 1.0f;
+      float scale = 0;  // largest corner gradient component: the size of the interpolation's inputs
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        AxisLines S;
+        load_axis(g, i, j, k, d, S);
+        float G[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+          float hi, lo;
+          corner_pair(c, S, d, q, hi, lo);
+          G[q] = (hi - lo) * g.inv2f[d];
+          scale = fmaxf(scale, fabsf(G[q]));
+        }
+        const float a0 = fmaf(p[0], G[1] - G[0], G[0]), a1 = fmaf(p[0], G[3] - G[2], G[2]);
+        const float a2 = fmaf(p[0], G[5] - G[4], G[4]), a3 = fmaf(p[0], G[7] - G[6], G[6]);
+        const float b0 = fmaf(p[1], a1 - a0, a0), b1 = fmaf(p[1], a3 - a2, a2);
+        nv3[d] = sgn * fmaf(p[2], b1 - b0, b0);
+      }
+      const float dot = nv3[0] * nv3[0] + nv3[1] * nv3[1] + nv3[2] * nv3[2];
+      // The float32 interpolation errs by a few ulps of `scale`; where the gradients cancel to below
+      // 1/16 of it (strongly uneven spacing, near critical points) that would exceed ~4e-6 of the
+      // unit normal: float pairs instead.
+      if (scale <= 16.0f * sqrtf(dot)) {
+        const float rn = rsqrtf(dot);
+#pragma unroll
+        for (int d = 0; d < 3; d++) nf[d] = ffx::ff_from(nv3[d] * rn);
+        pairs = true;
       }
     }
+    if (!pairs) pairs = normal_ff(g, i, j, k, c, p, flip, nf);
+  }
+  if (!pairs) {
+    const Normal64 n = normal_f64(g, i, j, k, p64 ? p64[0] : (double)p[0], p64 ? p64[1] : (double)p[1],
+                                  p64 ? p64[2] : (double)p[2], flip);
+#pragma unroll
+    for (int d = 0; d < 3; d++) nf[d] = ffx::ff_from_double(n.n[d]);
     st.normal_f64++;
-  } else if (kFF && keep64) {
-    ffx::ff Gq[8][3];
+  }
 #pragma unroll
-    for (int q = 0; q < 8; q++) point_diff_ff(g, i + (q & 1), j + ((q >> 1) & 1), k + ((q >> 2) & 1), Gq[q]);
-    ffx::ff nv3[3];
-    float scale = 0;  // largest |difference| * 1/(2 spacing): the size of the interpolation's inputs
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-      float md = 0;
-#pragma unroll
-      for (int q = 0; q < 8; q++) md = fmaxf(md, fabsf(Gq[q][d].hi));
-      scale = fmaxf(scale, md * G.inv2d[d]);
-      const ffx::ff a0 = ff_lerp(Gq[0][d], Gq[1][d], p[0]), a1 = ff_lerp(Gq[2][d], Gq[3][d], p[0]);
-      const ffx::ff a2 = ff_lerp(Gq[4][d], Gq[5][d], p[0]), a3 = ff_lerp(Gq[6][d], Gq[7][d], p[0]);
-      const ffx::ff b0 = ff_lerp(a0, a1, p[1]), b1 = ff_lerp(a2, a3, p[1]);
-      const ffx::ff t = ffx::ff_mul(ff_lerp(b0, b1, p[2]), G.inv2d_ff[d]);
-      nv3[d] = flip ? ffx::ff_neg(t) : t;
-    }
-    const ffx::ff dot =
-        ffx::ff_add(ffx::ff_add(ffx::ff_mul(nv3[0], nv3[0]), ffx::ff_mul(nv3[1], nv3[1])), ffx::ff_mul(nv3[2], nv3[2]));
-    // 1/sqrt(dot): float estimate and one Newton step in float-float
-    const float r0 = rsqrtf(dot.hi);
-    const ffx::ff h = ffx::ff_mul_f(ffx::ff_mul_f(dot, r0), r0);
-    const ffx::ff r = ffx::ff_mul_f(ffx::ff_sub(ffx::ff_from(1.5f), ffx::ff_mul_f(h, 0.5f)), r0);
-    if (scale <= 0x1p10f * sqrtf(dot.hi)) {
-      for (int d = 0; d < 3; d++) {
-        const ffx::ff x = ffx::ff_mul(nv3[d], r);
-        n2[o + d] = make_float2(x.hi, x.lo);
-      }
-    } else {
-      // the gradients cancel to below 2^-10 of their size: float64, as the reference
-      const Normal64 nf = normal_f64(g, i, j, k, p[0], p[1], p[2], flip);
-      for (int d = 0; d < 3; d++) {
-        const ffx::ff x = ffx::ff_from_double(nf.n[d]);
-        n2[o + d] = make_float2(x.hi, x.lo);
-      }
-      st.normal_f64++;
-    }
-  } else {
-    float Gq[8][3];
-#pragma unroll
-    for (int q = 0; q < 8; q++)
-      point_gradient_f(g, i + (q & 1), j + ((q >> 1) & 1), k + ((q >> 2) & 1), (float*)G.inv2d, Gq[q]);
-    float nv3[3];
-    const float uu = p[0], vv = p[1], ww = p[2];
-    const float sgn = flip ? -1.0f : 1.0f;
-    float scale = 0;  // largest corner gradient component: the size of the interpolation's inputs
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-#pragma unroll
-      for (int q = 0; q < 8; q++) scale = fmaxf(scale, fabsf(Gq[q][d]));
-      const float a0 = fmaf(uu, Gq[1][d] - Gq[0][d], Gq[0][d]), a1 = fmaf(uu, Gq[3][d] - Gq[2][d], Gq[2][d]);
-      const float a2 = fmaf(uu, Gq[5][d] - Gq[4][d], Gq[4][d]), a3 = fmaf(uu, Gq[7][d] - Gq[6][d], Gq[6][d]);
-      const float b0 = fmaf(vv, a1 - a0, a0), b1 = fmaf(vv, a3 - a2, a2);
-      nv3[d] = sgn * fmaf(ww, b1 - b0, b0);
-    }
-    const float dot = nv3[0] * nv3[0] + nv3[1] * nv3[1] + nv3[2] * nv3[2];
-    // The float32 interpolation errs by a few ulps of `scale`; where the gradients cancel to below
-    // 1/16 of it (strongly uneven spacing, near critical points) that would exceed ~4e-6 of the
-    // unit normal: the reference's float64 normal instead.
-    if (scale <= 16.0f * sqrtf(dot)) {
-      const float rn = rsqrtf(dot);
-      for (int d = 0; d < 3; d++) out.n[o + d] = nv3[d] * rn;
-    } else {
-      const Normal64 nf = normal_f64(g, i, j, k, (double)p[0], (double)p[1], (double)p[2], flip);
-      for (int d = 0; d < 3; d++) out.n[o + d] = (float)nf.n[d];
-      st.normal_f64++;
-    }
+  for (int d = 0; d < 3; d++) {
+    if (keep64) n2[o + d] = make_float2(nf[d].hi, nf[d].lo);
+    else out.n[o + d] = nf[d].hi;
   }
   if (out.vcell) {
     out.vcell[vidx] = cell;
@@ -473,7 +493,7 @@ __global__ void __launch_bounds__(kVertexThreads) dmc_vertex_kernel(CellSpace sp
       tail_list[atomicAdd(tail_count, 1u)] = (uint32_t)vidx;
       continue;
     }
-    vertex_outputs(G, i, j, k, cell, p, nullptr, vidx, out, flip_all | (g.flags & kGridFlip), st);
+    vertex_outputs(g, i, j, k, cell, p, nullptr, vidx, out, flip_all | (g.flags & kGridFlip), st);
   }
   flush_stats(st, stats);
 }
@@ -566,14 +586,14 @@ __global__ void __launch_bounds__(kVertexThreads) dmc_vertex_warp_kernel(CellSpa
       float p[3];
       if (b.q != repr::kNoSample) {
         repr::lane_point(P, su, sv, ns, b, p);
-        vertex_outputs(G, i, j, k, cell, p, nullptr, vidx, out, flip_all | (g.flags & kGridFlip), st);
+        vertex_outputs(g, i, j, k, cell, p, nullptr, vidx, out, flip_all | (g.flags & kGridFlip), st);
       } else {
         // nothing valid at 26x26 either: the reference keeps its float64 mean point, unrounded
         st.fail2++;
         const repr::Point64 pm = repr::mean_point_exact(pts, npts);
         for (int d = 0; d < 3; d++) p[d] = (float)pm.p[d];
         const bool exact = (double)p[0] == pm.p[0] && (double)p[1] == pm.p[1] && (double)p[2] == pm.p[2];
-        vertex_outputs(G, i, j, k, cell, p, exact ? nullptr : pm.p, vidx, out, flip_all | (g.flags & kGridFlip),
+        vertex_outputs(g, i, j, k, cell, p, exact ? nullptr : pm.p, vidx, out, flip_all | (g.flags & kGridFlip),
                        st);
       }
     }
@@ -754,26 +774,24 @@ __global__ void __launch_bounds__(kVertexThreads) dmc_vertex_w_kernel(CellSpace 
 }
 
 // Positions, normals and local coordinates of the projected vertices.
-template <bool kFF>
-__global__ void __launch_bounds__(kVertexThreads, 4) dmc_vertex_finish_kernel(CellSpace space, const uint16_t* cellof,
-                                                                            const uint32_t* vwork,
-                                                                            int64_t nv, const float4* vp,
-                                                                            DmcVertexOut out, int flip_all,
-                                                                            unsigned long long* stats) {
+template <bool kBatch, bool kFF>
+__global__ void __launch_bounds__(kVertexThreads) dmc_vertex_finish_kernel(CellSpace space, const uint16_t* cellof,
+                                                                         const uint32_t* vwork,
+                                                                         int64_t nv, const float4* vp,
+                                                                         DmcVertexOut out, int flip_all,
+                                                                         unsigned long long* stats) {
   repr::Stats st;
-  GridCache G;
   for (int64_t vidx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; vidx < nv;
        vidx += (int64_t)gridDim.x * blockDim.x) {
     const float4 q = vp[vidx];
     if (q.w != 0.0f) continue;  // done by the one-pass kernel
     const uint32_t vcell = slot_cell(cellof, vwork[vidx]);
-    G.load(space, vcell);
-    const Grid& g = G.g;
+    const Grid& g = kBatch ? space.grids[__ldg(space.tile_vol + vcell / kScanTile)] : space.one;
     const int64_t cell = vcell - g.vbase;
     int i, j, k;
     cell_ijk(g, cell, i, j, k);
     const float p[3] = {q.x, q.y, q.z};
-    vertex_outputs<kFF>(G, i, j, k, cell, p, nullptr, vidx, out, flip_all | (g.flags & kGridFlip), st);
+    vertex_outputs<kFF>(g, i, j, k, cell, p, nullptr, vidx, out, flip_all | (g.flags & kGridFlip), st);
   }
   flush_stats(st, stats);
 }
@@ -946,8 +964,6 @@ int dmc_front_emit(const CellSpace& space, DmcScratch& s, DmcVertexOut vo, int64
   static const int r_point = resident_blocks(dmc_vertex_point_kernel<false>, kVertexThreads);
   static const int r_point_batch = resident_blocks(dmc_vertex_point_kernel<true>, kVertexThreads);
   static const int r_w = resident_blocks(dmc_vertex_w_kernel, kVertexThreads);
-  static const int r_finish = resident_blocks(dmc_vertex_finish_kernel<true>, kVertexThreads);
-  static const int r_finish32 = resident_blocks(dmc_vertex_finish_kernel<false>, kVertexThreads);
   static const int r_quad = resident_blocks(dmc_quad_kernel<false>, kQuadThreads);
   static const int r_quad_batch = resident_blocks(dmc_quad_kernel<true>, kQuadThreads);
   auto vgrid = [&](int resident) {
@@ -968,13 +984,19 @@ int dmc_front_emit(const CellSpace& space, DmcScratch& s, DmcVertexOut vo, int64
   }
   {
     Stage t(prof, "dmc_vertex_finish", st);
-    // the float-float normals only when some volume keeps float64 normals (simplification)
-    if (vo.n64)
-      dmc_vertex_finish_kernel<true><<<vgrid(r_finish), kVertexThreads, 0, st>>>(space, s.cellof, s.vwork, nv, s.vp, vo, flip,
-                                                                                 s.stats);
-    else
-      dmc_vertex_finish_kernel<false><<<vgrid(r_finish32), kVertexThreads, 0, st>>>(space, s.cellof, s.vwork, nv, s.vp, vo, flip,
-                                                                                    s.stats);
+#define DMC_FINISH(B, F)                                                                              \
+  {                                                                                                   \
+    static const int res = resident_blocks(dmc_vertex_finish_kernel<B, F>, kVertexThreads);           \
+    dmc_vertex_finish_kernel<B, F><<<vgrid(res), kVertexThreads, 0, st>>>(space, s.cellof, s.vwork, nv, s.vp, vo, flip, \
+                                                                          s.stats);                   \
+  }
+    // the pair normals' storing path only when some volume keeps them (simplification)
+    if (space.grids) {
+      if (vo.n64) DMC_FINISH(true, true) else DMC_FINISH(true, false)
+    } else {
+      if (vo.n64) DMC_FINISH(false, true) else DMC_FINISH(false, false)
+    }
+#undef DMC_FINISH
   }
   {
     // the listed vertices: one thread each with every float64 fallback, the 26x26 retries one warp
