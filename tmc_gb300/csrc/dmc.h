@@ -19,7 +19,7 @@ struct DmcVertexOut {
 
 struct DmcScratch {
   uint32_t* rec;                  // per listed cell (slot)
-  int32_t* voff;                  // per listed cell (slot)
+  uint2* rv;                      // per listed cell (slot): record and vertex offset
   int32_t* qoff;                  // per listed cell (slot)
   uint32_t* vwork;                // per vertex: slot of the generating cell
   unsigned long long* tile_sums;  // per scan tile
@@ -31,12 +31,13 @@ struct DmcScratch {
   uint32_t* w_list;
   unsigned* fb_count;             // entries of [0] fb_list, [1] tail_list, [2] w_list
   uint32_t* tail_list;            // vertices without a valid 7x7 sample (26x26 retry)
-  // listed cells (common.cuh): rec, voff and qoff hold one entry per listed cell at its slot
+  // listed cells (common.cuh): rec, rv and qoff hold one entry per listed cell at its slot
   CellMask* mask;                 // per 32 cells of the space
   uint16_t* cellof;               // per slot: in-tile offset of the listed cell
   uint8_t* ccase;                 // per slot: the listed cell's MC case
   uint8_t* vrank;                 // per vertex: rank among its cell's vertices (vwork: the cell's slot)
-  unsigned* amb_n;                // listed cells with an ambiguous case (their slots wait in qoff)
+  unsigned* amb_n;                // [0] listed cells with an ambiguous case (their slots wait in qoff), [1] chunks
+  uint32_t* chunks;               // kScanTile / 32 per tile: the chunk list (scan.cuh)
 };
 
 // Each launcher returns the number of kernels it launched.

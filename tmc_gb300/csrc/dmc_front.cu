@@ -21,7 +21,7 @@
 //   dmc_vertex_kernel    the vertices those leave, with every float64 fallback
 //   dmc_vertex_warp_kernel  the reference's 26x26 retry (and short lists whole), one warp per vertex
 //   dmc_quad_kernel      each cell emits the quads of its crossed interior edges 0, 3, 8 by
-//                        looking up the four cells around the edge
+//                        looking up the cells around them
 #include <cstdio>
 
 #include "common.cuh"
@@ -130,18 +130,22 @@ __global__ void __launch_bounds__(128) dmc_amb_kernel(CellSpace space, const uin
   }
 }
 
-// In-tile exclusive scan of the listed cells' records -> their vertex and quad offsets (blocked:
-// 16-byte record loads and offset stores over the tile's slots, one block scan of the thread
-// totals), and two entries per vertex: the slot of the cell that generates it and its rank there.
+// In-tile exclusive scan of the listed cells' records -> per slot the record beside its vertex offset
+// (rv, what the quads need of a neighbour in one load) and the quad offset (blocked: 16-byte loads
+// and stores over the tile's slots), two entries per vertex (the slot of the cell that generates it
+// and its rank there), and the tile's chunks of 32 slots appended to the chunk list (scan.cuh).
 __global__ void __launch_bounds__(32 * kOffsetWarps) dmc_offsets_kernel(const CellMask* mask, const uint32_t* rec,
                                                                        const unsigned long long* tile_off,
-                                                                       int64_t tiles, int32_t* voff, int32_t* qoff,
-                                                                       uint32_t* vwork, uint8_t* vrank) {
+                                                                       int64_t tiles, uint2* rv, int32_t* qoff,
+                                                                       uint32_t* vwork, uint8_t* vrank,
+                                                                       uint32_t* chunks, unsigned* nchunks) {
   const int lane = threadIdx.x & 31;
   const int64_t tile = (int64_t)blockIdx.x * kOffsetWarps + (threadIdx.x >> 5);
+  const uint32_t listed = tile < tiles ? tile_listed(mask, tile) : 0;
+  list_chunks<kOffsetWarps>(tile, listed, chunks, nchunks);
   if (tile >= tiles) return;  // the whole warp
   const int64_t base = tile * kScanTile;
-  const int64_t end = base + tile_listed(mask, tile);
+  const int64_t end = base + listed;
   unsigned long long carry = tile_off[tile];
   for (int64_t step = base; step < end; step += kOffsetStep) {  // warp-uniform
     const int64_t first = step + (int64_t)lane * kScanItems;
@@ -153,14 +157,15 @@ __global__ void __launch_bounds__(32 * kOffsetWarps) dmc_offsets_kernel(const Ce
     const unsigned long long inc = warp_inclusive_scan(sum);
     unsigned long long pre = carry + inc - sum;
     carry += __shfl_sync(0xffffffffu, inc, 31);
-    int32_t vo[kScanItems], qo[kScanItems];
+    uint32_t vo[kScanItems];
+    int32_t qo[kScanItems];
 #pragma unroll
     for (int s = 0; s < kScanItems; s++) {
-      vo[s] = (int32_t)(pre >> 32);
+      vo[s] = (uint32_t)(pre >> 32);
       qo[s] = (int32_t)(pre & 0xffffffffull);
       pre += ((unsigned long long)rec_nv(r[s]) << 32) | rec_nq(r[s]);
     }
-    store8(voff, first, end, vo);
+    store8_pairs(rv, first, end, r, vo);
     store8(qoff, first, end, qo);
 #pragma unroll
     for (int s = 0; s < kScanItems; s++)
@@ -803,105 +808,85 @@ __global__ void __launch_bounds__(kVertexThreads) dmc_vertex_finish_kernel(CellS
 // ------------------------------------------------------------------------------------------
 // Quad corners are vertex indices within the quad's own volume: the space-wide offsets minus the
 // volume's first vertex (the scanned tile offset of its first tile; 0 for a single volume).
-// The quads a cell owns (one per crossed interior edge 0, 3, 8), from the records of the four
-// cells around each edge (listed cells: a crossed edge makes every cell around it listed).
-__device__ __forceinline__ void cell_quads(const Grid& g, int32_t vfirst, uint32_t slot, int64_t vc, unsigned cs,
-                                           const CellMask* mask, const uint32_t* rec, const int32_t* voff,
-                                           const int32_t* qoff, int32_t* quads, uint8_t* colors) {
-  // cell offsets (di, dj, dk) and local edge of the four cells around the owned edges 0, 3, 8
-  // x edge: (0,-1,-1) e6, (0,0,-1) e4, (0,-1,0) e2, (0,0,0) e0
-  // y edge: (-1,0,-1) e5, (0,0,-1) e7, (-1,0,0) e1, (0,0,0) e3
-  // z edge: (-1,-1,0) e10, (0,-1,0) e11, (-1,0,0) e9, (0,0,0) e8
-  const int64_t cell = vc - g.vbase;
-  int i, j, k;
-  cell_ijk(g, cell, i, j, k);
-  // from the cell's MC case (bit v: corner v at or above the isovalue): corner 0's side, and the
-  // crossings of edges 0 (corners 0-1), 3 (0-2) and 8 (0-4)
-  const int neg = !(cs & 1u);  // first end vertex below the isovalue
-  const bool crossed[3] = {((cs ^ (cs >> 1)) & 1u) != 0, ((cs ^ (cs >> 2)) & 1u) != 0, ((cs ^ (cs >> 4)) & 1u) != 0};
-  int32_t q = qoff[slot];
-  const int par = (i & 1) | ((j & 1) << 1) | ((k & 1) << 2);
-#pragma unroll
-  for (int a = 0; a < 3; a++) {
-    if (!crossed[a] || !edge_interior(g, i, j, k, a == 0 ? 0 : (a == 1 ? 3 : 8))) continue;
-    int di[4], dj[4], dk[4], le[4];
-    if (a == 0) {
-      di[0] = 0; dj[0] = -1; dk[0] = -1; le[0] = 6;
-      di[1] = 0; dj[1] = 0; dk[1] = -1; le[1] = 4;
-      di[2] = 0; dj[2] = -1; dk[2] = 0; le[2] = 2;
-      di[3] = 0; dj[3] = 0; dk[3] = 0; le[3] = 0;
-    } else if (a == 1) {
-      di[0] = -1; dj[0] = 0; dk[0] = -1; le[0] = 5;
-      di[1] = 0; dj[1] = 0; dk[1] = -1; le[1] = 7;
-      di[2] = -1; dj[2] = 0; dk[2] = 0; le[2] = 1;
-      di[3] = 0; dj[3] = 0; dk[3] = 0; le[3] = 3;
-    } else {
-      di[0] = -1; dj[0] = -1; dk[0] = 0; le[0] = 10;
-      di[1] = 0; dj[1] = -1; dk[1] = 0; le[1] = 11;
-      di[2] = -1; dj[2] = 0; dk[2] = 0; le[2] = 9;
-      di[3] = 0; dj[3] = 0; dk[3] = 0; le[3] = 8;
-    }
-    int32_t qv[4];
-#pragma unroll
-    for (int s = 0; s < 4; s++) {
-      const uint32_t ns = s == 3 ? slot : listed_slot(mask, (uint32_t)g.vcell(i + di[s], j + dj[s], k + dk[s]));
-      const uint32_t rn = rec[ns];
-      qv[quad_slot(le[s], neg)] = voff[ns] - vfirst + rec_rank(rn, le[s]);
-    }
-    reinterpret_cast<int4*>(quads)[q] = make_int4(qv[0], qv[1], qv[2], qv[3]);
-    if (colors) colors[q] = (uint8_t)(3 * par + a);
-    q++;
-  }
-}
-
-// Each warp walks chunks of 32 consecutive slots of the listed cells, queues those that own quads
-// (ballot) in shared memory and processes the queue 32 cells at a time, one per lane.  No block
-// barrier.
+//
+// One warp per chunk of 32 consecutive listed cells of one tile (the chunk list of the offsets pass),
+// a cell per lane.  A cell owns the quads of its crossed interior edges 0, 3 and 8; the cells around
+// them are six neighbours, each looked up once and independently (a mask word, then record and offset
+// in one load).  A crossed edge makes every cell around it listed.  Walking every tile's 64 possible
+// chunks, with up to nine dependent look-ups of three loads each, a smooth field took as long as a dense
+// one (512^3 periodic: 0.62 ms of a 2.81 ms call; 2.31 ms with the list).
 constexpr int kQuadThreads = 256;
+// quad around edge axis A from its four cells' vertices, in the order of their cells: the one across
+// both axes, then those below the edge along the second and the first, then the owner
+template <int E0, int E1, int E2, int E3>
+__device__ __forceinline__ int4 quad_corners(const int32_t v[4], int neg) {
+  constexpr int kE[4] = {E0, E1, E2, E3};
+  int32_t a[4], b[4];
+#pragma unroll
+  for (int s = 0; s < 4; s++) {
+    a[quad_slot(kE[s], 0)] = v[s];
+    b[quad_slot(kE[s], 1)] = v[s];
+  }
+  return neg ? make_int4(b[0], b[1], b[2], b[3]) : make_int4(a[0], a[1], a[2], a[3]);
+}
 template <bool kBatch>
 __global__ void __launch_bounds__(kQuadThreads) dmc_quad_kernel(CellSpace space, const CellMask* mask,
                                                                 const uint16_t* cellof, const uint8_t* ccase,
-                                                                const uint32_t* rec,
-                                                                const int32_t* voff, const int32_t* qoff,
-                                                                const unsigned long long* tile_off, int32_t* quads,
-                                                                uint8_t* colors) {
+                                                                const uint2* rv, const int32_t* qoff,
+                                                                const unsigned long long* tile_off,
+                                                                const uint32_t* chunks, const unsigned* nchunks,
+                                                                int32_t* quads, uint8_t* colors) {
   constexpr int kWarps = kQuadThreads / 32;
-  __shared__ uint32_t queue[kWarps][64];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  uint32_t* Q = queue[wid];
-  const int64_t tiles = ceil_div(space.n, kScanTile), chunks = tiles * (kScanTile / 32);
-  int qn = 0;  // queued cells (the same on every lane)
-  for (int64_t chunk = (int64_t)blockIdx.x * kWarps + wid;; chunk += (int64_t)gridDim.x * kWarps) {
-    const bool more = chunk < chunks;
-    if (more) {
-      int64_t tile;
-      uint32_t first;
-      slot_chunk(chunk, tiles, tile, first);
-      const uint32_t slot = first + lane, r = slot & (kScanTile - 1);
-      const bool own = r < tile_listed(mask, tile) && rec_nq(rec[slot]) != 0;
-      const unsigned bal = __ballot_sync(0xffffffffu, own);
-      if (own) Q[qn + __popc(bal & ((1u << lane) - 1u))] = slot;
-      qn += __popc(bal);
-      __syncwarp();
+  const unsigned n = *nchunks;
+  for (unsigned c = blockIdx.x * kWarps + wid; c < n; c += gridDim.x * kWarps) {
+    const uint32_t chunk = __ldg(chunks + c), slot = (chunk & ~31u) + lane;
+    if ((uint32_t)lane > (chunk & 31u)) continue;  // the chunk's number of cells minus one
+    const uint2 own = __ldg(rv + slot);
+    if (rec_nq(own.x) == 0) continue;
+    const unsigned cs = __ldg(ccase + slot);
+    const uint32_t vc = slot_cell(cellof, slot);
+    const Grid& g = kBatch ? space.grids[__ldg(space.tile_vol + vc / kScanTile)] : space.one;
+    const int32_t vfirst = kBatch ? (int32_t)(__ldg(tile_off + g.vbase / kScanTile) >> 32) : 0;
+    int i, j, k;
+    cell_ijk(g, vc - g.vbase, i, j, k);
+    // from the cell's MC case (bit v: corner v at or above the isovalue): corner 0's side, and the
+    // crossings of edges 0 (corners 0-1), 3 (0-2) and 8 (0-4); interior: off the lower borders (the
+    // edges at the cell's lower corner never lie on the upper ones)
+    const int neg = !(cs & 1u);  // first end vertex below the isovalue
+    const bool x = (((cs ^ (cs >> 1)) & 1u) != 0) && j > 0 && k > 0;
+    const bool y = (((cs ^ (cs >> 2)) & 1u) != 0) && i > 0 && k > 0;
+    const bool z = (((cs ^ (cs >> 4)) & 1u) != 0) && i > 0 && j > 0;
+    const uint32_t cx = (uint32_t)g.cx(), cxy = cx * (uint32_t)g.cy();
+    // neighbours (0,-1,-1), (0,0,-1), (-1,0,-1), (0,-1,0), (-1,0,0), (-1,-1,0)
+    const uint32_t off[6] = {cxy + cx, cxy, cxy + 1, cx, 1, cx + 1};
+    const bool want[6] = {x, x || y, y, x || z, y || z, z};
+    uint32_t ns[6];
+#pragma unroll
+    for (int s = 0; s < 6; s++) ns[s] = want[s] ? listed_slot(mask, vc - off[s]) : 0u;
+    uint2 o[6];
+#pragma unroll
+    for (int s = 0; s < 6; s++) o[s] = want[s] ? __ldg(rv + ns[s]) : make_uint2(0, 0);
+    auto vertex = [vfirst](uint2 r, int e) { return (int32_t)r.y - vfirst + rec_rank(r.x, e); };
+    int64_t q = __ldg(qoff + slot);
+    const int par = (i & 1) | ((j & 1) << 1) | ((k & 1) << 2);
+    if (x) {
+      const int32_t v[4] = {vertex(o[0], 6), vertex(o[1], 4), vertex(o[3], 2), vertex(own, 0)};
+      reinterpret_cast<int4*>(quads)[q] = quad_corners<6, 4, 2, 0>(v, neg);
+      if (colors) colors[q] = (uint8_t)(3 * par);
+      q++;
     }
-    while (qn >= 32 || (!more && qn > 0)) {
-      const int take = qn < 32 ? qn : 32;
-      if (lane < take) {
-        const uint32_t slot = Q[lane];
-        const uint32_t vc = slot_cell(cellof, slot);
-        const Grid& g = kBatch ? space.grids[__ldg(space.tile_vol + vc / kScanTile)] : space.one;
-        const int32_t vfirst = kBatch ? (int32_t)(tile_off[g.vbase / kScanTile] >> 32) : 0;
-        cell_quads(g, vfirst, slot, vc, __ldg(ccase + slot), mask, rec, voff, qoff, quads, colors);
-      }
-      __syncwarp();
-      const int rest = qn - take;  // at most 31: move them to the front
-      const uint32_t x = lane < rest ? Q[take + lane] : 0u;
-      __syncwarp();
-      if (lane < rest) Q[lane] = x;
-      __syncwarp();
-      qn = rest;
+    if (y) {
+      const int32_t v[4] = {vertex(o[2], 5), vertex(o[1], 7), vertex(o[4], 1), vertex(own, 3)};
+      reinterpret_cast<int4*>(quads)[q] = quad_corners<5, 7, 1, 3>(v, neg);
+      if (colors) colors[q] = (uint8_t)(3 * par + 1);
+      q++;
     }
-    if (!more) break;
+    if (z) {
+      const int32_t v[4] = {vertex(o[5], 10), vertex(o[3], 11), vertex(o[4], 9), vertex(own, 8)};
+      reinterpret_cast<int4*>(quads)[q] = quad_corners<10, 11, 9, 8>(v, neg);
+      if (colors) colors[q] = (uint8_t)(3 * par + 2);
+    }
   }
 }
 
@@ -917,7 +902,7 @@ int dmc_front_count(const CellSpace& space, DmcScratch& s, cudaStream_t st, Prof
   {
     Stage t(prof, "dmc_classify", st);
     // the ambiguous cells' list lives in qoff until the offsets kernel writes the quad offsets
-    cudaMemsetAsync(s.amb_n, 0, sizeof(unsigned), st);
+    cudaMemsetAsync(s.amb_n, 0, 2 * sizeof(unsigned), st);  // and the chunk counter behind it
     auto classify = [&](int64_t t0, int64_t t1) {
       if (t1 <= t0) return;
       if (space.one.gen)  // fused generation (single volumes)
@@ -958,7 +943,7 @@ int dmc_front_emit(const CellSpace& space, DmcScratch& s, DmcVertexOut vo, int64
     Stage t(prof, "dmc_scan", st);
     const int64_t tiles = ceil_div(n, kScanTile);
     dmc_offsets_kernel<<<(unsigned)ceil_div(tiles, kOffsetWarps), 32 * kOffsetWarps, 0, st>>>(
-        s.mask, s.rec, s.tile_sums, tiles, s.voff, s.qoff, s.vwork, s.vrank);
+        s.mask, s.rec, s.tile_sums, tiles, s.rv, s.qoff, s.vwork, s.vrank, s.chunks, s.amb_n + 1);
   }
   // per-vertex grids: whole waves of each kernel's resident blocks
   static const int r_point = resident_blocks(dmc_vertex_point_kernel<false>, kVertexThreads);
@@ -1012,16 +997,14 @@ int dmc_front_emit(const CellSpace& space, DmcScratch& s, DmcVertexOut vo, int64
         s.stats);
   }
   Stage t(prof, "dmc_quad", st);
-  // one wave: the kernel takes 32-cell chunks until none are left
-  if (space.grids)
-    dmc_quad_kernel<true><<<(unsigned)wave_grid(r_quad_batch, sms, tu.quad_blocks_per_sm, ceil_div(n, 32),
-                                                kQuadThreads / 32), kQuadThreads,
-                            0, st>>>(space, s.mask, s.cellof, s.ccase, s.rec, s.voff, s.qoff, s.tile_sums, quads, colors);
-  else
-    dmc_quad_kernel<false><<<(unsigned)wave_grid(r_quad, sms, tu.quad_blocks_per_sm, ceil_div(n, 32),
-                                                 kQuadThreads / 32), kQuadThreads, 0,
-                             st>>>(space, s.mask, s.cellof, s.ccase, s.rec, s.voff, s.qoff, s.tile_sums, quads,
-                                   colors);
+  // one wave: the number of chunks is only known on the device
+#define DMC_QUADS(B, R)                                                                                              \
+  dmc_quad_kernel<B><<<(unsigned)wave_grid(R, sms, tu.quad_blocks_per_sm, ceil_div(n, 32), kQuadThreads / 32),       \
+                       kQuadThreads, 0, st>>>(space, s.mask, s.cellof, s.ccase, s.rv, s.qoff, s.tile_sums, s.chunks, \
+                                              s.amb_n + 1, quads, colors)
+  if (space.grids) DMC_QUADS(true, r_quad_batch);
+  else DMC_QUADS(false, r_quad);
+#undef DMC_QUADS
   return 7;
 }
 

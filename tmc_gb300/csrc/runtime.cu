@@ -659,11 +659,12 @@ tmc_status dmc_extract(tmc_ctx* ctx, const tmc_volume* vol, double iso, uint32_t
 
   tmc::DmcScratch sc{};
   TMC_CUDA(ctx, al.get(&sc.rec, ncell));
-  TMC_CUDA(ctx, al.get(&sc.voff, ncell));
+  TMC_CUDA(ctx, al.get(&sc.rv, ncell));
   TMC_CUDA(ctx, al.get(&sc.qoff, ncell));
   TMC_CUDA(ctx, al.get(&sc.cellof, ncell));
   TMC_CUDA(ctx, al.get(&sc.ccase, ncell));
-  TMC_CUDA(ctx, al.get(&sc.amb_n, 1));
+  TMC_CUDA(ctx, al.get(&sc.amb_n, 2));
+  TMC_CUDA(ctx, al.get(&sc.chunks, tmc::dmc_tiles(space) * (tmc::kScanTile / 32)));
   TMC_CUDA(ctx, al.get(&sc.mask, tmc::dmc_tiles(space) * (tmc::kScanTile / 32)));
   TMC_CUDA(ctx, al.get(&sc.tile_sums, tmc::dmc_tiles(space)));
   TMC_CUDA(ctx, al.get(&sc.totals, 2));
@@ -995,7 +996,7 @@ tmc_status batch_run(tmc_ctx* ctx, const std::vector<int>& idx, const tmc_reques
 
   // ---- count ----
   uint32_t* rec = nullptr;
-  int32_t *voff = nullptr, *qoff = nullptr;
+  int32_t* qoff = nullptr;
   unsigned long long *tile_sums = nullptr, *totals = nullptr;
   tmc::CellMask* mask = nullptr;
   uint16_t* cellof = nullptr;
@@ -1010,11 +1011,12 @@ tmc_status batch_run(tmc_ctx* ctx, const std::vector<int>& idx, const tmc_reques
   tmc::TmcScratch tsc{};
   int64_t n_amb_rec = 0;
   if (dmc) {
-    TMC_CUDA(ctx, al.get(&voff, ncell));
-    dsc = tmc::DmcScratch{rec, voff, qoff, nullptr, tile_sums, totals, ctx->d_stats};
+    dsc = tmc::DmcScratch{rec, nullptr, qoff, nullptr, tile_sums, totals, ctx->d_stats};
     dsc.mask = mask;
     dsc.cellof = cellof;
-    TMC_CUDA(ctx, al.get(&dsc.amb_n, 1));
+    TMC_CUDA(ctx, al.get(&dsc.rv, ncell));
+    TMC_CUDA(ctx, al.get(&dsc.chunks, tiles * (tmc::kScanTile / 32)));
+    TMC_CUDA(ctx, al.get(&dsc.amb_n, 2));
     TMC_CUDA(ctx, al.get(&dsc.ccase, ncell));
     ctx->launches += tmc::dmc_front_count(space, dsc, st, &ctx->prof);
   } else {
