@@ -63,16 +63,23 @@ struct Grid {
   float iso_lo;   // the isovalue's remainder: (iso_f, iso_lo) as ffx::ff_from_double makes it
   bool iso_exact; // the isovalue is the float iso_f
   Div32 div_cx, div_cy;  // division by nx - 1 and ny - 1 (cell index -> i, j, k); set_divisors()
-  // fused generation (single-volume launches): the classification evaluates the field from `gen` at
-  // the float32 spacing gd instead of reading f, and writes each point once to gen_out (== f), which
-  // the later passes read
+  // the points' sides as bit rows of wpr words (listing.cuh); the words after the last row are padding
+  uint32_t* bits;
+  int wpr;
+  Div32 div_wpr;
+  // fused generation (single-volume launches): the pass that makes the bit rows evaluates the field from
+  // `gen` at the float32 spacing gd instead of reading f, and writes each point once to gen_out (== f),
+  // which the later passes read
   const GenParams* gen;
   float* gen_out;
   float gd[3];
   __host__ void set_divisors() {
     div_cx.init((uint32_t)(nx - 1));
     div_cy.init((uint32_t)(ny - 1));
+    wpr = (nx + 31) / 32;
+    div_wpr.init((uint32_t)wpr);
   }
+  __host__ int64_t bit_words() const { return (int64_t)nz * ny * wpr; }
   __host__ __device__ int cx() const { return nx - 1; }
   __host__ __device__ int cy() const { return ny - 1; }
   __host__ __device__ int cz() const { return nz - 1; }
@@ -101,6 +108,8 @@ struct CellSpace {
   const Grid* grids;        // batch: grid of each volume (vbase set), else nullptr
   const int32_t* tile_vol;  // batch: volume of each tile
   int64_t n;                // cells in the space, padding included
+  int n_volumes;            // batch
+  int64_t max_bit_words;    // batch: of the largest volume
   __device__ __forceinline__ Grid grid_of_tile(int64_t tile) const {
     if (!grids) return one;
     return grids[__ldg(tile_vol + tile)];
@@ -156,6 +165,8 @@ inline CellSpace single_space(const Grid& g) {
   cs.one.vbase = 0;
   cs.grids = nullptr;
   cs.tile_vol = nullptr;
+  cs.n_volumes = 1;
+  cs.max_bit_words = g.bit_words();
   cs.n = g.ncells();
   return cs;
 }
@@ -378,6 +389,7 @@ inline int64_t wave_grid(int resident, int sms, int64_t per_sm, int64_t items, i
 // the last one covers every tile.
 struct TileGate {
   int64_t tile_end;
+  int z_end;  // planes below it are on the device
   cudaEvent_t ready;
 };
 

@@ -45,7 +45,7 @@ struct DmcScratch {
 int64_t dmc_tiles(const CellSpace& space);  // scan tiles of the space
 // gates: classify the tiles of each gate once its event has completed (a host field arriving in
 // slabs); none: the whole field is on the device
-int dmc_front_count(const CellSpace& space, DmcScratch& s, cudaStream_t st, Prof* prof = nullptr,
+int dmc_front_count(const CellSpace& space, DmcScratch& s, int sms, cudaStream_t st, Prof* prof = nullptr,
                     const TileGate* gates = nullptr, int ngates = 0);
 // Quads hold vertex indices within their own volume; vertices and quads of the volumes follow one
 // another in the output arrays.

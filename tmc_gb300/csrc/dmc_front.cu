@@ -37,73 +37,115 @@ __constant__ uint64_t c_case_contour[256] = TMC_CASE_CONTOUR_INIT;
 // ------------------------------------------------------------------------------------------
 // classification (per-cell helpers in dmc_cell.cuh)
 // ------------------------------------------------------------------------------------------
-// One block per kScanTile consecutive cells (linear order).  Pass 1: every cell's MC case from the
-// warp-ballot corner rows (tile_cases: one coalesced load per corner row and warp, no per-cell
-// gather); the cells with a case other than 0 and 255 are listed in cell order (list_tile).  Pass 2:
-// the contours and records of the listed cells with an unambiguous case, written densely at their
-// slots with their in-tile offsets, and the tile's packed (vertices << 32 | quads) sum.  Listed cells
-// with an ambiguous case (the asymptotic decider, ~1 % of the cells) go by slot to amb_list for
-// dmc_amb_kernel, which runs them densely instead of stalling every warp here on a few lanes.
-template <bool kGen>
-__global__ void __launch_bounds__(kScanThreads, 6) dmc_classify_kernel(CellSpace space, int64_t tile0, uint32_t* rec,
-                                                                   uint16_t* cellof, uint8_t* ccase, CellMask* mask,
-                                                                   unsigned long long* tile_sums,
-                                                                   unsigned long long* stats, uint32_t* amb_list,
-                                                                   unsigned* amb_n) {
-  const int64_t tile = tile0 + blockIdx.x;
-  __shared__ uint64_t cc[256];
-  __shared__ uint16_t act_list[kScanTile];
-  __shared__ uint8_t case_of[kScanTile];
-  __shared__ uint32_t wmask[kScanTile / 32], wpre[kScanTile / 32];
-  __shared__ int total;
-  __shared__ unsigned long long tile_sum;
-  for (int c = threadIdx.x; c < 256; c += blockDim.x) cc[c] = c_case_contour[c];
-  if (threadIdx.x == 0) tile_sum = 0;
+// Records of cells whose edges are all interior (at least one cell away from every border), by case: an
+// unambiguous case has one contour, which is then used (rank 0 on every edge); 0 for the ambiguous ones.
+struct CaseRecords {
+  uint32_t r[256];
+};
+constexpr CaseRecords make_case_records() {
+  constexpr uint64_t contours[256] = TMC_CASE_CONTOUR_INIT;
+  CaseRecords t{};
+  for (int c = 1; c < 255; c++) {
+    if ((contours[c] & 0xF) == 0) continue;  // the contour's size
+    int nq = 0;
+    const int edge[3][2] = {{0, 1}, {0, 2}, {0, 4}};
+    for (int e = 0; e < 3; e++) nq += ((c >> edge[e][0]) ^ (c >> edge[e][1])) & 1;
+    t.r[c] = 1u | ((uint32_t)nq << 3);
+  }
+  return t;
+}
+__device__ const CaseRecords d_case_records = make_case_records();
+
+// One warp per tile of kScanTile consecutive cells (linear order): the crossed cells in cell order from
+// the bit rows (list_tile), then the records of those with an unambiguous case, a cell per lane,
+// written densely at their slots with their in-tile offsets and cases, and the tile's packed
+// (vertices << 32 | quads) sum.  Ambiguous cells (the asymptotic decider, ~1 % of the cells) go by slot
+// to amb_list for dmc_amb_kernel, which runs them densely instead of stalling every warp here on a
+// few lanes.
+template <int kPerTile>  // warps per tile (block_per_tile)
+__global__ void __launch_bounds__(kClassifyThreads) dmc_classify_kernel(CellSpace space, int64_t tile0, int64_t tile1,
+                                                                          uint32_t* rec, uint16_t* cellof,
+                                                                          uint8_t* ccase, CellMask* mask,
+                                                                          unsigned long long* tile_sums,
+                                                                          unsigned long long* stats,
+                                                                          uint32_t* amb_list, unsigned* amb_n) {
+  constexpr unsigned kAll = 0xffffffffu;
+  constexpr int kTiles = kClassifyThreads / 32 / kPerTile;  // tiles per block
+  __shared__ uint16_t lists[kTiles][kScanTile];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int share = kPerTile == 1 ? 0 : wid;  // the warp's share of its tile
+  const int64_t tile = tile0 + (int64_t)blockIdx.x * kTiles + (kPerTile == 1 ? wid : 0);
+  if (tile >= tile1) return;  // the whole warp, or the whole block
+  uint16_t* list = lists[kPerTile == 1 ? wid : 0];
   const Grid g = space.grid_of_tile(tile);
   const int64_t vbase = tile * kScanTile;  // first cell of the tile in the space
-  const int lane = threadIdx.x & 31;
-  const unsigned actbits = tile_cases<kGen>(g, space.n, vbase, case_of);
-  const int na = list_tile(actbits, tile, mask, wmask, wpre, act_list, &total);
-  // pass 2: records of the listed cells
-  unsigned long long local = 0, amb = 0, nact = 0;
-  for (int a = threadIdx.x; a < na; a += blockDim.x) {
-    const int off = act_list[a];
+  unsigned long long* tile_sum = nullptr;  // of the tile's warps, when there are several
+  int na = 0;
+  if (share == 0) na = list_tile(g, space.n, tile, mask, list);
+  if (kPerTile > 1) {
+    __shared__ int s_na;
+    __shared__ unsigned long long s_sum;
+    if (threadIdx.x == 0) {
+      s_na = na;
+      s_sum = 0;
+    }
+    __syncthreads();
+    na = s_na;
+    tile_sum = &s_sum;
+  }
+  unsigned long long local = 0;
+  unsigned nact = 0, amb = 0;
+  for (int a0 = 32 * share; a0 < na; a0 += 32 * kPerTile) {
+    const int a = a0 + lane;
     const uint32_t slot = (uint32_t)(vbase + a);
-    const unsigned cs = case_of[off];
-    const bool ambiguous = case_ambiguous(cs);
-    cellof[slot] = (uint16_t)off;
-    ccase[slot] = (uint8_t)cs;
-    if (!ambiguous) {
+    bool ambiguous = false;
+    uint32_t r = 0;
+    if (a < na) {
+      const int off = list[a];
       int i, j, k;
       cell_ijk(g, vbase + off - g.vbase, i, j, k);
-      const uint32_t r = record_from_contours(g, i, j, k, cs, table_contour(cc[cs]), false);
-      rec[slot] = r;
-      local += ((unsigned long long)rec_nv(r) << 32) | (unsigned long long)rec_nq(r);
-      nact += r != 0;
+      const unsigned cs = case_from_bits(g, i, j, k);
+      ambiguous = case_ambiguous(cs);
+      cellof[slot] = (uint16_t)off;
+      ccase[slot] = (uint8_t)cs;
+      if (!ambiguous) {
+        const bool inner = i >= 1 && j >= 1 && k >= 1 && i <= g.nx - 3 && j <= g.ny - 3 && k <= g.nz - 3;
+        r = inner ? __ldg(d_case_records.r + cs)
+                  : record_from_contours(g, i, j, k, cs, table_contour(c_case_contour[cs]), false);
+        rec[slot] = r;
+        local += ((unsigned long long)rec_nv(r) << 32) | (unsigned long long)rec_nq(r);
+      }
     }
-    amb += ambiguous;
-    const unsigned am = __activemask();
-    const unsigned bal = __ballot_sync(am, ambiguous);
+    nact += __popc(__ballot_sync(kAll, r != 0));
+    // ambiguous cells: their ranks to the front of the warp's share (its entries up to here are read)
+    const unsigned bal = __ballot_sync(kAll, ambiguous);
     if (bal) {
-      const int leader = __ffs(bal) - 1;
-      unsigned base = 0;
-      if (lane == leader) base = atomicAdd(amb_n, (unsigned)__popc(bal));
-      base = __shfl_sync(am, base, leader);
-      if (ambiguous) amb_list[base + __popc(bal & ((1u << lane) - 1u))] = slot;
+      __syncwarp();
+      if (ambiguous) list[share_entry<kPerTile>(share, amb + __popc(bal & ((1u << lane) - 1u)))] = (uint16_t)a;
+      amb += __popc(bal);
     }
   }
-  for (int o = 16; o; o >>= 1) {
-    local += __shfl_down_sync(0xffffffffu, local, o);
-    amb += __shfl_down_sync(0xffffffffu, amb, o);
-    nact += __shfl_down_sync(0xffffffffu, nact, o);
+  if (amb) {  // one atomic per warp: a single counter takes them all
+    unsigned base = 0;
+    if (lane == 0) base = atomicAdd(amb_n, amb);
+    base = __shfl_sync(kAll, base, 0);
+    __syncwarp();
+    for (unsigned x = lane; x < amb; x += 32)
+      amb_list[base + x] = (uint32_t)(vbase + list[share_entry<kPerTile>(share, x)]);
   }
-  if (lane == 0 && local) atomicAdd(&tile_sum, local);
-  // stats[0]: cells with a record (a used contour, an owned quad or the ambiguous flag); the
-  // ambiguous cells' records are never empty, so they count here too
-  if (lane == 0 && amb) atomicAdd(stats + 1, amb);
-  if (lane == 0 && (nact | amb)) atomicAdd(stats + 0, nact + amb);
-  __syncthreads();
-  if (threadIdx.x == 0) tile_sums[tile] = tile_sum;
+  for (int o = 16; o; o >>= 1) local += __shfl_down_sync(kAll, local, o);
+  if (lane == 0) {
+    if (kPerTile == 1) tile_sums[tile] = local;
+    else if (local) atomicAdd(tile_sum, local);
+    // stats[0]: cells with a record (a used contour, an owned quad or the ambiguous flag); the
+    // ambiguous cells' records are never empty, so they count here too
+    if (amb) atomicAdd(stats + 1, (unsigned long long)amb);
+    if (nact | amb) atomicAdd(stats + 0, (unsigned long long)(nact + amb));
+  }
+  if (kPerTile > 1) {
+    __syncthreads();
+    if (threadIdx.x == 0) tile_sums[tile] = *tile_sum;
+  }
 }
 
 // The ambiguous listed cells: MC polygon with the asymptotic decider (float-float, float64 near the
@@ -893,33 +935,35 @@ __global__ void __launch_bounds__(kQuadThreads) dmc_quad_kernel(CellSpace space,
 // ------------------------------------------------------------------------------------------
 // host-side launches
 // ------------------------------------------------------------------------------------------
-int dmc_front_count(const CellSpace& space, DmcScratch& s, cudaStream_t st, Prof* prof, const TileGate* gates,
-                    int ngates) {
+int dmc_front_count(const CellSpace& space, DmcScratch& s, int sms, cudaStream_t st, Prof* prof,
+                    const TileGate* gates, int ngates) {
   const int64_t tiles = ceil_div(space.n, kScanTile);
-  int k = 0, dev = 0, sms = 1;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  int k = 0;
   {
     Stage t(prof, "dmc_classify", st);
     // the ambiguous cells' list lives in qoff until the offsets kernel writes the quad offsets
     cudaMemsetAsync(s.amb_n, 0, 2 * sizeof(unsigned), st);  // and the chunk counter behind it
-    auto classify = [&](int64_t t0, int64_t t1) {
+    auto classify = [&](int64_t t0, int64_t t1, int z0, int z1) {
+      k += launch_point_bits(space, z0, z1, sms, st);
       if (t1 <= t0) return;
-      if (space.one.gen)  // fused generation (single volumes)
-        dmc_classify_kernel<true><<<(unsigned)(t1 - t0), kScanThreads, 0, st>>>(
-            space, t0, s.rec, s.cellof, s.ccase, s.mask, s.tile_sums, s.stats, reinterpret_cast<uint32_t*>(s.qoff), s.amb_n);
+      uint32_t* amb = reinterpret_cast<uint32_t*>(s.qoff);
+      if (block_per_tile(t1 - t0, sms))
+        dmc_classify_kernel<8><<<(unsigned)(t1 - t0), kClassifyThreads, 0, st>>>(
+            space, t0, t1, s.rec, s.cellof, s.ccase, s.mask, s.tile_sums, s.stats, amb, s.amb_n);
       else
-        dmc_classify_kernel<false><<<(unsigned)(t1 - t0), kScanThreads, 0, st>>>(
-            space, t0, s.rec, s.cellof, s.ccase, s.mask, s.tile_sums, s.stats, reinterpret_cast<uint32_t*>(s.qoff), s.amb_n);
+        dmc_classify_kernel<1><<<(unsigned)ceil_div(t1 - t0, kClassifyThreads / 32), kClassifyThreads, 0, st>>>(
+            space, t0, t1, s.rec, s.cellof, s.ccase, s.mask, s.tile_sums, s.stats, amb, s.amb_n);
       k++;
     };
-    if (ngates == 0) classify(0, tiles);
+    if (ngates == 0) classify(0, tiles, 0, space.one.nz);
     int64_t t0 = 0;
+    int z0 = 0;
     for (int q = 0; q < ngates; q++) {
       cudaStreamWaitEvent(st, gates[q].ready, 0);
       const int64_t t1 = (q == ngates - 1) ? tiles : std::min(gates[q].tile_end, tiles);
-      classify(t0, t1);
+      classify(t0, t1, z0, gates[q].z_end);
       t0 = std::max(t0, t1);
+      z0 = gates[q].z_end;
     }
     // one wave; the list length is only known on the device, so the grid follows the cell count
     static const int r_amb = resident_blocks(dmc_amb_kernel, 128);

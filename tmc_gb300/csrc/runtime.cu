@@ -233,7 +233,7 @@ tmc_status field_slabs(tmc_ctx* ctx, const tmc_volume* vol, Allocs& al, const fl
                                   cudaMemcpyHostToDevice, ctx->copy_stream));
     TMC_CUDA(ctx, cudaEventRecord(ctx->slab_events[q], ctx->copy_stream));
     // cells in planes z < z1 - 1 have all eight corners on the device; whole tiles only
-    gates.push_back({(int64_t)(z1 - 1) * cells_per_plane / tmc::kScanTile, ctx->slab_events[q]});
+    gates.push_back({(int64_t)(z1 - 1) * cells_per_plane / tmc::kScanTile, z1, ctx->slab_events[q]});
     z0 = z1;
   }
   *out = d;
@@ -654,6 +654,7 @@ tmc_status dmc_extract(tmc_ctx* ctx, const tmc_volume* vol, double iso, uint32_t
   tmc::Grid g = make_grid(vol, field, iso);
   if (fg) set_fused(g, *fg, dev_params);
   g.flags = ((flags & TMC_GRAD_FLIP) ? tmc::kGridFlip : 0) | (simplify ? tmc::kGridNormal64 : 0);
+  TMC_CUDA(ctx, al.get(&g.bits, g.bit_words() + 4));
   const tmc::CellSpace space = tmc::single_space(g);
   const int64_t ncell = g.ncells();
 
@@ -670,7 +671,7 @@ tmc_status dmc_extract(tmc_ctx* ctx, const tmc_volume* vol, double iso, uint32_t
   TMC_CUDA(ctx, al.get(&sc.totals, 2));
   sc.stats = ctx->d_stats;
   TMC_CUDA(ctx, cudaMemsetAsync(sc.stats, 0, 8 * sizeof(unsigned long long), st));
-  ctx->launches += tmc::dmc_front_count(space, sc, st, &ctx->prof, gates.data(), (int)gates.size());
+  ctx->launches += tmc::dmc_front_count(space, sc, ctx->sms, st, &ctx->prof, gates.data(), (int)gates.size());
   unsigned long long* h = (unsigned long long*)ctx->h_pinned;
   TMC_CUDA(ctx, cudaMemcpyAsync(h, sc.totals, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
   TMC_CUDA(ctx, tmc::host_wait(st));
@@ -819,6 +820,7 @@ tmc_status tmc_extract(tmc_ctx* ctx, const tmc_volume* vol, double iso, uint32_t
   tmc::Grid g = make_grid(vol, field, iso);
   if (fg) set_fused(g, *fg, dev_params);
   g.flags = (flags & TMC_OUT_POS_F64) ? tmc::kGridPos64 : 0;
+  TMC_CUDA(ctx, al.get(&g.bits, g.bit_words() + 4));
   const int64_t ncell = g.ncells();
   tmc::TmcScratch sc{};
   TMC_CUDA(ctx, al.get(&sc.rec, ncell));
@@ -834,7 +836,7 @@ tmc_status tmc_extract(tmc_ctx* ctx, const tmc_volume* vol, double iso, uint32_t
   TMC_CUDA(ctx, al.get(&sc.chunks, tmc::tmc_tiles(space) * (tmc::kScanTile / 32)));
   sc.stats = ctx->d_stats;
   TMC_CUDA(ctx, cudaMemsetAsync(sc.stats, 0, 8 * sizeof(unsigned long long), st));
-  ctx->launches += tmc::tmc_classify(space, sc, st, &ctx->prof, gates.data(), (int)gates.size());
+  ctx->launches += tmc::tmc_classify(space, sc, ctx->sms, st, &ctx->prof, gates.data(), (int)gates.size());
   unsigned long long* h = (unsigned long long*)ctx->h_pinned;
   int64_t n_amb = 0;
   TMC_CUDA(ctx, tmc_ambiguous_records(ctx, al, sc, n_amb));
@@ -982,6 +984,18 @@ tmc_status batch_run(tmc_ctx* ctx, const std::vector<int>& idx, const tmc_reques
   std::vector<int32_t> tile_vol((size_t)tiles);
   for (int q = 0; q < nb; q++)
     for (int64_t t = tile0[q]; t < tile0[q + 1]; t++) tile_vol[(size_t)t] = q;
+  // the volumes' bit rows one after another
+  int64_t bit_words = 0, max_bit_words = 0;
+  for (const tmc::Grid& g : grids) {
+    bit_words += g.bit_words();
+    max_bit_words = std::max(max_bit_words, g.bit_words());
+  }
+  uint32_t* bits = nullptr;
+  TMC_CUDA(ctx, al.get(&bits, bit_words + 4));
+  for (tmc::Grid& g : grids) {
+    g.bits = bits;
+    bits += g.bit_words();
+  }
   tmc::Grid* d_grids = nullptr;
   int32_t* d_tile_vol = nullptr;
   TMC_CUDA(ctx, al.get(&d_grids, nb));
@@ -992,6 +1006,8 @@ tmc_status batch_run(tmc_ctx* ctx, const std::vector<int>& idx, const tmc_reques
   space.one = grids[0];
   space.grids = d_grids;
   space.tile_vol = d_tile_vol;
+  space.n_volumes = nb;
+  space.max_bit_words = max_bit_words;
   space.n = ncell;
 
   // ---- count ----
@@ -1018,7 +1034,7 @@ tmc_status batch_run(tmc_ctx* ctx, const std::vector<int>& idx, const tmc_reques
     TMC_CUDA(ctx, al.get(&dsc.chunks, tiles * (tmc::kScanTile / 32)));
     TMC_CUDA(ctx, al.get(&dsc.amb_n, 2));
     TMC_CUDA(ctx, al.get(&dsc.ccase, ncell));
-    ctx->launches += tmc::dmc_front_count(space, dsc, st, &ctx->prof);
+    ctx->launches += tmc::dmc_front_count(space, dsc, ctx->sms, st, &ctx->prof);
   } else {
     tsc = tmc::TmcScratch{rec, nullptr, qoff, tile_sums, totals, ctx->d_stats};
     tsc.mask = mask;
@@ -1027,7 +1043,7 @@ tmc_status batch_run(tmc_ctx* ctx, const std::vector<int>& idx, const tmc_reques
     TMC_CUDA(ctx, al.get(&tsc.ccase, ncell));
     TMC_CUDA(ctx, al.get(&tsc.chunks, tiles * (tmc::kScanTile / 32)));
     TMC_CUDA(ctx, al.get(&tsc.amb_n, 2));
-    ctx->launches += tmc::tmc_classify(space, tsc, st, &ctx->prof);
+    ctx->launches += tmc::tmc_classify(space, tsc, ctx->sms, st, &ctx->prof);
     TMC_CUDA(ctx, tmc_ambiguous_records(ctx, al, tsc, n_amb_rec));
     ctx->launches += tmc::tmc_count(space, tsc, n_amb_rec, ctx->sms, st, &ctx->prof);
   }

@@ -604,65 +604,93 @@ __device__ void load_amb_cell(const Grid& g, int i, int j, int k, const float u[
 // ------------------------------------------------------------------------------------------
 // kernels
 // ------------------------------------------------------------------------------------------
-// One block per kScanTile consecutive cells.  Pass 1: MC cases from the warp-ballot corner rows
-// (warp_cases) and the listing of the crossed cells in cell order (list_tile).  Pass 2: the records
-// of the listed cells at their slots (owned crossed edges, table triangle counts); ambiguous cells are
-// listed by slot (amb_list, warp-aggregated appends) for the float64 counting pass.
-template <bool kGen>
-__global__ void __launch_bounds__(kScanThreads, 6) tmc_classify_kernel(CellSpace space, int64_t tile0, uint32_t* rec,
-                                                                   uint16_t* cellof, uint8_t* ccase, CellMask* mask,
-                                                                   unsigned long long* tile_sums,
-                                                                   unsigned long long* stats, uint32_t* amb_list,
-                                                                   unsigned* amb_n) {
-  const int64_t tile = tile0 + blockIdx.x;
-  __shared__ uint16_t act_list[kScanTile];
-  __shared__ uint8_t case_of[kScanTile];
-  __shared__ uint32_t wmask[kScanTile / 32], wpre[kScanTile / 32];
-  __shared__ int total;
-  __shared__ unsigned long long tile_sum;
-  if (threadIdx.x == 0) tile_sum = 0;
+// What the classification knows of a cell from its case alone, as the bits of its record: the crossed
+// edges among those it owns away from the lower borders, the table's triangles or the ambiguous flag.
+__device__ __forceinline__ uint32_t case_record(unsigned cs, uint32_t owned) {
+  return (case_edge_mask(cs) & owned) | (case_ambiguous(cs) ? (1u << 21) : (uint32_t)(c_tmc_tris[cs] & 0xF) << 15);
+}
+// One warp per tile of kScanTile consecutive cells: the crossed cells in cell order from the bit rows
+// (list_tile), then their records at their slots, a cell per lane; ambiguous cells are listed by slot
+// (amb_list) for the counting pass, which adds to this tile's sums.
+template <int kPerTile>  // warps per tile (block_per_tile)
+__global__ void __launch_bounds__(kClassifyThreads) tmc_classify_kernel(CellSpace space, int64_t tile0, int64_t tile1,
+                                                                          uint32_t* rec, uint16_t* cellof,
+                                                                          uint8_t* ccase, CellMask* mask,
+                                                                          unsigned long long* tile_sums,
+                                                                          unsigned long long* stats,
+                                                                          uint32_t* amb_list, unsigned* amb_n) {
+  constexpr unsigned kAll = 0xffffffffu;
+  constexpr int kTiles = kClassifyThreads / 32 / kPerTile;  // tiles per block
+  __shared__ uint16_t lists[kTiles][kScanTile];
+  __shared__ uint32_t inner_rec[256];  // records of cells off the lower borders
+  for (int c = threadIdx.x; c < 256; c += blockDim.x) inner_rec[c] = case_record(c, owned_edges(1, 1, 1));
+  __syncthreads();
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int share = kPerTile == 1 ? 0 : wid;  // the warp's share of its tile
+  const int64_t tile = tile0 + (int64_t)blockIdx.x * kTiles + (kPerTile == 1 ? wid : 0);
+  if (tile >= tile1) return;  // the whole warp, or the whole block
+  uint16_t* list = lists[kPerTile == 1 ? wid : 0];
   const Grid g = space.grid_of_tile(tile);
-  const int64_t n = g.ncells();
   const int64_t vbase = tile * kScanTile;
-  const int lane = threadIdx.x & 31;
-  const unsigned actbits = tile_cases<kGen>(g, space.n, vbase, case_of);
-  const int na = list_tile(actbits, tile, mask, wmask, wpre, act_list, &total);
-  unsigned long long local = 0, amb = 0;
-  for (int a = threadIdx.x; a < na; a += blockDim.x) {
-    const int off = act_list[a];
+  unsigned long long* tile_sum = nullptr;  // of the tile's warps, when there are several
+  int na = 0;
+  if (share == 0) na = list_tile(g, space.n, tile, mask, list);
+  if (kPerTile > 1) {
+    __shared__ int s_na;
+    __shared__ unsigned long long s_sum;
+    if (threadIdx.x == 0) {
+      s_na = na;
+      s_sum = 0;
+    }
+    __syncthreads();
+    na = s_na;
+    tile_sum = &s_sum;
+  }
+  unsigned long long local = 0;
+  unsigned amb = 0;
+  for (int a0 = 32 * share; a0 < na; a0 += 32 * kPerTile) {
+    const int a = a0 + lane;
     const uint32_t slot = (uint32_t)(vbase + a);
-    int i, j, k;
-    tcell_ijk(g, vbase + off - g.vbase, i, j, k);
-    const unsigned cs = case_of[off];
-    // away from the lower borders a cell owns a fixed set of edges (folded at compile time)
-    uint32_t r = case_edge_mask(cs) & ((i > 0 && j > 0 && k > 0) ? owned_edges(1, 1, 1) : owned_edges(i, j, k));
-    const bool listed = case_ambiguous(cs);
-    // ambiguous: counted by tmc_amb_count_kernel (float64), which adds to this tile's sums
-    r |= listed ? (1u << 21) : (uint32_t)(c_tmc_tris[cs] & 0xF) << 15;
-    amb += listed;
-    rec[slot] = r;
-    cellof[slot] = (uint16_t)off;
-    ccase[slot] = (uint8_t)cs;
-    local += ((unsigned long long)trec_nv(r) << 32) | (unsigned long long)trec_ntri(r);
-    const unsigned am = __activemask();
-    const unsigned bal = __ballot_sync(am, listed);
+    bool listed = false;
+    if (a < na) {
+      const int off = list[a];
+      int i, j, k;
+      tcell_ijk(g, vbase + off - g.vbase, i, j, k);
+      const unsigned cs = case_from_bits(g, i, j, k);
+      const uint32_t r = (i > 0 && j > 0 && k > 0) ? inner_rec[cs] : case_record(cs, owned_edges(i, j, k));
+      listed = (r >> 21) & 1;
+      rec[slot] = r;
+      cellof[slot] = (uint16_t)off;
+      ccase[slot] = (uint8_t)cs;
+      local += ((unsigned long long)trec_nv(r) << 32) | (unsigned long long)trec_ntri(r);
+    }
+    // ambiguous cells: their ranks to the front of the warp's share (its entries up to here are read)
+    const unsigned bal = __ballot_sync(kAll, listed);
     if (bal) {
-      const int leader = __ffs(bal) - 1;
-      unsigned base = 0;
-      if (lane == leader) base = atomicAdd(amb_n, (unsigned)__popc(bal));
-      base = __shfl_sync(am, base, leader);
-      if (listed) amb_list[base + __popc(bal & ((1u << lane) - 1u))] = slot;
+      __syncwarp();
+      if (listed) list[share_entry<kPerTile>(share, amb + __popc(bal & ((1u << lane) - 1u)))] = (uint16_t)a;
+      amb += __popc(bal);
     }
   }
-  for (int o = 16; o; o >>= 1) {
-    local += __shfl_down_sync(0xffffffffu, local, o);
-    amb += __shfl_down_sync(0xffffffffu, amb, o);
+  if (amb) {  // one atomic per warp: a single counter takes them all
+    unsigned base = 0;
+    if (lane == 0) base = atomicAdd(amb_n, amb);
+    base = __shfl_sync(kAll, base, 0);
+    __syncwarp();
+    for (unsigned x = lane; x < amb; x += 32)
+      amb_list[base + x] = (uint32_t)(vbase + list[share_entry<kPerTile>(share, x)]);
   }
-  if (lane == 0 && local) atomicAdd(&tile_sum, local);
-  if (lane == 0 && amb) atomicAdd(stats + 1, amb);
-  if (threadIdx.x == 0 && na) atomicAdd(stats + 0, (unsigned long long)na);
-  __syncthreads();
-  if (threadIdx.x == 0) tile_sums[tile] = tile_sum;
+  for (int o = 16; o; o >>= 1) local += __shfl_down_sync(kAll, local, o);
+  if (lane == 0) {
+    if (amb) atomicAdd(stats + 1, (unsigned long long)amb);
+    if (share == 0 && na) atomicAdd(stats + 0, (unsigned long long)na);
+    if (kPerTile == 1) tile_sums[tile] = local;
+    else if (local) atomicAdd(tile_sum, local);
+  }
+  if (kPerTile > 1) {
+    __syncthreads();
+    if (threadIdx.x == 0) tile_sums[tile] = *tile_sum;
+  }
 }
 
 // The classification lists the ambiguous cells in no useful order; p_slice's branches follow the MC
@@ -1523,7 +1551,7 @@ __global__ void __launch_bounds__(kEmitThreads, 4) tmc_emit_kernel(CellSpace spa
 // ------------------------------------------------------------------------------------------
 int64_t tmc_tiles(const CellSpace& space) { return ceil_div(space.n, kScanTile); }
 
-int tmc_classify(const CellSpace& space, TmcScratch& s, cudaStream_t st, Prof* prof, const TileGate* gates,
+int tmc_classify(const CellSpace& space, TmcScratch& s, int sms, cudaStream_t st, Prof* prof, const TileGate* gates,
                  int ngates) {
   const int64_t tiles = tmc_tiles(space);
   // the ambiguous-cell list lives in toff until the offsets kernel overwrites it
@@ -1532,23 +1560,26 @@ int tmc_classify(const CellSpace& space, TmcScratch& s, cudaStream_t st, Prof* p
   {
     Stage t(prof, "tmc_classify", st);
     cudaMemsetAsync(s.amb_n, 0, 2 * sizeof(unsigned), st);  // and the chunk counter behind it
-    auto classify = [&](int64_t t0, int64_t t1) {
+    auto classify = [&](int64_t t0, int64_t t1, int z0, int z1) {
+      k += launch_point_bits(space, z0, z1, sms, st);
       if (t1 <= t0) return;
-      if (space.one.gen)  // fused generation (single volumes)
-        tmc_classify_kernel<true><<<(unsigned)(t1 - t0), kScanThreads, 0, st>>>(
-            space, t0, s.rec, s.cellof, s.ccase, s.mask, s.tile_sums, s.stats, amb_cells, s.amb_n);
+      if (block_per_tile(t1 - t0, sms))
+        tmc_classify_kernel<8><<<(unsigned)(t1 - t0), kClassifyThreads, 0, st>>>(
+            space, t0, t1, s.rec, s.cellof, s.ccase, s.mask, s.tile_sums, s.stats, amb_cells, s.amb_n);
       else
-        tmc_classify_kernel<false><<<(unsigned)(t1 - t0), kScanThreads, 0, st>>>(
-            space, t0, s.rec, s.cellof, s.ccase, s.mask, s.tile_sums, s.stats, amb_cells, s.amb_n);
+        tmc_classify_kernel<1><<<(unsigned)ceil_div(t1 - t0, kClassifyThreads / 32), kClassifyThreads, 0, st>>>(
+            space, t0, t1, s.rec, s.cellof, s.ccase, s.mask, s.tile_sums, s.stats, amb_cells, s.amb_n);
       k++;
     };
-    if (ngates == 0) classify(0, tiles);
+    if (ngates == 0) classify(0, tiles, 0, space.one.nz);
     int64_t t0 = 0;
+    int z0 = 0;
     for (int q = 0; q < ngates; q++) {
       cudaStreamWaitEvent(st, gates[q].ready, 0);
       const int64_t t1 = (q == ngates - 1) ? tiles : std::min(gates[q].tile_end, tiles);
-      classify(t0, t1);
+      classify(t0, t1, z0, gates[q].z_end);
       t0 = std::max(t0, t1);
+      z0 = gates[q].z_end;
     }
   }
   return k;

@@ -43,7 +43,7 @@ struct TmcScratch {
 int64_t tmc_tiles(const CellSpace& space);
 // Classification: records of the crossed cells and the list of the ambiguous ones, whose number it
 // leaves in *s.amb_n.  gates: as dmc_front_count's (classification of a host field arriving in slabs).
-int tmc_classify(const CellSpace& space, TmcScratch& s, cudaStream_t st, Prof* prof = nullptr,
+int tmc_classify(const CellSpace& space, TmcScratch& s, int sms, cudaStream_t st, Prof* prof = nullptr,
                  const TileGate* gates = nullptr, int ngates = 0);
 // The ambiguous cells' counts (p_slice, float64) into their records and s.amb_rec (n_amb records,
 // n_amb = *s.amb_n), then the vertex and triangle offsets.
