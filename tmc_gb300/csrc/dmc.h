@@ -40,7 +40,8 @@ struct DmcScratch {
   uint32_t* chunks;               // kScanTile / 32 per tile: the chunk list (scan.cuh)
 };
 
-// Each launcher returns the number of kernels it launched.
+// Each launcher returns the number of kernels it launched.  The counters (stats, totals, amb_n,
+// fb_count) are zero when a call starts.
 // Per-cell scratch is indexed in the cell space (space.n cells, padding included).
 int64_t dmc_tiles(const CellSpace& space);  // scan tiles of the space
 // gates: classify the tiles of each gate once its event has completed (a host field arriving in

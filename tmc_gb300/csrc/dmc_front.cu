@@ -942,7 +942,6 @@ int dmc_front_count(const CellSpace& space, DmcScratch& s, int sms, cudaStream_t
   {
     Stage t(prof, "dmc_classify", st);
     // the ambiguous cells' list lives in qoff until the offsets kernel writes the quad offsets
-    cudaMemsetAsync(s.amb_n, 0, 2 * sizeof(unsigned), st);  // and the chunk counter behind it
     auto classify = [&](int64_t t0, int64_t t1, int z0, int z1) {
       k += launch_point_bits(space, z0, z1, sms, st);
       if (t1 <= t0) return;
@@ -1000,7 +999,6 @@ int dmc_front_emit(const CellSpace& space, DmcScratch& s, DmcVertexOut vo, int64
   };
   {
     Stage t(prof, "dmc_vertex_point", st);
-    cudaMemsetAsync(s.fb_count, 0, 3 * sizeof(unsigned), st);
     if (space.grids)
       dmc_vertex_point_kernel<true><<<vgrid(r_point_batch), kVertexThreads, 0, st>>>(
           space, s.cellof, s.ccase, s.rec, s.vrank, s.vwork, nv, s.vp, s.fb_list, s.w_list, s.fb_count);

@@ -485,10 +485,6 @@ __global__ void gather_live_quads_kernel(const uint8_t* alive, const int32_t* id
   }
 }
 
-__global__ void fill_i32_kernel(int32_t* p, int64_t n, int32_t v) {
-  FOR_EACH(i, n) p[i] = v;
-}
-
 // ---------------------------------------------------------------------------------------------
 // quad -> triangles (collectTriangles, :1387-1460; minAngle, DualMarchingCubes.h:746-756)
 // ---------------------------------------------------------------------------------------------
@@ -617,25 +613,41 @@ __global__ void triangles_kernel(const int32_t* q, const uint32_t* list, const u
 // ---------------------------------------------------------------------------------------------
 // driver helpers
 // ---------------------------------------------------------------------------------------------
+// Scratch of one call: arrays cut from one reserved block (256-byte aligned), on their own when it is
+// used up.
 struct Pool {
   cudaStream_t st;
   std::vector<void*> temp;
   cudaError_t err = cudaSuccess;
+  char* at = nullptr;
+  size_t left = 0;
+  explicit Pool(cudaStream_t s) : st(s) {}
+  void reserve(size_t bytes) {
+    void* p = nullptr;
+    if (err != cudaSuccess) return;
+    err = cudaMallocAsync(&p, bytes, st);
+    if (err != cudaSuccess) return;
+    temp.push_back(p);
+    at = (char*)p;
+    left = bytes;
+  }
   template <typename T>
   T* get(int64_t n) {
-    void* p = nullptr;
+    const size_t bytes = ((size_t)std::max<int64_t>(n, 4) * sizeof(T) + 255) & ~(size_t)255;
     if (err != cudaSuccess) return nullptr;
-    err = cudaMallocAsync(&p, (size_t)std::max<int64_t>(n, 4) * sizeof(T), st);
+    if (bytes <= left) {
+      void* p = at;
+      at += bytes;
+      left -= bytes;
+      return (T*)p;
+    }
+    void* p = nullptr;
+    err = cudaMallocAsync(&p, bytes, st);
     if (err == cudaSuccess) temp.push_back(p);
     return (T*)p;
   }
-  void drop(void* p) {
-    for (auto& q : temp)
-      if (q == p) q = nullptr;
-  }
   ~Pool() {
-    for (void* p : temp)
-      if (p) cudaFreeAsync(p, st);
+    for (void* p : temp) cudaFreeAsync(p, st);
   }
 };
 
@@ -644,6 +656,9 @@ struct HeBufs {
   uint8_t* flag = nullptr;
   int32_t* hv = nullptr;
   HeWork w{};
+  // counters, zeroed together: non-manifold edges, overflow, merge jobs of the passes, handle counts,
+  // quads of the exact triangle split, colour classes
+  unsigned long long* zero = nullptr;
   unsigned long long* nm = nullptr;
   unsigned* ovf = nullptr;
   // repairs after the simplification passes: vertices a pass touched (dold) and the dirty ones
@@ -658,13 +673,12 @@ struct HeBufs {
 // colorFaces (:714-844) on a mesh whose halfedges are built: the inherited colours in `col` become
 // the reduced ones, class by class (colours 5..23 to the lowest of 0..4 free among the neighbours,
 // then colour 4 to the lowest of 0..3).  Returns the number of kernels launched.
-int color_faces(const HeView& he, uint8_t* col, int64_t nq, Pool& pool, int sms, cudaStream_t st) {
-  int32_t* cnt = pool.get<int32_t>(24);
+// cnt: 24 zeroed words.
+int color_faces(const HeView& he, uint8_t* col, int64_t nq, int32_t* cnt, Pool& pool, int sms, cudaStream_t st) {
   int32_t* off = pool.get<int32_t>(24);
   int32_t* cursor = pool.get<int32_t>(24);
   int32_t* list = pool.get<int32_t>(std::max<int64_t>(nq, 1));
   if (pool.err) return 0;
-  cudaMemsetAsync(cnt, 0, 24 * sizeof(int32_t), st);
   const unsigned gc = (unsigned)std::max<int64_t>(1, ceil_div(nq, kColorTile));
   color_count_kernel<<<gc, kColorThreads, 0, st>>>(col, nq, cnt);
   color_offsets_kernel<<<1, 32, 0, st>>>(cnt, off, cursor);
@@ -684,6 +698,9 @@ int vertex_valence(const HeView& he, const int32_t* deg, int64_t nv, int64_t nq,
   return 1;
 }
 
+constexpr int kZeroWords = 32;  // [0,1] non-manifold, [2] overflow, [3..6] handles, [7] jobs, [8] split, [16..27] colours
+constexpr int kZeroJobs = 7, kZeroSplit = 8, kZeroColors = 16;
+
 HeBufs halfedge_buffers(Pool& pool, int64_t NV, int64_t NQ) {
   HeBufs hw;
   hw.twin = pool.get<int32_t>(4 * NQ);
@@ -696,26 +713,64 @@ HeBufs halfedge_buffers(Pool& pool, int64_t NV, int64_t NQ) {
   hw.w.hv_key = pool.get<unsigned long long>(NV);
   hw.w.tiles = pool.get<unsigned long long>(scan_tiles(NV) + 2);
   hw.w.total = pool.get<unsigned long long>(2);
-  hw.nm = pool.get<unsigned long long>(2);
+  hw.zero = pool.get<unsigned long long>(kZeroWords);
+  hw.nm = hw.zero;
   hw.w.non_manifold = hw.nm;
-  hw.ovf = pool.get<unsigned>(2);
-  hw.hcount = pool.get<unsigned long long>(4);
+  hw.ovf = reinterpret_cast<unsigned*>(hw.zero + 2);
+  hw.hcount = hw.zero + 3;
   return hw;
 }
 
-// buffers of the halfedge repairs and of the final compaction
-void update_buffers(Pool& pool, HeBufs& hw, int64_t NV, int64_t NQ) {
-  hw.dold = pool.get<uint8_t>(NV);
-  hw.dnew = pool.get<uint8_t>(NV);
+// Buffers of the simplification passes, their halfedge repairs and the final compaction.  What a pass
+// resets lies together: `fresh` (bucket sizes, merge marks, touched and dirty vertices) is zeroed and
+// `owner` (claims and merge targets) set to -1 by one fill each.
+struct PassBufs {
+  int32_t* val;
+  uint8_t *p, *em, *branch;   // p and em adjacent (both zero for P3333)
+  size_t face_stride;         // from p to em
+  uint8_t* fresh;
+  size_t fresh_bytes;
+  uint8_t* vm_first;
+  int32_t* owner;
+  int32_t *own_pos, *own_rm, *vm_second;
+  int4* jobs;
+  uint8_t *alive, *valive;    // adjacent
+  size_t alive_bytes;         // of both
+  int32_t *idx, *idx_q;
+};
+PassBufs pass_buffers(Pool& pool, HeBufs& hw, int64_t NV, int64_t NQ) {
+  PassBufs b;
+  const int64_t nv16 = (NV + 15) / 16 * 16, nq16 = (NQ + 15) / 16 * 16;
   hw.src = pool.get<int32_t>(NQ);
   hw.u.drank = pool.get<int32_t>(4 * NQ);
   hw.u.dmask = pool.get<uint8_t>(NQ);
-  hw.u.bcnt = pool.get<int32_t>(NV);
   hw.u.boff = hw.w.off;    // the build's scratch is idle after the one build
   hw.u.blist = hw.w.list;
   hw.u.bkey = pool.get<int32_t>(4 * NQ);
   hw.u.tiles = hw.w.tiles;
   hw.u.total = hw.w.total;
+  b.val = pool.get<int32_t>(NV);
+  b.face_stride = (size_t)nq16;
+  b.p = pool.get<uint8_t>(2 * nq16);
+  b.em = b.p + nq16;
+  b.branch = pool.get<uint8_t>(NQ);
+  b.fresh_bytes = (size_t)(7 * nv16);
+  b.fresh = pool.get<uint8_t>(7 * nv16);
+  hw.u.bcnt = reinterpret_cast<int32_t*>(b.fresh);
+  b.vm_first = b.fresh + 4 * nv16;
+  hw.dold = b.fresh + 5 * nv16;
+  hw.dnew = b.fresh + 6 * nv16;
+  b.owner = pool.get<int32_t>(3 * NV);
+  b.own_pos = b.owner;
+  b.own_rm = b.owner + NV;
+  b.vm_second = b.owner + 2 * NV;
+  b.jobs = pool.get<int4>(NQ);
+  b.alive_bytes = (size_t)(nq16 + NV);
+  b.alive = pool.get<uint8_t>(nq16 + NV);
+  b.valive = b.alive + nq16;
+  b.idx = pool.get<int32_t>(NV);
+  b.idx_q = pool.get<int32_t>(NQ);
+  return b;
 }
 
 }  // namespace
@@ -727,14 +782,15 @@ DmcPostStatus dmc_color_valence(const int32_t* quads, int64_t nq, int64_t nv, ui
     if (nv > 0) s.err = cudaMemsetAsync(valence, 0, nv * sizeof(int32_t), st);
     return s;
   }
-  Pool pool{st};
+  Pool pool(st);
+  pool.reserve(72 * (size_t)nq + 20 * (size_t)std::max<int64_t>(nv, 1) + 32 * 256);
   HeBufs hw = halfedge_buffers(pool, std::max<int64_t>(nv, 1), nq);
   if ((s.err = pool.err) != cudaSuccess) return s;
-  cudaMemsetAsync(hw.nm, 0, 2 * sizeof(unsigned long long), st);
+  cudaMemsetAsync(hw.zero, 0, kZeroWords * sizeof(unsigned long long), st);
   HeOut ho{hw.twin, hw.flag, hw.hv};
   s.launches += build_halfedges(quads, 4, nq, nv, ho, hw.w, sms, st, false);
   const HeView he{quads, hw.twin, hw.flag};
-  s.launches += color_faces(he, colors, nq, pool, sms, st);
+  s.launches += color_faces(he, colors, nq, reinterpret_cast<int32_t*>(hw.zero + kZeroColors), pool, sms, st);
   if ((s.err = pool.err) != cudaSuccess) return s;
   s.launches += vertex_valence(he, hw.w.deg, nv, nq, valence, sms, st);
   s.err = cudaGetLastError();
@@ -753,8 +809,11 @@ DmcPostStatus dmc_postprocess(const DmcMesh& in, uint32_t flags, int sms, cudaSt
     s.err = cudaErrorInvalidValue;
     return s;
   }
-  Pool pool{st};
+  Pool pool(st);
   const int64_t NV = std::max<int64_t>(in.nv, 1), NQ = std::max<int64_t>(in.nq, 1);
+  // what the buffers below add up to, per face and per vertex
+  const bool passes = (c3x3y || i3x3y || p3333) && in.nq > 0;
+  pool.reserve((passes ? 144 : 74) * (size_t)NQ + (passes ? 56 : 24) * (size_t)NV + 64 * 256);
 
   DmcMesh cur = in;
   HeBufs hw = halfedge_buffers(pool, NV, NQ);
@@ -764,12 +823,11 @@ DmcPostStatus dmc_postprocess(const DmcMesh& in, uint32_t flags, int sms, cudaSt
     s.err = pool.err;
     return s;
   }
-  if (hw.ovf) cudaMemsetAsync(hw.ovf, 0, 2 * sizeof(unsigned), st);
-  const unsigned gq = grid_for(NQ, sms), gv = grid_for(NV, sms);
+  cudaMemsetAsync(hw.zero, 0, kZeroWords * sizeof(unsigned long long), st);
+  const unsigned gq = grid_for(NQ, sms);
   const bool simplify = (c3x3y || i3x3y || p3333) && in.nq > 0;
   auto build_he = [&](bool handles) {
     Stage tm(prof, "dmc_halfedges", st);
-    cudaMemsetAsync(hw.nm, 0, 2 * sizeof(unsigned long long), st);
     HeOut ho{hw.twin, hw.flag, hw.hv};
     s.launches += build_halfedges(cur.quads, 4, cur.nq, cur.nv, ho, hw.w, sms, st, handles);
   };
@@ -797,24 +855,15 @@ DmcPostStatus dmc_postprocess(const DmcMesh& in, uint32_t flags, int sms, cudaSt
   int64_t nv0 = cur.nv, nq0 = cur.nq;  // the uncompacted mesh
   int32_t* q0 = cur.quads;
   if (simplify) {
-    update_buffers(pool, hw, NV, NQ);
-    int32_t* val = pool.get<int32_t>(NV);
-    uint8_t* p = pool.get<uint8_t>(NQ);
-    uint8_t* branch = pool.get<uint8_t>(NQ);
-    uint8_t* vm_first = pool.get<uint8_t>(NV);
-    uint8_t* em = pool.get<uint8_t>(NQ);
-    int32_t* own_pos = pool.get<int32_t>(NV);
-    int32_t* own_rm = pool.get<int32_t>(NV);
-    int32_t* vm_second = pool.get<int32_t>(NV);
-    int4* jobs = pool.get<int4>(NQ);
-    unsigned* njobs = pool.get<unsigned>(2);
-    alive = pool.get<uint8_t>(NQ);
-    valive = pool.get<uint8_t>(NV);
-    idx = pool.get<int32_t>(NV);
-    idx_q = pool.get<int32_t>(NQ);
+    const PassBufs b = pass_buffers(pool, hw, NV, NQ);
+    int32_t *val = b.val, *own_pos = b.own_pos, *own_rm = b.own_rm, *vm_second = b.vm_second;
+    uint8_t *p = b.p, *em = b.em, *branch = b.branch, *vm_first = b.vm_first;
+    alive = b.alive;
+    valive = b.valive;
+    idx = b.idx;
+    idx_q = b.idx_q;
     if ((s.err = pool.err) != cudaSuccess) return s;
-    cudaMemsetAsync(alive, 1, nq0, st);
-    cudaMemsetAsync(valive, 1, nv0, st);
+    cudaMemsetAsync(alive, 1, b.alive_bytes, st);
     build_he(false);
     const HeView he{q0, hw.twin, hw.flag};
     auto repair = [&]() {
@@ -827,27 +876,23 @@ DmcPostStatus dmc_postprocess(const DmcMesh& in, uint32_t flags, int sms, cudaSt
       if ((pass == 0 && !c3x3y) || (pass == 1 && !i3x3y)) continue;
       if (pass == 0) {
         Stage tm(prof, "dmc_color", st);
-        s.launches += color_faces(he, cur.colors, nq0, pool, sms, st);
+        s.launches += color_faces(he, cur.colors, nq0, reinterpret_cast<int32_t*>(hw.zero + kZeroColors), pool, sms, st);
         if ((s.err = pool.err) != cudaSuccess) return s;
       }
       {
         Stage tm(prof, "dmc_p3x3y", st);
         s.launches += vertex_valence(he, hw.w.deg, nv0, nq0, val, sms, st, alive);
         mark3x3y_kernel<<<gq, 256, 0, st>>>(q0, nq0, val, p, alive);
-        fill_i32_kernel<<<gv, 256, 0, st>>>(own_pos, nv0, -1);
-        fill_i32_kernel<<<gv, 256, 0, st>>>(own_rm, nv0, -1);
-        fill_i32_kernel<<<gv, 256, 0, st>>>(vm_second, nv0, -1);
-        cudaMemsetAsync(vm_first, 0, nv0, st);
-        cudaMemsetAsync(hw.dold, 0, nv0, st);
-        cudaMemsetAsync(hw.dnew, 0, nv0, st);
+        cudaMemsetAsync(b.owner, 0xff, 3 * (size_t)NV * sizeof(int32_t), st);
+        cudaMemsetAsync(b.fresh, 0, b.fresh_bytes, st);
         merge_claim_kernel<<<gq, 256, 0, st>>>(he, nq0, p, val, cur.colors, pass == 0, branch, own_pos, own_rm);
-        cudaMemsetAsync(njobs, 0, sizeof(unsigned), st);
+        unsigned* njobs = reinterpret_cast<unsigned*>(hw.zero + kZeroJobs) + pass;
         merge_apply_kernel<<<gq, kMergeThreads, 0, st>>>(he, nq0, branch, own_pos, own_rm, vm_first, vm_second, em,
-                                                         jobs, njobs, hw.dold, valive);
+                                                         b.jobs, njobs, hw.dold, valive);
         static const int r_mid = resident_blocks(midpoint_kernel, 256);  // one wave over the merge list
-        midpoint_kernel<<<(unsigned)wave_grid(r_mid, sms, 1, nq0, 256), 256, 0, st>>>(jobs, njobs, cur.v64, cur.n64);
+        midpoint_kernel<<<(unsigned)wave_grid(r_mid, sms, 1, nq0, 256), 256, 0, st>>>(b.jobs, njobs, cur.v64, cur.n64);
         apply_3x3y_kernel<<<gq, 256, 0, st>>>(q0, nq0, alive, em, vm_first, vm_second, hw.dold, hw.dnew, hw.w.deg);
-        s.launches += 11;
+        s.launches += 5;
       }
       repair();
     }
@@ -860,15 +905,12 @@ DmcPostStatus dmc_postprocess(const DmcMesh& in, uint32_t flags, int sms, cudaSt
         uint8_t* vm0 = vm_first;
         int32_t* vm1 = own_pos;
         s.launches += vertex_valence(he, hw.w.deg, nv0, nq0, val, sms, st, alive);
-        cudaMemsetAsync(p3, 0, nq0, st);
-        cudaMemsetAsync(rflag, 0, nq0, st);
-        cudaMemsetAsync(vm0, 0, nv0, st);
-        cudaMemsetAsync(hw.dold, 0, nv0, st);
-        cudaMemsetAsync(hw.dnew, 0, nv0, st);
-        fill_i32_kernel<<<gv, 256, 0, st>>>(vm1, nv0, -1);
+        cudaMemsetAsync(p3, 0, 2 * b.face_stride, st);  // and rflag behind it
+        cudaMemsetAsync(b.fresh, 0, b.fresh_bytes, st);
+        cudaMemsetAsync(vm1, 0xff, (size_t)NV * sizeof(int32_t), st);
         mark3333_kernel<<<gq, 256, 0, st>>>(he, nq0, val, p3, rflag, vm0, vm1, hw.dold, alive, valive);
         apply_3333_kernel<<<gq, 256, 0, st>>>(q0, nq0, alive, rflag, p3, vm1, hw.dold, hw.dnew, hw.w.deg);
-        s.launches += 3;
+        s.launches += 2;
       }
       repair();
     }
@@ -956,9 +998,9 @@ DmcPostStatus dmc_postprocess(const DmcMesh& in, uint32_t flags, int sms, cudaSt
         (*ready)(hv, (size_t)cur.nv * sizeof(int32_t));
         (*ready)(hf, (size_t)cur.nq * sizeof(int32_t));
       }
-      cudaMemcpyAsync(h_cnt + 1, hw.nm, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st);
-      host_wait(st);
-      out->non_manifold = (int64_t)h_cnt[1];
+      // read by the caller when the stream is done (the compaction's counts in h_cnt are read by now)
+      cudaMemcpyAsync(h_cnt + 2, hw.nm, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st);
+      out->non_manifold = h_cnt + 2;
       out->nhe = 4 * cur.nq;
       out->he = (int32_t*)he4;
       out->he_v = (int32_t*)hv;
@@ -971,9 +1013,8 @@ DmcPostStatus dmc_postprocess(const DmcMesh& in, uint32_t flags, int sms, cudaSt
       adopt(tr);
       Stage tm(prof, "dmc_triangles", st);
       uint32_t* tlist = pool.get<uint32_t>(std::max<int64_t>(cur.nq, 1));
-      unsigned* tcount = pool.get<unsigned>(2);
+      unsigned* tcount = reinterpret_cast<unsigned*>(hw.zero + kZeroSplit);
       if ((s.err = pool.err) == cudaSuccess) {
-        cudaMemsetAsync(tcount, 0, sizeof(unsigned), st);
         triangles_fast_kernel<<<grid_for(cur.nq, sms), 256, 0, st>>>(cur.quads, cur.nq, cur.v, (int32_t*)tr, tlist,
                                                                       tcount);
         triangles_kernel<<<grid_for(cur.nq, sms), 256, 0, st>>>(cur.quads, tlist, tcount, cur.v64, (int32_t*)tr,

@@ -27,7 +27,8 @@ struct DmcPostOut {
   int32_t* he = nullptr;        // 4 per halfedge
   int32_t* he_v = nullptr;
   int32_t* he_f = nullptr;
-  int64_t non_manifold = 0;
+  // three- and four-halfedge edges, when halfedges are built: a word of h_staging, there once `st` is done
+  const unsigned long long* non_manifold = nullptr;
   std::vector<void*> owned;     // new device buffers now owned by the result
   std::vector<void*> freed;     // input buffers released by the post-processing
 };

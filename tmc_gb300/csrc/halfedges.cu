@@ -506,7 +506,6 @@ int repair_halfedges(const int32_t* faces, int64_t nf, int64_t nv, const uint8_t
                      HeOut& o, int32_t* deg, HeUpdateWork& w, int sms, cudaStream_t st) {
   if (nf == 0) return 0;
   const int4* q4 = reinterpret_cast<const int4*>(faces);
-  cudaMemsetAsync(w.bcnt, 0, (size_t)nv * sizeof(int32_t), st);
   static const int r_mark = resident_blocks(he_repair_mark_kernel, 256);
   he_repair_mark_kernel<<<(unsigned)wave_grid(r_mark, sms, 8, nf, 256), 256, 0, st>>>(q4, nf, alive, dirty, deg, w.bcnt,
                                                                                       w.drank, w.dmask);

@@ -37,7 +37,7 @@ int build_halfedges(const int32_t* faces, int P, int64_t nf, int64_t nv, HeOut& 
 struct HeUpdateWork {
   int32_t* drank;             // 4 nf: rank of a halfedge with a dirty end in its bucket
   uint8_t* dmask;             // nf: the face's halfedges with a dirty end (bit r: halfedge 4f + r)
-  int32_t* bcnt;              // nv: bucket sizes
+  int32_t* bcnt;              // nv: bucket sizes (zero on entry)
   int32_t* boff;              // nv: bucket offsets
   int2* blist;                // 4 nf: (halfedge, other end) grouped by bucket
   int32_t* bkey;              // 4 nf: the bucket of each entry

@@ -2,8 +2,11 @@
 // scheduling of a context that has fewer threads than cores); a caller with several extractions
 // in flight, or a request server, has many threads waiting at once, and their spinning takes the
 // host's cores from the threads that have work.  A blocking-sync event (one per thread and device)
-// puts the waiting thread to sleep instead.
+// puts the waiting thread to sleep instead.  A sleeping thread takes some 20 us to come back, which a
+// small extraction would pay three times in a call of 200 us; so a wait polls for its first 60 us and
+// sleeps after that.
 #pragma once
+#include <chrono>
 #include <vector>
 #include <cuda_runtime.h>
 
@@ -27,7 +30,19 @@ inline cudaError_t host_wait(cudaStream_t st) {
       events[dev] = nullptr;
       break;
     }
-    if (cudaEventRecord(events[dev], st) == cudaSuccess) return cudaEventSynchronize(events[dev]);
+    if (cudaEventRecord(events[dev], st) == cudaSuccess) {
+      // a query that is not ready yet counts as the thread's last error: poll only when there is none to
+      // lose, and take each one back
+      if (cudaPeekAtLastError() == cudaSuccess) {
+        const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(60);
+        do {
+          const cudaError_t e = cudaEventQuery(events[dev]);
+          if (e != cudaErrorNotReady) return e;
+          (void)cudaGetLastError();
+        } while (std::chrono::steady_clock::now() < until);
+      }
+      return cudaEventSynchronize(events[dev]);
+    }
     (void)cudaGetLastError();
     events[dev] = nullptr;
   }

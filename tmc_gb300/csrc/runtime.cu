@@ -40,8 +40,9 @@ struct tmc_ctx {
   tmc_ctx_opts opts{};
   std::string err;
   std::atomic<int64_t> launches{0};
-  unsigned long long* d_stats = nullptr;  // 8 counters, reused per call
-  void* h_pinned = nullptr;               // small pinned staging area (totals, stats)
+  // the counters of one call (words of kStat..., zeroed together when it starts)
+  unsigned long long* d_stats = nullptr;
+  void* h_pinned = nullptr;               // small pinned staging area (totals, stats; a batch's tables)
   tmc::Prof prof;                         // stage timings (off unless enabled)
   // pinned host blocks for TMC_OUT_HOST results, reused across calls; shared by the worker contexts
   // of a request server (tmc::ctx_share_pinned)
@@ -51,6 +52,16 @@ struct tmc_ctx {
 };
 
 namespace {
+
+// tmc_ctx::d_stats, in 64-bit words
+constexpr int kStatTotals = 8;    // after the 8 statistics: [0] (vertices << 32) | faces, [1] overflow
+constexpr int kStatAmb = 10;      // 2 x u32: ambiguous cells, chunks
+constexpr int kStatFallback = 11; // 3 x u32: the DMC vertex lists
+constexpr int kStatAmbHist = 16;  // 514 x u32: the sort of TMC's ambiguous cells
+constexpr int kStatWords = kStatAmbHist + 257;
+constexpr size_t kPinnedBytes = 256 << 10;
+// a batch's grids and tile table go up from here, and its volume offsets come back (bytes)
+constexpr size_t kPinnedTables = 8192;
 
 // Device arrays shared by the meshes of one batch (each mesh points at its slice); released when
 // the last of those meshes is freed.
@@ -103,6 +114,27 @@ struct Allocs {
     *out = (T*)p;
     return e;
   }
+  // Scratch arrays of one stage in one allocation: plan() each, then commit() (a call's dozens of
+  // allocations cost some 1.5 us each, and on large ones the pool has mapped memory anew: 1.3 ms per
+  // 512^3 call).  Arrays are 256-byte aligned.
+  std::vector<std::pair<void**, size_t>> planned;
+  template <typename T>
+  void plan(T** out, int64_t count) {
+    planned.emplace_back(reinterpret_cast<void**>(out), (size_t)std::max<int64_t>(count, 1) * sizeof(T));
+  }
+  cudaError_t commit() {
+    size_t total = 0;
+    for (auto& a : planned) total += (a.second + 255) & ~(size_t)255;
+    char* base = nullptr;
+    const cudaError_t e = get(&base, total);
+    if (e == cudaSuccess)
+      for (auto& a : planned) {
+        *a.first = base;
+        base += (a.second + 255) & ~(size_t)255;
+      }
+    planned.clear();
+    return e;
+  }
   // hand ownership of p to the caller
   void release(void* p) {
     for (auto& q : ptrs)
@@ -122,12 +154,11 @@ cudaError_t tmc_ambiguous_records(tmc_ctx* ctx, Allocs& al, tmc::TmcScratch& sc,
   if (e == cudaSuccess) e = tmc::host_wait(ctx->stream);
   if (e != cudaSuccess) return e;
   n_amb = (int64_t)*h;
-  const size_t na = (size_t)std::max<int64_t>(n_amb, 1);
-  if ((e = al.get(&sc.amb_rec, na * tmc::kTmcAmbRecWords)) != cudaSuccess) return e;
-  if ((e = al.get(&sc.amb_sorted, na)) != cudaSuccess) return e;
-  if ((e = al.get(&sc.amb_key, na)) != cudaSuccess) return e;
-  if ((e = al.get(&sc.amb_doubt, na)) != cudaSuccess) return e;
-  return al.get(&sc.amb_hist, 514);
+  al.plan(&sc.amb_rec, n_amb * tmc::kTmcAmbRecWords);
+  al.plan(&sc.amb_sorted, n_amb);
+  al.plan(&sc.amb_key, n_amb);
+  al.plan(&sc.amb_doubt, n_amb);
+  return al.commit();
 }
 
 float iso_up(double iso) {
@@ -279,13 +310,46 @@ tmc::Grid make_grid(const tmc_volume* vol, const float* dev, double iso) {
 void mesh_reset(tmc_mesh* m) { std::memset(m, 0, sizeof(*m)); }
 
 // per-vertex scratch of the vertex kernels
-cudaError_t dmc_vertex_scratch(Allocs& al, tmc::DmcScratch& sc, int64_t nv) {
-  cudaError_t e = al.get(&sc.vp, nv);
-  if (e == cudaSuccess) e = al.get(&sc.fb_list, nv);
-  if (e == cudaSuccess) e = al.get(&sc.w_list, nv);
-  if (e == cudaSuccess) e = al.get(&sc.fb_count, 3);
-  if (e == cudaSuccess) e = al.get(&sc.tail_list, nv);
-  return e;
+void plan_dmc_vertices(Allocs& al, tmc::DmcScratch& sc, int64_t nv) {
+  al.plan(&sc.vwork, nv);
+  al.plan(&sc.vrank, nv);
+  al.plan(&sc.vp, nv);
+  al.plan(&sc.fb_list, nv);
+  al.plan(&sc.w_list, nv);
+  al.plan(&sc.tail_list, nv);
+}
+
+// per-cell scratch of the DMC / TMC front ends, and their counters (zeroed by start_counters)
+void plan_dmc_cells(tmc_ctx* ctx, Allocs& al, tmc::DmcScratch& sc, int64_t ncell, int64_t tiles) {
+  al.plan(&sc.rec, ncell);
+  al.plan(&sc.rv, ncell);
+  al.plan(&sc.qoff, ncell);
+  al.plan(&sc.cellof, ncell);
+  al.plan(&sc.ccase, ncell);
+  al.plan(&sc.chunks, tiles * (tmc::kScanTile / 32));
+  al.plan(&sc.mask, tiles * (tmc::kScanTile / 32));
+  al.plan(&sc.tile_sums, tiles);
+  sc.stats = ctx->d_stats;
+  sc.totals = ctx->d_stats + kStatTotals;
+  sc.amb_n = reinterpret_cast<unsigned*>(ctx->d_stats + kStatAmb);
+  sc.fb_count = reinterpret_cast<unsigned*>(ctx->d_stats + kStatFallback);
+}
+void plan_tmc_cells(tmc_ctx* ctx, Allocs& al, tmc::TmcScratch& sc, int64_t ncell, int64_t tiles) {
+  al.plan(&sc.rec, ncell);
+  al.plan(&sc.rv, ncell);
+  al.plan(&sc.toff, ncell);
+  al.plan(&sc.cellof, ncell);
+  al.plan(&sc.ccase, ncell);
+  al.plan(&sc.chunks, tiles * (tmc::kScanTile / 32));
+  al.plan(&sc.mask, tiles * (tmc::kScanTile / 32));
+  al.plan(&sc.tile_sums, tiles);
+  sc.stats = ctx->d_stats;
+  sc.totals = ctx->d_stats + kStatTotals;
+  sc.amb_n = reinterpret_cast<unsigned*>(ctx->d_stats + kStatAmb);
+  sc.amb_hist = reinterpret_cast<unsigned*>(ctx->d_stats + kStatAmbHist);
+}
+cudaError_t start_counters(tmc_ctx* ctx) {
+  return cudaMemsetAsync(ctx->d_stats, 0, kStatWords * sizeof(unsigned long long), ctx->stream);
 }
 
 // Early device-to-host copies for TMC_OUT_HOST: an array handed to issue() is final (no later
@@ -467,8 +531,8 @@ tmc_status tmc_ctx_create(int device, const tmc_ctx_opts* opts, tmc_ctx** out) {
     uint64_t thr = ctx->opts.reserve_bytes ? (uint64_t)ctx->opts.reserve_bytes : UINT64_MAX;
     cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &thr);
   }
-  if (cudaMalloc(&ctx->d_stats, 8 * sizeof(unsigned long long)) != cudaSuccess ||
-      cudaMallocHost(&ctx->h_pinned, 4096) != cudaSuccess) {
+  if (cudaMalloc(&ctx->d_stats, kStatWords * sizeof(unsigned long long)) != cudaSuccess ||
+      cudaMallocHost(&ctx->h_pinned, kPinnedBytes) != cudaSuccess) {
     tmc_ctx_destroy(ctx);
     return TMC_ERR_OOM;
   }
@@ -589,7 +653,7 @@ tmc_status tmc_mesh_free(tmc_ctx* ctx, tmc_mesh* mesh) {
     cudaSetDevice(ctx->device);
     for (void* p : mp->dev) cudaFreeAsync(p, ctx->stream);
     mp->shared.reset();
-    tmc::host_wait(ctx->stream);  // the next call may reuse these pinned blocks
+    if (!mp->host.empty()) tmc::host_wait(ctx->stream);  // the next call may reuse these pinned blocks
     for (void* p : mp->host) ctx->pinned_put(p);
     delete mp;
   }
@@ -654,23 +718,13 @@ tmc_status dmc_extract(tmc_ctx* ctx, const tmc_volume* vol, double iso, uint32_t
   tmc::Grid g = make_grid(vol, field, iso);
   if (fg) set_fused(g, *fg, dev_params);
   g.flags = ((flags & TMC_GRAD_FLIP) ? tmc::kGridFlip : 0) | (simplify ? tmc::kGridNormal64 : 0);
-  TMC_CUDA(ctx, al.get(&g.bits, g.bit_words() + 4));
-  const tmc::CellSpace space = tmc::single_space(g);
   const int64_t ncell = g.ncells();
-
   tmc::DmcScratch sc{};
-  TMC_CUDA(ctx, al.get(&sc.rec, ncell));
-  TMC_CUDA(ctx, al.get(&sc.rv, ncell));
-  TMC_CUDA(ctx, al.get(&sc.qoff, ncell));
-  TMC_CUDA(ctx, al.get(&sc.cellof, ncell));
-  TMC_CUDA(ctx, al.get(&sc.ccase, ncell));
-  TMC_CUDA(ctx, al.get(&sc.amb_n, 2));
-  TMC_CUDA(ctx, al.get(&sc.chunks, tmc::dmc_tiles(space) * (tmc::kScanTile / 32)));
-  TMC_CUDA(ctx, al.get(&sc.mask, tmc::dmc_tiles(space) * (tmc::kScanTile / 32)));
-  TMC_CUDA(ctx, al.get(&sc.tile_sums, tmc::dmc_tiles(space)));
-  TMC_CUDA(ctx, al.get(&sc.totals, 2));
-  sc.stats = ctx->d_stats;
-  TMC_CUDA(ctx, cudaMemsetAsync(sc.stats, 0, 8 * sizeof(unsigned long long), st));
+  al.plan(&g.bits, g.bit_words() + 4);
+  plan_dmc_cells(ctx, al, sc, ncell, tmc::ceil_div(ncell, tmc::kScanTile));
+  TMC_CUDA(ctx, al.commit());
+  const tmc::CellSpace space = tmc::single_space(g);
+  TMC_CUDA(ctx, start_counters(ctx));
   ctx->launches += tmc::dmc_front_count(space, sc, ctx->sms, st, &ctx->prof, gates.data(), (int)gates.size());
   unsigned long long* h = (unsigned long long*)ctx->h_pinned;
   TMC_CUDA(ctx, cudaMemcpyAsync(h, sc.totals, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
@@ -707,14 +761,9 @@ tmc_status dmc_extract(tmc_ctx* ctx, const tmc_volume* vol, double iso, uint32_t
     TMC_GET(vo.vuvw, 3 * nv);
   }
   TMC_GET(quads, 4 * nq);
-  ce = al.get(&colors, nq);
-  if (ce != cudaSuccess) {
-    delete mp;
-    TMC_CUDA(ctx, ce);
-  }
-  ce = al.get(&sc.vwork, nv);
-  if (ce == cudaSuccess) ce = al.get(&sc.vrank, nv);
-  if (ce == cudaSuccess) ce = dmc_vertex_scratch(al, sc, nv);
+  al.plan(&colors, nq);
+  plan_dmc_vertices(al, sc, nv);
+  ce = al.commit();
   if (ce != cudaSuccess) {
     delete mp;
     TMC_CUDA(ctx, ce);
@@ -792,10 +841,24 @@ tmc_status dmc_extract(tmc_ctx* ctx, const tmc_volume* vol, double iso, uint32_t
   TMC_CUDA(ctx, tmc::host_wait(st));
   for (int q = 0; q < 8; q++) out->stats[q] = (int64_t)h[q];
   ctx->prof.collect();
-  out->stats[4] = post.non_manifold;
+  out->stats[4] = post.non_manifold ? (int64_t)*post.non_manifold : 0;
   out->stats[6] = ncell;
 #undef TMC_GET
   return finish_mesh(ctx, flags, out, mp, &early);
+}
+
+// scratch of a TMC mesh's halfedge build (nv vertices, nh halfedges)
+void plan_tmc_halfedges(Allocs& al, tmc::HeWork& w, int32_t*& twin, uint8_t*& flag, int64_t nv, int64_t nh) {
+  al.plan(&w.deg, nv);
+  al.plan(&w.off, nv);
+  al.plan(&w.rank, nh);
+  al.plan(&w.list, nh);
+  al.plan(&w.hv_key, nv);
+  al.plan(&w.tiles, tmc::scan_tiles(nv) + 2);
+  al.plan(&w.total, 2);
+  al.plan(&w.non_manifold, 2);
+  al.plan(&twin, nh);
+  al.plan(&flag, nh);
 }
 
 // TMC extraction driver shared by the shared-vertex and halfedge entry points.
@@ -820,22 +883,13 @@ tmc_status tmc_extract(tmc_ctx* ctx, const tmc_volume* vol, double iso, uint32_t
   tmc::Grid g = make_grid(vol, field, iso);
   if (fg) set_fused(g, *fg, dev_params);
   g.flags = (flags & TMC_OUT_POS_F64) ? tmc::kGridPos64 : 0;
-  TMC_CUDA(ctx, al.get(&g.bits, g.bit_words() + 4));
   const int64_t ncell = g.ncells();
   tmc::TmcScratch sc{};
-  TMC_CUDA(ctx, al.get(&sc.rec, ncell));
-  TMC_CUDA(ctx, al.get(&sc.rv, ncell));
-  TMC_CUDA(ctx, al.get(&sc.toff, ncell));
-  TMC_CUDA(ctx, al.get(&sc.cellof, ncell));
-  TMC_CUDA(ctx, al.get(&sc.ccase, ncell));
+  al.plan(&g.bits, g.bit_words() + 4);
+  plan_tmc_cells(ctx, al, sc, ncell, tmc::ceil_div(ncell, tmc::kScanTile));
+  TMC_CUDA(ctx, al.commit());
   const tmc::CellSpace space = tmc::single_space(g);
-  TMC_CUDA(ctx, al.get(&sc.mask, tmc::tmc_tiles(space) * (tmc::kScanTile / 32)));
-  TMC_CUDA(ctx, al.get(&sc.tile_sums, tmc::tmc_tiles(space)));
-  TMC_CUDA(ctx, al.get(&sc.totals, 2));
-  TMC_CUDA(ctx, al.get(&sc.amb_n, 2));
-  TMC_CUDA(ctx, al.get(&sc.chunks, tmc::tmc_tiles(space) * (tmc::kScanTile / 32)));
-  sc.stats = ctx->d_stats;
-  TMC_CUDA(ctx, cudaMemsetAsync(sc.stats, 0, 8 * sizeof(unsigned long long), st));
+  TMC_CUDA(ctx, start_counters(ctx));
   ctx->launches += tmc::tmc_classify(space, sc, ctx->sms, st, &ctx->prof, gates.data(), (int)gates.size());
   unsigned long long* h = (unsigned long long*)ctx->h_pinned;
   int64_t n_amb = 0;
@@ -873,7 +927,7 @@ tmc_status tmc_extract(tmc_ctx* ctx, const tmc_volume* vol, double iso, uint32_t
   out->n = vo.n;
   out->v64 = vo.v64;
   out->tris = tris;
-  int64_t non_manifold = 0;
+  h[8] = 0;  // the halfedge build's count of non-manifold edges, when there is one
   EarlyCopies early{ctx, mp};
   if ((flags & TMC_OUT_HOST) && (flags & TMC_OUT_HALFEDGES)) {
     // the vertices and triangles are final: copy them out while the halfedges are built
@@ -893,16 +947,8 @@ tmc_status tmc_extract(tmc_ctx* ctx, const tmc_volume* vol, double iso, uint32_t
     int32_t *twin = nullptr, *he4 = nullptr, *hv = nullptr, *hf = nullptr;
     uint8_t* flag = nullptr;
     tmc::HeWork w{};
-    TMC_CUDA(ctx, al.get(&w.deg, nv));
-    TMC_CUDA(ctx, al.get(&w.off, nv));
-    TMC_CUDA(ctx, al.get(&w.rank, nh));
-    TMC_CUDA(ctx, al.get(&w.list, nh));
-    TMC_CUDA(ctx, al.get(&w.hv_key, nv));
-    TMC_CUDA(ctx, al.get(&w.tiles, tmc::scan_tiles(nv) + 2));
-    TMC_CUDA(ctx, al.get(&w.total, 2));
-    TMC_CUDA(ctx, al.get(&w.non_manifold, 2));
-    TMC_CUDA(ctx, al.get(&twin, nh));
-    TMC_CUDA(ctx, al.get(&flag, nh));
+    plan_tmc_halfedges(al, w, twin, flag, nv, nh);
+    TMC_CUDA(ctx, al.commit());
     TMC_CUDA(ctx, cudaMemsetAsync(w.non_manifold, 0, 2 * sizeof(unsigned long long), st));
     TMC_OWN(he4, 4 * nh);
     TMC_OWN(hv, nv);
@@ -913,8 +959,6 @@ tmc_status tmc_extract(tmc_ctx* ctx, const tmc_volume* vol, double iso, uint32_t
     ctx->launches += tmc::pack_halfedges4(tris, 3, twin, nh, he4, hf, ctx->sms, st);
     TMC_CUDA(ctx, cudaGetLastError());
     TMC_CUDA(ctx, cudaMemcpyAsync(h + 8, w.non_manifold, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-    TMC_CUDA(ctx, tmc::host_wait(st));
-    non_manifold = (int64_t)h[8];
     out->nr_he = nh;
     out->he = he4;
     out->he_v = hv;
@@ -925,9 +969,28 @@ tmc_status tmc_extract(tmc_ctx* ctx, const tmc_volume* vol, double iso, uint32_t
   TMC_CUDA(ctx, tmc::host_wait(st));
   for (int q = 0; q < 8; q++) out->stats[q] = (int64_t)h[q];
   ctx->prof.collect();
-  out->stats[4] = non_manifold;
+  out->stats[4] = (int64_t)h[8];
   out->stats[6] = ncell;
   return finish_mesh(ctx, flags, out, mp, &early);
+}
+
+// Batch tables on the device: each tile's volume, from the volumes' first tiles (tile0[nb]: the end).
+__global__ void tile_volume_kernel(const int64_t* tile0, int nb, int64_t tiles, int32_t* tile_vol) {
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= tiles) return;
+  int lo = 0, hi = nb - 1;  // the last volume whose first tile is at or before t
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) / 2;
+    if (tile0[mid] <= t) lo = mid;
+    else hi = mid - 1;
+  }
+  tile_vol[t] = lo;
+}
+// The scanned sums at the volumes' first tiles, then the totals (two words).
+__global__ void volume_offsets_kernel(const unsigned long long* tile_off, const int64_t* tile0, int nb,
+                                      const unsigned long long* totals, unsigned long long* out) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q < nb + 2) out[q] = q < nb ? tile_off[tile0[q]] : totals[q - nb];
 }
 
 // One batch of requests of one algorithm: all volumes share one cell space, so every stage is one
@@ -981,9 +1044,6 @@ tmc_status batch_run(tmc_ctx* ctx, const std::vector<int>& idx, const tmc_reques
   const int64_t ncell = tiles * tmc::kScanTile;
   if (ncell > ((int64_t)1 << 32) - tmc::kScanTile)
     return fail(ctx, TMC_ERR_CAPACITY, "batch of %lld cells: a batch holds at most 2^32 cells", (long long)ncell);
-  std::vector<int32_t> tile_vol((size_t)tiles);
-  for (int q = 0; q < nb; q++)
-    for (int64_t t = tile0[q]; t < tile0[q + 1]; t++) tile_vol[(size_t)t] = q;
   // the volumes' bit rows one after another
   int64_t bit_words = 0, max_bit_words = 0;
   for (const tmc::Grid& g : grids) {
@@ -991,17 +1051,40 @@ tmc_status batch_run(tmc_ctx* ctx, const std::vector<int>& idx, const tmc_reques
     max_bit_words = std::max(max_bit_words, g.bit_words());
   }
   uint32_t* bits = nullptr;
-  TMC_CUDA(ctx, al.get(&bits, bit_words + 4));
+  tmc::DmcScratch dsc{};
+  tmc::TmcScratch tsc{};
+  tmc::Grid* d_grids = nullptr;
+  int64_t* d_tile0 = nullptr;  // the volumes' first tiles, and the end
+  int32_t* d_tile_vol = nullptr;
+  unsigned long long* d_voff = nullptr;  // the scanned sums at the volumes' first tiles, and the totals
+  al.plan(&bits, bit_words + 4);
+  al.plan(&d_grids, nb);
+  al.plan(&d_tile0, nb + 1);
+  al.plan(&d_voff, nb + 2);
+  al.plan(&d_tile_vol, tiles);
+  if (dmc) plan_dmc_cells(ctx, al, dsc, ncell, tiles);
+  else plan_tmc_cells(ctx, al, tsc, ncell, tiles);
+  TMC_CUDA(ctx, al.commit());
   for (tmc::Grid& g : grids) {
     g.bits = bits;
     bits += g.bit_words();
   }
-  tmc::Grid* d_grids = nullptr;
-  int32_t* d_tile_vol = nullptr;
-  TMC_CUDA(ctx, al.get(&d_grids, nb));
-  TMC_CUDA(ctx, al.get(&d_tile_vol, tiles));
-  TMC_CUDA(ctx, cudaMemcpyAsync(d_grids, grids.data(), nb * sizeof(tmc::Grid), cudaMemcpyHostToDevice, st));
-  TMC_CUDA(ctx, cudaMemcpyAsync(d_tile_vol, tile_vol.data(), tiles * sizeof(int32_t), cudaMemcpyHostToDevice, st));
+  // the tables through pinned memory when they fit (a pageable copy blocks, and the volume offsets that
+  // come back do too)
+  const size_t grid_bytes = nb * sizeof(tmc::Grid), tile0_bytes = (nb + 1) * sizeof(int64_t);
+  char* staging = (char*)ctx->h_pinned + kPinnedTables;
+  const bool staged = grid_bytes + 2 * tile0_bytes + 64 <= kPinnedBytes - kPinnedTables;
+  const void *grid_src = grids.data(), *tile0_src = tile0.data();
+  if (staged) {
+    std::memcpy(staging, grids.data(), grid_bytes);
+    std::memcpy(staging + grid_bytes, tile0.data(), tile0_bytes);
+    grid_src = staging;
+    tile0_src = staging + grid_bytes;
+  }
+  TMC_CUDA(ctx, cudaMemcpyAsync(d_grids, grid_src, grid_bytes, cudaMemcpyHostToDevice, st));
+  TMC_CUDA(ctx, cudaMemcpyAsync(d_tile0, tile0_src, tile0_bytes, cudaMemcpyHostToDevice, st));
+  tile_volume_kernel<<<(unsigned)tmc::ceil_div(tiles, 256), 256, 0, st>>>(d_tile0, nb, tiles, d_tile_vol);
+  ctx->launches += 1;
   tmc::CellSpace space{};
   space.one = grids[0];
   space.grids = d_grids;
@@ -1011,54 +1094,33 @@ tmc_status batch_run(tmc_ctx* ctx, const std::vector<int>& idx, const tmc_reques
   space.n = ncell;
 
   // ---- count ----
-  uint32_t* rec = nullptr;
-  int32_t* qoff = nullptr;
-  unsigned long long *tile_sums = nullptr, *totals = nullptr;
-  tmc::CellMask* mask = nullptr;
-  uint16_t* cellof = nullptr;
-  TMC_CUDA(ctx, al.get(&rec, ncell));
-  TMC_CUDA(ctx, al.get(&qoff, ncell));
-  TMC_CUDA(ctx, al.get(&cellof, ncell));
-  TMC_CUDA(ctx, al.get(&mask, tiles * (tmc::kScanTile / 32)));
-  TMC_CUDA(ctx, al.get(&tile_sums, tiles));
-  TMC_CUDA(ctx, al.get(&totals, 2));
-  TMC_CUDA(ctx, cudaMemsetAsync(ctx->d_stats, 0, 8 * sizeof(unsigned long long), st));
-  tmc::DmcScratch dsc{};
-  tmc::TmcScratch tsc{};
+  TMC_CUDA(ctx, start_counters(ctx));
   int64_t n_amb_rec = 0;
   if (dmc) {
-    dsc = tmc::DmcScratch{rec, nullptr, qoff, nullptr, tile_sums, totals, ctx->d_stats};
-    dsc.mask = mask;
-    dsc.cellof = cellof;
-    TMC_CUDA(ctx, al.get(&dsc.rv, ncell));
-    TMC_CUDA(ctx, al.get(&dsc.chunks, tiles * (tmc::kScanTile / 32)));
-    TMC_CUDA(ctx, al.get(&dsc.amb_n, 2));
-    TMC_CUDA(ctx, al.get(&dsc.ccase, ncell));
     ctx->launches += tmc::dmc_front_count(space, dsc, ctx->sms, st, &ctx->prof);
   } else {
-    tsc = tmc::TmcScratch{rec, nullptr, qoff, tile_sums, totals, ctx->d_stats};
-    tsc.mask = mask;
-    tsc.cellof = cellof;
-    TMC_CUDA(ctx, al.get(&tsc.rv, ncell));
-    TMC_CUDA(ctx, al.get(&tsc.ccase, ncell));
-    TMC_CUDA(ctx, al.get(&tsc.chunks, tiles * (tmc::kScanTile / 32)));
-    TMC_CUDA(ctx, al.get(&tsc.amb_n, 2));
     ctx->launches += tmc::tmc_classify(space, tsc, ctx->sms, st, &ctx->prof);
     TMC_CUDA(ctx, tmc_ambiguous_records(ctx, al, tsc, n_amb_rec));
     ctx->launches += tmc::tmc_count(space, tsc, n_amb_rec, ctx->sms, st, &ctx->prof);
   }
-  std::vector<unsigned long long> toff((size_t)tiles + 1);
+  volume_offsets_kernel<<<(unsigned)tmc::ceil_div(nb + 2, 256), 256, 0, st>>>(
+      dmc ? dsc.tile_sums : tsc.tile_sums, d_tile0, nb, ctx->d_stats + kStatTotals, d_voff);
+  ctx->launches += 1;
+  std::vector<unsigned long long> voff_pageable(staged ? 0 : (size_t)nb + 2);
+  unsigned long long* toff =
+      staged ? reinterpret_cast<unsigned long long*>(staging + ((grid_bytes + tile0_bytes + 15) & ~(size_t)15))
+             : voff_pageable.data();
   unsigned long long* h = (unsigned long long*)ctx->h_pinned;
-  TMC_CUDA(ctx, cudaMemcpyAsync(toff.data(), tile_sums, tiles * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-  TMC_CUDA(ctx, cudaMemcpyAsync(h, totals, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+  TMC_CUDA(ctx, cudaMemcpyAsync(toff, d_voff, (nb + 2) * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
   TMC_CUDA(ctx, tmc::host_wait(st));
-  toff[(size_t)tiles] = h[0];
+  h[0] = toff[nb];
+  h[1] = toff[nb + 1];
   const int64_t NV = (int64_t)(h[0] >> 32), NF = (int64_t)(h[0] & 0xffffffffull);
   if (NV >= ((int64_t)1 << 31) || NF >= ((int64_t)1 << 31))
     return fail(ctx, TMC_ERR_CAPACITY, "batch output above 2^31 vertices or faces; split the batch");
   std::vector<int64_t> vb(nb + 1), fb(nb + 1);
   for (int q = 0; q <= nb; q++) {
-    const unsigned long long w = toff[(size_t)tile0[q]];
+    const unsigned long long w = toff[q];
     vb[q] = (int64_t)(w >> 32);
     fb[q] = (int64_t)(w & 0xffffffffull);
   }
@@ -1091,9 +1153,8 @@ tmc_status batch_run(tmc_ctx* ctx, const std::vector<int>& idx, const tmc_reques
     }
     TMC_CUDA(ctx, get_shared(&faces, 4 * NF));
     TMC_CUDA(ctx, get_shared(&colors, NF));
-    TMC_CUDA(ctx, al.get(&dsc.vwork, NV));
-    TMC_CUDA(ctx, al.get(&dsc.vrank, NV));
-    TMC_CUDA(ctx, dmc_vertex_scratch(al, dsc, NV));
+    plan_dmc_vertices(al, dsc, NV);
+    TMC_CUDA(ctx, al.commit());
     tmc::DmcVertexOut vo{v, nn, v64, n64, vcell, vuvw};
     ctx->launches += tmc::dmc_front_emit(space, dsc, vo, NV, faces, colors, 0, ctx->tune, st, &ctx->prof);
   } else {
@@ -1155,7 +1216,10 @@ tmc_status batch_run(tmc_ctx* ctx, const std::vector<int>& idx, const tmc_reques
         out->vcell = vcell + vb[q];
         out->vuvw = vuvw + 3 * vb[q];
       }
-      out->stats[4] = post.non_manifold;
+      if (post.non_manifold) {  // staged by the post-processing; the next mesh's uses the same words
+        TMC_CUDA(ctx, tmc::host_wait(st));
+        out->stats[4] = (int64_t)*post.non_manifold;
+      }
       // float64 arrays the post-processing made that are not outputs
       auto drop = [&](void* ptr) {
         if (!ptr) return;
@@ -1183,16 +1247,8 @@ tmc_status batch_run(tmc_ctx* ctx, const std::vector<int>& idx, const tmc_reques
         int32_t *twin = nullptr, *he4 = nullptr, *hv = nullptr, *hf = nullptr;
         uint8_t* flag = nullptr;
         tmc::HeWork w{};
-        TMC_CUDA(ctx, al.get(&w.deg, nv));
-        TMC_CUDA(ctx, al.get(&w.off, nv));
-        TMC_CUDA(ctx, al.get(&w.rank, nh));
-        TMC_CUDA(ctx, al.get(&w.list, nh));
-        TMC_CUDA(ctx, al.get(&w.hv_key, nv));
-        TMC_CUDA(ctx, al.get(&w.tiles, tmc::scan_tiles(nv) + 2));
-        TMC_CUDA(ctx, al.get(&w.total, 2));
-        TMC_CUDA(ctx, al.get(&w.non_manifold, 2));
-        TMC_CUDA(ctx, al.get(&twin, nh));
-        TMC_CUDA(ctx, al.get(&flag, nh));
+        plan_tmc_halfedges(al, w, twin, flag, nv, nh);
+        TMC_CUDA(ctx, al.commit());
         TMC_CUDA(ctx, cudaMemsetAsync(w.non_manifold, 0, 2 * sizeof(unsigned long long), st));
         TMC_CUDA(ctx, al.get(&he4, 4 * nh));
         al.release(he4);

@@ -1559,7 +1559,6 @@ int tmc_classify(const CellSpace& space, TmcScratch& s, int sms, cudaStream_t st
   int k = 0;
   {
     Stage t(prof, "tmc_classify", st);
-    cudaMemsetAsync(s.amb_n, 0, 2 * sizeof(unsigned), st);  // and the chunk counter behind it
     auto classify = [&](int64_t t0, int64_t t1, int z0, int z1) {
       k += launch_point_bits(space, z0, z1, sms, st);
       if (t1 <= t0) return;
@@ -1593,7 +1592,6 @@ int tmc_count(const CellSpace& space, TmcScratch& s, int64_t n_amb, int sms, cud
     Stage ta(prof, "tmc_amb_count", st);
     // the list sorted by MC case (the records follow its order, so the emission pass is sorted too)
     const unsigned gs = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n_amb, 256), (int64_t)sms * 8));
-    cudaMemsetAsync(s.amb_hist, 0, 514 * sizeof(unsigned), st);
     tmc_amb_key_kernel<<<gs, 256, 0, st>>>(space, s.cellof, amb_cells, n_amb, s.amb_key, s.amb_hist);
     tmc_amb_cursor_kernel<<<1, 256, 0, st>>>(s.amb_hist, s.amb_hist + 256);
     tmc_amb_sort_kernel<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n_amb, kSortTile), (int64_t)sms * 8)),

@@ -38,6 +38,7 @@ struct TmcScratch {
   uint32_t* chunks;     // kScanTile / 32 per tile: the chunk list (scan.cuh)
 };
 
+// The counters (stats, totals, amb_n, amb_hist) are zero when a call starts.
 // Per-cell scratch is indexed in the cell space; triangles hold vertex indices within their own
 // volume, and the volumes' vertices and triangles follow one another in the outputs.
 int64_t tmc_tiles(const CellSpace& space);
