@@ -1,6 +1,6 @@
 // CPU check of repr::vertex_point (tmc_gb300/csrc/dmc_repr.cuh): every contour it answers must get the
 // floats of the float64 restatement of the reference.  Built with nvcc as host code.
-//   point_check field.raw nx ny nz iso  -> prints "contours mismatches redone w64 excluded"
+//   point_check field.raw nx ny nz iso  -> prints "contours mismatches redone w64 excluded searched"
 #include <cstdio>
 #include <cstdlib>
 #include <vector>
@@ -33,7 +33,7 @@ int main(int argc, char** argv) {
   fclose(in);
   float iso_up = (float)iso;
   if ((double)iso_up < iso) iso_up = nextafterf(iso_up, INFINITY);
-  long contours = 0, mism = 0, redone = 0, w64 = 0, excluded = 0;
+  long contours = 0, mism = 0, redone = 0, w64 = 0, excluded = 0, searched = 0;
   for (int k = 0; k < nz - 1; k++)
     for (int j = 0; j < ny - 1; j++)
       for (int i = 0; i < nx - 1; i++) {
@@ -68,11 +68,55 @@ int main(int argc, char** argv) {
           const int sz = cnt_size(c, t);
           bool excl = false;
           for (int q = 0; q < n; q++) excl = excl || (sz != 3 && q != t && cnt_size(c, q) == 3);
+          const uint32_t em = repr::edges_of_rank(map, t, crossed);
+          // the whole search, as dmc_vertex_search_kernel runs it
+          {
+            float frame[repr::kFrameFloats];
+            for (int q = 0; q < 8; q++) frame[q] = u[q];
+            const repr::FrameCol F{frame, 1};
+            const ffx::ff iso_ff = ffx::ff_from_double(iso);
+            const bool exact_iso = (double)(float)iso == iso;
+            repr::Exclusion X;
+            bool ok = true;
+            if (sz != 3)
+              for (int q = 0; q < n; q++) {
+                if (q == t || cnt_size(c, q) != 3) continue;
+                ok = repr::contour_box(F, repr::edges_of_rank(map, q, crossed), iso, iso_ff, exact_iso, X.lo[X.n], X.hi[X.n]) && ok;
+                for (int d = 0; d < 3; d++)
+                  if (ok && (X.lo[X.n][d] != bx.b[q][d][0] || X.hi[X.n][d] != bx.b[q][d][1])) mism++;
+                X.n++;
+              }
+            ffx::ff mean[3];
+            auto mean64 = [&]() { return repr::mean_point_exact(pts[t], sz); };
+            const int prj = ok ? repr::vertex_frame<true>(F, em, sz, iso, iso_ff, exact_iso, mean, mean64) : -1;
+            if (prj >= 0) {
+              const int ax[3][3] = {{0, 1, 2}, {0, 2, 1}, {1, 2, 0}};
+              repr::Exclusion Y = X;
+              for (int b = 0; b < X.n; b++)
+                for (int d = 0; d < 3; d++) {
+                  Y.lo[b][d] = X.lo[b][ax[prj][d]];
+                  Y.hi[b][d] = X.hi[b][ax[prj][d]];
+                }
+              float p[3] = {0, 0, 0};
+              int f64 = 0;
+              const int what = repr::search_all(F, prj, mean, Y, iso, iso_ff, mean64, p, f64);
+              const repr::Point64 pm = repr::mean_point_exact(pts[t], sz);
+              double pe[3] = {pm.p[0], pm.p[1], pm.p[2]};
+              repr::Stats st;
+              repr::representative_exact(u, iso, c, t, pe, bx, st);
+              // not found exactly where the reference goes on to its 26x26 retry
+              if ((what == repr::kRedo) != (st.fail1 != 0) ||
+                  (what == repr::kFound && (pe[0] != (double)p[0] || pe[1] != (double)p[1] || pe[2] != (double)p[2]))) {
+                if (mism < 5) fprintf(stderr, "search: cell %d %d %d t %d (size %d, %d)\n", i, j, k, t, sz, what);
+                mism++;
+              }
+              searched++;
+            }
+          }
           if (excl) {
             excluded++;
             continue;
           }
-          const uint32_t em = repr::edges_of_rank(map, t, crossed);
           float p[3] = {0, 0, 0};
           int prj = 0;
           float frame[repr::kFrameFloats];
@@ -98,6 +142,6 @@ int main(int argc, char** argv) {
           }
         }
       }
-  printf("%ld %ld %ld %ld %ld\n", contours, mism, redone, w64, excluded);
+  printf("%ld %ld %ld %ld %ld %ld\n", contours, mism, redone, w64, excluded, searched);
   return 0;
 }

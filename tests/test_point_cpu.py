@@ -63,8 +63,9 @@ def test_vertex_point_matches_the_reference_arithmetic(checker, tmp_path, name):
     nz, ny, nx = data.shape
     r = subprocess.run([str(checker), str(f), str(nx), str(ny), str(nz), repr(iso)], capture_output=True, text=True,
                        check=True)
-    contours, mism, redone, w64, excluded = (int(x) for x in r.stdout.split())
+    contours, mism, redone, w64, excluded, searched = (int(x) for x in r.stdout.split())
     assert contours > 0
     assert mism == 0, r.stderr
     if name in ("noise", "noise_iso", "blobs", "periodic"):
-        assert redone < 0.02 * contours  # generic fields: the one-pass kernels get the rest
+        assert redone < 0.02 * contours  # generic fields: the rest takes the whole search
+        assert searched == contours

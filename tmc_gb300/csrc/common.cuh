@@ -360,7 +360,7 @@ struct Tuning {
     Tuning t;
     t.sms = sms;
     t.group_lanes = (int64_t)sms * 24 * 32;
-    t.warp_list_max = (int64_t)sms * 32;
+    t.warp_list_max = (int64_t)sms * 128;
     return t;
   }
 };

@@ -25,11 +25,13 @@ struct DmcScratch {
   unsigned long long* tile_sums;  // per scan tile
   unsigned long long* totals;     // [0] = (vertices << 32) | quads
   unsigned long long* stats;      // 8 counters
-  // per vertex: the projected points, the one-pass list, the points that lack a coordinate
+  // per vertex: the projected points, those that take the whole search, those that lack a coordinate,
+  // those left to the one-pass kernels
   float4* vp;
   uint32_t* fb_list;
   uint32_t* w_list;
-  unsigned* fb_count;             // entries of [0] fb_list, [1] tail_list, [2] w_list
+  uint32_t* hard_list;
+  unsigned* fb_count;             // entries of [0] fb_list, [1] tail_list, [2] w_list, [3] hard_list
   uint32_t* tail_list;            // vertices without a valid 7x7 sample (26x26 retry)
   // listed cells (common.cuh): rec, rv and qoff hold one entry per listed cell at its slot
   CellMask* mask;                 // per 32 cells of the space

@@ -18,6 +18,7 @@
 //   dmc_vertex_point_kernel, dmc_vertex_w_kernel, dmc_vertex_finish_kernel
 //                        vertex representatives (cpp_dmc representative/projection) in float32
 //                        and float-float, normals, positions
+//   dmc_vertex_search_kernel  the vertices that take the whole 7x7 search
 //   dmc_vertex_kernel    the vertices those leave, with every float64 fallback
 //   dmc_vertex_warp_kernel  the reference's 26x26 retry (and short lists whole), one warp per vertex
 //   dmc_quad_kernel      each cell emits the quads of its crossed interior edges 0, 3, 8 by
@@ -502,8 +503,8 @@ __device__ __forceinline__ void flush_stats(const repr::Stats& st, unsigned long
   if (st.fallback + st.normal_f64) atomicAdd(stats + 7, (unsigned long long)(st.fallback + st.normal_f64));
 }
 
-// One-pass vertex kernel over the vertices the two-pass kernels list (neighbour-contour exclusion,
-// a distance that needs float64): the 7x7 projection with every float64 fallback.  Contours
+// One-pass vertex kernel over the vertices that dmc_vertex_search_kernel leaves: the 7x7 projection with
+// every float64 fallback.  Contours
 // without a valid 7x7 sample go on to the tail list (the reference's 26x26 retry, one warp each).
 // A list of at most `warp_max` entries is left whole to the warp kernel: one thread's serial
 // projection (~0.1 ms) would set the latency of a small call.
@@ -820,6 +821,189 @@ __global__ void __launch_bounds__(kVertexThreads) dmc_vertex_w_kernel(CellSpace 
   if (blockIdx.x == 0 && threadIdx.x == 0 && n) atomicAdd(stats + 7, 3ull * n);
 }
 
+// The reference's float64 mean point of the contour with edge set em (n edges): its edge points summed in
+// the polygon's order.  Rare, out of line.
+__device__ __noinline__ repr::Point64 contour_mean_f64(const Grid& g, int i, int j, int k, unsigned cs, uint32_t em,
+                                                       int n) {
+  float u[8];
+  load_corners(g, i, j, k, u);
+  const uint64_t c = dmc_polygon(cs, u, g.iso, c_case_contour);
+  int at = 0;  // where the contour begins in the word
+  for (int t = 0; t < cnt_count(c) && !((em >> (2 * cnt_edge(c, at))) & 1); t++) at += cnt_size(c, t);
+  repr::Point64 r{{0, 0, 0}};
+  for (int q = 0; q < n; q++) {
+    float p[3];
+    const int e = cnt_edge(c, at + q);
+    repr::local_from_param(e, repr::edge_param_exact(e, u, g.iso), p);
+    for (int d = 0; d < 3; d++) r.p[d] += p[d];
+  }
+  for (int d = 0; d < 3; d++) r.p[d] /= n;
+  return r;
+}
+
+// The listed vertices that take the whole search: several samples as near as one another (exact ties of
+// symmetric contours), contours beside one that excludes samples, no sample surely valid.  The edge
+// sets, frame and bounds are the point kernel's; samples are evaluated exactly, in float64 where a
+// rounding is not certified.  What is left (no valid sample at 7x7, values at the ends of the float
+// range) goes to the one-pass kernels' list, which is empty on most fields.
+//
+// A list of more than `warp_max` entries takes one thread per vertex (bounds first, then the few
+// candidates); a shorter one takes a warp per vertex, the lanes splitting the 49 samples, because one
+// thread's search of a contour whose samples all tie lasts as long as the rest of a small call (85 us;
+// a warp's 14 us; lists of 19,000 take about as long either way).  Before, all of them took the one-pass
+// kernels (64^3 blobs 24 us, 512^3 noise 0.67 ms, 1024x1024x64 saddles 3.3 ms); now 14 us, 0.35 and
+// 0.96 ms, and the one-pass kernels get what is left (0.05 and 0.14 ms).
+// the edge sets of a cell whose record does not tell its contours apart (some unused): the contour of
+// vertex `rank`, and the other contours of three edges
+struct ContourSets {
+  uint32_t own, others[3];
+  int n_others;
+};
+__device__ __noinline__ ContourSets contour_sets(const Grid& g, int i, int j, int k, unsigned cs, int rank) {
+  float u[8];
+  load_corners(g, i, j, k, u);
+  const uint64_t c = dmc_polygon(cs, u, g.iso, c_case_contour);
+  ContourSets S{0, {0, 0, 0}, 0};
+  int flat = 0, seen = 0;
+  for (int t = 0; t < cnt_count(c); t++) {
+    const int sz = cnt_size(c, t);
+    uint32_t m = 0;
+    bool used = false;
+    for (int q = 0; q < sz; q++) {
+      const int e = cnt_edge(c, flat + q);
+      m |= 1u << (2 * e);
+      used = used || edge_interior(g, i, j, k, e);
+    }
+    if (used && seen++ == rank) S.own = m;
+    else if (sz == 3 && S.n_others < 3) S.others[S.n_others++] = m;
+    flat += sz;
+  }
+  return S;
+}
+__device__ __forceinline__ int vertex_search_frame(const Grid& g, const repr::FrameCol& F, uint32_t r, int rank,
+                                                   unsigned cs, int i, int j, int k, ffx::ff mean[3],
+                                                   repr::Exclusion& X, uint32_t& em, int& n) {
+  float c[8];
+  load_corners(g, i, j, k, c);
+#pragma unroll
+  for (int q = 0; q < 8; q++) F[q] = c[q];
+  ContourSets S{0, {0, 0, 0}, 0};
+  if (rec_unused(r)) {
+    S = contour_sets(g, i, j, k, cs, rank);
+  } else {
+    const uint32_t crossed = d_case_edges.m[cs];
+    S.own = repr::edges_of_rank(rec_map(r), rank, crossed);
+    for (int t = 0; t < rec_nv(r); t++) {
+      const uint32_t m = repr::edges_of_rank(rec_map(r), t, crossed);
+      if (t != rank && __popc(m) == 3 && S.n_others < 3) S.others[S.n_others++] = m;
+    }
+  }
+  em = S.own;
+  n = __popc(em);
+  const ffx::ff iso{g.iso_f, g.iso_lo};
+  // the boxes of the other contours of three edges
+  bool ok = true;
+  if (n != 3)
+    for (; X.n < S.n_others; X.n++)
+      ok = repr::contour_box(F, S.others[X.n], g.iso, iso, g.iso_exact, X.lo[X.n], X.hi[X.n]) && ok;
+  if (!ok) return -1;
+  const uint32_t own = em;
+  const int edges = n;
+  auto mean64 = [&g, i, j, k, cs, own, edges]() { return contour_mean_f64(g, i, j, k, cs, own, edges); };
+  const int prj = repr::vertex_frame<true>(F, em, n, g.iso, iso, g.iso_exact, mean, mean64);
+  if (prj > 0)  // the boxes in the frame's axes: (x, z, y) or (y, z, x)
+    for (int t = 0; t < X.n; t++) {
+      const float l0 = X.lo[t][0], h0 = X.hi[t][0], l1 = X.lo[t][1], h1 = X.hi[t][1];
+      X.lo[t][0] = prj == 1 ? l0 : l1;
+      X.hi[t][0] = prj == 1 ? h0 : h1;
+      X.lo[t][1] = X.lo[t][2];
+      X.hi[t][1] = X.hi[t][2];
+      X.lo[t][2] = prj == 1 ? l1 : l0;
+      X.hi[t][2] = prj == 1 ? h1 : h0;
+    }
+  return prj;
+}
+__global__ void __launch_bounds__(kVertexThreads) dmc_vertex_search_kernel(CellSpace space, const uint16_t* cellof,
+                                                                           const uint8_t* ccase, const uint32_t* rec,
+                                                                           const uint8_t* vrank, const uint32_t* vwork,
+                                                                           const uint32_t* list, unsigned* count,
+                                                                           unsigned warp_max, float4* vp, uint32_t* hard,
+                                                                           unsigned long long* stats) {
+  constexpr unsigned kAll = 0xffffffffu;
+  __shared__ float frames[repr::kFrameFloats * kVertexThreads];
+  const repr::FrameCol F{frames + threadIdx.x, kVertexThreads};
+  const unsigned total = count[0];
+  const bool warp = total <= warp_max;  // the lanes of a warp share a vertex
+  const int lane = threadIdx.x & 31;
+  int f64 = 0;
+  const unsigned tid = blockIdx.x * blockDim.x + threadIdx.x, threads = gridDim.x * blockDim.x;
+  for (unsigned a = warp ? tid >> 5 : tid; a < total; a += warp ? threads >> 5 : threads) {
+    const uint32_t vidx = list[a];
+    const uint32_t slot = vwork[vidx];
+    const uint32_t r = rec[slot];
+    const unsigned cs = __ldg(ccase + slot);
+    const uint32_t vcell = slot_cell(cellof, slot);
+    const Grid& g = space.grids ? space.grids[__ldg(space.tile_vol + vcell / kScanTile)] : space.one;
+    int i, j, k;
+    cell_ijk(g, vcell - g.vbase, i, j, k);
+    ffx::ff mean[3];
+    repr::Exclusion X;
+    uint32_t em;
+    int n;
+    const int prj = vertex_search_frame(g, F, r, vrank[vidx], cs, i, j, k, mean, X, em, n);
+    const ffx::ff iso{g.iso_f, g.iso_lo};
+    auto mean64 = [&]() { return contour_mean_f64(g, i, j, k, cs, em, n); };
+    float p[3] = {0, 0, 0};
+    int what = repr::kRedo;
+    if (warp) {
+      // each lane two of the 49 samples; the winner by distance, then loop order
+      repr::LaneBest b = repr::lane_none();
+      if (prj >= 0) {  // warp-uniform
+        repr::ExactSample s[2];
+        float u[2], v[2];
+        bool open = false;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const int q = lane + 32 * h;
+          s[h].state = 0;
+          if (q < 49) {
+            u[h] = repr::sample_coord_any(F[repr::kUlo], F[repr::kUhi], q / 7 + 1);
+            v[h] = repr::sample_coord_any(F[repr::kVlo], F[repr::kVhi], q - 7 * (q / 7) + 1);
+            s[h] = repr::exact_sample(F, u[h], v[h], mean, X, g.iso, iso, f64);
+            open = open || s[h].state == 2;
+          }
+        }
+        if (__any_sync(kAll, open)) {
+          const repr::Point64 pm = mean64();
+#pragma unroll
+          for (int h = 0; h < 2; h++)
+            if (s[h].state == 2) {
+              s[h].d = repr::distance_f64(pm, prj, u[h], v[h], s[h].w);
+              f64++;
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const repr::LaneBest x{s[h].d, s[h].w, lane + 32 * h};
+          if (s[h].state != 0 && repr::lane_better(x, b)) b = x;
+        }
+        b = warp_best(b);
+        if (b.q != repr::kNoSample) {
+          what = repr::kFound;
+          repr::frame_point(prj, repr::sample_coord_any(F[repr::kUlo], F[repr::kUhi], b.q / 7 + 1),
+                            repr::sample_coord_any(F[repr::kVlo], F[repr::kVhi], b.q - 7 * (b.q / 7) + 1), b.w, p);
+        }
+      }
+      if (lane != 0) continue;
+    } else if (prj >= 0) {
+      what = repr::search_all(F, prj, mean, X, g.iso, iso, mean64, p, f64);
+    }
+    if (what == repr::kFound) vp[vidx] = make_float4(p[0], p[1], p[2], 0.0f);
+    append(hard, count + 3, what != repr::kFound, vidx);
+  }
+  if (f64) atomicAdd(stats + 7, (unsigned long long)f64);
+}
+
 // Positions, normals and local coordinates of the projected vertices.
 template <bool kBatch, bool kFF>
 __global__ void __launch_bounds__(kVertexThreads) dmc_vertex_finish_kernel(CellSpace space, const uint16_t* cellof,
@@ -1005,7 +1189,12 @@ int dmc_front_emit(const CellSpace& space, DmcScratch& s, DmcVertexOut vo, int64
     else
       dmc_vertex_point_kernel<false><<<vgrid(r_point), kVertexThreads, 0, st>>>(
           space, s.cellof, s.ccase, s.rec, s.vrank, s.vwork, nv, s.vp, s.fb_list, s.w_list, s.fb_count);
-    // the list's length is only known on the device: one wave, sized for a tenth of the vertices
+    // the lists' lengths are only known on the device: one wave, sized for a tenth of the vertices
+    // (the search takes a warp per vertex when few are listed, so as many warps as vertices may use)
+    static const int r_search = resident_blocks(dmc_vertex_search_kernel, kVertexThreads);
+    dmc_vertex_search_kernel<<<(unsigned)wave_grid(r_search, sms, 1, nv, kVertexThreads), kVertexThreads, 0, st>>>(
+        space, s.cellof, s.ccase, s.rec, s.vrank, s.vwork, s.fb_list, s.fb_count,
+        (unsigned)std::min<int64_t>(tu.warp_list_max, 0x7fffffff), s.vp, s.hard_list, s.stats);
     dmc_vertex_w_kernel<<<(unsigned)wave_grid(r_w, sms, 1, ceil_div(nv, 10), kVertexThreads), kVertexThreads, 0, st>>>(
         space, s.cellof, s.vwork, s.w_list, s.fb_count, s.vp, s.stats);
   }
@@ -1032,10 +1221,10 @@ int dmc_front_emit(const CellSpace& space, DmcScratch& s, DmcVertexOut vo, int64
     const unsigned warp_max = (unsigned)std::min<int64_t>(tu.warp_list_max, 0x7fffffff);
     static const int r_vertex = resident_blocks(dmc_vertex_kernel, kVertexThreads);
     const unsigned fb = (unsigned)wave_grid(r_vertex, sms, 8, nv, kVertexThreads);
-    dmc_vertex_kernel<<<fb, kVertexThreads, 0, st>>>(space, s.cellof, s.vrank, s.vwork, s.fb_list, s.fb_count, s.tail_list,
+    dmc_vertex_kernel<<<fb, kVertexThreads, 0, st>>>(space, s.cellof, s.vrank, s.vwork, s.hard_list, s.fb_count + 3, s.tail_list,
                                                       s.fb_count + 1, warp_max, vo, flip, s.stats);
     dmc_vertex_warp_kernel<<<(unsigned)std::max(1, sms * 3), kVertexThreads, 0, st>>>(
-        space, s.cellof, s.vrank, s.vwork, s.fb_list, s.fb_count, s.tail_list, s.fb_count + 1, warp_max, vo, flip,
+        space, s.cellof, s.vrank, s.vwork, s.hard_list, s.fb_count + 3, s.tail_list, s.fb_count + 1, warp_max, vo, flip,
         s.stats);
   }
   Stage t(prof, "dmc_quad", st);
@@ -1047,7 +1236,7 @@ int dmc_front_emit(const CellSpace& space, DmcScratch& s, DmcVertexOut vo, int64
   if (space.grids) DMC_QUADS(true, r_quad_batch);
   else DMC_QUADS(false, r_quad);
 #undef DMC_QUADS
-  return 7;
+  return 8;
 }
 
 }  // namespace tmc

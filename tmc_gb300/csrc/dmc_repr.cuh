@@ -1063,6 +1063,11 @@ TMC_HD bool bilinear_certain(float f0, float f1, float f2, float f3, float sabs,
   return sabs > 0x1p-80f && ffx::ff_certain(G, sabs * 0x1p-43f);
 }
 
+// the same wherever the ends lie: float64 outside the exact range
+TMC_HD float sample_coord_any(float lo, float hi, int i) {
+  return sample_range_exact(lo, hi) ? sample_at(lo, hi, i) : sample_coord_f64(lo, hi, i);
+}
+
 // One contour's search, as the lanes of a warp share it: the projection frame (corners permuted so
 // that the plane's axes come first), the box and the mean point in it.  Kept as a column of floats
 // (shared memory on the GPU, one column per lane) so that any lane can estimate any lane's samples.
@@ -1075,8 +1080,16 @@ struct FrameCol {
 
 // The frame of the contour with edge set `em` (n edges) of the cell whose corners are the first
 // eight floats of the column; returns its projection plane, or -1 when the one-pass kernels must
-// decide.
-TMC_HD int vertex_frame(const FrameCol& F, uint32_t em, int n, double iso, ff iso_ff, bool exact_iso) {
+// decide.  kFull (the whole search): planes and sample coordinates that float pairs do not decide are
+// taken in float64 (mean64: the reference's float64 mean point; sample_coord_any), so that only values
+// at the ends of the float range are refused; mean: the mean point in the frame's axes, within 2^-44 of
+// the reference's.
+struct NoMean64 {
+  TMC_HD Point64 operator()() const { return Point64{{0, 0, 0}}; }
+};
+template <bool kFull = false, typename Mean64 = NoMean64>
+TMC_HD int vertex_frame(const FrameCol& F, uint32_t em, int n, double iso, ff iso_ff, bool exact_iso,
+                        ff* mean = nullptr, const Mean64& mean64 = Mean64()) {
   // edge parameters: sums and extremes per axis
   float sh[3] = {0, 0, 0}, sl[3] = {0, 0, 0}, mn[3] = {1, 1, 1}, mx[3] = {0, 0, 0};
   bool ok = true;
@@ -1116,8 +1129,23 @@ TMC_HD int vertex_frame(const FrameCol& F, uint32_t em, int n, double iso, ff is
   float f[8];
 #pragma unroll
   for (int q = 0; q < 8; q++) f[q] = F[q];
-  const int prj = n >= 6 ? plane_from_gradient_f(f, pm[0].hi, pm[1].hi, pm[2].hi) : plane_from_extent_box_ff(box);
-  if (prj < 0) return -1;
+  int prj = n >= 6 ? plane_from_gradient_f(f, pm[0].hi, pm[1].hi, pm[2].hi) : plane_from_extent_box_ff(box);
+  if (prj < 0) {
+    if (!kFull) return -1;
+    if (n >= 6) {
+      double fd[8];
+      for (int q = 0; q < 8; q++) fd[q] = f[q];
+      prj = plane_from_gradient(fd, mean64().p);
+    } else {
+      Box3 x;
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        x.b[d][0] = box[d][0];
+        x.b[d][1] = box[d][1];
+      }
+      prj = plane_from_extent_box_f64(x);
+    }
+  }
   // the frame's axes: (A, B, W) = (x, y, z), (x, z, y) or (y, z, x)
   if (prj != 0) {
     const float x1 = f[1], x2 = f[2], x3 = f[3], x5 = f[5], x6 = f[6];
@@ -1135,6 +1163,11 @@ TMC_HD int vertex_frame(const FrameCol& F, uint32_t em, int n, double iso, ff is
   F[kPu] = prj == 2 ? pm[1].hi : pm[0].hi;
   F[kPv] = prj == 0 ? pm[1].hi : pm[2].hi;
   F[kPw] = prj == 0 ? pm[2].hi : (prj == 1 ? pm[1].hi : pm[0].hi);
+  if (mean) {
+    mean[0] = prj == 2 ? pm[1] : pm[0];
+    mean[1] = prj == 0 ? pm[1] : pm[2];
+    mean[2] = prj == 0 ? pm[2] : (prj == 1 ? pm[1] : pm[0]);
+  }
   const float ulo = prj == 2 ? box[1][0] : box[0][0], uhi = prj == 2 ? box[1][1] : box[0][1];
   const float vlo = prj == 0 ? box[1][0] : box[2][0], vhi = prj == 0 ? box[1][1] : box[2][1];
   F[kUlo] = ulo;
@@ -1148,7 +1181,7 @@ TMC_HD int vertex_frame(const FrameCol& F, uint32_t em, int n, double iso, ff is
   F[kWhi] = whi;
   F[kIso] = iso_ff.hi;
   F[kIsoErr] = fabsf(iso_ff.lo) + fabsf(iso_ff.hi) * 0x1p-30f;
-  return sample_range_exact(ulo, uhi) && sample_range_exact(vlo, vhi) ? prj : -1;
+  return kFull || (sample_range_exact(ulo, uhi) && sample_range_exact(vlo, vhi)) ? prj : -1;
 }
 
 // Sample q = 7 i + j of a frame in float32.  Lower and upper bounds of its distance as the reference
@@ -1156,9 +1189,14 @@ TMC_HD int vertex_frame(const FrameCol& F, uint32_t em, int n, double iso, ff is
 struct SampleBound {
   float lb, ub;
 };
-TMC_HD SampleBound sample_bound(const FrameCol& F, int q) {
-  const int i = q / 7, j = q - 7 * i;
-  const float u = sample_at(F[kUlo], F[kUhi], i + 1), v = sample_at(F[kVlo], F[kVhi], j + 1);
+// The boxes (in the frame's axes) of the cell's other contours of three edges: the reference takes no
+// sample inside them (is_in_neighbor_bbox, cpp_dmc/DualMarchingCubes.cpp:248-268).
+struct Exclusion {
+  int n = 0;
+  float lo[3][3], hi[3][3];
+};
+template <bool kExclude>
+TMC_HD SampleBound sample_bound_at(const FrameCol& F, float u, float v, const Exclusion* X) {
   const float omu = 1 - u, omv = 1 - v;
   const float A1 = ffx::fma_rn(u, F[1], omu * F[0]), B1 = ffx::fma_rn(u, F[3], omu * F[2]);
   const float A2 = ffx::fma_rn(u, F[5], omu * F[4]), B2 = ffx::fma_rn(u, F[7], omu * F[6]);
@@ -1176,12 +1214,26 @@ TMC_HD SampleBound sample_bound(const FrameCol& F, int q) {
   const float Ew = ((Enum + aw * Eden) * ffx::rcp_est(ad - Eden) + aw * 0x1p-20f) * 1.0001f + 1e-30f;
   const float wlo = F[kWlo], whi = F[kWhi];
   if (w + Ew < wlo || w - Ew > whi) return SampleBound{INFINITY, INFINITY};
+  bool sure = w - Ew >= wlo && w + Ew <= whi;
+  if (kExclude) {
+    for (int b = 0; b < X->n; b++) {
+      if (u < X->lo[b][0] || X->hi[b][0] < u || v < X->lo[b][1] || X->hi[b][1] < v) continue;
+      const float lo = X->lo[b][2], hi = X->hi[b][2];
+      if (w + Ew < lo || w - Ew > hi) continue;                                           // surely outside
+      if (w - Ew >= lo && w + Ew <= hi) return SampleBound{INFINITY, INFINITY};           // surely inside
+      sure = false;
+    }
+  }
   const float Ep = 0x1p-22f;
   const float e0 = F[kPu] - u, e1 = F[kPv] - v, e2 = F[kPw] - w;
   const float D = e0 * e0 + e1 * e1 + e2 * e2;
   const float ED = (2 * (fabsf(e0) + fabsf(e1)) * Ep + 2 * fabsf(e2) * (Ew + Ep) + (Ew + Ep) * (Ew + Ep) +
                     2 * Ep * Ep + D * 0x1p-20f) * 1.0001f + 1e-30f;
-  return SampleBound{fmaxf(D - ED, 0.0f), w - Ew >= wlo && w + Ew <= whi ? D + ED : INFINITY};
+  return SampleBound{fmaxf(D - ED, 0.0f), sure ? D + ED : INFINITY};
+}
+TMC_HD SampleBound sample_bound(const FrameCol& F, int q) {
+  const int i = q / 7, j = q - 7 * i;
+  return sample_bound_at<false>(F, sample_at(F[kUlo], F[kUhi], i + 1), sample_at(F[kVlo], F[kVhi], j + 1), nullptr);
 }
 
 // The sample nearest to the mean point (a guess is enough: it is only where the search starts)
@@ -1259,6 +1311,141 @@ TMC_HD int sample_point(const FrameCol& F, int q, int prj, ff iso_ff, float p[3]
   p[1] = prj == 0 ? v : (prj == 1 ? W.hi : u);
   p[2] = prj == 0 ? W.hi : v;
   return ok ? kFound : kW64;
+}
+
+// The box of the contour with edge set `em` (corners in the first eight floats of the column, before
+// vertex_frame permutes them); false for values at the ends of the float range.
+TMC_HD bool contour_box(const FrameCol& F, uint32_t em, double iso, ff iso_ff, bool exact_iso, float lo[3], float hi[3]) {
+  float mn[3] = {1, 1, 1}, mx[3] = {0, 0, 0};
+  bool ok = true;
+#pragma unroll 1
+  for (uint32_t m = em; m; m &= m - 1) {
+    const int e = lowest_bit32(m) >> 1;
+    const int ax = e < 8 ? (e & 1) : 2;
+    const int v0 = nibr(EDGE_V0, e);
+    const float f0 = F[v0], f1 = F[v0 + (1 << ax)];
+    float l;
+    if (!edge_param_certain(f0, f1, iso_ff, exact_iso, l)) l = edge_param_f64(iso, f0, f1) + 0.0f;
+    ok = ok && l >= 0.0f && l <= 1.0f;
+#pragma unroll
+    for (int d = 0; d < 3; d++)
+      if (ax == d) {
+        mn[d] = fminf(mn[d], l);
+        mx[d] = fmaxf(mx[d], l);
+      }
+  }
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    lo[d] = (em & edges_zero(d)) ? 0.0f : mn[d];
+    hi[d] = (em & edges_one(d)) ? 1.0f : mx[d];
+  }
+  return ok;
+}
+
+// One sample of a frame as the reference evaluates it.  state: 0 not valid, 1 valid, 2 valid with a
+// distance whose rounding is not certified (distance_f64).  f64 counts the values computed in float64.
+struct ExactSample {
+  float d, w;
+  int state;
+};
+TMC_HD ExactSample exact_sample(const FrameCol& F, float u, float v, const ff mean[3], const Exclusion& X, double iso,
+                                ff iso_ff, int& f64) {
+  ExactSample r{0.0f, 0.0f, 0};
+  float g1, g2;
+  if (!bilinear_certain(F[0], F[1], F[2], F[3], F[kSabsLo], u, v, g1)) {
+    g1 = bilinear_f64(F[0], F[1], F[2], F[3], u, v);
+    f64++;
+  }
+  if (!bilinear_certain(F[4], F[5], F[6], F[7], F[kSabsHi], u, v, g2)) {
+    g2 = bilinear_f64(F[4], F[5], F[6], F[7], u, v);
+    f64++;
+  }
+  if (g1 == g2) return r;
+  const float den = g2 - g1, ad = fabsf(den);
+  ff t = ffx::two_sum(iso_ff.hi, -g1);
+  t.lo += iso_ff.lo;
+  const ff num = ffx::quick_two_sum(t.hi, t.lo);
+  const float rc = ffx::rcp_est(den);
+  const ff W = ffx::ff_quot(num, ffx::ff_from(den), rc);
+  r.w = W.hi;
+  if (!(ad > 0x1p-60f && ad < 0x1p120f && fabsf(num.hi) > 0x1p-90f &&
+        ffx::ff_certain(W, fabsf(W.hi) * 0x1p-42f + fmaxf(fabsf(iso_ff.hi), fabsf(g1)) * 0x1p-45f * fabsf(rc)))) {
+    r.w = w_f64(iso, g1, g2);
+    f64++;
+  }
+  const float w = r.w;
+  if (!(w >= F[kWlo] && w <= F[kWhi])) return r;
+  for (int x = 0; x < X.n; x++)
+    if (!(u < X.lo[x][0] || X.hi[x][0] < u || v < X.lo[x][1] || X.hi[x][1] < v || w < X.lo[x][2] || X.hi[x][2] < w))
+      return r;
+  const ff d0 = ffx::ff_sub(mean[0], ffx::ff_from(u)), d1 = ffx::ff_sub(mean[1], ffx::ff_from(v)),
+           d2 = ffx::ff_sub(mean[2], ffx::ff_from(w));
+  const ff D = ffx::ff_add(ffx::ff_add(ffx::ff_mul(d0, d0), ffx::ff_mul(d1, d1)), ffx::ff_mul(d2, d2));
+  r.d = D.hi;
+  r.state =
+      ffx::ff_certain(D, fabsf(D.hi) * 0x1p-40f + (fabsf(d0.hi) + fabsf(d1.hi) + fabsf(d2.hi)) * 0x1p-41f) ? 1 : 2;
+  return r;
+}
+// the reference's float of a sample's distance from its float64 mean point (cell axes)
+TMC_HD float distance_f64(const Point64& pm, int prj, float u, float v, float w) {
+  const double a = prj == 2 ? pm.p[1] : pm.p[0], b = prj == 0 ? pm.p[1] : pm.p[2],
+               c = prj == 0 ? pm.p[2] : (prj == 1 ? pm.p[1] : pm.p[0]);
+  return (float)((a - u) * (a - u) + (b - v) * (b - v) + (c - w) * (c - w));
+}
+TMC_HD void frame_point(int prj, float u, float v, float w, float p[3]) {
+  p[0] = prj == 2 ? w : u;
+  p[1] = prj == 0 ? v : (prj == 1 ? w : u);
+  p[2] = prj == 0 ? w : v;
+}
+
+// The whole 7x7 search of a framed contour with neighbour boxes X and any number of candidates: the
+// samples whose lower bound is within the smallest upper bound are evaluated exactly, in the
+// reference's loop order (strict minDistance > d).  mean: the frame's; mean64: the reference's float64
+// mean point, called when a distance's rounding is not certified.  kFound with p, or kRedo when no
+// sample is valid (the reference's 26x26 retry).
+template <typename Mean64>
+TMC_HD int search_all(const FrameCol& F, int prj, const ff mean[3], const Exclusion& X, double iso, ff iso_ff,
+                      const Mean64& mean64, float p[3], int& f64) {
+  const float ulo = F[kUlo], uhi = F[kUhi], vlo = F[kVlo], vhi = F[kVhi];
+  float m = INFINITY;
+  uint64_t seen = 0;
+  const int q0 = seed_sample(F);
+  // the seed, its neighbours when it is not certain, then all samples within the bound found
+#pragma unroll 1
+  for (int round = 0; round < 3; round++) {
+    if (round == 1 && m < INFINITY) continue;
+    uint64_t need = (round == 0 ? 1ull << q0 : (round == 1 ? ring_of(q0) : samples_within(F, m))) & ~seen;
+    seen |= need;
+#pragma unroll 1
+    for (; need; need &= need - 1) {
+      const int q = lowest_bit(need), i = q / 7, j = q - 7 * i;
+      m = fminf(m, sample_bound_at<true>(F, sample_coord_any(ulo, uhi, i + 1), sample_coord_any(vlo, vhi, j + 1), &X).ub);
+    }
+  }
+  // d < 100 always: both points lie in the cell (100 is where the reference's minimum starts)
+  float best = INFINITY;
+  bool found = false, have_mean = false;
+  Point64 pm{{0, 0, 0}};
+#pragma unroll 1
+  for (; seen; seen &= seen - 1) {
+    const int q = lowest_bit(seen), i = q / 7, j = q - 7 * i;
+    const float u = sample_coord_any(ulo, uhi, i + 1), v = sample_coord_any(vlo, vhi, j + 1);
+    const SampleBound b = sample_bound_at<true>(F, u, v, &X);
+    if (!(b.lb <= m) || b.lb == INFINITY) continue;
+    ExactSample s = exact_sample(F, u, v, mean, X, iso, iso_ff, f64);
+    if (s.state == 2) {
+      if (!have_mean) pm = mean64();
+      have_mean = true;
+      s.d = distance_f64(pm, prj, u, v, s.w);
+      f64++;
+    }
+    if (s.state != 0 && best > s.d) {
+      best = s.d;
+      frame_point(prj, u, v, s.w, p);
+      found = true;
+    }
+  }
+  return found ? kFound : kRedo;
 }
 
 // The search on one thread (the order of the kernel's rounds; the CPU checks run it).

@@ -56,7 +56,7 @@ namespace {
 // tmc_ctx::d_stats, in 64-bit words
 constexpr int kStatTotals = 8;    // after the 8 statistics: [0] (vertices << 32) | faces, [1] overflow
 constexpr int kStatAmb = 10;      // 2 x u32: ambiguous cells, chunks
-constexpr int kStatFallback = 11; // 3 x u32: the DMC vertex lists
+constexpr int kStatFallback = 11; // 4 x u32: the DMC vertex lists
 constexpr int kStatAmbHist = 16;  // 514 x u32: the sort of TMC's ambiguous cells
 constexpr int kStatWords = kStatAmbHist + 257;
 constexpr size_t kPinnedBytes = 256 << 10;
@@ -316,6 +316,7 @@ void plan_dmc_vertices(Allocs& al, tmc::DmcScratch& sc, int64_t nv) {
   al.plan(&sc.vp, nv);
   al.plan(&sc.fb_list, nv);
   al.plan(&sc.w_list, nv);
+  al.plan(&sc.hard_list, nv);
   al.plan(&sc.tail_list, nv);
 }
 
