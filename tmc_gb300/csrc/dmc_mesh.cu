@@ -489,18 +489,67 @@ __global__ void gather_live_quads_kernel(const uint8_t* alive, const int32_t* id
 // quad -> triangles (collectTriangles, :1387-1460; minAngle, DualMarchingCubes.h:746-756)
 // ---------------------------------------------------------------------------------------------
 // minAngle exactly as the reference: three float arc cosines of the host C library (the restated
-// kind of libm_acosf.h that the host's acosf is, bit for bit), float minimum in std::min's order
-__device__ __forceinline__ float min_angle_full(float a, float b, float c, int acos_kind) {
-  const float A = libm::acosf_kind((b * b + c * c - a * a) / (2 * b * c), acos_kind);
-  const float B = libm::acosf_kind((a * a + c * c - b * b) / (2 * a * c), acos_kind);
-  const float C = libm::acosf_kind((b * b + a * a - c * c) / (2 * b * a), acos_kind);
+// kind of libm_acosf.h that the host's acosf is, bit for bit), float minimum in std::min's order.
+template <int kAcos>
+__device__ __noinline__ float min_angle_all(float ca, float cb, float cc) {
+  const float A = libm::acosf_kind(ca, kAcos), B = libm::acosf_kind(cb, kAcos), C = libm::acosf_kind(cc, kAcos);
   const float mAB = (B < A) ? B : A;
   return (C < mAB) ? C : mAB;
 }
+// Where one cosine is clearly the largest (by 2^-18; all within [-1, 1]) its arc cosine is the minimum:
+// acos falls at least as fast as its argument grows, and the library's is within an ulp (2^-22).
+template <int kAcos>
+__device__ __forceinline__ float min_angle(float a, float b, float c) {
+  const float ca = (b * b + c * c - a * a) / (2 * b * c), cb = (a * a + c * c - b * b) / (2 * a * c),
+              cc = (b * b + a * a - c * c) / (2 * b * a);
+  const float m = fmaxf(ca, fmaxf(cb, cc)), low = fminf(ca, fminf(cb, cc));
+  const float mid = fmaxf(fminf(ca, cb), fminf(fmaxf(ca, cb), cc));
+  if (ca == ca && cb == cb && cc == cc && m <= 1.0f && low >= -1.0f && mid < m - 0x1p-18f)
+    return libm::acosf_kind(m, kAcos);
+  return min_angle_all<kAcos>(ca, cb, cc);
+}
 
-__device__ __forceinline__ float side(const double* p, const double* q) {
+// the reference's side length: the float of a float64 distance
+__device__ __forceinline__ float side_f64(const double* p, const double* q) {
   const double d = (p[0] - q[0]) * (p[0] - q[0]) + (p[1] - q[1]) * (p[1] - q[1]) + (p[2] - q[2]) * (p[2] - q[2]);
   return (float)sqrt(d);
+}
+// A float64 position as float pairs (2^-47 relative), taken apart with integer operations (a conversion
+// would run on the float64 pipe too).
+struct PairPoint {
+  ffx::ff x[3];
+};
+__device__ __forceinline__ ffx::ff split_f64(double x) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const int e = (int)(b >> 52) & 0x7ff;
+  if (e < 1023 - 60 || e > 1023 + 60) return ffx::ff_from_double(x);  // zero, or far from 1
+  const uint32_t sign = (uint32_t)(b >> 63) << 31;
+  const float hi = __uint_as_float(sign | (uint32_t)(e - 896) << 23 | ((uint32_t)(b >> 29) & 0x7fffffu));
+  const float lo = (float)((uint32_t)b & 0x1fffffffu) * __uint_as_float(sign | (uint32_t)(e - 896 - 52) << 23);
+  return ffx::ff{hi, lo};
+}
+__device__ __forceinline__ PairPoint load_pairs(const double* v) {
+  return PairPoint{{split_f64(v[0]), split_f64(v[1]), split_f64(v[2])}};
+}
+// |p - q|; false when its rounding is not certified.  The differences err by 2^-45.4 of the coordinates'
+// magnitudes, so the length by their sum's, and by 2^-43 of itself.
+__device__ __forceinline__ bool side_certain(const PairPoint& p, const PairPoint& q, float& out) {
+  ffx::ff sum{0, 0};
+  float mag = 0;
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    const ffx::ff s = ffx::two_sum(p.x[a].hi, -q.x[a].hi);
+    const ffx::ff d = ffx::quick_two_sum(s.hi, s.lo + (p.x[a].lo - q.x[a].lo));
+    sum = ffx::ff_add_abs(sum, ffx::ff_mul(d, d));
+    mag += fabsf(p.x[a].hi) + fabsf(q.x[a].hi);
+  }
+  if (!(sum.hi > 0x1p-80f && sum.hi < 0x1p80f)) return false;
+  // the rounded root and one Newton step
+  const float r = sqrtf(sum.hi);
+  const ffx::ff sq = ffx::two_prod(r, r);
+  const ffx::ff l = ffx::quick_two_sum(r, (((sum.hi - sq.hi) - sq.lo) + sum.lo) * (0.5f * ffx::rcp_est(r)));
+  out = l.hi;
+  return ffx::ff_certain(l, mag * 0x1p-45f + l.hi * 0x1p-42f);
 }
 
 __device__ __forceinline__ void write_split(int32_t* t, int64_t i, int v0, int v1, int v2, int v3, bool first) {
@@ -512,21 +561,23 @@ __device__ __forceinline__ void write_split(int32_t* t, int64_t i, int v0, int v
   }
 }
 
-// Largest cosine of a triangle from float sides with their error bounds, and the bound of the
-// result; false when the cosines are not surely inside [-1, 1].
-__device__ __forceinline__ bool max_cosine_bounded(float a, float b, float c, float ea, float eb, float ec, float& m,
-                                                   float& em) {
-  const float cA = (b * b + c * c - a * a) / (2 * b * c);
-  const float cB = (a * a + c * c - b * b) / (2 * a * c);
-  const float cC = (b * b + a * a - c * c) / (2 * b * a);
-  // first-order propagation of the side errors (doubled), plus the rounding of both evaluations
-  const float rel = ea / a + eb / b + ec / c;
-  const float eA = 2.0f * (2.0f * (a * ea + b * eb + c * ec) / (2 * b * c) + fabsf(cA) * rel) + 0x1p-20f;
-  const float eB = 2.0f * (2.0f * (a * ea + b * eb + c * ec) / (2 * a * c) + fabsf(cB) * rel) + 0x1p-20f;
-  const float eC = 2.0f * (2.0f * (a * ea + b * eb + c * ec) / (2 * b * a) + fabsf(cC) * rel) + 0x1p-20f;
-  if (!(cA - eA >= -1.f && cA + eA <= 1.f && cB - eB >= -1.f && cB + eB <= 1.f && cC - eC >= -1.f &&
-        cC + eC <= 1.f))
-    return false;
+// A side from float positions: its length, the reciprocal's estimate and its relative error bound.
+struct Side {
+  float d, r, e;
+};
+// Largest cosine of the triangle with sides a, b, c, and the bound of the result's distance to the
+// reference's; false when the cosines are not surely inside [-1, 1].
+__device__ __forceinline__ bool max_cosine_bounded(const Side& a, const Side& b, const Side& c, float& m, float& em) {
+  const float aa = a.d * a.d, bb = b.d * b.d, cc = c.d * c.d;
+  const float ab = 0.5f * a.r * b.r, ac = 0.5f * a.r * c.r, bc = 0.5f * b.r * c.r;
+  const float cA = (bb + cc - aa) * bc, cB = (aa + cc - bb) * ac, cC = (bb + aa - cc) * ab;
+  // first-order propagation of the side errors (doubled), plus the rounding of both evaluations (with
+  // the reciprocals' 2^-21)
+  const float rel = a.e + b.e + c.e, s = 2.0f * (aa * a.e + bb * b.e + cc * c.e);
+  const float eA = 2.0f * (s * bc + fabsf(cA) * rel) + 0x1p-19f;
+  const float eB = 2.0f * (s * ac + fabsf(cB) * rel) + 0x1p-19f;
+  const float eC = 2.0f * (s * ab + fabsf(cC) * rel) + 0x1p-19f;
+  if (!(fabsf(cA) + eA <= 1.f && fabsf(cB) + eB <= 1.f && fabsf(cC) + eC <= 1.f)) return false;
   m = fmaxf(cA, fmaxf(cB, cC));
   em = fmaxf(eA, fmaxf(eB, eC));
   return true;
@@ -535,78 +586,145 @@ __device__ __forceinline__ bool max_cosine_bounded(float a, float b, float c, fl
 // |p - q| from float positions and a bound of its distance to the reference's float (rounded from
 // the float64 length of the float64 difference); each float position is within 2^-24 |x| of its
 // float64 value.
-__device__ __forceinline__ float side_f(const float* p, const float* q, float& err) {
-  const float dx = p[0] - q[0], dy = p[1] - q[1], dz = p[2] - q[2];
-  const float d = sqrtf(dx * dx + dy * dy + dz * dz);
-  const float mag = fabsf(p[0]) + fabsf(q[0]) + fabsf(p[1]) + fabsf(q[1]) + fabsf(p[2]) + fabsf(q[2]);
-  err = mag * 0x1p-23f + d * 0x1p-20f;
-  return d;
+struct FloatPoint {
+  float x[3];
+};
+__device__ __forceinline__ FloatPoint load_point(const float* v, int64_t i) {
+  return FloatPoint{{v[3 * i], v[3 * i + 1], v[3 * i + 2]}};
+}
+__device__ __forceinline__ bool side_bounded(const FloatPoint& p, const FloatPoint& q, Side& out) {
+  const float dx = p.x[0] - q.x[0], dy = p.x[1] - q.x[1], dz = p.x[2] - q.x[2];
+  const float d2 = dx * dx + dy * dy + dz * dz;
+  const float mag = fabsf(p.x[0]) + fabsf(q.x[0]) + fabsf(p.x[1]) + fabsf(q.x[1]) + fabsf(p.x[2]) + fabsf(q.x[2]);
+  out.r = rsqrtf(d2);  // within two ulps
+  out.d = d2 * out.r;
+  out.e = mag * 0x1p-23f * out.r + 0x1p-20f;
+  return d2 > 0x1p-80f && d2 < 0x1p80f;
 }
 
-// collectTriangles (:1387-1460), first pass: decides the split from the float positions wherever
-// the two candidates' smallest angles are apart by more than the error bounds; the other quads are
-// listed for the exact pass.
+// The split of quad corners P, where the two candidates' smallest angles are apart by more than the
+// error bounds: 1 first (along v1-v3), 0 second, -1 in doubt.
+__device__ __forceinline__ int split_bounded(const FloatPoint& P0, const FloatPoint& P1, const FloatPoint& P2,
+                                             const FloatPoint& P3) {
+  Side d01, d12, d20, d23, d30, d13;
+  bool ok = side_bounded(P0, P1, d01);
+  ok = side_bounded(P1, P2, d12) && ok;
+  ok = side_bounded(P2, P0, d20) && ok;
+  ok = side_bounded(P2, P3, d23) && ok;
+  ok = side_bounded(P3, P0, d30) && ok;
+  ok = side_bounded(P1, P3, d13) && ok;
+  float m1, m2, m3, m4, x1, x2, x3, x4;
+  if (!(ok && max_cosine_bounded(d01, d12, d20, m1, x1) && max_cosine_bounded(d20, d23, d30, m2, x2) &&
+        max_cosine_bounded(d13, d30, d01, m3, x3) && max_cosine_bounded(d12, d23, d13, m4, x4)))
+    return -1;
+  // smallest angle of a split = acos of its largest cosine (acos decreasing): the first split wins when
+  // its largest cosine is smaller.  The bounds place the reference's largest cosines; a further 2^-20
+  // between them keeps its angles (acos has slope at least 1 in magnitude, and the library's float
+  // acos is within one ulp, at most 2^-22 below pi) strictly ordered the same way.
+  const float xb = fmaxf(m1, m2), eb = fmaxf(x1, x2), xc = fmaxf(m3, m4), ec = fmaxf(x3, x4);
+  if (xb + eb + 0x1p-20f < xc - ec) return 0;  // b1 > c1
+  if (xb - eb > xc + ec + 0x1p-20f) return 1;  // b1 < c1
+  return -1;
+}
+__device__ __forceinline__ void list_quad(uint32_t* list, unsigned* count, bool take, uint32_t x) {
+  const int lane = threadIdx.x & 31;
+  const unsigned am = __activemask();
+  const unsigned bal = __ballot_sync(am, take);
+  if (!bal) return;
+  const int leader = __ffs(bal) - 1;
+  unsigned base = 0;
+  if (lane == leader) base = atomicAdd(count, (unsigned)__popc(bal));
+  base = __shfl_sync(am, base, leader);
+  if (take) list[base + __popc(bal & ((1u << lane) - 1u))] = x;
+}
+
+// collectTriangles (:1387-1460), first pass: decides the split from the float positions wherever they
+// leave no doubt; the other quads are listed.
 __global__ void triangles_fast_kernel(const int32_t* q, int64_t nq, const float* v, int32_t* t, uint32_t* list,
                                       unsigned* count) {
-  const int lane = threadIdx.x & 31;
   FOR_EACH(i, nq) {
     const int v0 = q[4 * i], v1 = q[4 * i + 1], v2 = q[4 * i + 2], v3 = q[4 * i + 3];
-    const float *P0 = v + 3 * (int64_t)v0, *P1 = v + 3 * (int64_t)v1, *P2 = v + 3 * (int64_t)v2,
-                *P3 = v + 3 * (int64_t)v3;
-    float e01, e12, e20, e23, e30, e13;
-    const float d01 = side_f(P0, P1, e01), d12 = side_f(P1, P2, e12), d20 = side_f(P2, P0, e20),
-                d23 = side_f(P2, P3, e23), d30 = side_f(P3, P0, e30), d13 = side_f(P1, P3, e13);
-    float m1, m2, m3, m4, x1, x2, x3, x4;
-    bool sure = d01 > 0 && d12 > 0 && d20 > 0 && d23 > 0 && d30 > 0 && d13 > 0 &&
-                max_cosine_bounded(d01, d12, d20, e01, e12, e20, m1, x1) &&
-                max_cosine_bounded(d20, d23, d30, e20, e23, e30, m2, x2) &&
-                max_cosine_bounded(d13, d30, d01, e13, e30, e01, m3, x3) &&
-                max_cosine_bounded(d12, d23, d13, e12, e23, e13, m4, x4);
-    bool first = false;
-    if (sure) {
-      // smallest angle of a split = acos of its largest cosine (acos decreasing): the first split
-      // (along v1-v3) wins when its largest cosine is smaller
-      // The bounds place the reference's largest cosines; a further 2^-20 between them keeps its
-      // angles (acos has slope at least 1 in magnitude, and the library's float acos is within one
-      // ulp, at most 2^-22 below pi) strictly ordered the same way.
-      const float xb = fmaxf(m1, m2), eb = fmaxf(x1, x2), xc = fmaxf(m3, m4), ec = fmaxf(x3, x4);
-      if (xb + eb + 0x1p-20f < xc - ec) first = false;       // b1 > c1
-      else if (xb - eb > xc + ec + 0x1p-20f) first = true;  // b1 < c1
-      else sure = false;
-    }
-    if (sure) write_split(t, i, v0, v1, v2, v3, first);
-    const unsigned am = __activemask();
-    const unsigned bal = __ballot_sync(am, !sure);
-    if (bal) {
-      const int leader = __ffs(bal) - 1;
-      unsigned base = 0;
-      if (lane == leader) base = atomicAdd(count, (unsigned)__popc(bal));
-      base = __shfl_sync(am, base, leader);
-      if (!sure) list[base + __popc(bal & ((1u << lane) - 1u))] = (uint32_t)i;
-    }
+    const int s = split_bounded(load_point(v, v0), load_point(v, v1), load_point(v, v2), load_point(v, v3));
+    if (s >= 0) write_split(t, i, v0, v1, v2, v3, s == 1);
+    list_quad(list, count, s < 0, (uint32_t)i);
   }
+}
+
+// The reference's decision from the six side lengths: minAngle of the triangles (v0,v1,v2), (v0,v2,v3)
+// against (v1,v3,v0), (v1,v2,v3), each from the sides |p0p1|, |p1p2|, |p2p0|; true: the first split.
+template <int kAcos>
+__device__ __forceinline__ bool split_exact(float d01, float d12, float d20, float d23, float d30, float d13) {
+  float m[4];
+#pragma unroll 1  // one copy of the arc cosines: the pass is bound by instruction fetch otherwise
+  for (int t = 0; t < 4; t++) {
+    const float a = t == 0 ? d01 : (t == 1 ? d20 : (t == 2 ? d13 : d12));
+    const float b = t == 0 ? d12 : (t == 1 ? d23 : (t == 2 ? d30 : d23));
+    const float c = t == 0 ? d20 : (t == 1 ? d30 : (t == 2 ? d01 : d13));
+    const float x = min_angle<kAcos>(a, b, c);
+    if (t == 0) m[0] = x;
+    if (t == 1) m[1] = x;
+    if (t == 2) m[2] = x;
+    if (t == 3) m[3] = x;
+  }
+  // (the reference compares the floats as doubles)
+  const float b1 = m[1] < m[0] ? m[1] : m[0], b2 = m[0] < m[1] ? m[1] : m[0];
+  const float c1 = m[3] < m[2] ? m[3] : m[2], c2 = m[2] < m[3] ? m[3] : m[2];
+  return b1 < c1 || (b1 == c1 && b2 <= c2);
 }
 
 // collectTriangles (:1387-1460), exact pass over the listed quads: the reference's arithmetic
 // step by step.  Six side lengths (float of a float64 distance), minAngle of the four triangles with
-// the host library's float acos (libm_acosf.h, acos_kind), float64 comparisons of the two splits.
-__global__ void triangles_kernel(const int32_t* q, const uint32_t* list, const unsigned* count, const double* v64,
-                                 int32_t* t, int acos_kind) {
+// the host library's float acos (libm_acosf.h, kAcos), comparisons of the two splits.
+// The float positions are coarse beside a fine grid's cells, so many quads are listed (8 % of the 512^3
+// noise field's, 40 % of the 1024x1024x64 saddle field's).  The lengths come from float pairs with
+// certified rounding; the quads with one that is not certified (a few per cent) are gathered in shared
+// memory and taken in float64 densely, a few lanes of most warps would occupy that pipe otherwise.
+// With twelve arc cosines per quad and every length in float64 the pass took 0.28 ms (noise, 0.38 million
+// quads listed) and 4.64 ms (saddle); 0.16 and 2.18 ms so.
+constexpr int kSplitThreads = 256;
+template <int kAcos>
+__global__ void __launch_bounds__(kSplitThreads) triangles_kernel(const int32_t* q, const uint32_t* list,
+                                                                  const unsigned* count, const double* v64,
+                                                                  int32_t* t) {
+  __shared__ uint32_t open[2 * kSplitThreads];
+  __shared__ unsigned n_open;
+  if (threadIdx.x == 0) n_open = 0;
+  __syncthreads();
   const int64_t nl = *count;
-  FOR_EACH(a, nl) {
-    const int64_t i = list[a];
-    const int v0 = q[4 * i], v1 = q[4 * i + 1], v2 = q[4 * i + 2], v3 = q[4 * i + 3];
-    const double *P0 = v64 + 3 * (int64_t)v0, *P1 = v64 + 3 * (int64_t)v1, *P2 = v64 + 3 * (int64_t)v2,
-                 *P3 = v64 + 3 * (int64_t)v3;
-    const float d01 = side(P0, P1), d12 = side(P1, P2), d20 = side(P2, P0), d23 = side(P2, P3), d30 = side(P3, P0),
-                d13 = side(P1, P3);
-    // triangles (v0,v1,v2), (v0,v2,v3) | (v1,v3,v0), (v1,v2,v3); minAngle(a, b, c) takes the sides
-    // |p0p1|, |p1p2|, |p2p0| of its triangle (p0, p1, p2)
-    const double a1 = min_angle_full(d01, d12, d20, acos_kind), a2 = min_angle_full(d20, d23, d30, acos_kind);
-    const double b1 = a2 < a1 ? a2 : a1, b2 = a1 < a2 ? a2 : a1;
-    const double a3 = min_angle_full(d13, d30, d01, acos_kind), a4 = min_angle_full(d12, d23, d13, acos_kind);
-    const double c1 = a4 < a3 ? a4 : a3, c2 = a3 < a4 ? a4 : a3;
-    write_split(t, i, v0, v1, v2, v3, b1 < c1 || (b1 == c1 && b2 <= c2));
+  const int64_t step = (int64_t)gridDim.x * kSplitThreads;
+  for (int64_t base = (int64_t)blockIdx.x * kSplitThreads; base < nl; base += step) {  // block-uniform
+    const int64_t a = base + threadIdx.x;
+    if (a < nl) {
+      const int64_t i = list[a];
+      const int v0 = q[4 * i], v1 = q[4 * i + 1], v2 = q[4 * i + 2], v3 = q[4 * i + 3];
+      const PairPoint p0 = load_pairs(v64 + 3 * (int64_t)v0), p1 = load_pairs(v64 + 3 * (int64_t)v1),
+                      p2 = load_pairs(v64 + 3 * (int64_t)v2), p3 = load_pairs(v64 + 3 * (int64_t)v3);
+      float d01, d12, d20, d23, d30, d13;
+      bool ok = side_certain(p0, p1, d01);
+      ok = side_certain(p1, p2, d12) && ok;
+      ok = side_certain(p2, p0, d20) && ok;
+      ok = side_certain(p2, p3, d23) && ok;
+      ok = side_certain(p3, p0, d30) && ok;
+      ok = side_certain(p1, p3, d13) && ok;
+      if (ok) write_split(t, i, v0, v1, v2, v3, split_exact<kAcos>(d01, d12, d20, d23, d30, d13));
+      else open[atomicAdd(&n_open, 1u)] = (uint32_t)i;
+    }
+    __syncthreads();
+    const unsigned n = n_open;
+    if (n >= kSplitThreads || base + step >= nl) {  // block-uniform: a full round, or the last
+      for (unsigned x = threadIdx.x; x < n; x += kSplitThreads) {
+        const int64_t i = open[x];
+        const int v0 = q[4 * i], v1 = q[4 * i + 1], v2 = q[4 * i + 2], v3 = q[4 * i + 3];
+        const double *P0 = v64 + 3 * (int64_t)v0, *P1 = v64 + 3 * (int64_t)v1, *P2 = v64 + 3 * (int64_t)v2,
+                     *P3 = v64 + 3 * (int64_t)v3;
+        write_split(t, i, v0, v1, v2, v3,
+                    split_exact<kAcos>(side_f64(P0, P1), side_f64(P1, P2), side_f64(P2, P0), side_f64(P2, P3),
+                                       side_f64(P3, P0), side_f64(P1, P3)));
+      }
+      __syncthreads();
+      if (threadIdx.x == 0) n_open = 0;
+      __syncthreads();
+    }
   }
 }
 
@@ -1017,8 +1135,14 @@ DmcPostStatus dmc_postprocess(const DmcMesh& in, uint32_t flags, int sms, cudaSt
       if ((s.err = pool.err) == cudaSuccess) {
         triangles_fast_kernel<<<grid_for(cur.nq, sms), 256, 0, st>>>(cur.quads, cur.nq, cur.v, (int32_t*)tr, tlist,
                                                                       tcount);
-        triangles_kernel<<<grid_for(cur.nq, sms), 256, 0, st>>>(cur.quads, tlist, tcount, cur.v64, (int32_t*)tr,
-                                                                libm::host_acosf_kind());
+        const unsigned gt = grid_for(cur.nq, sms);
+        const int kind = libm::host_acosf_kind();
+#define TRIANGLES(K) \
+  triangles_kernel<K><<<gt, kSplitThreads, 0, st>>>(cur.quads, tlist, tcount, cur.v64, (int32_t*)tr)
+        if (kind == libm::kAcosfFused) TRIANGLES(libm::kAcosfFused);
+        else if (kind == libm::kAcosfSeparate) TRIANGLES(libm::kAcosfSeparate);
+        else TRIANGLES(libm::kAcosfCorrect);
+#undef TRIANGLES
         s.launches += 2;
         if (ready) (*ready)(tr, (size_t)cur.nq * 6 * sizeof(int32_t));
       }
