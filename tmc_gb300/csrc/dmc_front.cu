@@ -676,6 +676,47 @@ __device__ __forceinline__ void append(uint32_t* list, unsigned* count, bool tak
   if (take) list[base + __popc(bal & ((1u << lane) - 1u))] = x;
 }
 
+// A warp's entries for a list, gathered in shared memory and appended 32 at a time: one atomic per 32
+// entries.  (With one per warp and iteration the list's single counter took a fifth of the point kernel.)
+struct WarpList {
+  uint32_t* buf;  // 64 entries
+  int n = 0;      // the same on every lane
+  __device__ __forceinline__ void flush(uint32_t* list, unsigned* count, int k) {
+    const int lane = threadIdx.x & 31;
+    unsigned base = 0;
+    if (lane == 0) base = atomicAdd(count, (unsigned)k);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (lane < k) list[base + lane] = buf[lane];
+  }
+  // every lane of the warp calls it
+  __device__ __forceinline__ void add(uint32_t* list, unsigned* count, bool take, uint32_t x) {
+    const unsigned bal = __ballot_sync(0xffffffffu, take);
+    if (!bal) return;
+    const int lane = threadIdx.x & 31;
+    if (take) buf[n + __popc(bal & ((1u << lane) - 1u))] = x;
+    n += __popc(bal);
+    __syncwarp();
+    if (n >= 32) {
+      flush(list, count, 32);
+      n -= 32;
+      const uint32_t rest = buf[32 + lane];
+      __syncwarp();
+      buf[lane] = rest;
+      __syncwarp();
+    }
+  }
+  __device__ __forceinline__ void finish(uint32_t* list, unsigned* count) {
+    if (n) flush(list, count, n);
+  }
+};
+
+// copies a float to shared memory without waiting for it (cp_async_wait)
+__device__ __forceinline__ void cp_async4(float* dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // The vertices' projected points, one lane per vertex.  The contour's edge set comes from the cell's
 // record and case, so no polygon is walked again; the frame of the search (repr::vertex_frame) sits
 // in shared memory, a column per lane, and nothing is written to memory but the point.
@@ -686,11 +727,19 @@ __device__ __forceinline__ void append(uint32_t* list, unsigned* count, bool tak
 // vertices of the noise field, more than ten for 1 %): looping over its own, a lane would keep its
 // warp busy until the warp's largest number is reached (6 active lanes per instruction, measured).
 // So the warp lists all its lanes' samples and its lanes take them 32 at a time, whosever they are.
-// Bound by instruction issue (73 % active, 19 lanes per instruction, 68 registers, DRAM 210 MB).
-// 5.5 M vertices (320^3 noise field): 0.44 ms, 1.06 ms with the per-lane loops; the separate set-up
-// and projection kernels this replaces (a 144-byte record per vertex written and read in between,
-// nine samples bounded per vertex) took 1.15 + 0.85 ms.
-constexpr int kSampleWindow = 64;  // samples listed at a time
+// A lane with more than kFewSamples has its samples listed by the whole warp, and a sample's bounds go to
+// its lane's words in shared memory: the lanes' own loops over their samples took 43 % of the saddle
+// field's time, where a few lanes of most warps have dozens.  The first samples pass through the same code
+// (one copy of it: with two the warps waited for instructions a quarter of the time).  The chain vertex ->
+// slot -> record and cell -> corners runs one iteration ahead, the corners into shared memory.
+// Bound by instruction issue (80 % active, 23 lanes per instruction, 72 registers).  16.6 M vertices
+// (512^3 noise): 1.78 -> 1.48 ms; 47 M (1024x1024x64 saddles): 7.66 -> 5.54 ms, with 0.13 ms more for the
+// search of what stays open; 2.2 M (256^3 noise): 0.237 -> 0.200 ms.
+// The separate set-up and projection kernels before this one (a 144-byte record per vertex written and
+// read in between, nine samples bounded per vertex) took 1.15 + 0.85 ms for 5.5 M vertices, one kernel
+// with per-lane loops 1.06 ms.
+constexpr int kSampleWindow = 256;  // samples listed at a time
+constexpr int kFewSamples = 4;
 template <bool kBatch>
 __global__ void __launch_bounds__(kVertexThreads) dmc_vertex_point_kernel(CellSpace space, const uint16_t* cellof,
                                                                           const uint8_t* ccase, const uint32_t* rec,
@@ -700,32 +749,65 @@ __global__ void __launch_bounds__(kVertexThreads) dmc_vertex_point_kernel(CellSp
   constexpr int kWarps = kVertexThreads / 32;
   constexpr unsigned kAll = 0xffffffffu;
   __shared__ float frames[repr::kFrameFloats * kVertexThreads];
+  __shared__ float corners[8 * kVertexThreads];  // of the next iteration's cells
   __shared__ uint16_t items[kWarps][kSampleWindow];
-  __shared__ repr::SampleBound bounds[kWarps][kSampleWindow];
+  __shared__ float lowers[kWarps][kSampleWindow];
+  __shared__ unsigned per_lane[kWarps][2][32];
+  __shared__ uint32_t lists[kWarps][2][64];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   uint16_t* item = items[wid];
-  repr::SampleBound* bound = bounds[wid];
+  float* const lower = lowers[wid];
+  unsigned *const smallest = per_lane[wid][0], *const tally = per_lane[wid][1];
   float* const warp_frames = frames + 32 * wid;
   const repr::FrameCol F{warp_frames + lane, kVertexThreads};
+  WarpList redo_list{lists[wid][0]}, w_list{lists[wid][1]};
   const int64_t step = (int64_t)gridDim.x * kVertexThreads;
-  for (int64_t first = ((int64_t)blockIdx.x * kWarps + wid) * 32; first < nv; first += step) {  // warp-uniform
-    const int64_t vidx = first + lane;
-    const bool valid = vidx < nv;
+  int64_t first = ((int64_t)blockIdx.x * kWarps + wid) * 32;  // warp-uniform
+  auto grid_of = [&](uint32_t vcell) -> const Grid& {
+    return kBatch ? space.grids[__ldg(space.tile_vol + vcell / kScanTile)] : space.one;
+  };
+  auto fetch_corners = [&](uint32_t vcell) {
+    const Grid& g = grid_of(vcell);
+    int i, j, k;
+    cell_ijk(g, vcell - g.vbase, i, j, k);
+    const float* p = g.f + ((int64_t)k * g.ny + j) * g.nx + i;
+    const int64_t sy = g.nx, sz = (int64_t)g.nx * g.ny;
+    float* c = corners + threadIdx.x;
+#pragma unroll
+    for (int q = 0; q < 8; q++)
+      cp_async4(c + q * kVertexThreads, p + (q & 1) + (q & 2 ? sy : 0) + (q & 4 ? sz : 0));
+  };
+  // this iteration's record, crossed edges, rank and cell; the next one's slot
+  uint32_t r = 0, crossed = 0, vcell = 0, slot_next = 0;
+  int rank = 0;
+  if (first + lane < nv) {
+    const uint32_t slot = vwork[first + lane];
+    rank = vrank[first + lane];
+    r = rec[slot];
+    crossed = d_case_edges.m[__ldg(ccase + slot)];
+    vcell = slot_cell(cellof, slot);
+    fetch_corners(vcell);
+  }
+  if (first + step + lane < nv) slot_next = vwork[first + step + lane];
+  for (; first < nv; first += step) {
+    const int64_t vidx = first + lane, ahead = vidx + step;
+    const bool valid = vidx < nv, more = ahead < nv;
+    uint32_t r_next = 0, cs_next = 0, vcell_next = 0, slot_after = 0;
+    int rank_next = 0;
+    if (more) {
+      r_next = rec[slot_next];
+      cs_next = __ldg(ccase + slot_next);
+      vcell_next = slot_cell(cellof, slot_next);
+      rank_next = vrank[ahead];
+      if (ahead + step < nv) slot_after = vwork[ahead + step];
+    }
     int prj = -1;
     ffx::ff iso{0, 0};
+    cp_async_wait();
     if (valid) {
-      const uint32_t slot = vwork[vidx];
-      const int rank = vrank[vidx];
-      const uint32_t r = rec[slot];
-      const uint32_t crossed = d_case_edges.m[__ldg(ccase + slot)];
-      const uint32_t vcell = slot_cell(cellof, slot);
-      const Grid& g = kBatch ? space.grids[__ldg(space.tile_vol + vcell / kScanTile)] : space.one;
-      int i, j, k;
-      cell_ijk(g, vcell - g.vbase, i, j, k);
-      float c[8];
-      load_corners(g, i, j, k, c);
+      const Grid& g = grid_of(vcell);
 #pragma unroll
-      for (int q = 0; q < 8; q++) F[q] = c[q];
+      for (int q = 0; q < 8; q++) F[q] = corners[q * kVertexThreads + threadIdx.x];
       const uint32_t em = repr::edges_of_rank(rec_map(r), rank, crossed);
       const int n = __popc(em);
       // another contour of three edges excludes samples inside its box (one-pass kernels); in a cell
@@ -737,59 +819,103 @@ __global__ void __launch_bounds__(kVertexThreads) dmc_vertex_point_kernel(CellSp
       iso = ffx::ff{g.iso_f, g.iso_lo};
       if (!redo) prj = repr::vertex_frame(F, em, n, g.iso, iso, g.iso_exact);
     }
-    repr::SampleSet S;
-    uint64_t need = 0, seen = 0;
-    int q0 = 0;
-    bool ring = false;
-    if (prj >= 0) {
-      q0 = repr::seed_sample(F);
-      seen = 1ull << q0;
-      S.add(repr::sample_bound(F, q0), q0);
-      // the seed not surely valid: its neighbours before everything else
-      ring = !(S.m < INFINITY);
-      need = (ring ? repr::ring_of(q0) : repr::samples_within(F, S.m)) & ~seen;
+    uint32_t crossed_next = 0;
+    if (more) {
+      crossed_next = d_case_edges.m[cs_next];
+      fetch_corners(vcell_next);
     }
-    for (;;) {
-      const int c = __popcll(need);
+    // The search: the lane's first sample, then (shared) its neighbours when that one is not surely valid,
+    // then the samples whose in-plane distance is within the smallest upper bound.  smallest[lane] is
+    // that bound, tally[lane] counts the samples whose lower bound does not exceed it (a later window or
+    // round may lower it further: such a count is too large, never too small) and sums their numbers.
+    int q0 = 0;
+    if (prj >= 0) q0 = repr::seed_sample(F);
+    smallest[lane] = __float_as_uint(INFINITY);
+    tally[lane] = 0;
+    float seed_lb = INFINITY;
+    uint64_t need = 0, seen = 1ull << q0;
+    bool ring = false;
+    for (int round = 0;; round++) {
+      const int c = round ? __popcll(need) : 1;
       int upto = c;  // inclusive scan of the lanes' numbers
+      if (round) {
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(kAll, upto, o);
-        if (lane >= o) upto += y;
+        for (int o = 1; o < 32; o <<= 1) {
+          const int y = __shfl_up_sync(kAll, upto, o);
+          if (lane >= o) upto += y;
+        }
       }
-      const int from = upto - c, total = __shfl_sync(kAll, upto, 31);
+      const int from = upto - c, total = round ? __shfl_sync(kAll, upto, 31) : 32;
       for (int w = 0; w < total; w += kSampleWindow) {
         const int end = min(w + kSampleWindow, total);
-        __syncwarp();  // the frames are written, the previous window's bounds are read
-        if (from < end && upto > w) {
-          uint64_t m = need;
-          for (int k = from; k < min(upto, end); k++, m &= m - 1)
-            if (k >= w) item[k - w] = (uint16_t)(lane << 6 | (__ffsll((long long)m) - 1));
+        if (round) {
+          const int hi = min(upto, end);
+          __syncwarp();  // the frames are written, the previous window's entries are read
+          if (c <= kFewSamples && hi > w) {
+            uint64_t m = need;
+            for (int k = from; k < hi; k++, m &= m - 1)
+              if (k >= w) item[k - w] = (uint16_t)(lane << 6 | (__ffsll((long long)m) - 1));
+          }
+          for (unsigned x = __ballot_sync(kAll, c > kFewSamples && from < end && upto > w); x; x &= x - 1) {
+            const int o = __ffs(x) - 1;  // the owner
+            const unsigned m0 = __shfl_sync(kAll, (unsigned)need, o), m1 = __shfl_sync(kAll, (unsigned)(need >> 32), o);
+            const unsigned below = (1u << lane) - 1u;
+            const int k0 = __shfl_sync(kAll, from, o) - w + __popc(m0 & below);
+            const int k1 = __shfl_sync(kAll, from, o) - w + __popc(m0) + __popc(m1 & below);
+            if ((m0 >> lane & 1) && (unsigned)k0 < kSampleWindow) item[k0] = (uint16_t)(o << 6 | lane);
+            if ((m1 >> lane & 1) && (unsigned)k1 < kSampleWindow) item[k1] = (uint16_t)(o << 6 | 32 | lane);
+          }
+          __syncwarp();
         }
-        __syncwarp();
         for (int k = w + lane; k < end; k += 32) {
-          const int x = item[k - w];
-          bound[k - w] = repr::sample_bound(repr::FrameCol{warp_frames + (x >> 6), kVertexThreads}, x & 63);
+          const int x = round ? item[k - w] : lane << 6 | q0;
+          const repr::SampleBound b =
+              repr::sample_bound(repr::FrameCol{warp_frames + (x >> 6), kVertexThreads}, x & 63);
+          if (round) lower[k - w] = b.lb;
+          else seed_lb = b.lb;
+          if (b.ub < INFINITY) atomicMin(smallest + (x >> 6), __float_as_uint(b.ub));
         }
-        __syncwarp();
-        for (int k = max(from, w); k < min(upto, end); k++) S.add(bound[k - w], item[k - w] & 63);
+        if (round) {
+          __syncwarp();
+          for (int k = w + lane; k < end; k += 32) {
+            const int o = item[k - w] >> 6;
+            const float lb = lower[k - w];
+            if (lb < INFINITY && lb <= __uint_as_float(smallest[o])) atomicAdd(tally + o, 0x10000u + (item[k - w] & 63u));
+          }
+        }
       }
-      if (!__any_sync(kAll, ring)) break;
+      __syncwarp();
+      if (!__any_sync(kAll, round == 0 || ring)) break;
+      const float m = __uint_as_float(smallest[lane]);
+      // the seed not surely valid: its neighbours before everything else
+      const bool want = prj >= 0 && (round == 0 || ring);
+      ring = want && round == 0 && !(m < INFINITY);
+      need = 0;
+      if (want) need = (ring ? repr::ring_of(q0) : repr::samples_within(F, m)) & ~seen;
       seen |= need;
-      need = ring ? repr::samples_within(F, S.m) & ~seen : 0ull;
-      ring = false;
     }
+    const float m = __uint_as_float(smallest[lane]);
+    unsigned near = tally[lane];
+    if (seed_lb <= m) near += 0x10000u + q0;
     float p[3] = {0, 0, 0};
     int what = repr::kRedo;
-    if (prj >= 0 && S.decided()) what = repr::sample_point(F, S.q1, prj, iso, p);
+    // one sample's lower bound is within the smallest upper bound: it has that bound, is surely valid
+    // and the nearest
+    if (prj >= 0 && m < INFINITY && near >> 16 == 1) what = repr::sample_point(F, near & 0xffffu, prj, iso, p);
     __syncwarp();  // the frames are read
-    if (valid) {
-      append(list, count, what == repr::kRedo, (uint32_t)vidx);
-      append(wlist, count + 2, what == repr::kW64, (uint32_t)vidx);
+    if (valid)
       vp[vidx] =
           make_float4(p[0], p[1], p[2], what == repr::kFound ? 0.0f : (what == repr::kRedo ? 1.0f : 4.0f + prj));
-    }
+    redo_list.add(list, count, valid && what == repr::kRedo, (uint32_t)vidx);
+    w_list.add(wlist, count + 2, valid && what == repr::kW64, (uint32_t)vidx);
+    r = r_next;
+    crossed = crossed_next;
+    vcell = vcell_next;
+    rank = rank_next;
+    slot_next = slot_after;
   }
+  redo_list.finish(list, count);
+  w_list.finish(wlist, count + 2);
 }
 
 // The points whose last coordinate needs float64 (mostly bilinear values exactly on a float midpoint,
