@@ -342,28 +342,31 @@ __global__ void float_outputs_kernel(const double* v64, const double* n64, int64
 // ---------------------------------------------------------------------------------------------
 
 // removeVertices3X3Y / removeVertices3333 (:1096-1112, :1324-1338): kept vertices move to their
-// new index, which becomes their map entry.  One thread per vertex component (x, y or z of the
-// float64 positions and normals): every load and store is unit-stride across the warp.
-// vo, no: the float32 outputs of the kept vertices (the roundings float_outputs_kernel makes), or null
+// new index (idx[i] - idx[0]), which becomes their map entry.  One thread per vertex component (x, y or z):
+// every load and store is unit-stride across the warp.
+// Writes what the result keeps: the float32 positions and normals (roundings of the float64 positions and
+// float-pair normals) and, when they are an output (v64o), the float64 positions.  16.6 M vertices, 12 M
+// kept: 349 us with the float64 positions and the normals' pairs copied along (nothing reads them), 227 us.
 __global__ void gather_vertices_kernel(const uint8_t* keep, const int32_t* idx, int64_t nv, const double* v64,
-                                       const double* n64, double* v64o, double* n64o, int32_t* map, int64_t cap,
-                                       unsigned* overflow, float* vo, float* no) {
+                                       const double* n64, double* v64o, int32_t* map, int64_t cap, unsigned* overflow,
+                                       float* vo, float* no) {
+  const int first = idx[0];
   FOR_EACH(e, 3 * nv) {
-    const int64_t i = e / 3;
-    if (!keep[i]) continue;
-    const int64_t o = idx[i];
-    const int d = (int)(e - 3 * i);
+    const uint32_t i = (uint32_t)e / 3u, d = (uint32_t)e - 3u * i;  // 3 nv < 2^32
+    // all four loads before the first use: a third of the vertices goes, but a component read in vain
+    // costs less than one waited for
+    const uint8_t k = keep[i];
+    const int64_t o = (int64_t)idx[i] - first;
+    const double x = v64[e];
+    const float nn = reinterpret_cast<const float2*>(n64)[e].x;
+    if (!k) continue;
     if (o < 0 || o >= cap) {
       if (d == 0) atomicAdd(overflow, 1u);
       continue;
     }
-    const double x = v64[e], nn = n64[e];
-    v64o[3 * o + d] = x;
-    n64o[3 * o + d] = nn;
-    if (vo) {
-      vo[3 * o + d] = (float)x;
-      no[3 * o + d] = reinterpret_cast<const float2*>(n64)[e].x;
-    }
+    if (v64o) v64o[3 * o + d] = x;
+    vo[3 * o + d] = (float)x;
+    no[3 * o + d] = nn;
     if (d == 0) map[i] = (int32_t)o;
   }
 }
@@ -469,19 +472,22 @@ __global__ void apply_3333_kernel(int32_t* q, int64_t nq, uint8_t* alive, const 
 }
 
 // The live faces at their compacted indices, corners renumbered (vertex x -> vmap[x]); src[o]: the
-// face's index before.
-__global__ void gather_live_quads_kernel(const uint8_t* alive, const int32_t* idx, int64_t nq, const int32_t* q,
-                                         const int32_t* vmap, int32_t* qo, int32_t* src, int64_t cap,
-                                         unsigned* overflow) {
+// face's index before.  Bound by the latency of the gathers: 16-byte loads and stores (the arrays are
+// aligned), everything but the corners' numbers loaded before it is known whether the face is live.
+// 16.6 M faces: 164 -> 127 us.
+__global__ void gather_live_quads_kernel(const uint8_t* alive, const int32_t* idx, int64_t nq, const int4* q,
+                                         const int32_t* vmap, int4* qo, int32_t* src, int64_t cap, unsigned* overflow) {
   FOR_EACH(f, nq) {
-    if (!alive[f]) continue;
+    const uint8_t a = alive[f];
     const int64_t o = idx[f];
+    const int4 c = q[f];
+    if (!a) continue;
     if (o < 0 || o >= cap) {
       atomicAdd(overflow, 1u);
       continue;
     }
     src[o] = (int32_t)f;
-    for (int r = 0; r < 4; r++) qo[4 * o + r] = vmap[q[4 * f + r]];
+    qo[o] = make_int4(vmap[c.x], vmap[c.y], vmap[c.z], vmap[c.w]);
   }
 }
 
@@ -679,13 +685,15 @@ __device__ __forceinline__ bool split_exact(float d01, float d12, float d20, flo
 // noise field's, 40 % of the 1024x1024x64 saddle field's).  The lengths come from float pairs with
 // certified rounding; the quads with one that is not certified (a few per cent) are gathered in shared
 // memory and taken in float64 densely, a few lanes of most warps would occupy that pipe otherwise.
+// v64 and q64: the float64 positions and the quads that index them; src: the face there of each of q's
+// (null when they are the same mesh).
 // With twelve arc cosines per quad and every length in float64 the pass took 0.28 ms (noise, 0.38 million
 // quads listed) and 4.64 ms (saddle); 0.16 and 2.18 ms so.
 constexpr int kSplitThreads = 256;
 template <int kAcos>
 __global__ void __launch_bounds__(kSplitThreads) triangles_kernel(const int32_t* q, const uint32_t* list,
                                                                   const unsigned* count, const double* v64,
-                                                                  int32_t* t) {
+                                                                  const int32_t* q64, const int32_t* src, int32_t* t) {
   __shared__ uint32_t open[2 * kSplitThreads];
   __shared__ unsigned n_open;
   if (threadIdx.x == 0) n_open = 0;
@@ -697,8 +705,9 @@ __global__ void __launch_bounds__(kSplitThreads) triangles_kernel(const int32_t*
     if (a < nl) {
       const int64_t i = list[a];
       const int v0 = q[4 * i], v1 = q[4 * i + 1], v2 = q[4 * i + 2], v3 = q[4 * i + 3];
-      const PairPoint p0 = load_pairs(v64 + 3 * (int64_t)v0), p1 = load_pairs(v64 + 3 * (int64_t)v1),
-                      p2 = load_pairs(v64 + 3 * (int64_t)v2), p3 = load_pairs(v64 + 3 * (int64_t)v3);
+      const int32_t* c = q64 + 4 * (src ? (int64_t)src[i] : i);
+      const PairPoint p0 = load_pairs(v64 + 3 * (int64_t)c[0]), p1 = load_pairs(v64 + 3 * (int64_t)c[1]),
+                      p2 = load_pairs(v64 + 3 * (int64_t)c[2]), p3 = load_pairs(v64 + 3 * (int64_t)c[3]);
       float d01, d12, d20, d23, d30, d13;
       bool ok = side_certain(p0, p1, d01);
       ok = side_certain(p1, p2, d12) && ok;
@@ -715,8 +724,9 @@ __global__ void __launch_bounds__(kSplitThreads) triangles_kernel(const int32_t*
       for (unsigned x = threadIdx.x; x < n; x += kSplitThreads) {
         const int64_t i = open[x];
         const int v0 = q[4 * i], v1 = q[4 * i + 1], v2 = q[4 * i + 2], v3 = q[4 * i + 3];
-        const double *P0 = v64 + 3 * (int64_t)v0, *P1 = v64 + 3 * (int64_t)v1, *P2 = v64 + 3 * (int64_t)v2,
-                     *P3 = v64 + 3 * (int64_t)v3;
+        const int32_t* c = q64 + 4 * (src ? (int64_t)src[i] : i);
+        const double *P0 = v64 + 3 * (int64_t)c[0], *P1 = v64 + 3 * (int64_t)c[1], *P2 = v64 + 3 * (int64_t)c[2],
+                     *P3 = v64 + 3 * (int64_t)c[3];
         write_split(t, i, v0, v1, v2, v3,
                     split_exact<kAcos>(side_f64(P0, P1), side_f64(P1, P2), side_f64(P2, P0), side_f64(P2, P3),
                                        side_f64(P3, P0), side_f64(P1, P3)));
@@ -852,9 +862,8 @@ struct PassBufs {
   int32_t* owner;
   int32_t *own_pos, *own_rm, *vm_second;
   int4* jobs;
-  uint8_t *alive, *valive;    // adjacent
-  size_t alive_bytes;         // of both
-  int32_t *idx, *idx_q;
+  uint8_t *alive, *valive;    // faces, then vertices: one scan numbers both
+  int32_t *idx_q, *idx;       // likewise; vertex x becomes idx[x] - idx[0], and idx[0] faces are kept
 };
 PassBufs pass_buffers(Pool& pool, HeBufs& hw, int64_t NV, int64_t NQ) {
   PassBufs b;
@@ -883,11 +892,10 @@ PassBufs pass_buffers(Pool& pool, HeBufs& hw, int64_t NV, int64_t NQ) {
   b.own_rm = b.owner + NV;
   b.vm_second = b.owner + 2 * NV;
   b.jobs = pool.get<int4>(NQ);
-  b.alive_bytes = (size_t)(nq16 + NV);
-  b.alive = pool.get<uint8_t>(nq16 + NV);
-  b.valive = b.alive + nq16;
-  b.idx = pool.get<int32_t>(NV);
-  b.idx_q = pool.get<int32_t>(NQ);
+  b.alive = pool.get<uint8_t>(NQ + NV);
+  b.valive = b.alive + NQ;
+  b.idx_q = pool.get<int32_t>(NQ + NV);
+  b.idx = b.idx_q + NQ;
   return b;
 }
 
@@ -935,7 +943,7 @@ DmcPostStatus dmc_postprocess(const DmcMesh& in, uint32_t flags, int sms, cudaSt
 
   DmcMesh cur = in;
   HeBufs hw = halfedge_buffers(pool, NV, NQ);
-  unsigned long long* tiles = pool.get<unsigned long long>(scan_tiles(std::max(NV, NQ)) + 2);
+  unsigned long long* tiles = pool.get<unsigned long long>(scan_tiles(NV + NQ) + 2);
   unsigned long long* total = pool.get<unsigned long long>(2);
   if (pool.err) {
     s.err = pool.err;
@@ -969,8 +977,9 @@ DmcPostStatus dmc_postprocess(const DmcMesh& in, uint32_t flags, int sms, cudaSt
   // of what remains, and every rule that compares indices compares them in the same order).
   bool compacted = false;
   uint8_t *alive = nullptr, *valive = nullptr;
-  int32_t *idx = nullptr, *idx_q = nullptr;
+  int32_t *idx = nullptr, *idx_q = nullptr, *map = nullptr;
   int64_t nv0 = cur.nv, nq0 = cur.nq;  // the uncompacted mesh
+  int64_t nv2 = nv0, nq2 = nq0;        // and what is left of it
   int32_t* q0 = cur.quads;
   if (simplify) {
     const PassBufs b = pass_buffers(pool, hw, NV, NQ);
@@ -980,10 +989,21 @@ DmcPostStatus dmc_postprocess(const DmcMesh& in, uint32_t flags, int sms, cudaSt
     valive = b.valive;
     idx = b.idx;
     idx_q = b.idx_q;
+    map = b.vm_second;
     if ((s.err = pool.err) != cudaSuccess) return s;
-    cudaMemsetAsync(alive, 1, b.alive_bytes, st);
+    cudaMemsetAsync(alive, 1, (size_t)(NQ + NV), st);
     build_he(false);
     const HeView he{q0, hw.twin, hw.flag};
+    // what is left after the last pass, counted before its repair and the handles: they run while the host
+    // takes the counts and makes room for the result
+    cudaEvent_t counted = nullptr;
+    auto count_live = [&]() {
+      Stage tm(prof, "dmc_compact", st);
+      s.launches += scan_flags(alive, nq0 + nv0, idx_q, tiles, total, st);
+      cudaMemcpyAsync(h_cnt, total, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st);
+      cudaMemcpyAsync(h_cnt + 1, idx, sizeof(int32_t), cudaMemcpyDeviceToHost, st);
+      counted = host_mark(st);
+    };
     auto repair = [&]() {
       Stage tm(prof, "dmc_halfedges", st);
       HeOut ho{hw.twin, hw.flag, nullptr};
@@ -1012,6 +1032,7 @@ DmcPostStatus dmc_postprocess(const DmcMesh& in, uint32_t flags, int sms, cudaSt
         apply_3x3y_kernel<<<gq, 256, 0, st>>>(q0, nq0, alive, em, vm_first, vm_second, hw.dold, hw.dnew, hw.w.deg);
         s.launches += 5;
       }
+      if (!p3333 && (pass == 1 || !i3x3y)) count_live();
       repair();
     }
     // P3333
@@ -1030,6 +1051,7 @@ DmcPostStatus dmc_postprocess(const DmcMesh& in, uint32_t flags, int sms, cudaSt
         apply_3333_kernel<<<gq, 256, 0, st>>>(q0, nq0, alive, rflag, p3, vm1, hw.dold, hw.dnew, hw.w.deg);
         s.launches += 2;
       }
+      count_live();
       repair();
     }
     // the output's vertex handles and edge counts, on the uncompacted mesh (before it is released)
@@ -1038,52 +1060,73 @@ DmcPostStatus dmc_postprocess(const DmcMesh& in, uint32_t flags, int sms, cudaSt
       s.launches += halfedge_handles(q0, 4, nq0, nv0, alive, hw.twin, hw.flag, hw.hv, hw.w, hw.hcount, sms, st);
     }
     // ---- the one compaction: live vertices and faces, in order ----
-    Stage tm(prof, "dmc_compact", st);
-    s.launches += scan_flags(valive, nv0, idx, tiles, total, st);
-    s.launches += scan_flags(alive, nq0, idx_q, tiles, total + 1, st);
-    cudaMemcpyAsync(h_cnt, total, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st);
-    host_wait(st);
-    const int64_t nv2 = (int64_t)h_cnt[0], nq2 = (int64_t)h_cnt[1];
+    if ((s.err = host_wait_mark(counted, st)) != cudaSuccess) return s;
+    nq2 = (int64_t) * reinterpret_cast<const int32_t*>(h_cnt + 1);
+    nv2 = (int64_t)h_cnt[0] - nq2;
     // nothing died: no pass changed the mesh, and it stays as it is (with its halfedges)
-    if (nv2 != nv0 || nq2 != nq0) {
-      DmcMesh nx = cur;
-      void *a = nullptr, *b = nullptr, *c = nullptr, *d = nullptr, *qn = nullptr;
-      const size_t nvb = (size_t)std::max<int64_t>(nv2, 1) * 3;
-      if ((s.err = cudaMallocAsync(&a, nvb * sizeof(double), st)) != cudaSuccess) return s;
-      adopt(a);
-      if ((s.err = cudaMallocAsync(&b, nvb * sizeof(float), st)) != cudaSuccess) return s;
-      adopt(b);
-      if ((s.err = cudaMallocAsync(&c, nvb * sizeof(float), st)) != cudaSuccess) return s;
-      adopt(c);
-      if ((s.err = cudaMallocAsync(&d, nvb * sizeof(double), st)) != cudaSuccess) return s;
-      adopt(d);
-      if ((s.err = cudaMallocAsync(&qn, (size_t)std::max<int64_t>(nq2, 1) * 4 * sizeof(int32_t), st)) != cudaSuccess)
-        return s;
-      adopt(qn);
-      nx.v64 = (double*)a;
-      nx.v = (float*)b;
-      nx.n = (float*)c;
-      nx.n64 = (double*)d;
-      nx.quads = (int32_t*)qn;
-      nx.nv = nv2;
-      nx.nq = nq2;
-      // vertex map into vm_second (free after the passes)
-      gather_vertices_kernel<<<grid_for(3 * nv0, sms), 256, 0, st>>>(valive, idx, nv0, cur.v64, cur.n64, nx.v64,
-                                                                     nx.n64, vm_second, nv2, hw.ovf, nx.v, nx.n);
-      gather_live_quads_kernel<<<gq, 256, 0, st>>>(alive, idx_q, nq0, q0, vm_second, nx.quads, hw.src, nq2, hw.ovf);
-      s.launches += 2;
-      // the inherited colours are only read by the colour pass; they are not carried along
-      retire(cur.v64);
+    compacted = nv2 != nv0 || nq2 != nq0;
+    if (compacted) {  // made anew below
       retire(cur.v);
       retire(cur.n);
-      retire(cur.n64);
-      retire(cur.quads);
-      cur = nx;
-      compacted = true;
+      cur.v = cur.n = nullptr;
     }
   }
-  // the float32 outputs of the simplified mesh (the compaction's gather writes them when it ran)
-  if (s.err == cudaSuccess && simplify && !compacted && cur.nv > 0) {
+  // The result's arrays in one allocation: made one by one behind the frees of what they replace, the pool
+  // mapped memory anew for them (1.4 ms of a 512^3 call's 12.4, the GPU waiting).
+  struct Part {
+    void** p;
+    size_t bytes;
+  };
+  std::vector<Part> parts;
+  auto part = [&](auto** p, int64_t count) {
+    parts.push_back(Part{reinterpret_cast<void**>(p), ((size_t)std::max<int64_t>(count, 1) * sizeof(**p) + 255) & ~(size_t)255});
+  };
+  DmcMesh nx = cur;
+  nx.nv = nv2;
+  nx.nq = nq2;
+  const bool new_floats = !cur.v;  // compacted, or left to be made here
+  if (new_floats) {
+    part(&nx.v, 3 * nv2);
+    part(&nx.n, 3 * nv2);
+  }
+  if (compacted) {
+    nx.v64 = nx.n64 = nullptr;
+    if (flags & TMC_OUT_POS_F64) part(&nx.v64, 3 * nv2);
+    part(&nx.quads, 4 * nq2);
+  }
+  int32_t *he4 = nullptr, *hv = nullptr, *hf = nullptr, *tr = nullptr;
+  if (want_he) {
+    part(&he4, 16 * nq2);
+    part(&hv, nv2);
+    part(&hf, nq2);
+  }
+  if (want_t) part(&tr, 6 * nq2);
+  if (!parts.empty()) {
+    size_t bytes = 0;
+    for (const Part& x : parts) bytes += x.bytes;
+    void* block = nullptr;
+    if ((s.err = cudaMallocAsync(&block, bytes, st)) != cudaSuccess) return s;
+    adopt(block);
+    char* at = (char*)block;
+    for (const Part& x : parts) {
+      *x.p = at;
+      at += x.bytes;
+    }
+  }
+  const DmcMesh old = cur;  // the uncompacted mesh
+  cur = nx;
+  if (compacted) {
+    Stage tm(prof, "dmc_compact", st);
+    // vertex map into vm_second (free after the passes)
+    gather_vertices_kernel<<<grid_for(3 * nv0, sms), 256, 0, st>>>(valive, idx, nv0, old.v64, old.n64, cur.v64, map, nv2,
+                                                                   hw.ovf, cur.v, cur.n);
+    gather_live_quads_kernel<<<gq, 256, 0, st>>>(alive, idx_q, nq0, reinterpret_cast<const int4*>(q0), map,
+                                                 reinterpret_cast<int4*>(cur.quads), hw.src, nq2, hw.ovf);
+    s.launches += 2;
+    // the inherited colours are only read by the colour pass; they are not carried along
+    retire(old.n64);
+  } else if ((simplify || new_floats) && cur.nv > 0) {
+    // the float32 outputs of a mesh no pass changed
     float_outputs_kernel<<<grid_for(3 * cur.nv, sms), 256, 0, st>>>(cur.v64, cur.n64, 3 * cur.nv, cur.v, cur.n);
     s.launches += 1;
   }
@@ -1094,61 +1137,53 @@ DmcPostStatus dmc_postprocess(const DmcMesh& in, uint32_t flags, int sms, cudaSt
     if (flags & TMC_OUT_POS_F64) (*ready)(cur.v64, (size_t)cur.nv * 3 * sizeof(double));
     (*ready)(cur.quads, (size_t)cur.nq * 4 * sizeof(int32_t));
   }
-  if (s.err == cudaSuccess && want_he) {
+  if (want_he) {
     if (!simplify) build_he(true);  // the front-end mesh as it is: one build with the handles
-    void *he4 = nullptr, *hv = nullptr, *hf = nullptr;
-    if ((s.err = cudaMallocAsync(&he4, std::max<int64_t>(4 * cur.nq, 1) * 4 * sizeof(int32_t), st)) == cudaSuccess &&
-        (s.err = cudaMallocAsync(&hv, std::max<int64_t>(cur.nv, 1) * sizeof(int32_t), st)) == cudaSuccess &&
-        (s.err = cudaMallocAsync(&hf, std::max<int64_t>(cur.nq, 1) * sizeof(int32_t), st)) == cudaSuccess) {
-      adopt(he4);
-      adopt(hv);
-      adopt(hf);
-      Stage tm(prof, "dmc_halfedges", st);
-      if (compacted) {
-        s.launches += pack_compacted_halfedges(cur.quads, cur.nq, hw.src, idx_q, hw.twin, (int32_t*)he4, (int32_t*)hf,
-                                               valive, idx, nv0, hw.hv, (int32_t*)hv, sms, st);
-      } else {
-        s.launches += pack_halfedges4(cur.quads, 4, hw.twin, 4 * cur.nq, (int32_t*)he4, (int32_t*)hf, sms, st);
-        cudaMemcpyAsync(hv, hw.hv, cur.nv * sizeof(int32_t), cudaMemcpyDeviceToDevice, st);
-      }
-      if (ready) {
-        (*ready)(he4, (size_t)cur.nq * 16 * sizeof(int32_t));
-        (*ready)(hv, (size_t)cur.nv * sizeof(int32_t));
-        (*ready)(hf, (size_t)cur.nq * sizeof(int32_t));
-      }
-      // read by the caller when the stream is done (the compaction's counts in h_cnt are read by now)
-      cudaMemcpyAsync(h_cnt + 2, hw.nm, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st);
-      out->non_manifold = h_cnt + 2;
-      out->nhe = 4 * cur.nq;
-      out->he = (int32_t*)he4;
-      out->he_v = (int32_t*)hv;
-      out->he_f = (int32_t*)hf;
+    Stage tm(prof, "dmc_halfedges", st);
+    if (compacted) {
+      s.launches += pack_compacted_halfedges(cur.quads, cur.nq, hw.src, idx_q, hw.twin, he4, hf, valive, idx, nv0, hw.hv,
+                                             hv, sms, st);
+    } else {
+      s.launches += pack_halfedges4(cur.quads, 4, hw.twin, 4 * cur.nq, he4, hf, sms, st);
+      cudaMemcpyAsync(hv, hw.hv, cur.nv * sizeof(int32_t), cudaMemcpyDeviceToDevice, st);
     }
+    if (ready) {
+      (*ready)(he4, (size_t)cur.nq * 16 * sizeof(int32_t));
+      (*ready)(hv, (size_t)cur.nv * sizeof(int32_t));
+      (*ready)(hf, (size_t)cur.nq * sizeof(int32_t));
+    }
+    // read by the caller when the stream is done (the compaction's counts in h_cnt are read by now)
+    cudaMemcpyAsync(h_cnt + 2, hw.nm, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st);
+    out->non_manifold = h_cnt + 2;
+    out->nhe = 4 * cur.nq;
+    out->he = he4;
+    out->he_v = hv;
+    out->he_f = hf;
   }
-  if (s.err == cudaSuccess && want_t) {
-    void* tr = nullptr;
-    if ((s.err = cudaMallocAsync(&tr, std::max<int64_t>(2 * cur.nq, 1) * 3 * sizeof(int32_t), st)) == cudaSuccess) {
-      adopt(tr);
-      Stage tm(prof, "dmc_triangles", st);
-      uint32_t* tlist = pool.get<uint32_t>(std::max<int64_t>(cur.nq, 1));
-      unsigned* tcount = reinterpret_cast<unsigned*>(hw.zero + kZeroSplit);
-      if ((s.err = pool.err) == cudaSuccess) {
-        triangles_fast_kernel<<<grid_for(cur.nq, sms), 256, 0, st>>>(cur.quads, cur.nq, cur.v, (int32_t*)tr, tlist,
-                                                                      tcount);
-        const unsigned gt = grid_for(cur.nq, sms);
-        const int kind = libm::host_acosf_kind();
-#define TRIANGLES(K) \
-  triangles_kernel<K><<<gt, kSplitThreads, 0, st>>>(cur.quads, tlist, tcount, cur.v64, (int32_t*)tr)
-        if (kind == libm::kAcosfFused) TRIANGLES(libm::kAcosfFused);
-        else if (kind == libm::kAcosfSeparate) TRIANGLES(libm::kAcosfSeparate);
-        else TRIANGLES(libm::kAcosfCorrect);
+  if (want_t) {
+    Stage tm(prof, "dmc_triangles", st);
+    uint32_t* tlist = pool.get<uint32_t>(std::max<int64_t>(cur.nq, 1));
+    unsigned* tcount = reinterpret_cast<unsigned*>(hw.zero + kZeroSplit);
+    if ((s.err = pool.err) == cudaSuccess) {
+      triangles_fast_kernel<<<grid_for(cur.nq, sms), 256, 0, st>>>(cur.quads, cur.nq, cur.v, tr, tlist, tcount);
+      const unsigned gt = grid_for(cur.nq, sms);
+      const int kind = libm::host_acosf_kind();
+      // positions from the uncompacted mesh, by its quads
+#define TRIANGLES(K)                                                                                               \
+  triangles_kernel<K><<<gt, kSplitThreads, 0, st>>>(cur.quads, tlist, tcount, old.v64, q0, compacted ? hw.src : nullptr, tr)
+      if (kind == libm::kAcosfFused) TRIANGLES(libm::kAcosfFused);
+      else if (kind == libm::kAcosfSeparate) TRIANGLES(libm::kAcosfSeparate);
+      else TRIANGLES(libm::kAcosfCorrect);
 #undef TRIANGLES
-        s.launches += 2;
-        if (ready) (*ready)(tr, (size_t)cur.nq * 6 * sizeof(int32_t));
-      }
-      out->nt = 2 * cur.nq;
-      out->tris = (int32_t*)tr;
+      s.launches += 2;
+      if (ready) (*ready)(tr, (size_t)cur.nq * 6 * sizeof(int32_t));
     }
+    out->nt = 2 * cur.nq;
+    out->tris = tr;
+  }
+  if (compacted) {
+    retire(old.v64);
+    retire(old.quads);
   }
   {
     std::vector<void*> keepv;

@@ -12,7 +12,7 @@ namespace tmc {
 
 struct DmcMesh {
   int64_t nv = 0, nq = 0;
-  float* v = nullptr;
+  float* v = nullptr;  // null on entry to a simplification: made from v64 and n64 after the passes
   float* n = nullptr;
   double* v64 = nullptr;
   double* n64 = nullptr;  // normals while simplifying, float pairs (hi, lo) per 8-byte slot (merges average them in float64)

@@ -437,13 +437,14 @@ __global__ void he_pack_compacted_kernel(const int32_t* faces, int64_t nh, const
   }
 }
 
-// handles of the kept vertices in the compacted numbering (vertex x became vidx[x])
+// handles of the kept vertices in the compacted numbering (vertex x became vidx[x] - vidx[0])
 __global__ void he_handles_compacted_kernel(const uint8_t* vkeep, const int32_t* vidx, int64_t nv, const int32_t* hv,
                                             const int32_t* fidx, int32_t* hv_out) {
+  const int first = vidx[0];
   for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < nv; x += (int64_t)gridDim.x * blockDim.x) {
     if (!vkeep[x]) continue;
     const int h = hv[x];
-    hv_out[vidx[x]] = h < 0 ? -1 : 4 * fidx[h >> 2] + (h & 3);
+    hv_out[vidx[x] - first] = h < 0 ? -1 : 4 * fidx[h >> 2] + (h & 3);
   }
 }
 

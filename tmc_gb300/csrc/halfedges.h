@@ -60,7 +60,7 @@ int halfedge_handles(const int32_t* faces, int P, int64_t nf, int64_t nv, const 
                      const uint8_t* flag, int32_t* hv, HeWork& w, unsigned long long* counts, int sms,
                      cudaStream_t st);
 // Output halfedge records, face handles and vertex handles of a compacted quad mesh (faces: its nf
-// quads; new face f was face src[f], kept face g became fidx[g], kept vertex x became vidx[x]) from
+// quads; new face f was face src[f], kept face g became fidx[g], kept vertex x became vidx[x] - vidx[0]) from
 // the twins and handles (hv) built on the uncompacted mesh.
 int pack_compacted_halfedges(const int32_t* faces, int64_t nf, const int32_t* src, const int32_t* fidx,
                              const int32_t* twin, int32_t* he4, int32_t* hf, const uint8_t* vkeep, const int32_t* vidx,

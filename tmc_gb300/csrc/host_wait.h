@@ -12,14 +12,14 @@
 
 namespace tmc {
 
-// Waits for the work queued on `st` so far.  The event belongs to the current device; when it
-// cannot be recorded on `st` (a stream of another device, or an event left from before a device
-// reset, which is replaced once) the wait falls back to cudaStreamSynchronize.
-inline cudaError_t host_wait(cudaStream_t st) {
+// Marks the work queued on `st` so far, for host_wait_mark on the same thread (before its next mark).
+// The event belongs to the current device; null when it cannot be recorded on `st` (a stream of another
+// device, or an event left from before a device reset, which is replaced once).
+inline cudaEvent_t host_mark(cudaStream_t st) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) {
     (void)cudaGetLastError();
-    return cudaStreamSynchronize(st);
+    return nullptr;
   }
   thread_local std::vector<cudaEvent_t> events;  // by device
   if ((int)events.size() <= dev) events.resize(dev + 1, nullptr);
@@ -30,23 +30,30 @@ inline cudaError_t host_wait(cudaStream_t st) {
       events[dev] = nullptr;
       break;
     }
-    if (cudaEventRecord(events[dev], st) == cudaSuccess) {
-      // a query that is not ready yet counts as the thread's last error: poll only when there is none to
-      // lose, and take each one back
-      if (cudaPeekAtLastError() == cudaSuccess) {
-        const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(60);
-        do {
-          const cudaError_t e = cudaEventQuery(events[dev]);
-          if (e != cudaErrorNotReady) return e;
-          (void)cudaGetLastError();
-        } while (std::chrono::steady_clock::now() < until);
-      }
-      return cudaEventSynchronize(events[dev]);
-    }
+    if (cudaEventRecord(events[dev], st) == cudaSuccess) return events[dev];
     (void)cudaGetLastError();
     events[dev] = nullptr;
   }
-  return cudaStreamSynchronize(st);
+  return nullptr;
 }
+
+// Waits for the marked work; without a mark, for all of the stream's.
+inline cudaError_t host_wait_mark(cudaEvent_t mark, cudaStream_t st) {
+  if (!mark) return cudaStreamSynchronize(st);
+  // a query that is not ready yet counts as the thread's last error: poll only when there is none to
+  // lose, and take each one back
+  if (cudaPeekAtLastError() == cudaSuccess) {
+    const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(60);
+    do {
+      const cudaError_t e = cudaEventQuery(mark);
+      if (e != cudaErrorNotReady) return e;
+      (void)cudaGetLastError();
+    } while (std::chrono::steady_clock::now() < until);
+  }
+  return cudaEventSynchronize(mark);
+}
+
+// Waits for the work queued on `st` so far.
+inline cudaError_t host_wait(cudaStream_t st) { return host_wait_mark(host_mark(st), st); }
 
 }  // namespace tmc

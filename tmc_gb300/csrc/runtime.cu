@@ -751,8 +751,10 @@ tmc_status dmc_extract(tmc_ctx* ctx, const tmc_volume* vol, double iso, uint32_t
     }                                       \
     own(ptr);                               \
   } while (0)
-  TMC_GET(vo.v, 3 * nv);
-  TMC_GET(vo.n, 3 * nv);
+  if (!simplify) {  // the post-processing makes a simplified mesh's float32 arrays
+    TMC_GET(vo.v, 3 * nv);
+    TMC_GET(vo.n, 3 * nv);
+  }
   // simplification and the triangle split work on float64 positions, as the reference does
   const bool need_f64 = (flags & (TMC_OUT_POS_F64 | TMC_OUT_TRIANGLES)) || simplify;
   if (need_f64) TMC_GET(vo.v64, 3 * nv);
