@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include "ffloat.cuh"
+#include "launch.cuh"
 #include "mc_tables.h"
 
 namespace tmc {
@@ -112,7 +113,7 @@ struct CellSpace {
   int64_t max_bit_words;    // batch: of the largest volume
   __device__ __forceinline__ Grid grid_of_tile(int64_t tile) const {
     if (!grids) return one;
-    return grids[__ldg(tile_vol + tile)];
+    return grids[ld(tile_vol + tile)];
   }
 };
 
@@ -129,12 +130,12 @@ struct CellMask {
 };
 constexpr int kTileShift = 11;  // kScanTile = 2048 cells per scan tile
 __device__ __forceinline__ uint32_t listed_slot(const CellMask* mask, uint32_t vc) {
-  const uint2 a = __ldg(reinterpret_cast<const uint2*>(mask) + (vc >> 5));
+  const uint2 a = ld(reinterpret_cast<const uint2*>(mask) + (vc >> 5));
   return ((vc >> kTileShift) << kTileShift) + a.y + __popc(a.x & ((1u << (vc & 31)) - 1u));
 }
 // number of listed cells of a tile
 __device__ __forceinline__ uint32_t tile_listed(const CellMask* mask, int64_t tile) {
-  const uint2 a = __ldg(reinterpret_cast<const uint2*>(mask) + (tile << (kTileShift - 5)) + 63);
+  const uint2 a = ld(reinterpret_cast<const uint2*>(mask) + (tile << (kTileShift - 5)) + 63);
   return a.y + __popc(a.x);
 }
 // Chunk q of 32 slots when the chunks of all tiles are walked without a list of the non-empty ones (the
@@ -156,7 +157,7 @@ __host__ __device__ __forceinline__ void slot_chunk(int64_t q, int64_t tiles, in
 }
 // the cell behind a slot (cell: in-tile cell offsets of the listed cells)
 __device__ __forceinline__ uint32_t slot_cell(const uint16_t* cell, uint32_t slot) {
-  return ((slot >> kTileShift) << kTileShift) + __ldg(cell + slot);
+  return ((slot >> kTileShift) << kTileShift) + ld(cell + slot);
 }
 
 inline CellSpace single_space(const Grid& g) {

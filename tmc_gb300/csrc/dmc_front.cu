@@ -70,6 +70,7 @@ __global__ void __launch_bounds__(kClassifyThreads) dmc_classify_kernel(CellSpac
                                                                           unsigned long long* tile_sums,
                                                                           unsigned long long* stats,
                                                                           uint32_t* amb_list, unsigned* amb_n) {
+  pdl_begin();
   constexpr unsigned kAll = 0xffffffffu;
   constexpr int kTiles = kClassifyThreads / 32 / kPerTile;  // tiles per block
   __shared__ uint16_t lists[kTiles][kScanTile];
@@ -154,6 +155,7 @@ __global__ void __launch_bounds__(kClassifyThreads) dmc_classify_kernel(CellSpac
 __global__ void __launch_bounds__(128) dmc_amb_kernel(CellSpace space, const uint16_t* cellof, uint32_t* rec,
                                                       unsigned long long* tile_sums, const uint32_t* list,
                                                       const unsigned* count) {
+  pdl_begin();
   __shared__ uint64_t cc[256];
   for (int c = threadIdx.x; c < 256; c += blockDim.x) cc[c] = c_case_contour[c];
   __syncthreads();
@@ -182,6 +184,7 @@ __global__ void __launch_bounds__(32 * kOffsetWarps) dmc_offsets_kernel(const Ce
                                                                        int64_t tiles, uint2* rv, int32_t* qoff,
                                                                        uint32_t* vwork, uint8_t* vrank,
                                                                        uint32_t* chunks, unsigned* nchunks) {
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const int64_t tile = (int64_t)blockIdx.x * kOffsetWarps + (threadIdx.x >> 5);
   const uint32_t listed = tile < tiles ? tile_listed(mask, tile) : 0;
@@ -341,7 +344,7 @@ struct GridCache {
   Grid g{};
   ffx::ff iso_ff{0, 0};
   __device__ __forceinline__ void load(const CellSpace& space, uint32_t vcell) {
-    const int v = space.grids ? __ldg(space.tile_vol + vcell / kScanTile) : 0;
+    const int v = space.grids ? ld(space.tile_vol + vcell / kScanTile) : 0;
     if (v == vol) return;
     vol = v;
     g = space.grids ? space.grids[v] : space.one;
@@ -514,6 +517,7 @@ __global__ void __launch_bounds__(kVertexThreads) dmc_vertex_kernel(CellSpace sp
                                                                      unsigned* tail_count, unsigned warp_max,
                                                                      DmcVertexOut out, int flip_all,
                                                                      unsigned long long* stats) {
+  pdl_begin();
   __shared__ uint64_t cc[256];
   __shared__ float sample_lb[49 * kVertexThreads];  // per-thread sample bounds, column per thread
   const unsigned n = *count;
@@ -571,6 +575,7 @@ __global__ void __launch_bounds__(kVertexThreads) dmc_vertex_warp_kernel(CellSpa
                                                                           const unsigned* tail_count,
                                                                           unsigned warp_max, DmcVertexOut out,
                                                                           int flip_all, unsigned long long* stats) {
+  pdl_begin();
   constexpr int kWarps = kVertexThreads / 32;
   __shared__ uint64_t cc[256];
   __shared__ float coords[kWarps][2][26];  // each warp's sample coordinates
@@ -746,6 +751,7 @@ __global__ void __launch_bounds__(kVertexThreads) dmc_vertex_point_kernel(CellSp
                                                                           const uint8_t* vrank, const uint32_t* vwork,
                                                                           int64_t nv, float4* vp, uint32_t* list,
                                                                           uint32_t* wlist, unsigned* count) {
+  pdl_begin();
   constexpr int kWarps = kVertexThreads / 32;
   constexpr unsigned kAll = 0xffffffffu;
   __shared__ float frames[repr::kFrameFloats * kVertexThreads];
@@ -764,7 +770,7 @@ __global__ void __launch_bounds__(kVertexThreads) dmc_vertex_point_kernel(CellSp
   const int64_t step = (int64_t)gridDim.x * kVertexThreads;
   int64_t first = ((int64_t)blockIdx.x * kWarps + wid) * 32;  // warp-uniform
   auto grid_of = [&](uint32_t vcell) -> const Grid& {
-    return kBatch ? space.grids[__ldg(space.tile_vol + vcell / kScanTile)] : space.one;
+    return kBatch ? space.grids[ld(space.tile_vol + vcell / kScanTile)] : space.one;
   };
   auto fetch_corners = [&](uint32_t vcell) {
     const Grid& g = grid_of(vcell);
@@ -784,7 +790,7 @@ __global__ void __launch_bounds__(kVertexThreads) dmc_vertex_point_kernel(CellSp
     const uint32_t slot = vwork[first + lane];
     rank = vrank[first + lane];
     r = rec[slot];
-    crossed = d_case_edges.m[__ldg(ccase + slot)];
+    crossed = d_case_edges.m[ld(ccase + slot)];
     vcell = slot_cell(cellof, slot);
     fetch_corners(vcell);
   }
@@ -796,7 +802,7 @@ __global__ void __launch_bounds__(kVertexThreads) dmc_vertex_point_kernel(CellSp
     int rank_next = 0;
     if (more) {
       r_next = rec[slot_next];
-      cs_next = __ldg(ccase + slot_next);
+      cs_next = ld(ccase + slot_next);
       vcell_next = slot_cell(cellof, slot_next);
       rank_next = vrank[ahead];
       if (ahead + step < nv) slot_after = vwork[ahead + step];
@@ -926,11 +932,12 @@ __global__ void __launch_bounds__(kVertexThreads) dmc_vertex_w_kernel(CellSpace 
                                                                       const uint32_t* vwork, const uint32_t* wlist,
                                                                       const unsigned* count, float4* vp,
                                                                       unsigned long long* stats) {
+  pdl_begin();
   const unsigned n = count[2];
   for (unsigned a = blockIdx.x * blockDim.x + threadIdx.x; a < n; a += gridDim.x * blockDim.x) {
     const uint32_t vidx = wlist[a];
     const uint32_t vcell = slot_cell(cellof, vwork[vidx]);
-    const Grid& g = space.grids ? space.grids[__ldg(space.tile_vol + vcell / kScanTile)] : space.one;
+    const Grid& g = space.grids ? space.grids[ld(space.tile_vol + vcell / kScanTile)] : space.one;
     int i, j, k;
     cell_ijk(g, vcell - g.vbase, i, j, k);
     float u[8];
@@ -1055,6 +1062,7 @@ __global__ void __launch_bounds__(kVertexThreads) dmc_vertex_search_kernel(CellS
                                                                            const uint32_t* list, unsigned* count,
                                                                            unsigned warp_max, float4* vp, uint32_t* hard,
                                                                            unsigned long long* stats) {
+  pdl_begin();
   constexpr unsigned kAll = 0xffffffffu;
   __shared__ float frames[repr::kFrameFloats * kVertexThreads];
   const repr::FrameCol F{frames + threadIdx.x, kVertexThreads};
@@ -1067,9 +1075,9 @@ __global__ void __launch_bounds__(kVertexThreads) dmc_vertex_search_kernel(CellS
     const uint32_t vidx = list[a];
     const uint32_t slot = vwork[vidx];
     const uint32_t r = rec[slot];
-    const unsigned cs = __ldg(ccase + slot);
+    const unsigned cs = ld(ccase + slot);
     const uint32_t vcell = slot_cell(cellof, slot);
-    const Grid& g = space.grids ? space.grids[__ldg(space.tile_vol + vcell / kScanTile)] : space.one;
+    const Grid& g = space.grids ? space.grids[ld(space.tile_vol + vcell / kScanTile)] : space.one;
     int i, j, k;
     cell_ijk(g, vcell - g.vbase, i, j, k);
     ffx::ff mean[3];
@@ -1137,13 +1145,14 @@ __global__ void __launch_bounds__(kVertexThreads) dmc_vertex_finish_kernel(CellS
                                                                          int64_t nv, const float4* vp,
                                                                          DmcVertexOut out, int flip_all,
                                                                          unsigned long long* stats) {
+  pdl_begin();
   repr::Stats st;
   for (int64_t vidx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; vidx < nv;
        vidx += (int64_t)gridDim.x * blockDim.x) {
     const float4 q = vp[vidx];
     if (q.w != 0.0f) continue;  // done by the one-pass kernel
     const uint32_t vcell = slot_cell(cellof, vwork[vidx]);
-    const Grid& g = kBatch ? space.grids[__ldg(space.tile_vol + vcell / kScanTile)] : space.one;
+    const Grid& g = kBatch ? space.grids[ld(space.tile_vol + vcell / kScanTile)] : space.one;
     const int64_t cell = vcell - g.vbase;
     int i, j, k;
     cell_ijk(g, cell, i, j, k);
@@ -1188,18 +1197,19 @@ __global__ void __launch_bounds__(kQuadThreads) dmc_quad_kernel(CellSpace space,
                                                                 const unsigned long long* tile_off,
                                                                 const uint32_t* chunks, const unsigned* nchunks,
                                                                 int32_t* quads, uint8_t* colors) {
+  pdl_begin();
   constexpr int kWarps = kQuadThreads / 32;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const unsigned n = *nchunks;
   for (unsigned c = blockIdx.x * kWarps + wid; c < n; c += gridDim.x * kWarps) {
-    const uint32_t chunk = __ldg(chunks + c), slot = (chunk & ~31u) + lane;
+    const uint32_t chunk = ld(chunks + c), slot = (chunk & ~31u) + lane;
     if ((uint32_t)lane > (chunk & 31u)) continue;  // the chunk's number of cells minus one
-    const uint2 own = __ldg(rv + slot);
+    const uint2 own = ld(rv + slot);
     if (rec_nq(own.x) == 0) continue;
-    const unsigned cs = __ldg(ccase + slot);
+    const unsigned cs = ld(ccase + slot);
     const uint32_t vc = slot_cell(cellof, slot);
-    const Grid& g = kBatch ? space.grids[__ldg(space.tile_vol + vc / kScanTile)] : space.one;
-    const int32_t vfirst = kBatch ? (int32_t)(__ldg(tile_off + g.vbase / kScanTile) >> 32) : 0;
+    const Grid& g = kBatch ? space.grids[ld(space.tile_vol + vc / kScanTile)] : space.one;
+    const int32_t vfirst = kBatch ? (int32_t)(ld(tile_off + g.vbase / kScanTile) >> 32) : 0;
     int i, j, k;
     cell_ijk(g, vc - g.vbase, i, j, k);
     // from the cell's MC case (bit v: corner v at or above the isovalue): corner 0's side, and the
@@ -1218,9 +1228,9 @@ __global__ void __launch_bounds__(kQuadThreads) dmc_quad_kernel(CellSpace space,
     for (int s = 0; s < 6; s++) ns[s] = want[s] ? listed_slot(mask, vc - off[s]) : 0u;
     uint2 o[6];
 #pragma unroll
-    for (int s = 0; s < 6; s++) o[s] = want[s] ? __ldg(rv + ns[s]) : make_uint2(0, 0);
+    for (int s = 0; s < 6; s++) o[s] = want[s] ? ld(rv + ns[s]) : make_uint2(0, 0);
     auto vertex = [vfirst](uint2 r, int e) { return (int32_t)r.y - vfirst + rec_rank(r.x, e); };
-    int64_t q = __ldg(qoff + slot);
+    int64_t q = ld(qoff + slot);
     const int par = (i & 1) | ((j & 1) << 1) | ((k & 1) << 2);
     if (x) {
       const int32_t v[4] = {vertex(o[0], 6), vertex(o[1], 4), vertex(o[3], 2), vertex(own, 0)};
@@ -1257,10 +1267,10 @@ int dmc_front_count(const CellSpace& space, DmcScratch& s, int sms, cudaStream_t
       if (t1 <= t0) return;
       uint32_t* amb = reinterpret_cast<uint32_t*>(s.qoff);
       if (block_per_tile(t1 - t0, sms))
-        dmc_classify_kernel<8><<<(unsigned)(t1 - t0), kClassifyThreads, 0, st>>>(
+        launch(dmc_classify_kernel<8>, (unsigned)(t1 - t0), kClassifyThreads, st, 
             space, t0, t1, s.rec, s.cellof, s.ccase, s.mask, s.tile_sums, s.stats, amb, s.amb_n);
       else
-        dmc_classify_kernel<1><<<(unsigned)ceil_div(t1 - t0, kClassifyThreads / 32), kClassifyThreads, 0, st>>>(
+        launch(dmc_classify_kernel<1>, (unsigned)ceil_div(t1 - t0, kClassifyThreads / 32), kClassifyThreads, st, 
             space, t0, t1, s.rec, s.cellof, s.ccase, s.mask, s.tile_sums, s.stats, amb, s.amb_n);
       k++;
     };
@@ -1276,12 +1286,12 @@ int dmc_front_count(const CellSpace& space, DmcScratch& s, int sms, cudaStream_t
     }
     // one wave; the list length is only known on the device, so the grid follows the cell count
     static const int r_amb = resident_blocks(dmc_amb_kernel, 128);
-    dmc_amb_kernel<<<(unsigned)wave_grid(r_amb, sms, 16, ceil_div(space.n, 128), 128), 128, 0, st>>>(
+    launch(dmc_amb_kernel, (unsigned)wave_grid(r_amb, sms, 16, ceil_div(space.n, 128), 128), 128, st, 
         space, s.cellof, s.rec, s.tile_sums, reinterpret_cast<const uint32_t*>(s.qoff), s.amb_n);
     k++;
   }
   Stage t(prof, "dmc_scan", st);
-  scan_tile_sums_kernel<<<1, 1024, 0, st>>>(s.tile_sums, tiles, s.totals);
+  launch(scan_tile_sums_kernel, 1, 1024, st, s.tile_sums, tiles, s.totals);
   return k + 1;
 }
 
@@ -1295,7 +1305,7 @@ int dmc_front_emit(const CellSpace& space, DmcScratch& s, DmcVertexOut vo, int64
     // per-cell offsets and the vertex work list (needs the vertex count for its size)
     Stage t(prof, "dmc_scan", st);
     const int64_t tiles = ceil_div(n, kScanTile);
-    dmc_offsets_kernel<<<(unsigned)ceil_div(tiles, kOffsetWarps), 32 * kOffsetWarps, 0, st>>>(
+    launch(dmc_offsets_kernel, (unsigned)ceil_div(tiles, kOffsetWarps), 32 * kOffsetWarps, st, 
         s.mask, s.rec, s.tile_sums, tiles, s.rv, s.qoff, s.vwork, s.vrank, s.chunks, s.amb_n + 1);
   }
   // per-vertex grids: whole waves of each kernel's resident blocks
@@ -1310,18 +1320,18 @@ int dmc_front_emit(const CellSpace& space, DmcScratch& s, DmcVertexOut vo, int64
   {
     Stage t(prof, "dmc_vertex_point", st);
     if (space.grids)
-      dmc_vertex_point_kernel<true><<<vgrid(r_point_batch), kVertexThreads, 0, st>>>(
+      launch(dmc_vertex_point_kernel<true>, vgrid(r_point_batch), kVertexThreads, st, 
           space, s.cellof, s.ccase, s.rec, s.vrank, s.vwork, nv, s.vp, s.fb_list, s.w_list, s.fb_count);
     else
-      dmc_vertex_point_kernel<false><<<vgrid(r_point), kVertexThreads, 0, st>>>(
+      launch(dmc_vertex_point_kernel<false>, vgrid(r_point), kVertexThreads, st, 
           space, s.cellof, s.ccase, s.rec, s.vrank, s.vwork, nv, s.vp, s.fb_list, s.w_list, s.fb_count);
     // the lists' lengths are only known on the device: one wave, sized for a tenth of the vertices
     // (the search takes a warp per vertex when few are listed, so as many warps as vertices may use)
     static const int r_search = resident_blocks(dmc_vertex_search_kernel, kVertexThreads);
-    dmc_vertex_search_kernel<<<(unsigned)wave_grid(r_search, sms, 1, nv, kVertexThreads), kVertexThreads, 0, st>>>(
+    launch(dmc_vertex_search_kernel, (unsigned)wave_grid(r_search, sms, 1, nv, kVertexThreads), kVertexThreads, st, 
         space, s.cellof, s.ccase, s.rec, s.vrank, s.vwork, s.fb_list, s.fb_count,
         (unsigned)std::min<int64_t>(tu.warp_list_max, 0x7fffffff), s.vp, s.hard_list, s.stats);
-    dmc_vertex_w_kernel<<<(unsigned)wave_grid(r_w, sms, 1, ceil_div(nv, 10), kVertexThreads), kVertexThreads, 0, st>>>(
+    launch(dmc_vertex_w_kernel, (unsigned)wave_grid(r_w, sms, 1, ceil_div(nv, 10), kVertexThreads), kVertexThreads, st, 
         space, s.cellof, s.vwork, s.w_list, s.fb_count, s.vp, s.stats);
   }
   {
@@ -1329,7 +1339,7 @@ int dmc_front_emit(const CellSpace& space, DmcScratch& s, DmcVertexOut vo, int64
 #define DMC_FINISH(B, F)                                                                              \
   {                                                                                                   \
     static const int res = resident_blocks(dmc_vertex_finish_kernel<B, F>, kVertexThreads);           \
-    dmc_vertex_finish_kernel<B, F><<<vgrid(res), kVertexThreads, 0, st>>>(space, s.cellof, s.vwork, nv, s.vp, vo, flip, \
+    launch(dmc_vertex_finish_kernel<B, F>, vgrid(res), kVertexThreads, st, space, s.cellof, s.vwork, nv, s.vp, vo, flip, \
                                                                           s.stats);                   \
   }
     // the pair normals' storing path only when some volume keeps them (simplification)
@@ -1347,17 +1357,16 @@ int dmc_front_emit(const CellSpace& space, DmcScratch& s, DmcVertexOut vo, int64
     const unsigned warp_max = (unsigned)std::min<int64_t>(tu.warp_list_max, 0x7fffffff);
     static const int r_vertex = resident_blocks(dmc_vertex_kernel, kVertexThreads);
     const unsigned fb = (unsigned)wave_grid(r_vertex, sms, 8, nv, kVertexThreads);
-    dmc_vertex_kernel<<<fb, kVertexThreads, 0, st>>>(space, s.cellof, s.vrank, s.vwork, s.hard_list, s.fb_count + 3, s.tail_list,
+    launch(dmc_vertex_kernel, fb, kVertexThreads, st, space, s.cellof, s.vrank, s.vwork, s.hard_list, s.fb_count + 3, s.tail_list,
                                                       s.fb_count + 1, warp_max, vo, flip, s.stats);
-    dmc_vertex_warp_kernel<<<(unsigned)std::max(1, sms * 3), kVertexThreads, 0, st>>>(
+    launch(dmc_vertex_warp_kernel, (unsigned)std::max(1, sms * 3), kVertexThreads, st, 
         space, s.cellof, s.vrank, s.vwork, s.hard_list, s.fb_count + 3, s.tail_list, s.fb_count + 1, warp_max, vo, flip,
         s.stats);
   }
   Stage t(prof, "dmc_quad", st);
   // one wave: the number of chunks is only known on the device
 #define DMC_QUADS(B, R)                                                                                              \
-  dmc_quad_kernel<B><<<(unsigned)wave_grid(R, sms, tu.quad_blocks_per_sm, ceil_div(n, 32), kQuadThreads / 32),       \
-                       kQuadThreads, 0, st>>>(space, s.mask, s.cellof, s.ccase, s.rv, s.qoff, s.tile_sums, s.chunks, \
+  launch(dmc_quad_kernel<B>, (unsigned)wave_grid(R, sms, tu.quad_blocks_per_sm, ceil_div(n, 32), kQuadThreads / 32),  kQuadThreads, st, space, s.mask, s.cellof, s.ccase, s.rv, s.qoff, s.tile_sums, s.chunks, \
                                               s.amb_n + 1, quads, colors)
   if (space.grids) DMC_QUADS(true, r_quad_batch);
   else DMC_QUADS(false, r_quad);

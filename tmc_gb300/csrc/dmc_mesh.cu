@@ -78,6 +78,7 @@ __device__ __forceinline__ int color_class(int c) { return c > 4 ? c - 5 : (c ==
 constexpr int kColorThreads = 256, kColorItems = 8, kColorTile = kColorThreads * kColorItems;
 
 __global__ void __launch_bounds__(kColorThreads) color_count_kernel(const uint8_t* col, int64_t nq, int32_t* cnt) {
+  pdl_begin();
   __shared__ int h[20];
   if (threadIdx.x < 20) h[threadIdx.x] = 0;
   __syncthreads();
@@ -95,6 +96,7 @@ __global__ void __launch_bounds__(kColorThreads) color_count_kernel(const uint8_
 }
 
 __global__ void color_offsets_kernel(const int32_t* cnt, int32_t* off, int32_t* cursor) {
+  pdl_begin();
   if (threadIdx.x == 0 && blockIdx.x == 0) {
     int s = 0;
     for (int k = 0; k < 20; k++) {
@@ -108,6 +110,7 @@ __global__ void color_offsets_kernel(const int32_t* cnt, int32_t* off, int32_t* 
 
 __global__ void __launch_bounds__(kColorThreads) color_scatter_kernel(const uint8_t* col, int64_t nq, int32_t* cursor,
                                                                      int32_t* list) {
+  pdl_begin();
   __shared__ int h[20], at[20];
   if (threadIdx.x < 20) h[threadIdx.x] = 0;
   __syncthreads();
@@ -129,6 +132,7 @@ __global__ void __launch_bounds__(kColorThreads) color_scatter_kernel(const uint
 
 __global__ void color_reduce_kernel(HeView he, uint8_t* col, const int32_t* list, const int32_t* off, int k,
                                     int lim) {
+  pdl_begin();
   const int64_t b = off[k], e = off[k + 1];
   FOR_EACH(idx, e - b) {
     const int f = list[b + idx];
@@ -154,6 +158,7 @@ __global__ void color_reduce_kernel(HeView he, uint8_t* col, const int32_t* list
 // One thread per face (16-byte twin loads; the corners only for a face with a boundary halfedge);
 // alive: the live faces (all when NULL).  A caller's quads need not be 16-byte aligned.
 __global__ void valence_boundary_kernel(HeView he, int64_t nq, int32_t* val, const uint8_t* alive) {
+  pdl_begin();
   const bool vec = ((reinterpret_cast<uintptr_t>(he.q) | reinterpret_cast<uintptr_t>(he.twin)) & 15) == 0;
   FOR_EACH(f, nq) {
     if (alive && !alive[f]) continue;
@@ -172,6 +177,7 @@ __global__ void valence_boundary_kernel(HeView he, int64_t nq, int32_t* val, con
 
 // mark3X3Y (:889-913)
 __global__ void mark3x3y_kernel(const int32_t* q, int64_t nq, const int32_t* val, uint8_t* p, const uint8_t* alive) {
+  pdl_begin();
   FOR_EACH(f, nq) {
     if (!alive[f]) {
       p[f] = 0;
@@ -186,6 +192,7 @@ __global__ void mark3x3y_kernel(const int32_t* q, int64_t nq, const int32_t* val
 __global__ void merge_claim_kernel(HeView he, int64_t nq, const uint8_t* p, const int32_t* val,
                                    const uint8_t* col, int color_pass, uint8_t* branch, int32_t* own_pos,
                                    int32_t* own_rm) {
+  pdl_begin();
   FOR_EACH(f, nq) {
     branch[f] = 0;
     if (!p[f]) continue;
@@ -271,6 +278,7 @@ __global__ void __launch_bounds__(kMergeThreads) merge_apply_kernel(HeView he, i
                                                                    uint8_t* vm_first, int32_t* vm_second, uint8_t* em,
                                                                    int4* jobs, unsigned* njobs, uint8_t* dold,
                                                                    uint8_t* valive) {
+  pdl_begin();
   __shared__ int4 s_jobs[kMergeThreads];
   __shared__ unsigned s_n, s_base;
   // block-uniform loop: every thread reaches the barriers
@@ -319,6 +327,7 @@ __global__ void __launch_bounds__(kMergeThreads) merge_apply_kernel(HeView he, i
 }
 
 __global__ void midpoint_kernel(const int4* jobs, const unsigned* njobs, double* v64, double* n64) {
+  pdl_begin();
   const int64_t nj = *njobs;
   FOR_EACH(a, nj) {
     const int4 j = jobs[a];
@@ -330,6 +339,7 @@ __global__ void midpoint_kernel(const int4* jobs, const unsigned* njobs, double*
 // front end writes float32 values that are the same roundings, so that the passes only carry the
 // float64 arrays).
 __global__ void float_outputs_kernel(const double* v64, const double* n64, int64_t n, float* v, float* nf) {
+  pdl_begin();
   const float2* n2 = reinterpret_cast<const float2*>(n64);
   FOR_EACH(e, n) {
     v[e] = (float)v64[e];
@@ -350,6 +360,7 @@ __global__ void float_outputs_kernel(const double* v64, const double* n64, int64
 __global__ void gather_vertices_kernel(const uint8_t* keep, const int32_t* idx, int64_t nv, const double* v64,
                                        const double* n64, double* v64o, int32_t* map, int64_t cap, unsigned* overflow,
                                        float* vo, float* no) {
+  pdl_begin();
   const int first = idx[0];
   FOR_EACH(e, 3 * nv) {
     const uint32_t i = (uint32_t)e / 3u, d = (uint32_t)e - 3u * i;  // 3 nv < 2^32
@@ -394,6 +405,7 @@ __device__ __forceinline__ void touch_corner(int x, int y, const uint8_t* dold, 
 // Faces and vertices keep their indices; the compaction runs once after the last pass.
 __global__ void apply_3x3y_kernel(int32_t* q, int64_t nq, uint8_t* alive, const uint8_t* em, const uint8_t* vm_first,
                                   const int32_t* vm_second, const uint8_t* dold, uint8_t* dirty, int32_t* deg) {
+  pdl_begin();
   FOR_EACH(f, nq) {
     if (!alive[f]) continue;
     if (em[f]) {
@@ -413,6 +425,7 @@ __global__ void apply_3x3y_kernel(int32_t* q, int64_t nq, uint8_t* alive, const 
 // mark3333 (:1189-1322)
 __global__ void mark3333_kernel(HeView he, int64_t nq, const int32_t* val, uint8_t* p3, uint8_t* rflag,
                                 uint8_t* vm0, int32_t* vm1, uint8_t* dold, const uint8_t* alive, uint8_t* valive) {
+  pdl_begin();
   FOR_EACH(f, nq) {
     if (!alive[f] || non_manifold(he, f)) continue;
     int vq[4], fo[4], vo[4];
@@ -454,6 +467,7 @@ __global__ void mark3333_kernel(HeView he, int64_t nq, const int32_t* val, uint8
 // marked face die and its corners move to the neighbours' far vertices (kept: their valence is not 3).
 __global__ void apply_3333_kernel(int32_t* q, int64_t nq, uint8_t* alive, const uint8_t* rflag, const uint8_t* p3,
                                   const int32_t* vm1, const uint8_t* dold, uint8_t* dirty, int32_t* deg) {
+  pdl_begin();
   FOR_EACH(f, nq) {
     if (!alive[f]) continue;
     if (rflag[f]) {
@@ -477,6 +491,7 @@ __global__ void apply_3333_kernel(int32_t* q, int64_t nq, uint8_t* alive, const 
 // 16.6 M faces: 164 -> 127 us.
 __global__ void gather_live_quads_kernel(const uint8_t* alive, const int32_t* idx, int64_t nq, const int4* q,
                                          const int32_t* vmap, int4* qo, int32_t* src, int64_t cap, unsigned* overflow) {
+  pdl_begin();
   FOR_EACH(f, nq) {
     const uint8_t a = alive[f];
     const int64_t o = idx[f];
@@ -648,6 +663,7 @@ __device__ __forceinline__ void list_quad(uint32_t* list, unsigned* count, bool 
 // leave no doubt; the other quads are listed.
 __global__ void triangles_fast_kernel(const int32_t* q, int64_t nq, const float* v, int32_t* t, uint32_t* list,
                                       unsigned* count) {
+  pdl_begin();
   FOR_EACH(i, nq) {
     const int v0 = q[4 * i], v1 = q[4 * i + 1], v2 = q[4 * i + 2], v3 = q[4 * i + 3];
     const int s = split_bounded(load_point(v, v0), load_point(v, v1), load_point(v, v2), load_point(v, v3));
@@ -694,6 +710,7 @@ template <int kAcos>
 __global__ void __launch_bounds__(kSplitThreads) triangles_kernel(const int32_t* q, const uint32_t* list,
                                                                   const unsigned* count, const double* v64,
                                                                   const int32_t* q64, const int32_t* src, int32_t* t) {
+  pdl_begin();
   __shared__ uint32_t open[2 * kSplitThreads];
   __shared__ unsigned n_open;
   if (threadIdx.x == 0) n_open = 0;
@@ -808,12 +825,12 @@ int color_faces(const HeView& he, uint8_t* col, int64_t nq, int32_t* cnt, Pool& 
   int32_t* list = pool.get<int32_t>(std::max<int64_t>(nq, 1));
   if (pool.err) return 0;
   const unsigned gc = (unsigned)std::max<int64_t>(1, ceil_div(nq, kColorTile));
-  color_count_kernel<<<gc, kColorThreads, 0, st>>>(col, nq, cnt);
-  color_offsets_kernel<<<1, 32, 0, st>>>(cnt, off, cursor);
-  color_scatter_kernel<<<gc, kColorThreads, 0, st>>>(col, nq, cursor, list);
+  launch(color_count_kernel, gc, kColorThreads, st, col, nq, cnt);
+  launch(color_offsets_kernel, 1, 32, st, cnt, off, cursor);
+  launch(color_scatter_kernel, gc, kColorThreads, st, col, nq, cursor, list);
   const unsigned gq = grid_for(std::max<int64_t>(nq, 1), sms);
-  for (int k = 0; k < 19; k++) color_reduce_kernel<<<gq, 256, 0, st>>>(he, col, list, off, k, 4);
-  color_reduce_kernel<<<gq, 256, 0, st>>>(he, col, list, off, 19, 3);
+  for (int k = 0; k < 19; k++) launch(color_reduce_kernel, gq, 256, st, he, col, list, off, k, 4);
+  launch(color_reduce_kernel, gq, 256, st, he, col, list, off, 19, 3);
   return 23;
 }
 
@@ -822,7 +839,7 @@ int color_faces(const HeView& he, uint8_t* col, int64_t nq, int32_t* cnt, Pool& 
 int vertex_valence(const HeView& he, const int32_t* deg, int64_t nv, int64_t nq, int32_t* val, int sms,
                    cudaStream_t st, const uint8_t* alive = nullptr) {
   cudaMemcpyAsync(val, deg, nv * sizeof(int32_t), cudaMemcpyDeviceToDevice, st);
-  valence_boundary_kernel<<<grid_for(std::max<int64_t>(nq, 1), sms), 256, 0, st>>>(he, nq, val, alive);
+  launch(valence_boundary_kernel, grid_for(std::max<int64_t>(nq, 1), sms), 256, st, he, nq, val, alive);
   return 1;
 }
 
@@ -1020,16 +1037,16 @@ DmcPostStatus dmc_postprocess(const DmcMesh& in, uint32_t flags, int sms, cudaSt
       {
         Stage tm(prof, "dmc_p3x3y", st);
         s.launches += vertex_valence(he, hw.w.deg, nv0, nq0, val, sms, st, alive);
-        mark3x3y_kernel<<<gq, 256, 0, st>>>(q0, nq0, val, p, alive);
+        launch(mark3x3y_kernel, gq, 256, st, q0, nq0, val, p, alive);
         cudaMemsetAsync(b.owner, 0xff, 3 * (size_t)NV * sizeof(int32_t), st);
         cudaMemsetAsync(b.fresh, 0, b.fresh_bytes, st);
-        merge_claim_kernel<<<gq, 256, 0, st>>>(he, nq0, p, val, cur.colors, pass == 0, branch, own_pos, own_rm);
+        launch(merge_claim_kernel, gq, 256, st, he, nq0, p, val, cur.colors, pass == 0, branch, own_pos, own_rm);
         unsigned* njobs = reinterpret_cast<unsigned*>(hw.zero + kZeroJobs) + pass;
-        merge_apply_kernel<<<gq, kMergeThreads, 0, st>>>(he, nq0, branch, own_pos, own_rm, vm_first, vm_second, em,
+        launch(merge_apply_kernel, gq, kMergeThreads, st, he, nq0, branch, own_pos, own_rm, vm_first, vm_second, em,
                                                          b.jobs, njobs, hw.dold, valive);
         static const int r_mid = resident_blocks(midpoint_kernel, 256);  // one wave over the merge list
-        midpoint_kernel<<<(unsigned)wave_grid(r_mid, sms, 1, nq0, 256), 256, 0, st>>>(b.jobs, njobs, cur.v64, cur.n64);
-        apply_3x3y_kernel<<<gq, 256, 0, st>>>(q0, nq0, alive, em, vm_first, vm_second, hw.dold, hw.dnew, hw.w.deg);
+        launch(midpoint_kernel, (unsigned)wave_grid(r_mid, sms, 1, nq0, 256), 256, st, b.jobs, njobs, cur.v64, cur.n64);
+        launch(apply_3x3y_kernel, gq, 256, st, q0, nq0, alive, em, vm_first, vm_second, hw.dold, hw.dnew, hw.w.deg);
         s.launches += 5;
       }
       if (!p3333 && (pass == 1 || !i3x3y)) count_live();
@@ -1047,8 +1064,8 @@ DmcPostStatus dmc_postprocess(const DmcMesh& in, uint32_t flags, int sms, cudaSt
         cudaMemsetAsync(p3, 0, 2 * b.face_stride, st);  // and rflag behind it
         cudaMemsetAsync(b.fresh, 0, b.fresh_bytes, st);
         cudaMemsetAsync(vm1, 0xff, (size_t)NV * sizeof(int32_t), st);
-        mark3333_kernel<<<gq, 256, 0, st>>>(he, nq0, val, p3, rflag, vm0, vm1, hw.dold, alive, valive);
-        apply_3333_kernel<<<gq, 256, 0, st>>>(q0, nq0, alive, rflag, p3, vm1, hw.dold, hw.dnew, hw.w.deg);
+        launch(mark3333_kernel, gq, 256, st, he, nq0, val, p3, rflag, vm0, vm1, hw.dold, alive, valive);
+        launch(apply_3333_kernel, gq, 256, st, q0, nq0, alive, rflag, p3, vm1, hw.dold, hw.dnew, hw.w.deg);
         s.launches += 2;
       }
       count_live();
@@ -1118,16 +1135,16 @@ DmcPostStatus dmc_postprocess(const DmcMesh& in, uint32_t flags, int sms, cudaSt
   if (compacted) {
     Stage tm(prof, "dmc_compact", st);
     // vertex map into vm_second (free after the passes)
-    gather_vertices_kernel<<<grid_for(3 * nv0, sms), 256, 0, st>>>(valive, idx, nv0, old.v64, old.n64, cur.v64, map, nv2,
+    launch(gather_vertices_kernel, grid_for(3 * nv0, sms), 256, st, valive, idx, nv0, old.v64, old.n64, cur.v64, map, nv2,
                                                                    hw.ovf, cur.v, cur.n);
-    gather_live_quads_kernel<<<gq, 256, 0, st>>>(alive, idx_q, nq0, reinterpret_cast<const int4*>(q0), map,
+    launch(gather_live_quads_kernel, gq, 256, st, alive, idx_q, nq0, reinterpret_cast<const int4*>(q0), map,
                                                  reinterpret_cast<int4*>(cur.quads), hw.src, nq2, hw.ovf);
     s.launches += 2;
     // the inherited colours are only read by the colour pass; they are not carried along
     retire(old.n64);
   } else if ((simplify || new_floats) && cur.nv > 0) {
     // the float32 outputs of a mesh no pass changed
-    float_outputs_kernel<<<grid_for(3 * cur.nv, sms), 256, 0, st>>>(cur.v64, cur.n64, 3 * cur.nv, cur.v, cur.n);
+    launch(float_outputs_kernel, grid_for(3 * cur.nv, sms), 256, st, cur.v64, cur.n64, 3 * cur.nv, cur.v, cur.n);
     s.launches += 1;
   }
   // ---- final halfedges and triangles ----
@@ -1165,12 +1182,12 @@ DmcPostStatus dmc_postprocess(const DmcMesh& in, uint32_t flags, int sms, cudaSt
     uint32_t* tlist = pool.get<uint32_t>(std::max<int64_t>(cur.nq, 1));
     unsigned* tcount = reinterpret_cast<unsigned*>(hw.zero + kZeroSplit);
     if ((s.err = pool.err) == cudaSuccess) {
-      triangles_fast_kernel<<<grid_for(cur.nq, sms), 256, 0, st>>>(cur.quads, cur.nq, cur.v, tr, tlist, tcount);
+      launch(triangles_fast_kernel, grid_for(cur.nq, sms), 256, st, cur.quads, cur.nq, cur.v, tr, tlist, tcount);
       const unsigned gt = grid_for(cur.nq, sms);
       const int kind = libm::host_acosf_kind();
       // positions from the uncompacted mesh, by its quads
 #define TRIANGLES(K)                                                                                               \
-  triangles_kernel<K><<<gt, kSplitThreads, 0, st>>>(cur.quads, tlist, tcount, old.v64, q0, compacted ? hw.src : nullptr, tr)
+  launch(triangles_kernel<K>, gt, kSplitThreads, st, cur.quads, tlist, tcount, old.v64, q0, compacted ? hw.src : nullptr, tr)
       if (kind == libm::kAcosfFused) TRIANGLES(libm::kAcosfFused);
       else if (kind == libm::kAcosfSeparate) TRIANGLES(libm::kAcosfSeparate);
       else TRIANGLES(libm::kAcosfCorrect);

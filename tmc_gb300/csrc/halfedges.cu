@@ -30,6 +30,7 @@ namespace {
 
 __global__ void he_vertex_init_kernel(unsigned long long* hv_key, int32_t* deg, int32_t* hv, int64_t nv,
                                       unsigned long long* lone_count) {
+  pdl_begin();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += (int64_t)gridDim.x * blockDim.x) {
     hv_key[i] = 0;
     deg[i] = 0;
@@ -44,6 +45,7 @@ __global__ void he_vertex_init_kernel(unsigned long long* hv_key, int32_t* deg, 
 // he_twin_kernel, every entry once.
 template <bool kHandles>
 __global__ void he_build_kernel(const int32_t* faces, int64_t nh, int32_t* deg, int32_t* rank, int32_t* hv) {
+  pdl_begin();
   for (int64_t h = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; h < nh; h += (int64_t)gridDim.x * blockDim.x) {
     const int v = faces[h];
     rank[h] = atomicAdd(deg + v, 1);
@@ -55,6 +57,7 @@ __global__ void he_build_kernel(const int32_t* faces, int64_t nh, int32_t* deg, 
 template <int P>  // a compile-time face size: h / P without a run-time 64-bit division
 __global__ void __launch_bounds__(256, 8) he_scatter_kernel(const int32_t* faces, int64_t nf, const int32_t* off,
                                                             const int32_t* rank, int2* list) {
+  pdl_begin();
   const int64_t nh = nf * P;
   for (int64_t h = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; h < nh; h += (int64_t)gridDim.x * blockDim.x) {
     const int64_t f = h / P;
@@ -135,6 +138,7 @@ template <int P, bool kHandles>
 __global__ void he_twin_kernel(const int32_t* faces, int64_t nf, const int2* list, const int32_t* off, int nv,
                                int32_t* twin, uint8_t* flag, unsigned long long* hv_key,
                                unsigned long long* non_manifold, int32_t* lone, unsigned long long* lone_count) {
+  pdl_begin();
   const int nh = (int)(nf * P);
   // 16-byte face loads and twin stores only on aligned arrays (a caller's mesh may be a slice)
   const bool vec = P == 4 && ((reinterpret_cast<uintptr_t>(faces) | reinterpret_cast<uintptr_t>(twin)) & 15) == 0 &&
@@ -213,6 +217,7 @@ __global__ void he_twin_kernel(const int32_t* faces, int64_t nf, const int2* lis
 // (the lone halfedges are listed by he_twin_kernel)
 __global__ void he_override_kernel(const int32_t* faces, int P, const int32_t* lone, const unsigned long long* lone_count,
                                    int32_t* hv, const unsigned long long* hv_key) {
+  pdl_begin();
   const int64_t n = (int64_t)*lone_count;
   for (int64_t a = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; a < n; a += (int64_t)gridDim.x * blockDim.x) {
     const int64_t h = lone[a];
@@ -275,6 +280,7 @@ __device__ __forceinline__ int bucket_of(int o, int t, bool dout, bool din) {
 __global__ void __launch_bounds__(256) he_repair_mark_kernel(const int4* faces, int64_t nf, const uint8_t* alive,
                                                              const uint8_t* dirty, int32_t* deg, int32_t* bcnt,
                                                              int32_t* drank, uint8_t* dmask) {
+  pdl_begin();
   for (int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; f < nf; f += (int64_t)gridDim.x * blockDim.x) {
     unsigned m = 0;
     if (alive[f]) {
@@ -301,6 +307,7 @@ __global__ void __launch_bounds__(256) he_repair_mark_kernel(const int4* faces, 
 // bucket entries: (halfedge, the edge's other end)
 __global__ void he_bucket_scatter_kernel(const int4* faces, int64_t nf, const uint8_t* dirty, const uint8_t* dmask,
                                          const int32_t* drank, const int32_t* boff, int2* blist, int32_t* bkey) {
+  pdl_begin();
   for (int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; f < nf; f += (int64_t)gridDim.x * blockDim.x) {
     const unsigned m = dmask[f];
     if (!m) continue;
@@ -322,6 +329,7 @@ __global__ void he_bucket_scatter_kernel(const int4* faces, int64_t nf, const ui
 // lanes of one bucket load the same entries (one broadcast load per step), all from L1.
 __global__ void he_pair_kernel(const int32_t* faces, int nv, const unsigned long long* total, const int32_t* boff,
                                const int2* blist, const int32_t* bkey, int32_t* twin, uint8_t* flag) {
+  pdl_begin();
   const int n = (int)*total;
   for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < n; a += gridDim.x * blockDim.x) {
     const int2 x = blist[a];
@@ -346,6 +354,7 @@ __global__ void he_pair_kernel(const int32_t* faces, int nv, const unsigned long
 // member of a three-halfedge edge in edge-key order (he_override_kernel).
 __global__ void he_handles_init_kernel(int32_t* hv, unsigned long long* hv_key, int64_t nv,
                                        unsigned long long* counts) {
+  pdl_begin();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += (int64_t)gridDim.x * blockDim.x) {
     hv[i] = -1;
     hv_key[i] = 0;
@@ -357,6 +366,7 @@ template <int P>
 __global__ void he_handles_kernel(const int32_t* faces, int64_t nh, const uint8_t* alive, const int32_t* twin,
                                   const uint8_t* flag, int32_t* hv, unsigned long long* hv_key, int32_t* lone,
                                   unsigned long long* counts) {
+  pdl_begin();
   unsigned long long n1 = 0, n2 = 0;
   for (int64_t h = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; h < nh; h += (int64_t)gridDim.x * blockDim.x) {
     if (alive && !alive[h / P]) continue;
@@ -387,6 +397,7 @@ __global__ void he_handles_kernel(const int32_t* faces, int64_t nh, const uint8_
 __global__ void he_handles4_kernel(const int4* faces, int64_t nf, const uint8_t* alive, const int32_t* twin,
                                    const uint32_t* flag4, int32_t* hv, unsigned long long* hv_key, int32_t* lone,
                                    unsigned long long* counts) {
+  pdl_begin();
   unsigned long long n1 = 0, n2 = 0;
   for (int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; f < nf; f += (int64_t)gridDim.x * blockDim.x) {
     if (alive && !alive[f]) continue;
@@ -420,6 +431,7 @@ __global__ void he_handles4_kernel(const int4* faces, int64_t nf, const uint8_t*
 
 // edges with four halfedges (flag 1 on each) and with three (flag 2 on each)
 __global__ void he_group_count_kernel(const unsigned long long* counts, unsigned long long* non_manifold) {
+  pdl_begin();
   if (blockIdx.x == 0 && threadIdx.x == 0) *non_manifold = counts[0] / 4 + counts[1] / 3;
 }
 
@@ -427,6 +439,7 @@ __global__ void he_group_count_kernel(const unsigned long long* counts, unsigned
 // was face src[f], kept face g became fidx[g]; twins move with their faces.
 __global__ void he_pack_compacted_kernel(const int32_t* faces, int64_t nh, const int32_t* src, const int32_t* fidx,
                                          const int32_t* twin, int32_t* he4, int32_t* hf) {
+  pdl_begin();
   for (int64_t h = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; h < nh; h += (int64_t)gridDim.x * blockDim.x) {
     const int64_t f = h >> 2;
     const int r = (int)(h & 3);
@@ -440,6 +453,7 @@ __global__ void he_pack_compacted_kernel(const int32_t* faces, int64_t nh, const
 // handles of the kept vertices in the compacted numbering (vertex x became vidx[x] - vidx[0])
 __global__ void he_handles_compacted_kernel(const uint8_t* vkeep, const int32_t* vidx, int64_t nv, const int32_t* hv,
                                             const int32_t* fidx, int32_t* hv_out) {
+  pdl_begin();
   const int first = vidx[0];
   for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < nv; x += (int64_t)gridDim.x * blockDim.x) {
     if (!vkeep[x]) continue;
@@ -451,6 +465,7 @@ __global__ void he_handles_compacted_kernel(const uint8_t* vkeep, const int32_t*
 template <int P>
 __global__ void __launch_bounds__(256, 8) he_pack4_kernel(const int32_t* faces, const int32_t* twin, int64_t nh,
                                                           int32_t* he4, int32_t* hf) {
+  pdl_begin();
   for (int64_t h = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; h < nh; h += (int64_t)gridDim.x * blockDim.x) {
     const int64_t f = h / P;
     const int r = (int)(h - f * P);
@@ -471,22 +486,22 @@ int build_halfedges(const int32_t* faces, int P, int64_t nf, int64_t nv, HeOut& 
   // the lone-halfedge list reuses the slot array, which is dead once the lists are scattered
   unsigned long long* lone_count = w.total + 1;
   if (handles) {
-    he_vertex_init_kernel<<<grid(nv), 256, 0, st>>>(w.hv_key, w.deg, o.hv, nv, lone_count);
-    he_build_kernel<true><<<grid(nh), 256, 0, st>>>(faces, nh, w.deg, w.rank, o.hv);
+    launch(he_vertex_init_kernel, grid(nv), 256, st, w.hv_key, w.deg, o.hv, nv, lone_count);
+    launch(he_build_kernel<true>, grid(nh), 256, st, faces, nh, w.deg, w.rank, o.hv);
     k += 2;
   } else {
     cudaMemsetAsync(w.deg, 0, (size_t)nv * sizeof(int32_t), st);
-    he_build_kernel<false><<<grid(nh), 256, 0, st>>>(faces, nh, w.deg, w.rank, nullptr);
+    launch(he_build_kernel<false>, grid(nh), 256, st, faces, nh, w.deg, w.rank, nullptr);
     k += 1;
   }
   k += scan_i32(w.deg, nv, w.off, w.tiles, w.total, st);
-  if (P == 4) he_scatter_kernel<4><<<grid(nh), 256, 0, st>>>(faces, nf, w.off, w.rank, w.list);
-  else he_scatter_kernel<3><<<grid(nh), 256, 0, st>>>(faces, nf, w.off, w.rank, w.list);
+  if (P == 4) launch(he_scatter_kernel<4>, grid(nh), 256, st, faces, nf, w.off, w.rank, w.list);
+  else launch(he_scatter_kernel<3>, grid(nh), 256, st, faces, nf, w.off, w.rank, w.list);
   // one thread per face, whole waves of the kernel's resident blocks
 #define HE_TWIN(PP, HH)                                                                                     \
   {                                                                                                         \
     static const int res = resident_blocks(he_twin_kernel<PP, HH>, 256);                                    \
-    he_twin_kernel<PP, HH><<<(unsigned)wave_grid(res, sms, 8, nf, 256), 256, 0, st>>>(                       \
+    launch(he_twin_kernel<PP, HH>, (unsigned)wave_grid(res, sms, 8, nf, 256), 256, st,                        \
         faces, nf, w.list, w.off, (int)nv, o.twin, o.flag, HH ? w.hv_key : nullptr, w.non_manifold,          \
         HH ? w.rank : nullptr, HH ? lone_count : nullptr);                                                  \
   }
@@ -497,7 +512,7 @@ int build_halfedges(const int32_t* faces, int P, int64_t nf, int64_t nv, HeOut& 
   }
 #undef HE_TWIN
   if (handles) {
-    he_override_kernel<<<(unsigned)std::max(1, sms), 256, 0, st>>>(faces, P, w.rank, lone_count, o.hv, w.hv_key);
+    launch(he_override_kernel, (unsigned)std::max(1, sms), 256, st, faces, P, w.rank, lone_count, o.hv, w.hv_key);
     return k + 3;
   }
   return k + 2;
@@ -508,15 +523,15 @@ int repair_halfedges(const int32_t* faces, int64_t nf, int64_t nv, const uint8_t
   if (nf == 0) return 0;
   const int4* q4 = reinterpret_cast<const int4*>(faces);
   static const int r_mark = resident_blocks(he_repair_mark_kernel, 256);
-  he_repair_mark_kernel<<<(unsigned)wave_grid(r_mark, sms, 8, nf, 256), 256, 0, st>>>(q4, nf, alive, dirty, deg, w.bcnt,
+  launch(he_repair_mark_kernel, (unsigned)wave_grid(r_mark, sms, 8, nf, 256), 256, st, q4, nf, alive, dirty, deg, w.bcnt,
                                                                                       w.drank, w.dmask);
   int k = 1 + scan_i32(w.bcnt, nv, w.boff, w.tiles, w.total, st);
   static const int r_sc = resident_blocks(he_bucket_scatter_kernel, 256);
-  he_bucket_scatter_kernel<<<(unsigned)wave_grid(r_sc, sms, 8, nf, 256), 256, 0, st>>>(q4, nf, dirty, w.dmask, w.drank,
+  launch(he_bucket_scatter_kernel, (unsigned)wave_grid(r_sc, sms, 8, nf, 256), 256, st, q4, nf, dirty, w.dmask, w.drank,
                                                                                       w.boff, w.blist, w.bkey);
   // the entries are counted on the device: whole waves, as many as the halfedges could need
   static const int r_pair = resident_blocks(he_pair_kernel, 256);
-  he_pair_kernel<<<(unsigned)wave_grid(r_pair, sms, 8, 4 * nf, 256), 256, 0, st>>>(faces, (int)nv, w.total, w.boff,
+  launch(he_pair_kernel, (unsigned)wave_grid(r_pair, sms, 8, 4 * nf, 256), 256, st, faces, (int)nv, w.total, w.boff,
                                                                                   w.blist, w.bkey, o.twin, o.flag);
   return k + 2;
 }
@@ -528,17 +543,17 @@ int halfedge_handles(const int32_t* faces, int P, int64_t nf, int64_t nv, const 
   auto grid = [&](int64_t n) {
     return (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n, 256), (int64_t)sms * 8));
   };
-  he_handles_init_kernel<<<grid(nv), 256, 0, st>>>(hv, w.hv_key, nv, counts);
+  launch(he_handles_init_kernel, grid(nv), 256, st, hv, w.hv_key, nv, counts);
   if (P == 4) {  // quad arrays are 16-byte aligned (pool allocations)
     static const int r4 = resident_blocks(he_handles4_kernel, 256);
-    he_handles4_kernel<<<(unsigned)wave_grid(r4, sms, 8, nf, 256), 256, 0, st>>>(
+    launch(he_handles4_kernel, (unsigned)wave_grid(r4, sms, 8, nf, 256), 256, st, 
         reinterpret_cast<const int4*>(faces), nf, alive, twin, reinterpret_cast<const uint32_t*>(flag), hv, w.hv_key,
         w.rank, counts);
   } else {
-    he_handles_kernel<3><<<grid(nh), 256, 0, st>>>(faces, nh, alive, twin, flag, hv, w.hv_key, w.rank, counts);
+    launch(he_handles_kernel<3>, grid(nh), 256, st, faces, nh, alive, twin, flag, hv, w.hv_key, w.rank, counts);
   }
-  he_override_kernel<<<(unsigned)std::max(1, sms), 256, 0, st>>>(faces, P, w.rank, counts + 2, hv, w.hv_key);
-  he_group_count_kernel<<<1, 32, 0, st>>>(counts, w.non_manifold);
+  launch(he_override_kernel, (unsigned)std::max(1, sms), 256, st, faces, P, w.rank, counts + 2, hv, w.hv_key);
+  launch(he_group_count_kernel, 1, 32, st, counts, w.non_manifold);
   return 4;
 }
 
@@ -548,16 +563,16 @@ int pack_compacted_halfedges(const int32_t* faces, int64_t nf, const int32_t* sr
   auto grid = [&](int64_t n) {
     return (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n, 256), (int64_t)sms * 8));
   };
-  if (nf > 0) he_pack_compacted_kernel<<<grid(4 * nf), 256, 0, st>>>(faces, 4 * nf, src, fidx, twin, he4, hf);
-  he_handles_compacted_kernel<<<grid(nv), 256, 0, st>>>(vkeep, vidx, nv, hv, fidx, hv_out);
+  if (nf > 0) launch(he_pack_compacted_kernel, grid(4 * nf), 256, st, faces, 4 * nf, src, fidx, twin, he4, hf);
+  launch(he_handles_compacted_kernel, grid(nv), 256, st, vkeep, vidx, nv, hv, fidx, hv_out);
   return 2;
 }
 
 int pack_halfedges4(const int32_t* faces, int P, const int32_t* twin, int64_t nh, int32_t* he4, int32_t* hf, int sms,
                     cudaStream_t st) {
   const unsigned g = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(nh, 256), (int64_t)sms * 8));
-  if (P == 4) he_pack4_kernel<4><<<g, 256, 0, st>>>(faces, twin, nh, he4, hf);
-  else he_pack4_kernel<3><<<g, 256, 0, st>>>(faces, twin, nh, he4, hf);
+  if (P == 4) launch(he_pack4_kernel<4>, g, 256, st, faces, twin, nh, he4, hf);
+  else launch(he_pack4_kernel<3>, g, 256, st, faces, twin, nh, he4, hf);
   return 1;
 }
 

@@ -24,6 +24,7 @@ static_assert(kScanTile == 1 << kTileShift, "listed-cell slots assume 2048-cell 
 constexpr int kBitThreads = 256;
 template <bool kGen>
 __global__ void __launch_bounds__(kBitThreads) point_bits_kernel(Grid one, const Grid* grids, int z0, int z1) {
+  pdl_begin();
   const Grid& g = grids ? grids[blockIdx.y] : one;
   const int lane = threadIdx.x & 31;
   const uint32_t wpr = (uint32_t)g.wpr;
@@ -104,7 +105,7 @@ inline int launch_point_bits(const CellSpace& space, int z0, int z1, int sms, cu
 // Bits x .. x + 31 of a row (lo) and x + 1 .. x + 32 (hi); x within the row.  Reads the word after
 // x's, which may belong to the next row (its bits are not used then) or be the padding at the end.
 __device__ __forceinline__ void row_bits(const uint32_t* row, int x, uint32_t& lo, uint32_t& hi) {
-  const uint32_t a = __ldg(row + (x >> 5)), b = __ldg(row + (x >> 5) + 1);
+  const uint32_t a = ld(row + (x >> 5)), b = ld(row + (x >> 5) + 1);
   const int s = x & 31;
   lo = __funnelshift_r(a, b, s);
   hi = (lo >> 1) | ((b >> s) << 31);
@@ -119,7 +120,7 @@ __device__ __forceinline__ unsigned case_from_bits(const Grid& g, int i, int j, 
 #pragma unroll
   for (int q = 0; q < 4; q++) {
     const uint32_t* p = r + (q & 1 ? py : 0) + (q & 2 ? pz : 0);
-    c |= (__funnelshift_r(__ldg(p), __ldg(p + 1), s) & 3u) << (2 * q);
+    c |= (__funnelshift_r(ld(p), ld(p + 1), s) & 3u) << (2 * q);
   }
   return c;
 }

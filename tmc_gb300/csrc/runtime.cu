@@ -979,6 +979,7 @@ tmc_status tmc_extract(tmc_ctx* ctx, const tmc_volume* vol, double iso, uint32_t
 
 // Batch tables on the device: each tile's volume, from the volumes' first tiles (tile0[nb]: the end).
 __global__ void tile_volume_kernel(const int64_t* tile0, int nb, int64_t tiles, int32_t* tile_vol) {
+  tmc::pdl_begin();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= tiles) return;
   int lo = 0, hi = nb - 1;  // the last volume whose first tile is at or before t
@@ -992,6 +993,7 @@ __global__ void tile_volume_kernel(const int64_t* tile0, int nb, int64_t tiles, 
 // The scanned sums at the volumes' first tiles, then the totals (two words).
 __global__ void volume_offsets_kernel(const unsigned long long* tile_off, const int64_t* tile0, int nb,
                                       const unsigned long long* totals, unsigned long long* out) {
+  tmc::pdl_begin();
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q < nb + 2) out[q] = q < nb ? tile_off[tile0[q]] : totals[q - nb];
 }
@@ -1086,7 +1088,7 @@ tmc_status batch_run(tmc_ctx* ctx, const std::vector<int>& idx, const tmc_reques
   }
   TMC_CUDA(ctx, cudaMemcpyAsync(d_grids, grid_src, grid_bytes, cudaMemcpyHostToDevice, st));
   TMC_CUDA(ctx, cudaMemcpyAsync(d_tile0, tile0_src, tile0_bytes, cudaMemcpyHostToDevice, st));
-  tile_volume_kernel<<<(unsigned)tmc::ceil_div(tiles, 256), 256, 0, st>>>(d_tile0, nb, tiles, d_tile_vol);
+  tmc::launch(tile_volume_kernel, (unsigned)tmc::ceil_div(tiles, 256), 256, st, d_tile0, nb, tiles, d_tile_vol);
   ctx->launches += 1;
   tmc::CellSpace space{};
   space.one = grids[0];
@@ -1106,7 +1108,7 @@ tmc_status batch_run(tmc_ctx* ctx, const std::vector<int>& idx, const tmc_reques
     TMC_CUDA(ctx, tmc_ambiguous_records(ctx, al, tsc, n_amb_rec));
     ctx->launches += tmc::tmc_count(space, tsc, n_amb_rec, ctx->sms, st, &ctx->prof);
   }
-  volume_offsets_kernel<<<(unsigned)tmc::ceil_div(nb + 2, 256), 256, 0, st>>>(
+  tmc::launch(volume_offsets_kernel, (unsigned)tmc::ceil_div(nb + 2, 256), 256, st, 
       dmc ? dsc.tile_sums : tsc.tile_sums, d_tile0, nb, ctx->d_stats + kStatTotals, d_voff);
   ctx->launches += 1;
   std::vector<unsigned long long> voff_pageable(staged ? 0 : (size_t)nb + 2);

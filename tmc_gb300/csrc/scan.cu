@@ -6,6 +6,7 @@ namespace tmc {
 // 32 * rounds sums and walks it in rounds of 32 consecutive sums (coalesced), carrying its running
 // sum; the warps' totals are scanned in shared memory, then each warp writes its exclusive prefixes.
 __global__ void scan_tile_sums_kernel(unsigned long long* sums, int64_t ntiles, unsigned long long* totals) {
+  pdl_begin();
   constexpr int T = 1024, W = T / 32;
   __shared__ unsigned long long wsum[W];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -56,6 +57,7 @@ namespace tmc {
 // Generic compaction scan of 0/1 flags (one byte each): out[i] = number of set flags before i.
 __global__ void __launch_bounds__(kScanThreads) flag_tile_sum_kernel(const uint8_t* flags, int64_t n,
                                                                     unsigned long long* tile_sums) {
+  pdl_begin();
   uint32_t f[kScanItems];
   load8(flags, (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems, n, f);
   unsigned long long s = 0;
@@ -68,6 +70,7 @@ __global__ void __launch_bounds__(kScanThreads) flag_tile_sum_kernel(const uint8
 
 __global__ void __launch_bounds__(kScanThreads) flag_offsets_kernel(const uint8_t* flags, int64_t n,
                                                                    const unsigned long long* tile_off, int32_t* out) {
+  pdl_begin();
   const int64_t first = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
   uint32_t f[kScanItems];
   load8(flags, first, n, f);
@@ -93,9 +96,9 @@ int scan_flags(const uint8_t* flags, int64_t n, int32_t* out, unsigned long long
     cudaMemsetAsync(total, 0, sizeof(unsigned long long), st);
     return 0;
   }
-  flag_tile_sum_kernel<<<(unsigned)tiles, kScanThreads, 0, st>>>(flags, n, tile_sums);
-  scan_tile_sums_kernel<<<1, 1024, 0, st>>>(tile_sums, tiles, total);
-  flag_offsets_kernel<<<(unsigned)tiles, kScanThreads, 0, st>>>(flags, n, tile_sums, out);
+  launch(flag_tile_sum_kernel, (unsigned)tiles, kScanThreads, st, flags, n, tile_sums);
+  launch(scan_tile_sums_kernel, 1, 1024, st, tile_sums, tiles, total);
+  launch(flag_offsets_kernel, (unsigned)tiles, kScanThreads, st, flags, n, tile_sums, out);
   return 3;
 }
 
@@ -106,6 +109,7 @@ namespace tmc {
 // Exclusive scan of non-negative int32 values: out[i] = sum of in[0..i).
 __global__ void __launch_bounds__(kScanThreads) i32_tile_sum_kernel(const int32_t* in, int64_t n,
                                                                    unsigned long long* tile_sums) {
+  pdl_begin();
   uint32_t x[kScanItems];
   load8(reinterpret_cast<const uint32_t*>(in), (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems, n,
         x);
@@ -119,6 +123,7 @@ __global__ void __launch_bounds__(kScanThreads) i32_tile_sum_kernel(const int32_
 
 __global__ void __launch_bounds__(kScanThreads) i32_offsets_kernel(const int32_t* in, int64_t n,
                                                                   const unsigned long long* tile_off, int32_t* out) {
+  pdl_begin();
   const int64_t first = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
   uint32_t x[kScanItems];
   load8(reinterpret_cast<const uint32_t*>(in), first, n, x);
@@ -143,9 +148,9 @@ int scan_i32(const int32_t* in, int64_t n, int32_t* out, unsigned long long* til
     cudaMemsetAsync(total, 0, sizeof(unsigned long long), st);
     return 0;
   }
-  i32_tile_sum_kernel<<<(unsigned)tiles, kScanThreads, 0, st>>>(in, n, tile_sums);
-  scan_tile_sums_kernel<<<1, 1024, 0, st>>>(tile_sums, tiles, total);
-  i32_offsets_kernel<<<(unsigned)tiles, kScanThreads, 0, st>>>(in, n, tile_sums, out);
+  launch(i32_tile_sum_kernel, (unsigned)tiles, kScanThreads, st, in, n, tile_sums);
+  launch(scan_tile_sums_kernel, 1, 1024, st, tile_sums, tiles, total);
+  launch(i32_offsets_kernel, (unsigned)tiles, kScanThreads, st, in, n, tile_sums, out);
   return 3;
 }
 

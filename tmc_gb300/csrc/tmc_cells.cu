@@ -619,6 +619,7 @@ __global__ void __launch_bounds__(kClassifyThreads) tmc_classify_kernel(CellSpac
                                                                           unsigned long long* tile_sums,
                                                                           unsigned long long* stats,
                                                                           uint32_t* amb_list, unsigned* amb_n) {
+  pdl_begin();
   constexpr unsigned kAll = 0xffffffffu;
   constexpr int kTiles = kClassifyThreads / 32 / kPerTile;  // tiles per block
   __shared__ uint16_t lists[kTiles][kScanTile];
@@ -699,6 +700,7 @@ __global__ void __launch_bounds__(kClassifyThreads) tmc_classify_kernel(CellSpac
 // whatever its active lanes).  Key pass: each cell's case and the per-case counts.
 __global__ void __launch_bounds__(256) tmc_amb_key_kernel(CellSpace space, const uint16_t* cellof, const uint32_t* list,
                                                           int64_t n, uint8_t* key, unsigned* hist) {
+  pdl_begin();
   __shared__ unsigned h[256];
   h[threadIdx.x] = 0;
   __syncthreads();
@@ -721,6 +723,7 @@ __global__ void __launch_bounds__(256) tmc_amb_key_kernel(CellSpace space, const
 
 // exclusive scan of the 256 counts into the scatter cursors (one block of 256 threads)
 __global__ void tmc_amb_cursor_kernel(const unsigned* hist, unsigned* cursor) {
+  pdl_begin();
   __shared__ unsigned x[256];
   x[threadIdx.x] = hist[threadIdx.x];
   __syncthreads();
@@ -739,6 +742,7 @@ __global__ void tmc_amb_cursor_kernel(const unsigned* hist, unsigned* cursor) {
 constexpr int kSortItems = 8, kSortTile = 256 * kSortItems;
 __global__ void __launch_bounds__(256) tmc_amb_sort_kernel(const uint32_t* list, const uint8_t* key, int64_t n,
                                                            unsigned* cursor, uint32_t* sorted) {
+  pdl_begin();
   __shared__ unsigned h[256];
   for (int64_t base = (int64_t)blockIdx.x * kSortTile; base < n; base += (int64_t)gridDim.x * kSortTile) {
     h[threadIdx.x] = 0;
@@ -929,10 +933,11 @@ __global__ void __launch_bounds__(128) tmc_amb_decide_kernel(CellSpace space, co
                                                              unsigned long long* tile_sums, const uint32_t* list,
                                                              unsigned na, AmbRec* recs, uint32_t* doubt,
                                                              unsigned* ndoubt) {
+  pdl_begin();
   for (unsigned a = blockIdx.x * blockDim.x + threadIdx.x; a < na; a += gridDim.x * blockDim.x) {
     const uint32_t slot = list[a];
     const int64_t vcell = slot_cell(cellof, slot);
-    const Grid& g = space.grids ? space.grids[__ldg(space.tile_vol + vcell / kScanTile)] : space.one;
+    const Grid& g = space.grids ? space.grids[ld(space.tile_vol + vcell / kScanTile)] : space.one;
     int i, j, k;
     tcell_ijk(g, vcell - g.vbase, i, j, k);
     float f[8];
@@ -998,6 +1003,7 @@ __global__ void __launch_bounds__(128) tmc_amb_count_kernel(CellSpace space, con
                                                             unsigned long long* stats, const uint32_t* list,
                                                             const uint32_t* doubt, const unsigned* count,
                                                             AmbRec* recs, unsigned* overflow) {
+  pdl_begin();
   const unsigned na = *count;
   unsigned long long sing = 0;
   for (unsigned x = blockIdx.x * blockDim.x + threadIdx.x; x < na; x += gridDim.x * blockDim.x) {
@@ -1041,6 +1047,7 @@ __global__ void __launch_bounds__(32 * kOffsetWarps) tmc_offsets_kernel(const Ce
                                                                        uint32_t* chunks, unsigned* nchunks,
                                                                        const unsigned* overflow,
                                                                        unsigned long long* totals) {
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const int64_t tile = (int64_t)blockIdx.x * kOffsetWarps + (threadIdx.x >> 5);
   const uint32_t listed = tile < tiles ? tile_listed(mask, tile) : 0;
@@ -1238,7 +1245,7 @@ __device__ __forceinline__ int32_t border_vertex_id(const Grid& g, int i, int j,
   if (own & (1u << e)) return first - vfirst + __popc(own & ((1u << e) - 1u));
   int oi, oj, ok, oe = 0;
   edge_owner(i, j, k, e, oi, oj, ok, oe);
-  const uint2 o = __ldg(rv + listed_slot(mask, (uint32_t)g.vcell(oi, oj, ok)));  // crossed edge: listed owner
+  const uint2 o = ld(rv + listed_slot(mask, (uint32_t)g.vcell(oi, oj, ok)));  // crossed edge: listed owner
   return (int32_t)o.y - vfirst + __popc(trec_owned(o.x) & ((1u << oe) - 1u));
 }
 // The same for all crossed edges (em) of a cell.
@@ -1273,7 +1280,7 @@ __device__ __forceinline__ void interior_vertex_ids(int64_t vcell, int cx, int64
   }
   uint2 o[6];
 #pragma unroll
-  for (int q = 0; q < 6; q++) o[q] = slot[q] != 0xffffffffu ? __ldg(rv + slot[q]) : make_uint2(0, 0);
+  for (int q = 0; q < 6; q++) o[q] = slot[q] != 0xffffffffu ? ld(rv + slot[q]) : make_uint2(0, 0);
 #pragma unroll
   for (int q = 0; q < 6; q++)
 #pragma unroll
@@ -1306,6 +1313,7 @@ __global__ void __launch_bounds__(kAmbThreads) tmc_ambiguous_kernel(CellSpace sp
                                                                     const unsigned long long* tile_off,
                                                                     TmcVertexOut out, int32_t* tris,
                                                                     const AmbRec* recs, const unsigned* count) {
+  pdl_begin();
   constexpr int kWarps = kAmbThreads / 32;
   constexpr unsigned kAll = 0xffffffffu;
   __shared__ int32_t vids[kWarps][18 * 32];     // local code (edge, then inner vertex), cell
@@ -1326,10 +1334,10 @@ __global__ void __launch_bounds__(kAmbThreads) tmc_ambiguous_kernel(CellSpace sp
       ni = (int)((info >> 14) & 7);
       const uint32_t slot = recs[a].slot;
       const int64_t vcell = slot_cell(cellof, slot);
-      const uint2 r = __ldg(rv + slot);
-      vol = space.grids ? __ldg(space.tile_vol + vcell / kScanTile) : 0;
+      const uint2 r = ld(rv + slot);
+      vol = space.grids ? ld(space.tile_vol + vcell / kScanTile) : 0;
       const Grid& g = space.grids ? space.grids[vol] : space.one;
-      vfirst = (int32_t)(__ldg(tile_off + g.vbase / kScanTile) >> 32);
+      vfirst = (int32_t)(ld(tile_off + g.vbase / kScanTile) >> 32);
       int i, j, k;
       tcell_ijk(g, vcell - g.vbase, i, j, k);
       const uint32_t em = case_edge_mask(info & 0xFF), own = trec_owned(r.x);
@@ -1356,7 +1364,7 @@ __global__ void __launch_bounds__(kAmbThreads) tmc_ambiguous_kernel(CellSpace sp
     }
     tupto[wid][lane] = tu;
     iupto[wid][lane] = iu;
-    tbase[wid][lane] = nt ? __ldg(toff + recs[a].slot) - (tu - nt) : 0;
+    tbase[wid][lane] = nt ? ld(toff + recs[a].slot) - (tu - nt) : 0;
     const int ttotal = __shfl_sync(kAll, tu, 31), itotal = __shfl_sync(kAll, iu, 31);
     __syncwarp();
     for (int t = lane; t < ttotal; t += 32) {
@@ -1378,7 +1386,7 @@ __global__ void __launch_bounds__(kAmbThreads) tmc_ambiguous_kernel(CellSpace sp
         const float2* x = reinterpret_cast<const float2*>(prm);
         const ffx::ff U{x[0].x, x[0].y}, V{x[1].x, x[1].y}, W{x[2].x, x[2].y};
         inner_vertex_ff(g, c.x, c.y, c.z, U, V, W, out,
-                        (int64_t)vid[32 * 12 + o] + (int32_t)(__ldg(tile_off + g.vbase / kScanTile) >> 32));
+                        (int64_t)vid[32 * 12 + o] + (int32_t)(ld(tile_off + g.vbase / kScanTile) >> 32));
         continue;
       }
       double u = prm[0], v = prm[1], w = prm[2];
@@ -1388,7 +1396,7 @@ __global__ void __launch_bounds__(kAmbThreads) tmc_ambiguous_kernel(CellSpace sp
         w = prm[4 + ((0x0E >> q) & 1)];
       }
       // vertices are numbered within the volume; the outputs start at its first one
-      const int64_t at = (int64_t)vid[32 * (12 + q) + o] + (int32_t)(__ldg(tile_off + g.vbase / kScanTile) >> 32);
+      const int64_t at = (int64_t)vid[32 * (12 + q) + o] + (int32_t)(ld(tile_off + g.vbase / kScanTile) >> 32);
       // float64 outputs requested for this volume: the reference's float64 arithmetic
       if (g.flags & kGridPos64) inner_vertex_f64(g, c.x, c.y, c.z, u, v, w, out, at);
       else inner_vertex_ff(g, c.x, c.y, c.z, ffx::ff_from_double(u), ffx::ff_from_double(v), ffx::ff_from_double(w), out, at);
@@ -1404,6 +1412,7 @@ __global__ void __launch_bounds__(128) tmc_ambiguous_again_kernel(CellSpace spac
                                                             const int32_t* toff,
                                                             const unsigned long long* tile_off, TmcVertexOut out,
                                                             int32_t* tris, const AmbRec* recs, const unsigned* count) {
+  pdl_begin();
   const unsigned na = *count;
   for (unsigned a = blockIdx.x * blockDim.x + threadIdx.x; a < na; a += gridDim.x * blockDim.x) {
     const AmbRec& R = recs[a];
@@ -1457,6 +1466,7 @@ __global__ void __launch_bounds__(kEmitThreads, 4) tmc_emit_kernel(CellSpace spa
                                                                 const unsigned long long* tile_off,
                                                                 const uint32_t* chunks, const unsigned* nchunks,
                                                                 TmcVertexOut out, int32_t* tris) {
+  pdl_begin();
   constexpr int kWarps = kEmitThreads / 32;
   constexpr unsigned kAll = 0xffffffffu;
   __shared__ int32_t vids[kWarps][12 * 32];    // edge, cell
@@ -1471,15 +1481,15 @@ __global__ void __launch_bounds__(kEmitThreads, 4) tmc_emit_kernel(CellSpace spa
     const uint32_t chunk = chunks[q], slot0 = chunk & ~31u, slot = slot0 + lane;
     const bool in = (uint32_t)lane <= (chunk & 31u);  // the chunk's number of cells minus one
     const int64_t tile = slot0 >> kTileShift;
-    const Grid& g = kBatch ? space.grids[__ldg(space.tile_vol + tile)] : space.one;
-    const int32_t vfirst = kBatch ? (int32_t)(__ldg(tile_off + g.vbase / kScanTile) >> 32) : 0;
+    const Grid& g = kBatch ? space.grids[ld(space.tile_vol + tile)] : space.one;
+    const int32_t vfirst = kBatch ? (int32_t)(ld(tile_off + g.vbase / kScanTile) >> 32) : 0;
     uint2 r = make_uint2(0, 0);
     unsigned cs = 0;
     int64_t vcell = 0;
     int i = 0, j = 0, k = 0;
     if (in) {
-      r = __ldg(rv + slot);
-      cs = __ldg(ccase + slot);
+      r = ld(rv + slot);
+      cs = ld(ccase + slot);
       vcell = slot_cell(cellof, slot);
       tcell_ijk(g, vcell - g.vbase, i, j, k);
     }
@@ -1526,7 +1536,7 @@ __global__ void __launch_bounds__(kEmitThreads, 4) tmc_emit_kernel(CellSpace spa
     }
     from = upto - nt;
     total = __shfl_sync(kAll, upto, 31);
-    const int32_t to = nt ? __ldg(toff + slot) - from : 0;
+    const int32_t to = nt ? ld(toff + slot) - from : 0;
     for (int t = 0; t < nt; t++) item[from + t] = (uint16_t)(lane << 4 | t);
     __syncwarp();
     for (int t0 = 0; t0 < total; t0 += 32) {  // warp-uniform: the shuffles need every lane
@@ -1563,10 +1573,10 @@ int tmc_classify(const CellSpace& space, TmcScratch& s, int sms, cudaStream_t st
       k += launch_point_bits(space, z0, z1, sms, st);
       if (t1 <= t0) return;
       if (block_per_tile(t1 - t0, sms))
-        tmc_classify_kernel<8><<<(unsigned)(t1 - t0), kClassifyThreads, 0, st>>>(
+        launch(tmc_classify_kernel<8>, (unsigned)(t1 - t0), kClassifyThreads, st, 
             space, t0, t1, s.rec, s.cellof, s.ccase, s.mask, s.tile_sums, s.stats, amb_cells, s.amb_n);
       else
-        tmc_classify_kernel<1><<<(unsigned)ceil_div(t1 - t0, kClassifyThreads / 32), kClassifyThreads, 0, st>>>(
+        launch(tmc_classify_kernel<1>, (unsigned)ceil_div(t1 - t0, kClassifyThreads / 32), kClassifyThreads, st, 
             space, t0, t1, s.rec, s.cellof, s.ccase, s.mask, s.tile_sums, s.stats, amb_cells, s.amb_n);
       k++;
     };
@@ -1592,23 +1602,22 @@ int tmc_count(const CellSpace& space, TmcScratch& s, int64_t n_amb, int sms, cud
     Stage ta(prof, "tmc_amb_count", st);
     // the list sorted by MC case (the records follow its order, so the emission pass is sorted too)
     const unsigned gs = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n_amb, 256), (int64_t)sms * 8));
-    tmc_amb_key_kernel<<<gs, 256, 0, st>>>(space, s.cellof, amb_cells, n_amb, s.amb_key, s.amb_hist);
-    tmc_amb_cursor_kernel<<<1, 256, 0, st>>>(s.amb_hist, s.amb_hist + 256);
-    tmc_amb_sort_kernel<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n_amb, kSortTile), (int64_t)sms * 8)),
-                          256, 0, st>>>(amb_cells, s.amb_key, n_amb, s.amb_hist + 256, s.amb_sorted);
+    launch(tmc_amb_key_kernel, gs, 256, st, space, s.cellof, amb_cells, n_amb, s.amb_key, s.amb_hist);
+    launch(tmc_amb_cursor_kernel, 1, 256, st, s.amb_hist, s.amb_hist + 256);
+    launch(tmc_amb_sort_kernel, (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n_amb, kSortTile), (int64_t)sms * 8)), 256, st, amb_cells, s.amb_key, n_amb, s.amb_hist + 256, s.amb_sorted);
     static const int r_decide = resident_blocks(tmc_amb_decide_kernel, 128);
-    tmc_amb_decide_kernel<<<(unsigned)wave_grid(r_decide, sms, 16, n_amb, 128), 128, 0, st>>>(
+    launch(tmc_amb_decide_kernel, (unsigned)wave_grid(r_decide, sms, 16, n_amb, 128), 128, st, 
         space, s.cellof, s.rec, s.tile_sums, s.amb_sorted, (unsigned)n_amb, reinterpret_cast<AmbRec*>(s.amb_rec),
         s.amb_doubt, s.amb_hist + 513);
     static const int r_amb = resident_blocks(tmc_amb_count_kernel, 128);
-    tmc_amb_count_kernel<<<(unsigned)wave_grid(r_amb, sms, 4, n_amb, 128), 128, 0, st>>>(
+    launch(tmc_amb_count_kernel, (unsigned)wave_grid(r_amb, sms, 4, n_amb, 128), 128, st, 
         space, s.cellof, s.rec, s.tile_sums, s.stats, s.amb_sorted, s.amb_doubt, s.amb_hist + 513,
         reinterpret_cast<AmbRec*>(s.amb_rec), s.amb_hist + 512);
     k += 5;
   }
   Stage t(prof, "tmc_scan", st);
-  scan_tile_sums_kernel<<<1, 1024, 0, st>>>(s.tile_sums, tiles, s.totals);
-  tmc_offsets_kernel<<<(unsigned)ceil_div(tiles, kOffsetWarps), 32 * kOffsetWarps, 0, st>>>(s.mask, s.rec, s.tile_sums,
+  launch(scan_tile_sums_kernel, 1, 1024, st, s.tile_sums, tiles, s.totals);
+  launch(tmc_offsets_kernel, (unsigned)ceil_div(tiles, kOffsetWarps), 32 * kOffsetWarps, st, s.mask, s.rec, s.tile_sums,
                                                                                            tiles, s.rv, s.toff,
                                                                                            s.chunks, s.amb_n + 1,
                                                                                            n_amb > 0 ? s.amb_hist + 512 : nullptr,
@@ -1626,7 +1635,7 @@ int tmc_emit(const CellSpace& space, TmcScratch& s, int64_t n_amb, int64_t n_ove
   {                                                                                                             \
     static const int res = resident_blocks(tmc_emit_kernel<B, P>, kEmitThreads);                                \
     const int64_t blocks = wave_grid(res, sms, tu.emit_blocks_per_sm, ceil_div(space.n, 32), kEmitThreads / 32); \
-    tmc_emit_kernel<B, P><<<(unsigned)blocks, kEmitThreads, 0, st>>>(space, s.mask, s.cellof, s.ccase, s.rv, s.toff, \
+    launch(tmc_emit_kernel<B, P>, (unsigned)blocks, kEmitThreads, st, space, s.mask, s.cellof, s.ccase, s.rv, s.toff, \
                                                                      s.tile_sums, s.chunks, s.amb_n + 1, vo, tris);  \
   }
     const bool pos64 = vo.v64 != nullptr;
@@ -1640,12 +1649,11 @@ int tmc_emit(const CellSpace& space, TmcScratch& s, int64_t n_amb, int64_t n_ove
   if (n_amb == 0) return 1;
   Stage t2(prof, "tmc_ambiguous", st);
   static const int r_amb = resident_blocks(tmc_ambiguous_kernel, kAmbThreads);
-  tmc_ambiguous_kernel<<<(unsigned)wave_grid(r_amb, sms, 8, n_amb, kAmbThreads), kAmbThreads, 0, st>>>(
+  launch(tmc_ambiguous_kernel, (unsigned)wave_grid(r_amb, sms, 8, n_amb, kAmbThreads), kAmbThreads, st, 
       space, s.mask, s.cellof, s.rv, s.toff, s.tile_sums, vo, tris, reinterpret_cast<const AmbRec*>(s.amb_rec),
       s.amb_n);
   if (n_overflow == 0) return 2;
-  tmc_ambiguous_again_kernel<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n_amb, 128), (int64_t)sms * 2)),
-                               128, 0, st>>>(space, s.mask, s.cellof, s.rv, s.toff, s.tile_sums, vo, tris,
+  launch(tmc_ambiguous_again_kernel, (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n_amb, 128), (int64_t)sms * 2)), 128, st, space, s.mask, s.cellof, s.rv, s.toff, s.tile_sums, vo, tris,
                                              reinterpret_cast<const AmbRec*>(s.amb_rec), s.amb_n);
   return 3;
 }
