@@ -941,7 +941,8 @@ DmcPostStatus dmc_color_valence(const int32_t* quads, int64_t nq, int64_t nv, ui
 }
 
 DmcPostStatus dmc_postprocess(const DmcMesh& in, uint32_t flags, int sms, cudaStream_t st, DmcPostOut* out,
-                              unsigned long long* h_cnt, Prof* prof, bool borrowed, const ReadyFn* ready) {
+                              unsigned long long* h_cnt, Prof* prof, bool borrowed, const ReadyFn* ready,
+                              const TwinsFn* twins) {
   DmcPostStatus s;
   out->mesh = in;
   const bool c3x3y = flags & TMC_DMC_P3X3Y_COLOR, i3x3y = flags & TMC_DMC_P3X3Y_ISOLATED,
@@ -972,7 +973,14 @@ DmcPostStatus dmc_postprocess(const DmcMesh& in, uint32_t flags, int sms, cudaSt
   auto build_he = [&](bool handles) {
     Stage tm(prof, "dmc_halfedges", st);
     HeOut ho{hw.twin, hw.flag, hw.hv};
-    s.launches += build_halfedges(cur.quads, 4, cur.nq, cur.nv, ho, hw.w, sms, st, handles);
+    if (!twins || cur.nq == 0) {
+      s.launches += build_halfedges(cur.quads, 4, cur.nq, cur.nv, ho, hw.w, sms, st, handles);
+      return;
+    }
+    s.launches += (*twins)(hw.twin, hw.flag, hw.w.deg);
+    if (handles)
+      s.launches +=
+          halfedge_handles(cur.quads, 4, cur.nq, cur.nv, nullptr, hw.twin, hw.flag, hw.hv, hw.w, hw.hcount, sms, st);
   };
   auto retire = [&](void* ptr) {
     if (!ptr) return;

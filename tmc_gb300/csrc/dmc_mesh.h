@@ -44,12 +44,16 @@ struct DmcPostStatus {
 // halfedge arrays, then the triangles.  The caller may start copying them out.
 using ReadyFn = std::function<void(const void* dev, size_t bytes)>;
 
+// Twins, flags (4 per quad) and out-degrees of the input mesh's halfedges by the caller, who knows the cells
+// its quads come from; returns the number of kernels launched.
+using TwinsFn = std::function<int(int32_t* twin, uint8_t* flag, int32_t* deg)>;
+
 // borrowed: the input arrays belong to the caller (e.g. slices of a batch's shared arrays) and are
 // never freed here; they are still listed in out->freed once the result no longer uses them.
 // h_staging: pinned host memory for 4 words (counts read back between the passes).
 DmcPostStatus dmc_postprocess(const DmcMesh& in, uint32_t flags, int sms, cudaStream_t st, DmcPostOut* out,
                               unsigned long long* h_staging, Prof* prof = nullptr, bool borrowed = false,
-                              const ReadyFn* ready = nullptr);
+                              const ReadyFn* ready = nullptr, const TwinsFn* twins = nullptr);
 
 // The face colouring and vertex valence stage alone (colorFaces + vertexValence,
 // cpp_dmc/DualMarchingCubes.cpp:714-871): colors holds the inherited colours on entry and the reduced
