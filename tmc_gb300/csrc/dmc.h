@@ -40,6 +40,7 @@ struct DmcScratch {
   uint8_t* vrank;                 // per vertex: rank among its cell's vertices (vwork: the cell's slot)
   unsigned* amb_n;                // [0] listed cells with an ambiguous case (their slots wait in qoff), [1] chunks
   uint32_t* chunks;               // kScanTile / 32 per tile: the chunk list (scan.cuh)
+  int64_t vcap;                   // vertices that vwork and vrank have room for
 };
 
 // Each launcher returns the number of kernels it launched.  The counters (stats, totals, amb_n,
@@ -50,6 +51,9 @@ int64_t dmc_tiles(const CellSpace& space);  // scan tiles of the space
 // slabs); none: the whole field is on the device
 int dmc_front_count(const CellSpace& space, DmcScratch& s, int sms, cudaStream_t st, Prof* prof = nullptr,
                     const TileGate* gates = nullptr, int ngates = 0);
+// Offsets of the listed cells and the vertices' cells (vwork, vrank), after dmc_front_count; nothing when there
+// are more than vcap vertices.
+int dmc_front_offsets(const CellSpace& space, DmcScratch& s, cudaStream_t st, Prof* prof = nullptr);
 // Quads hold vertex indices within their own volume; vertices and quads of the volumes follow one
 // another in the output arrays.
 int dmc_front_emit(const CellSpace& space, DmcScratch& s, DmcVertexOut vo, int64_t nv, int32_t* quads,

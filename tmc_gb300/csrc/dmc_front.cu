@@ -179,12 +179,17 @@ __global__ void __launch_bounds__(128) dmc_amb_kernel(CellSpace space, const uin
 // (rv, what the quads need of a neighbour in one load) and the quad offset (blocked: 16-byte loads
 // and stores over the tile's slots), two entries per vertex (the slot of the cell that generates it
 // and its rank there), and the tile's chunks of 32 slots appended to the chunk list (scan.cuh).
+// Launched before the host knows the counts, with room for vcap vertices, so that it runs while the host
+// wakes, reads them and makes room for the results (70 to 90 us that the GPU waited); with more vertices it
+// does nothing and is launched again.
 __global__ void __launch_bounds__(32 * kOffsetWarps) dmc_offsets_kernel(const CellMask* mask, const uint32_t* rec,
                                                                        const unsigned long long* tile_off,
                                                                        int64_t tiles, uint2* rv, int32_t* qoff,
                                                                        uint32_t* vwork, uint8_t* vrank,
-                                                                       uint32_t* chunks, unsigned* nchunks) {
+                                                                       uint32_t* chunks, unsigned* nchunks,
+                                                                       const unsigned long long* totals, int64_t vcap) {
   pdl_begin();
+  if ((int64_t)(*totals >> 32) > vcap) return;  // the whole grid
   const int lane = threadIdx.x & 31;
   const int64_t tile = (int64_t)blockIdx.x * kOffsetWarps + (threadIdx.x >> 5);
   const uint32_t listed = tile < tiles ? tile_listed(mask, tile) : 0;
@@ -1474,17 +1479,18 @@ int dmc_front_count(const CellSpace& space, DmcScratch& s, int sms, cudaStream_t
 
 int64_t dmc_tiles(const CellSpace& space) { return ceil_div(space.n, kScanTile); }
 
+int dmc_front_offsets(const CellSpace& space, DmcScratch& s, cudaStream_t st, Prof* prof) {
+  Stage t(prof, "dmc_scan", st);
+  const int64_t tiles = ceil_div(space.n, kScanTile);
+  launch(dmc_offsets_kernel, (unsigned)ceil_div(tiles, kOffsetWarps), 32 * kOffsetWarps, st, s.mask, s.rec, s.tile_sums,
+         tiles, s.rv, s.qoff, s.vwork, s.vrank, s.chunks, s.amb_n + 1, s.totals, s.vcap);
+  return 1;
+}
+
 int dmc_front_emit(const CellSpace& space, DmcScratch& s, DmcVertexOut vo, int64_t nv, int32_t* quads,
                    uint8_t* colors, int flip, const Tuning& tu, cudaStream_t st, Prof* prof) {
   const int sms = tu.sms;
   const int64_t n = space.n;
-  {
-    // per-cell offsets and the vertex work list (needs the vertex count for its size)
-    Stage t(prof, "dmc_scan", st);
-    const int64_t tiles = ceil_div(n, kScanTile);
-    launch(dmc_offsets_kernel, (unsigned)ceil_div(tiles, kOffsetWarps), 32 * kOffsetWarps, st, 
-        s.mask, s.rec, s.tile_sums, tiles, s.rv, s.qoff, s.vwork, s.vrank, s.chunks, s.amb_n + 1);
-  }
   // per-vertex grids: whole waves of each kernel's resident blocks
   static const int r_point = resident_blocks(dmc_vertex_point_kernel<false>, kVertexThreads);
   static const int r_point_batch = resident_blocks(dmc_vertex_point_kernel<true>, kVertexThreads);
@@ -1548,7 +1554,7 @@ int dmc_front_emit(const CellSpace& space, DmcScratch& s, DmcVertexOut vo, int64
   if (space.grids) DMC_QUADS(true, r_quad_batch);
   else DMC_QUADS(false, r_quad);
 #undef DMC_QUADS
-  return 8;
+  return 7;
 }
 
 int dmc_front_twins(const CellSpace& space, const DmcScratch& s, int64_t nq, int32_t* twin, uint8_t* flag, int32_t* deg,

@@ -310,14 +310,21 @@ tmc::Grid make_grid(const tmc_volume* vol, const float* dev, double iso) {
 void mesh_reset(tmc_mesh* m) { std::memset(m, 0, sizeof(*m)); }
 
 // per-vertex scratch of the vertex kernels
-void plan_dmc_vertices(Allocs& al, tmc::DmcScratch& sc, int64_t nv) {
-  al.plan(&sc.vwork, nv);
-  al.plan(&sc.vrank, nv);
+// Scratch per vertex.  vwork and vrank come with the cells', with room for a vertex per cell, because the
+// offsets pass runs before the host knows nv; it is launched again with these when there are more.
+bool plan_dmc_vertices(Allocs& al, tmc::DmcScratch& sc, int64_t nv) {
+  const bool more = nv > sc.vcap;
+  if (more) {
+    al.plan(&sc.vwork, nv);
+    al.plan(&sc.vrank, nv);
+    sc.vcap = nv;
+  }
   al.plan(&sc.vp, nv);
   al.plan(&sc.fb_list, nv);
   al.plan(&sc.w_list, nv);
   al.plan(&sc.hard_list, nv);
   al.plan(&sc.tail_list, nv);
+  return more;
 }
 
 // per-cell scratch of the DMC / TMC front ends, and their counters (zeroed by start_counters)
@@ -330,6 +337,9 @@ void plan_dmc_cells(tmc_ctx* ctx, Allocs& al, tmc::DmcScratch& sc, int64_t ncell
   al.plan(&sc.chunks, tiles * (tmc::kScanTile / 32));
   al.plan(&sc.mask, tiles * (tmc::kScanTile / 32));
   al.plan(&sc.tile_sums, tiles);
+  al.plan(&sc.vwork, ncell);
+  al.plan(&sc.vrank, ncell);
+  sc.vcap = ncell;
   sc.stats = ctx->d_stats;
   sc.totals = ctx->d_stats + kStatTotals;
   sc.amb_n = reinterpret_cast<unsigned*>(ctx->d_stats + kStatAmb);
@@ -729,7 +739,9 @@ tmc_status dmc_extract(tmc_ctx* ctx, const tmc_volume* vol, double iso, uint32_t
   ctx->launches += tmc::dmc_front_count(space, sc, ctx->sms, st, &ctx->prof, gates.data(), (int)gates.size());
   unsigned long long* h = (unsigned long long*)ctx->h_pinned;
   TMC_CUDA(ctx, cudaMemcpyAsync(h, sc.totals, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-  TMC_CUDA(ctx, tmc::host_wait(st));
+  const cudaEvent_t counted = tmc::host_mark(st);
+  ctx->launches += tmc::dmc_front_offsets(space, sc, st, &ctx->prof);
+  TMC_CUDA(ctx, tmc::host_wait_mark(counted, st));
   const int64_t nv = (int64_t)(h[0] >> 32), nq = (int64_t)(h[0] & 0xffffffffull);
 
   MeshPriv* mp = new (std::nothrow) MeshPriv();
@@ -765,12 +777,13 @@ tmc_status dmc_extract(tmc_ctx* ctx, const tmc_volume* vol, double iso, uint32_t
   }
   TMC_GET(quads, 4 * nq);
   al.plan(&colors, nq);
-  plan_dmc_vertices(al, sc, nv);
+  const bool again = plan_dmc_vertices(al, sc, nv);
   ce = al.commit();
   if (ce != cudaSuccess) {
     delete mp;
     TMC_CUDA(ctx, ce);
   }
+  if (again) ctx->launches += tmc::dmc_front_offsets(space, sc, st, &ctx->prof);
   ctx->launches += tmc::dmc_front_emit(space, sc, vo, nv, quads, colors, (flags & TMC_GRAD_FLIP) ? 1 : 0, ctx->tune, st,
                                        &ctx->prof);
   TMC_CUDA(ctx, cudaGetLastError());
@@ -902,7 +915,9 @@ tmc_status tmc_extract(tmc_ctx* ctx, const tmc_volume* vol, double iso, uint32_t
   TMC_CUDA(ctx, tmc_ambiguous_records(ctx, al, sc, n_amb));
   ctx->launches += tmc::tmc_count(space, sc, n_amb, ctx->sms, st, &ctx->prof);
   TMC_CUDA(ctx, cudaMemcpyAsync(h, sc.totals, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-  TMC_CUDA(ctx, tmc::host_wait(st));
+  const cudaEvent_t counted = tmc::host_mark(st);
+  ctx->launches += tmc::tmc_offsets(space, sc, st, &ctx->prof);
+  TMC_CUDA(ctx, tmc::host_wait_mark(counted, st));
   const int64_t nv = (int64_t)(h[0] >> 32), nt = (int64_t)(h[0] & 0xffffffffull);
   const int64_t n_overflow = (int64_t)h[1];
 
@@ -1120,7 +1135,9 @@ tmc_status batch_run(tmc_ctx* ctx, const std::vector<int>& idx, const tmc_reques
              : voff_pageable.data();
   unsigned long long* h = (unsigned long long*)ctx->h_pinned;
   TMC_CUDA(ctx, cudaMemcpyAsync(toff, d_voff, (nb + 2) * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-  TMC_CUDA(ctx, tmc::host_wait(st));
+  const cudaEvent_t counted = tmc::host_mark(st);
+  ctx->launches += dmc ? tmc::dmc_front_offsets(space, dsc, st, &ctx->prof) : tmc::tmc_offsets(space, tsc, st, &ctx->prof);
+  TMC_CUDA(ctx, tmc::host_wait_mark(counted, st));
   h[0] = toff[nb];
   h[1] = toff[nb + 1];
   const int64_t NV = (int64_t)(h[0] >> 32), NF = (int64_t)(h[0] & 0xffffffffull);
@@ -1161,8 +1178,9 @@ tmc_status batch_run(tmc_ctx* ctx, const std::vector<int>& idx, const tmc_reques
     }
     TMC_CUDA(ctx, get_shared(&faces, 4 * NF));
     TMC_CUDA(ctx, get_shared(&colors, NF));
-    plan_dmc_vertices(al, dsc, NV);
+    const bool again = plan_dmc_vertices(al, dsc, NV);
     TMC_CUDA(ctx, al.commit());
+    if (again) ctx->launches += tmc::dmc_front_offsets(space, dsc, st, &ctx->prof);
     tmc::DmcVertexOut vo{v, nn, v64, n64, vcell, vuvw};
     ctx->launches += tmc::dmc_front_emit(space, dsc, vo, NV, faces, colors, 0, ctx->tune, st, &ctx->prof);
   } else {

@@ -1044,15 +1044,11 @@ __global__ void __launch_bounds__(128) tmc_amb_count_kernel(CellSpace space, con
 __global__ void __launch_bounds__(32 * kOffsetWarps) tmc_offsets_kernel(const CellMask* mask, const uint32_t* rec,
                                                                        const unsigned long long* tile_off,
                                                                        int64_t tiles, uint2* rv, int32_t* toff,
-                                                                       uint32_t* chunks, unsigned* nchunks,
-                                                                       const unsigned* overflow,
-                                                                       unsigned long long* totals) {
+                                                                       uint32_t* chunks, unsigned* nchunks) {
   pdl_begin();
   const int lane = threadIdx.x & 31;
   const int64_t tile = (int64_t)blockIdx.x * kOffsetWarps + (threadIdx.x >> 5);
   const uint32_t listed = tile < tiles ? tile_listed(mask, tile) : 0;
-  // read by the host with the totals: cells whose triangles overflow their records
-  if (blockIdx.x == 0 && threadIdx.x == 0) totals[1] = overflow ? *overflow : 0u;
   list_chunks<kOffsetWarps>(tile, listed, chunks, nchunks);
   if (tile >= tiles) return;  // the whole warp
   const int64_t base = tile * kScanTile;
@@ -1608,21 +1604,24 @@ int tmc_count(const CellSpace& space, TmcScratch& s, int64_t n_amb, int sms, cud
     static const int r_decide = resident_blocks(tmc_amb_decide_kernel, 128);
     launch(tmc_amb_decide_kernel, (unsigned)wave_grid(r_decide, sms, 16, n_amb, 128), 128, st, 
         space, s.cellof, s.rec, s.tile_sums, s.amb_sorted, (unsigned)n_amb, reinterpret_cast<AmbRec*>(s.amb_rec),
-        s.amb_doubt, s.amb_hist + 513);
+        s.amb_doubt, s.amb_hist + 512);
     static const int r_amb = resident_blocks(tmc_amb_count_kernel, 128);
     launch(tmc_amb_count_kernel, (unsigned)wave_grid(r_amb, sms, 4, n_amb, 128), 128, st, 
-        space, s.cellof, s.rec, s.tile_sums, s.stats, s.amb_sorted, s.amb_doubt, s.amb_hist + 513,
-        reinterpret_cast<AmbRec*>(s.amb_rec), s.amb_hist + 512);
+        space, s.cellof, s.rec, s.tile_sums, s.stats, s.amb_sorted, s.amb_doubt, s.amb_hist + 512,
+        reinterpret_cast<AmbRec*>(s.amb_rec), reinterpret_cast<unsigned*>(s.totals + 1));
     k += 5;
   }
   Stage t(prof, "tmc_scan", st);
   launch(scan_tile_sums_kernel, 1, 1024, st, s.tile_sums, tiles, s.totals);
+  return k + 1;
+}
+
+int tmc_offsets(const CellSpace& space, TmcScratch& s, cudaStream_t st, Prof* prof) {
+  Stage t(prof, "tmc_scan", st);
+  const int64_t tiles = tmc_tiles(space);
   launch(tmc_offsets_kernel, (unsigned)ceil_div(tiles, kOffsetWarps), 32 * kOffsetWarps, st, s.mask, s.rec, s.tile_sums,
-                                                                                           tiles, s.rv, s.toff,
-                                                                                           s.chunks, s.amb_n + 1,
-                                                                                           n_amb > 0 ? s.amb_hist + 512 : nullptr,
-                                                                                           s.totals);
-  return k + 2;
+         tiles, s.rv, s.toff, s.chunks, s.amb_n + 1);
+  return 1;
 }
 
 int tmc_emit(const CellSpace& space, TmcScratch& s, int64_t n_amb, int64_t n_overflow, TmcVertexOut vo, int32_t* tris,

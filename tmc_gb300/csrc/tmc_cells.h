@@ -29,7 +29,7 @@ struct TmcScratch {
   uint32_t* amb_sorted; // the ambiguous cells' slots sorted by MC case (one per ambiguous cell)
   uint8_t* amb_key;     // their cases, in list order (one per ambiguous cell)
   uint32_t* amb_doubt;  // places in amb_sorted that float pairs could not decide (one per ambiguous cell)
-  unsigned* amb_hist;   // 514: per-case counts, scatter cursors, cells that overflow their records, cells in doubt
+  unsigned* amb_hist;   // 513: per-case counts, scatter cursors, cells in doubt
   // listed cells (common.cuh): rec, rv and toff hold one entry per listed cell at its slot, the
   // ambiguous-cell list holds slots
   CellMask* mask;       // per 32 cells of the space
@@ -47,9 +47,12 @@ int64_t tmc_tiles(const CellSpace& space);
 int tmc_classify(const CellSpace& space, TmcScratch& s, int sms, cudaStream_t st, Prof* prof = nullptr,
                  const TileGate* gates = nullptr, int ngates = 0);
 // The ambiguous cells' counts (p_slice, float64) into their records and s.amb_rec (n_amb records,
-// n_amb = *s.amb_n), then the vertex and triangle offsets.
+// n_amb = *s.amb_n), then the totals: totals[0] = (vertices << 32) | triangles, totals[1] = cells with more
+// triangles than their records hold (tmc_emit's n_overflow).
 int tmc_count(const CellSpace& space, TmcScratch& s, int64_t n_amb, int sms, cudaStream_t st, Prof* prof = nullptr);
-// totals[1] after it: cells with more triangles than their records hold (tmc_emit's n_overflow)
+// Vertex and triangle offsets of the listed cells, after tmc_count.  The host reads the totals and makes room
+// for the results while it runs.
+int tmc_offsets(const CellSpace& space, TmcScratch& s, cudaStream_t st, Prof* prof = nullptr);
 int tmc_emit(const CellSpace& space, TmcScratch& s, int64_t n_amb, int64_t n_overflow, TmcVertexOut vo, int32_t* tris,
              const Tuning& tu, cudaStream_t st, Prof* prof = nullptr);
 
