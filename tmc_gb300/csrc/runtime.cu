@@ -146,20 +146,17 @@ struct Allocs {
   }
 };
 
-// The ambiguous cells the TMC classification listed (one host read) and their records for the
-// counting pass to fill.
-cudaError_t tmc_ambiguous_records(tmc_ctx* ctx, Allocs& al, tmc::TmcScratch& sc, int64_t& n_amb) {
-  unsigned* h = (unsigned*)ctx->h_pinned + 320;
-  cudaError_t e = cudaMemcpyAsync(h, sc.amb_n, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream);
-  if (e == cudaSuccess) e = tmc::host_wait(ctx->stream);
-  if (e != cudaSuccess) return e;
-  n_amb = (int64_t)*h;
-  al.plan(&sc.amb_rec, n_amb * tmc::kTmcAmbRecWords);
-  al.plan(&sc.amb_sorted, n_amb);
-  al.plan(&sc.amb_key, n_amb);
-  al.plan(&sc.amb_doubt, n_amb);
-  return al.commit();
+// The records of TMC's ambiguous cells, for `cap` of them.
+void plan_tmc_ambiguous(Allocs& al, tmc::TmcScratch& sc, int64_t cap) {
+  al.plan(&sc.amb_rec, cap * tmc::kTmcAmbRecWords);
+  al.plan(&sc.amb_sorted, cap);
+  al.plan(&sc.amb_key, cap);
+  al.plan(&sc.amb_doubt, cap);
+  sc.amb_cap = cap;
 }
+// What is planned before their number is known: one cell in 64, which holds the ambiguous cells of fields
+// of smooth surfaces and of dense noise (1 % of the cells); fields of saddles (15 %) take a second round.
+int64_t tmc_ambiguous_cap(int64_t ncell) { return std::min<int64_t>(ncell, std::max<int64_t>(4096, ncell / 64)); }
 
 float iso_up(double iso) {
   float f = (float)iso;
@@ -354,6 +351,7 @@ void plan_tmc_cells(tmc_ctx* ctx, Allocs& al, tmc::TmcScratch& sc, int64_t ncell
   al.plan(&sc.chunks, tiles * (tmc::kScanTile / 32));
   al.plan(&sc.mask, tiles * (tmc::kScanTile / 32));
   al.plan(&sc.tile_sums, tiles);
+  plan_tmc_ambiguous(al, sc, tmc_ambiguous_cap(ncell));
   sc.stats = ctx->d_stats;
   sc.totals = ctx->d_stats + kStatTotals;
   sc.amb_n = reinterpret_cast<unsigned*>(ctx->d_stats + kStatAmb);
@@ -912,12 +910,18 @@ tmc_status tmc_extract(tmc_ctx* ctx, const tmc_volume* vol, double iso, uint32_t
   ctx->launches += tmc::tmc_classify(space, sc, ctx->sms, st, &ctx->prof, gates.data(), (int)gates.size());
   unsigned long long* h = (unsigned long long*)ctx->h_pinned;
   int64_t n_amb = 0;
-  TMC_CUDA(ctx, tmc_ambiguous_records(ctx, al, sc, n_amb));
-  ctx->launches += tmc::tmc_count(space, sc, n_amb, ctx->sms, st, &ctx->prof);
-  TMC_CUDA(ctx, cudaMemcpyAsync(h, sc.totals, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-  const cudaEvent_t counted = tmc::host_mark(st);
-  ctx->launches += tmc::tmc_offsets(space, sc, st, &ctx->prof);
-  TMC_CUDA(ctx, tmc::host_wait_mark(counted, st));
+  for (;;) {
+    ctx->launches += tmc::tmc_count(space, sc, ctx->sms, st, &ctx->prof);
+    // the totals and, behind them, the number of ambiguous cells
+    TMC_CUDA(ctx, cudaMemcpyAsync(h, sc.totals, 3 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+    const cudaEvent_t counted = tmc::host_mark(st);
+    ctx->launches += tmc::tmc_offsets(space, sc, st, &ctx->prof);
+    TMC_CUDA(ctx, tmc::host_wait_mark(counted, st));
+    n_amb = (int64_t)(uint32_t)h[kStatAmb - kStatTotals];
+    if (n_amb <= sc.amb_cap) break;
+    plan_tmc_ambiguous(al, sc, n_amb);
+    TMC_CUDA(ctx, al.commit());
+  }
   const int64_t nv = (int64_t)(h[0] >> 32), nt = (int64_t)(h[0] & 0xffffffffull);
   const int64_t n_overflow = (int64_t)h[1];
 
@@ -1008,12 +1012,12 @@ __global__ void tile_volume_kernel(const int64_t* tile0, int nb, int64_t tiles, 
   }
   tile_vol[t] = lo;
 }
-// The scanned sums at the volumes' first tiles, then the totals (two words).
+// The scanned sums at the volumes' first tiles, then the totals (two words) and the listed cells' counters.
 __global__ void volume_offsets_kernel(const unsigned long long* tile_off, const int64_t* tile0, int nb,
                                       const unsigned long long* totals, unsigned long long* out) {
   tmc::pdl_begin();
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q < nb + 2) out[q] = q < nb ? tile_off[tile0[q]] : totals[q - nb];
+  if (q < nb + 3) out[q] = q < nb ? tile_off[tile0[q]] : totals[q - nb];
 }
 
 // One batch of requests of one algorithm: all volumes share one cell space, so every stage is one
@@ -1083,7 +1087,7 @@ tmc_status batch_run(tmc_ctx* ctx, const std::vector<int>& idx, const tmc_reques
   al.plan(&bits, bit_words + 4);
   al.plan(&d_grids, nb);
   al.plan(&d_tile0, nb + 1);
-  al.plan(&d_voff, nb + 2);
+  al.plan(&d_voff, nb + 3);
   al.plan(&d_tile_vol, tiles);
   if (dmc) plan_dmc_cells(ctx, al, dsc, ncell, tiles);
   else plan_tmc_cells(ctx, al, tsc, ncell, tiles);
@@ -1096,7 +1100,7 @@ tmc_status batch_run(tmc_ctx* ctx, const std::vector<int>& idx, const tmc_reques
   // come back do too)
   const size_t grid_bytes = nb * sizeof(tmc::Grid), tile0_bytes = (nb + 1) * sizeof(int64_t);
   char* staging = (char*)ctx->h_pinned + kPinnedTables;
-  const bool staged = grid_bytes + 2 * tile0_bytes + 64 <= kPinnedBytes - kPinnedTables;
+  const bool staged = grid_bytes + 2 * tile0_bytes + 80 <= kPinnedBytes - kPinnedTables;
   const void *grid_src = grids.data(), *tile0_src = tile0.data();
   if (staged) {
     std::memcpy(staging, grids.data(), grid_bytes);
@@ -1118,26 +1122,30 @@ tmc_status batch_run(tmc_ctx* ctx, const std::vector<int>& idx, const tmc_reques
 
   // ---- count ----
   TMC_CUDA(ctx, start_counters(ctx));
-  int64_t n_amb_rec = 0;
-  if (dmc) {
-    ctx->launches += tmc::dmc_front_count(space, dsc, ctx->sms, st, &ctx->prof);
-  } else {
-    ctx->launches += tmc::tmc_classify(space, tsc, ctx->sms, st, &ctx->prof);
-    TMC_CUDA(ctx, tmc_ambiguous_records(ctx, al, tsc, n_amb_rec));
-    ctx->launches += tmc::tmc_count(space, tsc, n_amb_rec, ctx->sms, st, &ctx->prof);
-  }
-  tmc::launch(volume_offsets_kernel, (unsigned)tmc::ceil_div(nb + 2, 256), 256, st, 
-      dmc ? dsc.tile_sums : tsc.tile_sums, d_tile0, nb, ctx->d_stats + kStatTotals, d_voff);
-  ctx->launches += 1;
-  std::vector<unsigned long long> voff_pageable(staged ? 0 : (size_t)nb + 2);
+  if (dmc) ctx->launches += tmc::dmc_front_count(space, dsc, ctx->sms, st, &ctx->prof);
+  else ctx->launches += tmc::tmc_classify(space, tsc, ctx->sms, st, &ctx->prof);
+  std::vector<unsigned long long> voff_pageable(staged ? 0 : (size_t)nb + 3);
   unsigned long long* toff =
       staged ? reinterpret_cast<unsigned long long*>(staging + ((grid_bytes + tile0_bytes + 15) & ~(size_t)15))
              : voff_pageable.data();
   unsigned long long* h = (unsigned long long*)ctx->h_pinned;
-  TMC_CUDA(ctx, cudaMemcpyAsync(toff, d_voff, (nb + 2) * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-  const cudaEvent_t counted = tmc::host_mark(st);
-  ctx->launches += dmc ? tmc::dmc_front_offsets(space, dsc, st, &ctx->prof) : tmc::tmc_offsets(space, tsc, st, &ctx->prof);
-  TMC_CUDA(ctx, tmc::host_wait_mark(counted, st));
+  int64_t n_amb_rec = 0;
+  for (;;) {
+    if (!dmc) ctx->launches += tmc::tmc_count(space, tsc, ctx->sms, st, &ctx->prof);
+    // the volumes' offsets, the totals and, behind them, the number of ambiguous cells
+    tmc::launch(volume_offsets_kernel, (unsigned)tmc::ceil_div(nb + 3, 256), 256, st,
+                dmc ? dsc.tile_sums : tsc.tile_sums, d_tile0, nb, ctx->d_stats + kStatTotals, d_voff);
+    ctx->launches += 1;
+    TMC_CUDA(ctx, cudaMemcpyAsync(toff, d_voff, (nb + 3) * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+    const cudaEvent_t counted = tmc::host_mark(st);
+    ctx->launches += dmc ? tmc::dmc_front_offsets(space, dsc, st, &ctx->prof) : tmc::tmc_offsets(space, tsc, st, &ctx->prof);
+    TMC_CUDA(ctx, tmc::host_wait_mark(counted, st));
+    if (dmc) break;
+    n_amb_rec = (int64_t)(uint32_t)toff[nb + (kStatAmb - kStatTotals)];
+    if (n_amb_rec <= tsc.amb_cap) break;
+    plan_tmc_ambiguous(al, tsc, n_amb_rec);
+    TMC_CUDA(ctx, al.commit());
+  }
   h[0] = toff[nb];
   h[1] = toff[nb + 1];
   const int64_t NV = (int64_t)(h[0] >> 32), NF = (int64_t)(h[0] & 0xffffffffull);

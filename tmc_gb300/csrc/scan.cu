@@ -5,8 +5,10 @@ namespace tmc {
 // One block of 1024 threads scans all tile sums in place.  Warp w owns a contiguous segment of
 // 32 * rounds sums and walks it in rounds of 32 consecutive sums (coalesced), carrying its running
 // sum; the warps' totals are scanned in shared memory, then each warp writes its exclusive prefixes.
-__global__ void scan_tile_sums_kernel(unsigned long long* sums, int64_t ntiles, unsigned long long* totals) {
+__global__ void scan_tile_sums_kernel(unsigned long long* sums, int64_t ntiles, unsigned long long* totals,
+                                      const unsigned* gate, unsigned cap) {
   pdl_begin();
+  if (gate && *gate > cap) return;  // the whole block
   constexpr int T = 1024, W = T / 32;
   __shared__ unsigned long long wsum[W];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -97,7 +99,7 @@ int scan_flags(const uint8_t* flags, int64_t n, int32_t* out, unsigned long long
     return 0;
   }
   launch(flag_tile_sum_kernel, (unsigned)tiles, kScanThreads, st, flags, n, tile_sums);
-  launch(scan_tile_sums_kernel, 1, 1024, st, tile_sums, tiles, total);
+  launch(scan_tile_sums_kernel, 1, 1024, st, tile_sums, tiles, total, nullptr, 0u);
   launch(flag_offsets_kernel, (unsigned)tiles, kScanThreads, st, flags, n, tile_sums, out);
   return 3;
 }
@@ -149,7 +151,7 @@ int scan_i32(const int32_t* in, int64_t n, int32_t* out, unsigned long long* til
     return 0;
   }
   launch(i32_tile_sum_kernel, (unsigned)tiles, kScanThreads, st, in, n, tile_sums);
-  launch(scan_tile_sums_kernel, 1, 1024, st, tile_sums, tiles, total);
+  launch(scan_tile_sums_kernel, 1, 1024, st, tile_sums, tiles, total, nullptr, 0u);
   launch(i32_offsets_kernel, (unsigned)tiles, kScanThreads, st, in, n, tile_sums, out);
   return 3;
 }

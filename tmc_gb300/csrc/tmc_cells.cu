@@ -698,22 +698,20 @@ __global__ void __launch_bounds__(kClassifyThreads) tmc_classify_kernel(CellSpac
 // case, so the list is sorted by case (counting sort over the 256 cases) before the float64 passes:
 // the lanes of a warp then mostly take the same branches (the float64 pipe issues for the whole warp
 // whatever its active lanes).  Key pass: each cell's case and the per-case counts.
-__global__ void __launch_bounds__(256) tmc_amb_key_kernel(CellSpace space, const uint16_t* cellof, const uint32_t* list,
-                                                          int64_t n, uint8_t* key, unsigned* hist) {
+//
+// The passes over the list are launched before the host knows how many cells it has, with records for `cap`
+// of them; a longer list (amb_cells) makes them do nothing, and the host launches them again with more.
+// Waiting for the number first cost 30 us (small calls) to 85 us.
+__device__ __forceinline__ unsigned amb_cells(const unsigned* n, unsigned cap) { return *n > cap ? 0u : *n; }
+__global__ void __launch_bounds__(256) tmc_amb_key_kernel(const uint8_t* ccase, const uint32_t* list, const unsigned* count,
+                                                          unsigned cap, uint8_t* key, unsigned* hist) {
   pdl_begin();
   __shared__ unsigned h[256];
+  const unsigned n = amb_cells(count, cap);
   h[threadIdx.x] = 0;
   __syncthreads();
-  for (int64_t a = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; a < n; a += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t vcell = slot_cell(cellof, list[a]);
-    const Grid g = space.grid_of_tile(vcell / kScanTile);
-    int i, j, k;
-    tcell_ijk(g, vcell - g.vbase, i, j, k);
-    float u[8];
-    tload_corners(g, i, j, k, u);
-    unsigned cs = 0;
-#pragma unroll
-    for (int v = 0; v < 8; v++) cs |= (unsigned)(u[v] >= g.iso_up) << v;
+  for (unsigned a = blockIdx.x * blockDim.x + threadIdx.x; a < n; a += gridDim.x * blockDim.x) {
+    const unsigned cs = ccase[list[a]];
     key[a] = (uint8_t)cs;
     atomicAdd(&h[cs], 1u);
   }
@@ -740,10 +738,12 @@ __global__ void tmc_amb_cursor_kernel(const unsigned* hist, unsigned* cursor) {
 // per-case cursors are few and hot (one atomic per cell: 1.58 ms for the 11 M ambiguous cells of the
 // 1024x1024x64 saddle field, 0.31 ms for the 1.3 M of the 512^3 noise field; 0.08 and 0.02 ms so).
 constexpr int kSortItems = 8, kSortTile = 256 * kSortItems;
-__global__ void __launch_bounds__(256) tmc_amb_sort_kernel(const uint32_t* list, const uint8_t* key, int64_t n,
-                                                           unsigned* cursor, uint32_t* sorted) {
+__global__ void __launch_bounds__(256) tmc_amb_sort_kernel(const uint32_t* list, const uint8_t* key,
+                                                           const unsigned* count, unsigned cap, unsigned* cursor,
+                                                           uint32_t* sorted) {
   pdl_begin();
   __shared__ unsigned h[256];
+  const int64_t n = amb_cells(count, cap);
   for (int64_t base = (int64_t)blockIdx.x * kSortTile; base < n; base += (int64_t)gridDim.x * kSortTile) {
     h[threadIdx.x] = 0;
     __syncthreads();
@@ -931,9 +931,10 @@ __device__ __forceinline__ bool slice_center(unsigned q_sol, const Root u[2], co
 // them, or their place in the list appended to `doubt` for that kernel.
 __global__ void __launch_bounds__(128) tmc_amb_decide_kernel(CellSpace space, const uint16_t* cellof, uint32_t* rec,
                                                              unsigned long long* tile_sums, const uint32_t* list,
-                                                             unsigned na, AmbRec* recs, uint32_t* doubt,
-                                                             unsigned* ndoubt) {
+                                                             const unsigned* count, unsigned cap, AmbRec* recs,
+                                                             uint32_t* doubt, unsigned* ndoubt) {
   pdl_begin();
+  const unsigned na = amb_cells(count, cap);
   for (unsigned a = blockIdx.x * blockDim.x + threadIdx.x; a < na; a += gridDim.x * blockDim.x) {
     const uint32_t slot = list[a];
     const int64_t vcell = slot_cell(cellof, slot);
@@ -1044,8 +1045,10 @@ __global__ void __launch_bounds__(128) tmc_amb_count_kernel(CellSpace space, con
 __global__ void __launch_bounds__(32 * kOffsetWarps) tmc_offsets_kernel(const CellMask* mask, const uint32_t* rec,
                                                                        const unsigned long long* tile_off,
                                                                        int64_t tiles, uint2* rv, int32_t* toff,
-                                                                       uint32_t* chunks, unsigned* nchunks) {
+                                                                       uint32_t* chunks, unsigned* nchunks,
+                                                                       const unsigned* gate, unsigned cap) {
   pdl_begin();
+  if (*gate > cap) return;  // the whole grid: the counts are not complete
   const int lane = threadIdx.x & 31;
   const int64_t tile = (int64_t)blockIdx.x * kOffsetWarps + (threadIdx.x >> 5);
   const uint32_t listed = tile < tiles ? tile_listed(mask, tile) : 0;
@@ -1590,37 +1593,40 @@ int tmc_classify(const CellSpace& space, TmcScratch& s, int sms, cudaStream_t st
   return k;
 }
 
-int tmc_count(const CellSpace& space, TmcScratch& s, int64_t n_amb, int sms, cudaStream_t st, Prof* prof) {
+int tmc_count(const CellSpace& space, TmcScratch& s, int sms, cudaStream_t st, Prof* prof) {
   const int64_t tiles = tmc_tiles(space);
-  const uint32_t* amb_cells = reinterpret_cast<const uint32_t*>(s.toff);
-  int k = 0;
-  if (n_amb > 0) {
+  const uint32_t* amb_list = reinterpret_cast<const uint32_t*>(s.toff);
+  const int64_t cap = s.amb_cap;
+  const unsigned cap32 = (unsigned)cap;
+  {
     Stage ta(prof, "tmc_amb_count", st);
     // the list sorted by MC case (the records follow its order, so the emission pass is sorted too)
-    const unsigned gs = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n_amb, 256), (int64_t)sms * 8));
-    launch(tmc_amb_key_kernel, gs, 256, st, space, s.cellof, amb_cells, n_amb, s.amb_key, s.amb_hist);
+    auto blocks = [&](int64_t per) {
+      return (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(cap, per), (int64_t)sms * 8));
+    };
+    launch(tmc_amb_key_kernel, blocks(256), 256, st, s.ccase, amb_list, s.amb_n, cap32, s.amb_key, s.amb_hist);
     launch(tmc_amb_cursor_kernel, 1, 256, st, s.amb_hist, s.amb_hist + 256);
-    launch(tmc_amb_sort_kernel, (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n_amb, kSortTile), (int64_t)sms * 8)), 256, st, amb_cells, s.amb_key, n_amb, s.amb_hist + 256, s.amb_sorted);
+    launch(tmc_amb_sort_kernel, blocks(kSortTile), 256, st, amb_list, s.amb_key, s.amb_n, cap32, s.amb_hist + 256,
+           s.amb_sorted);
     static const int r_decide = resident_blocks(tmc_amb_decide_kernel, 128);
-    launch(tmc_amb_decide_kernel, (unsigned)wave_grid(r_decide, sms, 16, n_amb, 128), 128, st, 
-        space, s.cellof, s.rec, s.tile_sums, s.amb_sorted, (unsigned)n_amb, reinterpret_cast<AmbRec*>(s.amb_rec),
-        s.amb_doubt, s.amb_hist + 512);
+    launch(tmc_amb_decide_kernel, (unsigned)wave_grid(r_decide, sms, 16, cap, 128), 128, st, space, s.cellof, s.rec,
+           s.tile_sums, s.amb_sorted, s.amb_n, cap32, reinterpret_cast<AmbRec*>(s.amb_rec), s.amb_doubt,
+           s.amb_hist + 512);
     static const int r_amb = resident_blocks(tmc_amb_count_kernel, 128);
-    launch(tmc_amb_count_kernel, (unsigned)wave_grid(r_amb, sms, 4, n_amb, 128), 128, st, 
-        space, s.cellof, s.rec, s.tile_sums, s.stats, s.amb_sorted, s.amb_doubt, s.amb_hist + 512,
-        reinterpret_cast<AmbRec*>(s.amb_rec), reinterpret_cast<unsigned*>(s.totals + 1));
-    k += 5;
+    launch(tmc_amb_count_kernel, (unsigned)wave_grid(r_amb, sms, 4, cap, 128), 128, st, space, s.cellof, s.rec,
+           s.tile_sums, s.stats, s.amb_sorted, s.amb_doubt, s.amb_hist + 512, reinterpret_cast<AmbRec*>(s.amb_rec),
+           reinterpret_cast<unsigned*>(s.totals + 1));
   }
   Stage t(prof, "tmc_scan", st);
-  launch(scan_tile_sums_kernel, 1, 1024, st, s.tile_sums, tiles, s.totals);
-  return k + 1;
+  launch(scan_tile_sums_kernel, 1, 1024, st, s.tile_sums, tiles, s.totals, s.amb_n, cap32);
+  return 6;
 }
 
 int tmc_offsets(const CellSpace& space, TmcScratch& s, cudaStream_t st, Prof* prof) {
   Stage t(prof, "tmc_scan", st);
   const int64_t tiles = tmc_tiles(space);
   launch(tmc_offsets_kernel, (unsigned)ceil_div(tiles, kOffsetWarps), 32 * kOffsetWarps, st, s.mask, s.rec, s.tile_sums,
-         tiles, s.rv, s.toff, s.chunks, s.amb_n + 1);
+         tiles, s.rv, s.toff, s.chunks, s.amb_n + 1, s.amb_n, (unsigned)s.amb_cap);
   return 1;
 }
 

@@ -36,6 +36,7 @@ struct TmcScratch {
   uint16_t* cellof;     // per slot: in-tile offset of the listed cell
   uint8_t* ccase;       // per slot: its MC case
   uint32_t* chunks;     // kScanTile / 32 per tile: the chunk list (scan.cuh)
+  int64_t amb_cap;      // ambiguous cells that amb_rec, amb_sorted, amb_key and amb_doubt have room for
 };
 
 // The counters (stats, totals, amb_n, amb_hist) are zero when a call starts.
@@ -46,10 +47,10 @@ int64_t tmc_tiles(const CellSpace& space);
 // leaves in *s.amb_n.  gates: as dmc_front_count's (classification of a host field arriving in slabs).
 int tmc_classify(const CellSpace& space, TmcScratch& s, int sms, cudaStream_t st, Prof* prof = nullptr,
                  const TileGate* gates = nullptr, int ngates = 0);
-// The ambiguous cells' counts (p_slice, float64) into their records and s.amb_rec (n_amb records,
-// n_amb = *s.amb_n), then the totals: totals[0] = (vertices << 32) | triangles, totals[1] = cells with more
-// triangles than their records hold (tmc_emit's n_overflow).
-int tmc_count(const CellSpace& space, TmcScratch& s, int64_t n_amb, int sms, cudaStream_t st, Prof* prof = nullptr);
+// The ambiguous cells' counts (p_slice) into their records and s.amb_rec, then the totals: totals[0] =
+// (vertices << 32) | triangles, totals[1] = cells with more triangles than their records hold (tmc_emit's
+// n_overflow).  With more than s.amb_cap ambiguous cells it does nothing, and neither does tmc_offsets.
+int tmc_count(const CellSpace& space, TmcScratch& s, int sms, cudaStream_t st, Prof* prof = nullptr);
 // Vertex and triangle offsets of the listed cells, after tmc_count.  The host reads the totals and makes room
 // for the results while it runs.
 int tmc_offsets(const CellSpace& space, TmcScratch& s, cudaStream_t st, Prof* prof = nullptr);
