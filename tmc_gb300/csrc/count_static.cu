@@ -164,7 +164,7 @@ extern "C" tmc_status tmc_dmc_count_static(tmc_ctx* ctx, const tmc_volume* vol, 
   e = cudaMemsetAsync(scratch + kActiveWord, 0, 2 * sizeof(unsigned long long), st);
   if (e != cudaSuccess) return cuda_fail(ctx, "clearing the counters", e);
   dmc_count_static_kernel<<<(unsigned)tiles, kScanThreads, 0, st>>>(g, scratch);
-  scan_tile_sums_kernel<<<1, 1024, 0, st>>>(scratch, tiles, scratch + kTotalWord);
+  scan_tile_sums(scratch, tiles, scratch + kTotalWord, st);
   ctx_count_launches(ctx, 2);
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(ctx, "kernel launch", e);

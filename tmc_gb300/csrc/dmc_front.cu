@@ -1473,7 +1473,7 @@ int dmc_front_count(const CellSpace& space, DmcScratch& s, int sms, cudaStream_t
     k++;
   }
   Stage t(prof, "dmc_scan", st);
-  launch(scan_tile_sums_kernel, 1, 1024, st, s.tile_sums, tiles, s.totals, nullptr, 0u);
+  scan_tile_sums(s.tile_sums, tiles, s.totals, st);
   return k + 1;
 }
 

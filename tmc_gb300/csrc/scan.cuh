@@ -153,11 +153,11 @@ struct Pair {
   uint64_t w;
 };
 
-// Pass 2 of a device-wide scan: exclusive scan of the per-tile sums in place, in one block.
-// sums holds `ntiles` 64-bit packed pairs; totals[0..1] get the grand totals as 64-bit.  Nothing when
-// `gate` holds more than `cap` (the sums are not complete then, and the pass runs again).
-__global__ void scan_tile_sums_kernel(unsigned long long* sums, int64_t ntiles, unsigned long long* totals,
-                                      const unsigned* gate = nullptr, unsigned cap = 0);
+// Pass 2 of a device-wide scan: exclusive scan of the per-tile sums in place, one launch.
+// sums holds `ntiles` 64-bit packed pairs; totals[0] gets the grand total.  Nothing when `gate` holds more
+// than `cap` (the sums are not complete then, and the pass runs again).
+void scan_tile_sums(unsigned long long* sums, int64_t ntiles, unsigned long long* totals, cudaStream_t st,
+                    const unsigned* gate = nullptr, unsigned cap = 0);
 
 // Device-wide compaction scan of byte flags; tile_sums needs scan_tiles(n) words.  Returns the
 // number of kernels launched.

@@ -1618,7 +1618,7 @@ int tmc_count(const CellSpace& space, TmcScratch& s, int sms, cudaStream_t st, P
            reinterpret_cast<unsigned*>(s.totals + 1));
   }
   Stage t(prof, "tmc_scan", st);
-  launch(scan_tile_sums_kernel, 1, 1024, st, s.tile_sums, tiles, s.totals, s.amb_n, cap32);
+  scan_tile_sums(s.tile_sums, tiles, s.totals, st, s.amb_n, cap32);
   return 6;
 }
 
