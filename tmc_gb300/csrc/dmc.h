@@ -59,9 +59,9 @@ int dmc_front_offsets(const CellSpace& space, DmcScratch& s, cudaStream_t st, Pr
 int dmc_front_emit(const CellSpace& space, DmcScratch& s, DmcVertexOut vo, int64_t nv, int32_t* quads,
                    uint8_t* colors, int flip, const Tuning& tu, cudaStream_t st, Prof* prof = nullptr);
 
-// Twins and flags of the halfedges of a single volume's nq quads (as build_halfedges makes them) and the number
-// of quads around each vertex, after dmc_front_emit.
-int dmc_front_twins(const CellSpace& space, const DmcScratch& s, int64_t nq, int32_t* twin, uint8_t* flag, int32_t* deg,
-                    int sms, cudaStream_t st);
+// Twins and flags (zero on entry) of the halfedges of a single volume's quads, as build_halfedges makes them,
+// and the number of quads around each vertex, after dmc_front_emit.
+int dmc_front_twins(const CellSpace& space, const DmcScratch& s, int32_t* twin, uint8_t* flag, int32_t* deg, int sms,
+                    cudaStream_t st);
 
 }  // namespace tmc

@@ -1557,9 +1557,8 @@ int dmc_front_emit(const CellSpace& space, DmcScratch& s, DmcVertexOut vo, int64
   return 7;
 }
 
-int dmc_front_twins(const CellSpace& space, const DmcScratch& s, int64_t nq, int32_t* twin, uint8_t* flag, int32_t* deg,
-                    int sms, cudaStream_t st) {
-  cudaMemsetAsync(flag, 0, (size_t)(4 * nq), st);
+int dmc_front_twins(const CellSpace& space, const DmcScratch& s, int32_t* twin, uint8_t* flag, int32_t* deg, int sms,
+                    cudaStream_t st) {
   static const int res = resident_blocks(dmc_twin_kernel, kQuadThreads);
   launch(dmc_twin_kernel, (unsigned)wave_grid(res, sms, 32, ceil_div(space.n, 32), kQuadThreads / 32), kQuadThreads, st,
          space, s.mask, s.cellof, s.ccase, s.rv, s.qoff, s.chunks, s.amb_n + 1, twin, flag, deg);

@@ -36,6 +36,7 @@ inline unsigned grid_for(int64_t n, int sms) {
   return (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n, 256), (int64_t)sms * 8));
 }
 
+// (kernels on grids of grid_for keep to the 32 registers at which its blocks are one wave)
 #define FOR_EACH(i, n) for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (n); i += (int64_t)gridDim.x * blockDim.x)
 
 // Halfedges of a quad mesh: halfedge r of face f is 4f + r; its origin is quad corner r and its
@@ -157,7 +158,7 @@ __global__ void color_reduce_kernel(HeView he, uint8_t* col, const int32_t* list
 // (rare) add with atomics.
 // One thread per face (16-byte twin loads; the corners only for a face with a boundary halfedge);
 // alive: the live faces (all when NULL).  A caller's quads need not be 16-byte aligned.
-__global__ void valence_boundary_kernel(HeView he, int64_t nq, int32_t* val, const uint8_t* alive) {
+__global__ void __launch_bounds__(256, 8) valence_boundary_kernel(HeView he, int64_t nq, int32_t* val, const uint8_t* alive) {
   pdl_begin();
   const bool vec = ((reinterpret_cast<uintptr_t>(he.q) | reinterpret_cast<uintptr_t>(he.twin)) & 15) == 0;
   FOR_EACH(f, nq) {
@@ -176,20 +177,21 @@ __global__ void valence_boundary_kernel(HeView he, int64_t nq, int32_t* val, con
 }
 
 // mark3X3Y (:889-913)
-__global__ void mark3x3y_kernel(const int32_t* q, int64_t nq, const int32_t* val, uint8_t* p, const uint8_t* alive) {
+__global__ void __launch_bounds__(256, 8) mark3x3y_kernel(const int4* q, int64_t nq, const int32_t* val, uint8_t* p, const uint8_t* alive) {
   pdl_begin();
   FOR_EACH(f, nq) {
+    const int4 v = q[f];
     if (!alive[f]) {
       p[f] = 0;
       continue;
     }
-    const int a = val[q[4 * f]], b = val[q[4 * f + 1]], c = val[q[4 * f + 2]], d = val[q[4 * f + 3]];
+    const int a = val[v.x], b = val[v.y], c = val[v.z], d = val[v.w];
     p[f] = (a == 3 && b >= 5 && c == 3 && d >= 5) || (a >= 5 && b == 3 && c >= 5 && d == 3);
   }
 }
 
 // mergeVertices3X3Y, both variants (:916-1094): decide removal, claim written vertices
-__global__ void merge_claim_kernel(HeView he, int64_t nq, const uint8_t* p, const int32_t* val,
+__global__ void __launch_bounds__(256, 8) merge_claim_kernel(HeView he, int64_t nq, const uint8_t* p, const int32_t* val,
                                    const uint8_t* col, int color_pass, uint8_t* branch, int32_t* own_pos,
                                    int32_t* own_rm) {
   pdl_begin();
@@ -292,20 +294,26 @@ __device__ __forceinline__ void midpoint(double* v64, double* n64, int dst, int 
   }
 }
 
+// What a pass does to a vertex, in one byte (two arrays cost the next pass two gathers per corner).  Two faces
+// may mark one vertex differently, hence the atomic.
+constexpr unsigned kTouched = 1, kRemoved = 2;
+__device__ __forceinline__ void mark(uint8_t* marks, int v, unsigned m) {
+  atomicOr(reinterpret_cast<unsigned*>(marks) + (v >> 2), m << (8 * (v & 3)));
+}
+
 // Marks the removed vertices and lists the midpoint merges (destination, two sources); the
 // float64 midpoints run densely in midpoint_kernel (a few merging faces per warp would otherwise
 // pay the float64 pipe for the whole warp).  Each destination has one owner, and the sources are
 // never destinations (valence >= 5 vs valence 3), so the merges are independent.
-// dold: the valence-3 corners of the removed faces (merge targets and removed vertices), the
+// marks: the valence-3 corners of the removed faces (merge targets and removed vertices) are touched, the
 // vertices the halfedge repair re-pairs around; valive: the removed vertices die.
 // The jobs of a block's faces are gathered in shared memory and appended with one global atomic
 // per block and iteration (per-warp appends to the one counter serialise on it).
 constexpr int kMergeThreads = 256;
 __global__ void __launch_bounds__(kMergeThreads) merge_apply_kernel(HeView he, int64_t nq, const uint8_t* branch,
                                                                    const int32_t* own_pos, const int32_t* own_rm,
-                                                                   uint8_t* vm_first, int32_t* vm_second, uint8_t* em,
-                                                                   int4* jobs, unsigned* njobs, uint8_t* dold,
-                                                                   uint8_t* valive) {
+                                                                   int32_t* vm_second, uint8_t* em, int4* jobs,
+                                                                   unsigned* njobs, uint8_t* marks, uint8_t* valive) {
   pdl_begin();
   __shared__ int4 s_jobs[kMergeThreads];
   __shared__ unsigned s_n, s_base;
@@ -327,9 +335,8 @@ __global__ void __launch_bounds__(kMergeThreads) merge_apply_kernel(HeView he, i
             job = true;
             jv = make_int4(v0, v1, v3, 0);
           }
-          dold[v0] = 1;
-          dold[v2] = 1;
-          vm_first[v2] = 1;
+          mark(marks, v0, kTouched);
+          mark(marks, v2, kTouched | kRemoved);
           valive[v2] = 0;
           if (own_rm[v2] == f) vm_second[v2] = v0;
         } else {
@@ -337,9 +344,8 @@ __global__ void __launch_bounds__(kMergeThreads) merge_apply_kernel(HeView he, i
             job = true;
             jv = make_int4(v1, v0, v2, 0);
           }
-          dold[v1] = 1;
-          dold[v3] = 1;
-          vm_first[v3] = 1;
+          mark(marks, v1, kTouched);
+          mark(marks, v3, kTouched | kRemoved);
           valive[v3] = 0;
           if (own_rm[v3] == f) vm_second[v3] = v1;
         }
@@ -385,7 +391,7 @@ __global__ void float_outputs_kernel(const double* v64, const double* n64, int64
 // Writes what the result keeps: the float32 positions and normals (roundings of the float64 positions and
 // float-pair normals) and, when they are an output (v64o), the float64 positions.  16.6 M vertices, 12 M
 // kept: 349 us with the float64 positions and the normals' pairs copied along (nothing reads them), 227 us.
-__global__ void gather_vertices_kernel(const uint8_t* keep, const int32_t* idx, int64_t nv, const double* v64,
+__global__ void __launch_bounds__(256, 8) gather_vertices_kernel(const uint8_t* keep, const int32_t* idx, int64_t nv, const double* v64,
                                        const double* n64, double* v64o, int32_t* map, int64_t cap, unsigned* overflow,
                                        float* vo, float* no) {
   pdl_begin();
@@ -411,17 +417,13 @@ __global__ void gather_vertices_kernel(const uint8_t* keep, const int32_t* idx, 
 }
 
 // A killed face's corners that stay clean lose one outgoing halfedge each.
-__device__ __forceinline__ void killed_face_degrees(const int32_t* q, int64_t f, const uint8_t* dold, int32_t* deg) {
-  for (int r = 0; r < 4; r++) {
-    const int x = q[4 * f + r];
-    if (!dold[x]) atomicSub(deg + x, 1);
-  }
+// A live face's corner x, now y, is marked for the halfedge repair: y is dirty when x was touched by the
+// pass, and then its out-degree is recounted from zero.
+__device__ __forceinline__ void killed_corner(int x, unsigned m, int32_t* deg) {
+  if (!(m & kTouched)) atomicSub(deg + x, 1);
 }
-
-// Marks a live face's corner x, now y, for the halfedge repair: y is dirty when x was touched by the
-// pass (dold), and then its out-degree is recounted from zero.
-__device__ __forceinline__ void touch_corner(int x, int y, const uint8_t* dold, uint8_t* dirty, int32_t* deg) {
-  if (dold[x] && y >= 0) {
+__device__ __forceinline__ void live_corner(int y, unsigned m, uint8_t* dirty, int32_t* deg) {
+  if ((m & kTouched) && y >= 0) {
     dirty[y] = 1;
     deg[y] = 0;
   }
@@ -431,28 +433,39 @@ __device__ __forceinline__ void touch_corner(int x, int y, const uint8_t* dold, 
 // corners on removed vertices move to their merge target (which a merge always keeps: the faces
 // around a valence-3 vertex are pairwise adjacent and no two adjacent faces merge in one pass).
 // Faces and vertices keep their indices; the compaction runs once after the last pass.
-__global__ void apply_3x3y_kernel(int32_t* q, int64_t nq, uint8_t* alive, const uint8_t* em, const uint8_t* vm_first,
-                                  const int32_t* vm_second, const uint8_t* dold, uint8_t* dirty, int32_t* deg) {
+// Bound by the latency of the corners' gathers (the four marks are loaded together): 16.6 M faces 216 -> 143 us
+// in the first pass, 156 -> 85 us in the second, 178 -> 122 us for apply_3333_kernel, with two bytes per
+// corner and the corners one by one before.
+__global__ void __launch_bounds__(256, 8) apply_3x3y_kernel(int4* q, int64_t nq, uint8_t* alive, const uint8_t* em, const uint8_t* marks,
+                                  const int32_t* vm_second, uint8_t* dirty, int32_t* deg) {
   pdl_begin();
   FOR_EACH(f, nq) {
-    if (!alive[f]) continue;
-    if (em[f]) {
+    const uint8_t a = alive[f], e = em[f];
+    const int4 c = q[f];
+    if (!a) continue;
+    const unsigned m0 = marks[c.x], m1 = marks[c.y], m2 = marks[c.z], m3 = marks[c.w];
+    if (e) {
       alive[f] = 0;
-      killed_face_degrees(q, f, dold, deg);
+      killed_corner(c.x, m0, deg);
+      killed_corner(c.y, m1, deg);
+      killed_corner(c.z, m2, deg);
+      killed_corner(c.w, m3, deg);
       continue;
     }
-    for (int r = 0; r < 4; r++) {
-      const int x = q[4 * f + r];
-      const int y = vm_first[x] ? vm_second[x] : x;
-      if (y != x) q[4 * f + r] = y;
-      touch_corner(x, y, dold, dirty, deg);
-    }
+    if (!((m0 | m1 | m2 | m3) & kTouched)) continue;  // a removed vertex is a touched one
+    const int4 y = make_int4(m0 & kRemoved ? vm_second[c.x] : c.x, m1 & kRemoved ? vm_second[c.y] : c.y,
+                             m2 & kRemoved ? vm_second[c.z] : c.z, m3 & kRemoved ? vm_second[c.w] : c.w);
+    if ((m0 | m1 | m2 | m3) & kRemoved) q[f] = y;
+    live_corner(y.x, m0, dirty, deg);
+    live_corner(y.y, m1, dirty, deg);
+    live_corner(y.z, m2, dirty, deg);
+    live_corner(y.w, m3, dirty, deg);
   }
 }
 
 // mark3333 (:1189-1322)
-__global__ void mark3333_kernel(HeView he, int64_t nq, const int32_t* val, uint8_t* p3, uint8_t* rflag,
-                                uint8_t* vm0, int32_t* vm1, uint8_t* dold, const uint8_t* alive, uint8_t* valive) {
+__global__ void __launch_bounds__(256, 8) mark3333_kernel(HeView he, int64_t nq, const int32_t* val, uint8_t* p3, uint8_t* rflag,
+                                int32_t* vm1, uint8_t* marks, const uint8_t* alive, uint8_t* valive) {
   pdl_begin();
   FOR_EACH(f, nq) {
     if (!alive[f] || non_manifold(he, f)) continue;
@@ -480,10 +493,9 @@ __global__ void mark3333_kernel(HeView he, int64_t nq, const int32_t* val, uint8
     if (a == 3 || b == 3 || c == 3 || d == 3) continue;
     if (a == 4 && b == 4 && c == 4 && d == 4) continue;
     for (int r = 0; r < 4; r++) {
-      vm0[vq[r]] = 1;
       vm1[vq[r]] = vo[r];
-      dold[vq[r]] = 1;
-      dold[vo[r]] = 1;
+      marks[vq[r]] = kTouched;
+      marks[vo[r]] = kTouched;
       valive[vq[r]] = 0;
     }
     p3[f] = 1;
@@ -493,23 +505,32 @@ __global__ void mark3333_kernel(HeView he, int64_t nq, const int32_t* val, uint8
 
 // removeVertices3333 + removeQuadrilaterals3333 (:1324-1382) in place: the four neighbours of a
 // marked face die and its corners move to the neighbours' far vertices (kept: their valence is not 3).
-__global__ void apply_3333_kernel(int32_t* q, int64_t nq, uint8_t* alive, const uint8_t* rflag, const uint8_t* p3,
-                                  const int32_t* vm1, const uint8_t* dold, uint8_t* dirty, int32_t* deg) {
+__global__ void __launch_bounds__(256, 8) apply_3333_kernel(int4* q, int64_t nq, uint8_t* alive, const uint8_t* rflag, const uint8_t* p3,
+                                  const int32_t* vm1, const uint8_t* marks, uint8_t* dirty, int32_t* deg) {
   pdl_begin();
   FOR_EACH(f, nq) {
-    if (!alive[f]) continue;
-    if (rflag[f]) {
+    const uint8_t a = alive[f], e = rflag[f], moved = p3[f];
+    const int4 c = q[f];
+    if (!a) continue;
+    const unsigned m0 = marks[c.x], m1 = marks[c.y], m2 = marks[c.z], m3 = marks[c.w];
+    if (e) {
       alive[f] = 0;
-      killed_face_degrees(q, f, dold, deg);
+      killed_corner(c.x, m0, deg);
+      killed_corner(c.y, m1, deg);
+      killed_corner(c.z, m2, deg);
+      killed_corner(c.w, m3, deg);
       continue;
     }
-    const bool moved = p3[f] != 0;
-    for (int r = 0; r < 4; r++) {
-      const int x = q[4 * f + r];
-      const int y = moved ? vm1[x] : x;
-      if (y != x) q[4 * f + r] = y;
-      touch_corner(x, y, dold, dirty, deg);
+    if (!((m0 | m1 | m2 | m3) & kTouched)) continue;  // a moved face's corners are touched
+    int4 y = c;
+    if (moved) {
+      y = make_int4(vm1[c.x], vm1[c.y], vm1[c.z], vm1[c.w]);
+      q[f] = y;
     }
+    live_corner(y.x, m0, dirty, deg);
+    live_corner(y.y, m1, dirty, deg);
+    live_corner(y.z, m2, dirty, deg);
+    live_corner(y.w, m3, dirty, deg);
   }
 }
 
@@ -834,9 +855,9 @@ struct HeBufs {
   unsigned long long* zero = nullptr;
   unsigned long long* nm = nullptr;
   unsigned* ovf = nullptr;
-  // repairs after the simplification passes: vertices a pass touched (dold) and the dirty ones
+  // repairs after the simplification passes: what a pass did to the vertices (marks) and the dirty ones
   // (dnew); the compacted faces' indices before (src); handle counters
-  uint8_t* dold = nullptr;
+  uint8_t* marks = nullptr;
   uint8_t* dnew = nullptr;
   int32_t* src = nullptr;
   HeUpdateWork u{};
@@ -860,6 +881,41 @@ int color_faces(const HeView& he, uint8_t* col, int64_t nq, int32_t* cnt, Pool& 
   for (int k = 0; k < 19; k++) launch(color_reduce_kernel, gq, 256, st, he, col, list, off, k, 4);
   launch(color_reduce_kernel, gq, 256, st, he, col, list, off, 19, 3);
   return 23;
+}
+
+// Fills and one copy in one launch (16 bytes at a time; the arrays' pool blocks are whole multiples, so a
+// last partial one stays inside).  As fills and copies of the stream's own they cost 5 to 6 us each between
+// short kernels, three or four per pass: 131x117x140 with all outputs 648 -> 595 us with one launch each.
+struct Fill {
+  uint4* p;
+  int64_t n;  // of 16 bytes
+  uint32_t v;
+};
+Fill fill(void* p, size_t bytes, uint32_t v) {
+  return Fill{reinterpret_cast<uint4*>(p), (int64_t)((bytes + 15) / 16), v};
+}
+struct Fills {
+  Fill f[4];
+};
+__global__ void __launch_bounds__(256) fill_and_copy_kernel(Fills fills, const uint4* from, uint4* to, int64_t n) {
+  pdl_begin();
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const uint32_t v = fills.f[q].v;
+    FOR_EACH(i, fills.f[q].n) fills.f[q].p[i] = make_uint4(v, v, v, v);
+  }
+  FOR_EACH(i, n) to[i] = from[i];
+}
+int fill_and_copy(const std::vector<Fill>& fills, const void* from, void* to, size_t bytes, int sms, cudaStream_t st) {
+  Fills f{};
+  int64_t most = (int64_t)((bytes + 15) / 16);
+  for (size_t q = 0; q < fills.size(); q++) {  // at most four
+    f.f[q] = fills[q];
+    most = std::max(most, fills[q].n);
+  }
+  launch(fill_and_copy_kernel, grid_for(std::max<int64_t>(most, 1), sms), 256, st, f,
+         reinterpret_cast<const uint4*>(from), reinterpret_cast<uint4*>(to), (int64_t)((bytes + 15) / 16));
+  return 1;
 }
 
 // vertexValence (:847-871): the out-degrees of the halfedge build plus the boundary corrections
@@ -895,15 +951,14 @@ HeBufs halfedge_buffers(Pool& pool, int64_t NV, int64_t NQ) {
 }
 
 // Buffers of the simplification passes, their halfedge repairs and the final compaction.  What a pass
-// resets lies together: `fresh` (bucket sizes, merge marks, touched and dirty vertices) is zeroed and
-// `owner` (claims and merge targets) set to -1 by one fill each.
+// resets lies together: `fresh` (bucket sizes, marks and dirty vertices) is zeroed and `owner` (claims and
+// merge targets) set to -1.
 struct PassBufs {
   int32_t* val;
   uint8_t *p, *em, *branch;   // p and em adjacent (both zero for P3333)
   size_t face_stride;         // from p to em
   uint8_t* fresh;
   size_t fresh_bytes;
-  uint8_t* vm_first;
   int32_t* owner;
   int32_t *own_pos, *own_rm, *vm_second;
   int4* jobs;
@@ -926,12 +981,11 @@ PassBufs pass_buffers(Pool& pool, HeBufs& hw, int64_t NV, int64_t NQ) {
   b.p = pool.get<uint8_t>(2 * nq16);
   b.em = b.p + nq16;
   b.branch = pool.get<uint8_t>(NQ);
-  b.fresh_bytes = (size_t)(7 * nv16);
-  b.fresh = pool.get<uint8_t>(7 * nv16);
+  b.fresh_bytes = (size_t)(6 * nv16);
+  b.fresh = pool.get<uint8_t>(6 * nv16);
   hw.u.bcnt = reinterpret_cast<int32_t*>(b.fresh);
-  b.vm_first = b.fresh + 4 * nv16;
-  hw.dold = b.fresh + 5 * nv16;
-  hw.dnew = b.fresh + 6 * nv16;
+  hw.marks = b.fresh + 4 * nv16;
+  hw.dnew = b.fresh + 5 * nv16;
   b.owner = pool.get<int32_t>(3 * NV);
   b.own_pos = b.owner;
   b.own_rm = b.owner + NV;
@@ -995,9 +1049,14 @@ DmcPostStatus dmc_postprocess(const DmcMesh& in, uint32_t flags, int sms, cudaSt
     s.err = pool.err;
     return s;
   }
-  cudaMemsetAsync(hw.zero, 0, kZeroWords * sizeof(unsigned long long), st);
   const unsigned gq = grid_for(NQ, sms);
   const bool simplify = (c3x3y || i3x3y || p3333) && in.nq > 0;
+  // the counters and what else a call starts from
+  auto start = [&](std::vector<Fill> fills) {
+    fills.push_back(fill(hw.zero, kZeroWords * sizeof(unsigned long long), 0u));
+    if (twins && cur.nq > 0) fills.push_back(fill(hw.flag, 4 * (size_t)NQ, 0u));
+    s.launches += fill_and_copy(fills, nullptr, nullptr, 0, sms, st);
+  };
   auto build_he = [&](bool handles) {
     Stage tm(prof, "dmc_halfedges", st);
     HeOut ho{hw.twin, hw.flag, hw.hv};
@@ -1037,14 +1096,14 @@ DmcPostStatus dmc_postprocess(const DmcMesh& in, uint32_t flags, int sms, cudaSt
   if (simplify) {
     const PassBufs b = pass_buffers(pool, hw, NV, NQ);
     int32_t *val = b.val, *own_pos = b.own_pos, *own_rm = b.own_rm, *vm_second = b.vm_second;
-    uint8_t *p = b.p, *em = b.em, *branch = b.branch, *vm_first = b.vm_first;
+    uint8_t *p = b.p, *em = b.em, *branch = b.branch;
     alive = b.alive;
     valive = b.valive;
     idx = b.idx;
     idx_q = b.idx_q;
     map = b.vm_second;
     if ((s.err = pool.err) != cudaSuccess) return s;
-    cudaMemsetAsync(alive, 1, (size_t)(NQ + NV), st);
+    start({fill(alive, (size_t)(NQ + NV), 0x01010101u)});
     build_he(false);
     const HeView he{q0, hw.twin, hw.flag};
     // what is left after the last pass, counted before its repair and the handles: they run while the host
@@ -1056,6 +1115,12 @@ DmcPostStatus dmc_postprocess(const DmcMesh& in, uint32_t flags, int sms, cudaSt
       cudaMemcpyAsync(h_cnt, total, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st);
       cudaMemcpyAsync(h_cnt + 1, idx, sizeof(int32_t), cudaMemcpyDeviceToHost, st);
       counted = host_mark(st);
+    };
+    // what a pass starts from: its marks and the vertices' valences (vertexValence :847-871)
+    auto begin_pass = [&](const std::vector<Fill>& fills) {
+      s.launches += fill_and_copy(fills, hw.w.deg, val, (size_t)nv0 * sizeof(int32_t), sms, st);
+      launch(valence_boundary_kernel, gq, 256, st, he, nq0, val, alive);
+      s.launches += 2;
     };
     auto repair = [&]() {
       Stage tm(prof, "dmc_halfedges", st);
@@ -1072,17 +1137,16 @@ DmcPostStatus dmc_postprocess(const DmcMesh& in, uint32_t flags, int sms, cudaSt
       }
       {
         Stage tm(prof, "dmc_p3x3y", st);
-        s.launches += vertex_valence(he, hw.w.deg, nv0, nq0, val, sms, st, alive);
-        launch(mark3x3y_kernel, gq, 256, st, q0, nq0, val, p, alive);
-        cudaMemsetAsync(b.owner, 0xff, 3 * (size_t)NV * sizeof(int32_t), st);
-        cudaMemsetAsync(b.fresh, 0, b.fresh_bytes, st);
+        begin_pass({fill(b.owner, 3 * (size_t)NV * sizeof(int32_t), 0xffffffffu), fill(b.fresh, b.fresh_bytes, 0u)});
+        launch(mark3x3y_kernel, gq, 256, st, reinterpret_cast<const int4*>(q0), nq0, val, p, alive);
         launch(merge_claim_kernel, gq, 256, st, he, nq0, p, val, cur.colors, pass == 0, branch, own_pos, own_rm);
         unsigned* njobs = reinterpret_cast<unsigned*>(hw.zero + kZeroJobs) + pass;
-        launch(merge_apply_kernel, gq, kMergeThreads, st, he, nq0, branch, own_pos, own_rm, vm_first, vm_second, em,
-                                                         b.jobs, njobs, hw.dold, valive);
+        launch(merge_apply_kernel, gq, kMergeThreads, st, he, nq0, branch, own_pos, own_rm, vm_second, em, b.jobs, njobs,
+               hw.marks, valive);
         static const int r_mid = resident_blocks(midpoint_kernel, 256);  // one wave over the merge list
         launch(midpoint_kernel, (unsigned)wave_grid(r_mid, sms, 1, nq0, 256), 256, st, b.jobs, njobs, cur.v64, cur.n64);
-        launch(apply_3x3y_kernel, gq, 256, st, q0, nq0, alive, em, vm_first, vm_second, hw.dold, hw.dnew, hw.w.deg);
+        launch(apply_3x3y_kernel, gq, 256, st, reinterpret_cast<int4*>(q0), nq0, alive, em, hw.marks, vm_second, hw.dnew,
+               hw.w.deg);
         s.launches += 5;
       }
       if (!p3333 && (pass == 1 || !i3x3y)) count_live();
@@ -1094,14 +1158,12 @@ DmcPostStatus dmc_postprocess(const DmcMesh& in, uint32_t flags, int sms, cudaSt
         Stage tm(prof, "dmc_p3333", st);
         uint8_t* p3 = p;
         uint8_t* rflag = em;
-        uint8_t* vm0 = vm_first;
         int32_t* vm1 = own_pos;
-        s.launches += vertex_valence(he, hw.w.deg, nv0, nq0, val, sms, st, alive);
-        cudaMemsetAsync(p3, 0, 2 * b.face_stride, st);  // and rflag behind it
-        cudaMemsetAsync(b.fresh, 0, b.fresh_bytes, st);
-        cudaMemsetAsync(vm1, 0xff, (size_t)NV * sizeof(int32_t), st);
-        launch(mark3333_kernel, gq, 256, st, he, nq0, val, p3, rflag, vm0, vm1, hw.dold, alive, valive);
-        launch(apply_3333_kernel, gq, 256, st, q0, nq0, alive, rflag, p3, vm1, hw.dold, hw.dnew, hw.w.deg);
+        begin_pass({fill(p3, 2 * b.face_stride, 0u) /* and rflag behind it */, fill(b.fresh, b.fresh_bytes, 0u),
+                    fill(vm1, (size_t)NV * sizeof(int32_t), 0xffffffffu)});
+        launch(mark3333_kernel, gq, 256, st, he, nq0, val, p3, rflag, vm1, hw.marks, alive, valive);
+        launch(apply_3333_kernel, gq, 256, st, reinterpret_cast<int4*>(q0), nq0, alive, rflag, p3, vm1, hw.marks, hw.dnew,
+               hw.w.deg);
         s.launches += 2;
       }
       count_live();
@@ -1190,6 +1252,7 @@ DmcPostStatus dmc_postprocess(const DmcMesh& in, uint32_t flags, int sms, cudaSt
     if (flags & TMC_OUT_POS_F64) (*ready)(cur.v64, (size_t)cur.nv * 3 * sizeof(double));
     (*ready)(cur.quads, (size_t)cur.nq * 4 * sizeof(int32_t));
   }
+  if (!simplify) start({});
   if (want_he) {
     if (!simplify) build_he(true);  // the front-end mesh as it is: one build with the handles
     Stage tm(prof, "dmc_halfedges", st);
@@ -1218,7 +1281,9 @@ DmcPostStatus dmc_postprocess(const DmcMesh& in, uint32_t flags, int sms, cudaSt
     uint32_t* tlist = pool.get<uint32_t>(std::max<int64_t>(cur.nq, 1));
     unsigned* tcount = reinterpret_cast<unsigned*>(hw.zero + kZeroSplit);
     if ((s.err = pool.err) == cudaSuccess) {
-      launch(triangles_fast_kernel, grid_for(cur.nq, sms), 256, st, cur.quads, cur.nq, cur.v, tr, tlist, tcount);
+      static const int r_fast = resident_blocks(triangles_fast_kernel, 256);
+      launch(triangles_fast_kernel, (unsigned)wave_grid(r_fast, sms, 8, cur.nq, 256), 256, st, cur.quads, cur.nq, cur.v, tr,
+             tlist, tcount);
       const unsigned gt = grid_for(cur.nq, sms);
       const int kind = libm::host_acosf_kind();
       // positions from the uncompacted mesh, by its quads

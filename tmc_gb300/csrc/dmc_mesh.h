@@ -44,7 +44,7 @@ struct DmcPostStatus {
 // halfedge arrays, then the triangles.  The caller may start copying them out.
 using ReadyFn = std::function<void(const void* dev, size_t bytes)>;
 
-// Twins, flags (4 per quad) and out-degrees of the input mesh's halfedges by the caller, who knows the cells
+// Twins, flags (4 per quad, zero on entry) and out-degrees of the input mesh's halfedges by the caller, who knows the cells
 // its quads come from; returns the number of kernels launched.
 using TwinsFn = std::function<int(int32_t* twin, uint8_t* flag, int32_t* deg)>;
 

@@ -799,7 +799,7 @@ tmc_status dmc_extract(tmc_ctx* ctx, const tmc_volume* vol, double iso, uint32_t
   EarlyCopies early{ctx, mp};
   const tmc::ReadyFn ready = [&early](const void* dev, size_t bytes) { early.issue(dev, bytes); };
   const tmc::TwinsFn twins = [&](int32_t* twin, uint8_t* flag, int32_t* deg) {
-    return tmc::dmc_front_twins(space, sc, nq, twin, flag, deg, ctx->sms, st);
+    return tmc::dmc_front_twins(space, sc, twin, flag, deg, ctx->sms, st);
   };
   tmc::DmcPostStatus ps =
       tmc::dmc_postprocess(mesh, flags, ctx->sms, st, &post, (unsigned long long*)ctx->h_pinned + 64, &ctx->prof,
