@@ -21,6 +21,7 @@
 #include <cmath>
 
 #include "../../include/tmc_gb300.h"
+#include "color_groups.h"
 #include "dmc_mesh.h"
 #include "ffloat.cuh"
 #include "halfedges.h"
@@ -70,14 +71,27 @@ __device__ __forceinline__ bool non_manifold(const HeView& he, int64_t f) {
 // ---------------------------------------------------------------------------------------------
 // colouring
 // ---------------------------------------------------------------------------------------------
-// class of an inherited colour: 0..18 for colours 5..23, 19 for colour 4, -1 otherwise
-__device__ __forceinline__ int color_class(int c) { return c > 4 ? c - 5 : (c == 4 ? 19 : -1); }
+// The group a face's inherited colour is reduced in, -1 for colours 0..3.  Of any mesh: a group per colour,
+// 5..23 in order, then 4.  Of the front end's own (kFront): inherited colours are those of grid edges, and two
+// faces share an edge only when their grid edges lie on one grid face, so most pairs of colours never meet;
+// a colour's group is one after the last earlier colour it can meet, which leaves 14 groups, each as
+// independent as one colour (tests/test_color_groups_cpu.py derives them).  Small meshes pay per launch:
+// 0.4 M faces 57 -> 39 us, 2.2 M 84 -> 65 us; 16.6 M 0.26 ms either way.
+constexpr int kColorGroups = 20, kFrontGroups = 14;
+template <bool kFront>
+__device__ __forceinline__ int color_class(int c) {
+  if (!kFront) return c > 4 ? c - 5 : (c == 4 ? 19 : -1);
+  // group of colours 4..23, four bits each: 4..19, then 20..23
+  constexpr uint64_t lo = TMC_FRONT_GROUPS_LO, hi = TMC_FRONT_GROUPS_HI;
+  return c < 4 ? -1 : (int)((c < 20 ? lo >> (4 * (c - 4)) : hi >> (4 * (c - 20))) & 15);
+}
 
 // Class histograms and lists are aggregated per block (shared-memory ranks, one global atomic per
 // class and block): 20 global counters hit by every face serialise the whole pass otherwise.  The
 // order of faces within a class list does not matter (faces of one class never touch).
 constexpr int kColorThreads = 256, kColorItems = 8, kColorTile = kColorThreads * kColorItems;
 
+template <bool kFront>
 __global__ void __launch_bounds__(kColorThreads) color_count_kernel(const uint8_t* col, int64_t nq, int32_t* cnt) {
   pdl_begin();
   __shared__ int h[20];
@@ -88,7 +102,7 @@ __global__ void __launch_bounds__(kColorThreads) color_count_kernel(const uint8_
   for (int s = 0; s < kColorItems; s++) {
     const int64_t f = base + s * kColorThreads + threadIdx.x;
     if (f < nq) {
-      const int k = color_class(col[f]);
+      const int k = color_class<kFront>(col[f]);
       if (k >= 0) atomicAdd(&h[k], 1);
     }
   }
@@ -109,6 +123,7 @@ __global__ void color_offsets_kernel(const int32_t* cnt, int32_t* off, int32_t* 
   }
 }
 
+template <bool kFront>
 __global__ void __launch_bounds__(kColorThreads) color_scatter_kernel(const uint8_t* col, int64_t nq, int32_t* cursor,
                                                                      int32_t* list) {
   pdl_begin();
@@ -120,7 +135,7 @@ __global__ void __launch_bounds__(kColorThreads) color_scatter_kernel(const uint
 #pragma unroll
   for (int s = 0; s < kColorItems; s++) {
     const int64_t f = base + s * kColorThreads + threadIdx.x;
-    ks[s] = (f < nq) ? color_class(col[f]) : -1;
+    ks[s] = (f < nq) ? color_class<kFront>(col[f]) : -1;
     rs[s] = (ks[s] >= 0) ? atomicAdd(&h[ks[s]], 1) : 0;
   }
   __syncthreads();
@@ -865,22 +880,25 @@ struct HeBufs {
 };
 
 // colorFaces (:714-844) on a mesh whose halfedges are built: the inherited colours in `col` become
-// the reduced ones, class by class (colours 5..23 to the lowest of 0..4 free among the neighbours,
-// then colour 4 to the lowest of 0..3).  Returns the number of kernels launched.
-// cnt: 24 zeroed words.
-int color_faces(const HeView& he, uint8_t* col, int64_t nq, int32_t* cnt, Pool& pool, int sms, cudaStream_t st) {
+// the reduced ones, group by group (colours 5..23 to the lowest of 0..4 free among the neighbours,
+// then colour 4, the last group, to the lowest of 0..3).  Returns the number of kernels launched.
+// cnt: 24 zeroed words; front: the mesh is as the front end made it.
+int color_faces(const HeView& he, uint8_t* col, int64_t nq, int32_t* cnt, bool front, Pool& pool, int sms,
+                cudaStream_t st) {
   int32_t* off = pool.get<int32_t>(24);
   int32_t* cursor = pool.get<int32_t>(24);
   int32_t* list = pool.get<int32_t>(std::max<int64_t>(nq, 1));
   if (pool.err) return 0;
   const unsigned gc = (unsigned)std::max<int64_t>(1, ceil_div(nq, kColorTile));
-  launch(color_count_kernel, gc, kColorThreads, st, col, nq, cnt);
+  if (front) launch(color_count_kernel<true>, gc, kColorThreads, st, col, nq, cnt);
+  else launch(color_count_kernel<false>, gc, kColorThreads, st, col, nq, cnt);
   launch(color_offsets_kernel, 1, 32, st, cnt, off, cursor);
-  launch(color_scatter_kernel, gc, kColorThreads, st, col, nq, cursor, list);
+  if (front) launch(color_scatter_kernel<true>, gc, kColorThreads, st, col, nq, cursor, list);
+  else launch(color_scatter_kernel<false>, gc, kColorThreads, st, col, nq, cursor, list);
   const unsigned gq = grid_for(std::max<int64_t>(nq, 1), sms);
-  for (int k = 0; k < 19; k++) launch(color_reduce_kernel, gq, 256, st, he, col, list, off, k, 4);
-  launch(color_reduce_kernel, gq, 256, st, he, col, list, off, 19, 3);
-  return 23;
+  const int groups = front ? kFrontGroups : kColorGroups;
+  for (int k = 0; k < groups; k++) launch(color_reduce_kernel, gq, 256, st, he, col, list, off, k, k + 1 < groups ? 4 : 3);
+  return groups + 3;
 }
 
 // Fills and one copy in one launch (16 bytes at a time; the arrays' pool blocks are whole multiples, so a
@@ -1015,7 +1033,7 @@ DmcPostStatus dmc_color_valence(const int32_t* quads, int64_t nq, int64_t nv, ui
   HeOut ho{hw.twin, hw.flag, hw.hv};
   s.launches += build_halfedges(quads, 4, nq, nv, ho, hw.w, sms, st, false);
   const HeView he{quads, hw.twin, hw.flag};
-  s.launches += color_faces(he, colors, nq, reinterpret_cast<int32_t*>(hw.zero + kZeroColors), pool, sms, st);
+  s.launches += color_faces(he, colors, nq, reinterpret_cast<int32_t*>(hw.zero + kZeroColors), false, pool, sms, st);
   if ((s.err = pool.err) != cudaSuccess) return s;
   s.launches += vertex_valence(he, hw.w.deg, nv, nq, valence, sms, st);
   s.err = cudaGetLastError();
@@ -1132,7 +1150,8 @@ DmcPostStatus dmc_postprocess(const DmcMesh& in, uint32_t flags, int sms, cudaSt
       if ((pass == 0 && !c3x3y) || (pass == 1 && !i3x3y)) continue;
       if (pass == 0) {
         Stage tm(prof, "dmc_color", st);
-        s.launches += color_faces(he, cur.colors, nq0, reinterpret_cast<int32_t*>(hw.zero + kZeroColors), pool, sms, st);
+        s.launches += color_faces(he, cur.colors, nq0, reinterpret_cast<int32_t*>(hw.zero + kZeroColors), true, pool, sms,
+                                  st);
         if ((s.err = pool.err) != cudaSuccess) return s;
       }
       {
