@@ -15,10 +15,10 @@
 //   dmc_classify_kernel  case, contours, per-cell record (counts + edge->vertex rank map) and
 //                        per-tile sums for the scan
 //   dmc_offsets_kernel   in-tile scan -> per-cell vertex / quad offsets
-//   dmc_vertex_point_kernel, dmc_vertex_w_kernel, dmc_vertex_finish_kernel
+//   dmc_vertex_point_kernel, dmc_vertex_finish_kernel
 //                        vertex representatives (cpp_dmc representative/projection) in float32
 //                        and float-float, normals, positions
-//   dmc_vertex_search_kernel  the vertices that take the whole 7x7 search
+//   dmc_vertex_search_kernel  the vertices that take the whole 7x7 search, or a coordinate in float64
 //   dmc_vertex_kernel    the vertices those leave, with every float64 fallback
 //   dmc_vertex_warp_kernel  the reference's 26x26 retry (and short lists whole), one warp per vertex
 //   dmc_quad_kernel      each cell emits the quads of its crossed interior edges 0, 3, 8 by
@@ -731,7 +731,7 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_al
 // record and case, so no polygon is walked again; the frame of the search (repr::vertex_frame) sits
 // in shared memory, a column per lane, and nothing is written to memory but the point.
 // p (local coordinates) goes to vp, or w != 0 marks what is still open: 1 the one-pass kernels' list,
-// 4 + plane the missing coordinate of dmc_vertex_w_kernel's list.
+// 4 + plane the missing coordinate of the second list (last_coordinates).
 //
 // The number of samples a lane still has to bound after its first one varies (none for 70 % of the
 // vertices of the noise field, more than ten for 1 %): looping over its own, a lane would keep its
@@ -932,14 +932,13 @@ __global__ void __launch_bounds__(kVertexThreads) dmc_vertex_point_kernel(CellSp
 // The points whose last coordinate needs float64 (mostly bilinear values exactly on a float midpoint,
 // where a box spans the whole cell and the sample coordinates are eighths), listed by
 // dmc_vertex_point_kernel: a few per cent of the vertices, so that there nearly every warp would
-// wait for the float64 pipe; here every lane has one.
-__global__ void __launch_bounds__(kVertexThreads) dmc_vertex_w_kernel(CellSpace space, const uint16_t* cellof,
-                                                                      const uint32_t* vwork, const uint32_t* wlist,
-                                                                      const unsigned* count, float4* vp,
-                                                                      unsigned long long* stats) {
-  pdl_begin();
-  const unsigned n = count[2];
-  for (unsigned a = blockIdx.x * blockDim.x + threadIdx.x; a < n; a += gridDim.x * blockDim.x) {
+// wait for the float64 pipe; here every lane has one.  It is the second half of the search kernel's launch:
+// the two lists are apart, and short ones are latency, which here runs beside the search's.  Both passes: 64^3
+// blobs 20 -> 14 us, 20-volume batch 62 -> 45 us, 131x117x140 35 -> 17 us, 512^3 noise 0.53 -> 0.48 ms.
+__device__ __forceinline__ void last_coordinates(const CellSpace& space, const uint16_t* cellof, const uint32_t* vwork,
+                                                 const uint32_t* wlist, unsigned n, float4* vp) {
+  // from the grid's end: a short search list keeps its first threads
+  for (unsigned a = (gridDim.x - 1 - blockIdx.x) * blockDim.x + threadIdx.x; a < n; a += gridDim.x * blockDim.x) {
     const uint32_t vidx = wlist[a];
     const uint32_t vcell = slot_cell(cellof, vwork[vidx]);
     const Grid& g = space.grids ? space.grids[ld(space.tile_vol + vcell / kScanTile)] : space.one;
@@ -956,7 +955,6 @@ __global__ void __launch_bounds__(kVertexThreads) dmc_vertex_w_kernel(CellSpace 
       if (d == 2 - prj) p[d] = w;
     vp[vidx] = make_float4(p[0], p[1], p[2], 0.0f);
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0 && n) atomicAdd(stats + 7, 3ull * n);
 }
 
 // The reference's float64 mean point of the contour with edge set em (n edges): its edge points summed in
@@ -1064,7 +1062,8 @@ __device__ __forceinline__ int vertex_search_frame(const Grid& g, const repr::Fr
 __global__ void __launch_bounds__(kVertexThreads) dmc_vertex_search_kernel(CellSpace space, const uint16_t* cellof,
                                                                            const uint8_t* ccase, const uint32_t* rec,
                                                                            const uint8_t* vrank, const uint32_t* vwork,
-                                                                           const uint32_t* list, unsigned* count,
+                                                                           const uint32_t* list, const uint32_t* wlist,
+                                                                           unsigned* count,
                                                                            unsigned warp_max, float4* vp, uint32_t* hard,
                                                                            unsigned long long* stats) {
   pdl_begin();
@@ -1141,6 +1140,9 @@ __global__ void __launch_bounds__(kVertexThreads) dmc_vertex_search_kernel(CellS
     append(hard, count + 3, what != repr::kFound, vidx);
   }
   if (f64) atomicAdd(stats + 7, (unsigned long long)f64);
+  const unsigned open = count[2];
+  last_coordinates(space, cellof, vwork, wlist, open, vp);
+  if (tid == 0 && open) atomicAdd(stats + 7, 3ull * open);
 }
 
 // Positions, normals and local coordinates of the projected vertices.
@@ -1494,7 +1496,6 @@ int dmc_front_emit(const CellSpace& space, DmcScratch& s, DmcVertexOut vo, int64
   // per-vertex grids: whole waves of each kernel's resident blocks
   static const int r_point = resident_blocks(dmc_vertex_point_kernel<false>, kVertexThreads);
   static const int r_point_batch = resident_blocks(dmc_vertex_point_kernel<true>, kVertexThreads);
-  static const int r_w = resident_blocks(dmc_vertex_w_kernel, kVertexThreads);
   static const int r_quad = resident_blocks(dmc_quad_kernel<false>, kQuadThreads);
   static const int r_quad_batch = resident_blocks(dmc_quad_kernel<true>, kQuadThreads);
   auto vgrid = [&](int resident) {
@@ -1512,10 +1513,8 @@ int dmc_front_emit(const CellSpace& space, DmcScratch& s, DmcVertexOut vo, int64
     // (the search takes a warp per vertex when few are listed, so as many warps as vertices may use)
     static const int r_search = resident_blocks(dmc_vertex_search_kernel, kVertexThreads);
     launch(dmc_vertex_search_kernel, (unsigned)wave_grid(r_search, sms, 1, nv, kVertexThreads), kVertexThreads, st, 
-        space, s.cellof, s.ccase, s.rec, s.vrank, s.vwork, s.fb_list, s.fb_count,
+        space, s.cellof, s.ccase, s.rec, s.vrank, s.vwork, s.fb_list, s.w_list, s.fb_count,
         (unsigned)std::min<int64_t>(tu.warp_list_max, 0x7fffffff), s.vp, s.hard_list, s.stats);
-    launch(dmc_vertex_w_kernel, (unsigned)wave_grid(r_w, sms, 1, ceil_div(nv, 10), kVertexThreads), kVertexThreads, st, 
-        space, s.cellof, s.vwork, s.w_list, s.fb_count, s.vp, s.stats);
   }
   {
     Stage t(prof, "dmc_vertex_finish", st);
@@ -1554,7 +1553,7 @@ int dmc_front_emit(const CellSpace& space, DmcScratch& s, DmcVertexOut vo, int64
   if (space.grids) DMC_QUADS(true, r_quad_batch);
   else DMC_QUADS(false, r_quad);
 #undef DMC_QUADS
-  return 7;
+  return 6;
 }
 
 int dmc_front_twins(const CellSpace& space, const DmcScratch& s, int32_t* twin, uint8_t* flag, int32_t* deg, int sms,
