@@ -977,19 +977,7 @@ __device__ __noinline__ repr::Point64 contour_mean_f64(const Grid& g, int i, int
   return r;
 }
 
-// The listed vertices that take the whole search: several samples as near as one another (exact ties of
-// symmetric contours), contours beside one that excludes samples, no sample surely valid.  The edge
-// sets, frame and bounds are the point kernel's; samples are evaluated exactly, in float64 where a
-// rounding is not certified.  What is left (no valid sample at 7x7, values at the ends of the float
-// range) goes to the one-pass kernels' list, which is empty on most fields.
-//
-// A list of more than `warp_max` entries takes one thread per vertex (bounds first, then the few
-// candidates); a shorter one takes a warp per vertex, the lanes splitting the 49 samples, because one
-// thread's search of a contour whose samples all tie lasts as long as the rest of a small call (85 us;
-// a warp's 14 us; lists of 19,000 take about as long either way).  Before, all of them took the one-pass
-// kernels (64^3 blobs 24 us, 512^3 noise 0.67 ms, 1024x1024x64 saddles 3.3 ms); now 14 us, 0.35 and
-// 0.96 ms, and the one-pass kernels get what is left (0.05 and 0.14 ms).
-// the edge sets of a cell whose record does not tell its contours apart (some unused): the contour of
+// The edge sets of a cell whose record does not tell its contours apart (some unused): the contour of
 // vertex `rank`, and the other contours of three edges
 struct ContourSets {
   uint32_t own, others[3];
@@ -1059,6 +1047,18 @@ __device__ __forceinline__ int vertex_search_frame(const Grid& g, const repr::Fr
     }
   return prj;
 }
+// The listed vertices that take the whole search: several samples as near as one another (exact ties of
+// symmetric contours), contours beside one that excludes samples, no sample surely valid.  The edge
+// sets, frame and bounds are the point kernel's; samples are evaluated exactly, in float64 where a
+// rounding is not certified.  What is left (no valid sample at 7x7, values at the ends of the float
+// range) goes to the one-pass kernels' list, which is empty on most fields.
+//
+// A list of more than `warp_max` entries takes one thread per vertex (bounds first, then the few
+// candidates); a shorter one takes a warp per vertex, the lanes splitting the 49 samples, because one
+// thread's search of a contour whose samples all tie lasts as long as the rest of a small call (85 us;
+// a warp's 14 us; lists of 19,000 take about as long either way).  Before, all of them took the one-pass
+// kernels (64^3 blobs 24 us, 512^3 noise 0.67 ms, 1024x1024x64 saddles 3.3 ms); now 14 us, 0.35 and
+// 0.96 ms, and the one-pass kernels get what is left (0.05 and 0.14 ms).
 __global__ void __launch_bounds__(kVertexThreads) dmc_vertex_search_kernel(CellSpace space, const uint16_t* cellof,
                                                                            const uint8_t* ccase, const uint32_t* rec,
                                                                            const uint8_t* vrank, const uint32_t* vwork,
