@@ -742,7 +742,7 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_al
 // field's time, where a few lanes of most warps have dozens.  The first samples pass through the same code
 // (one copy of it: with two the warps waited for instructions a quarter of the time).  The chain vertex ->
 // slot -> record and cell -> corners runs one iteration ahead, the corners into shared memory.
-// Bound by instruction issue (80 % active, 23 lanes per instruction, 72 registers).  16.6 M vertices
+// Bound by instruction issue (80 % active, 23 lanes per instruction, 64 registers).  16.6 M vertices
 // (512^3 noise): 1.78 -> 1.48 ms; 47 M (1024x1024x64 saddles): 7.66 -> 5.54 ms, with 0.13 ms more for the
 // search of what stays open; 2.2 M (256^3 noise): 0.237 -> 0.200 ms.
 // The separate set-up and projection kernels before this one (a 144-byte record per vertex written and
@@ -751,7 +751,7 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_al
 constexpr int kSampleWindow = 256;  // samples listed at a time
 constexpr int kFewSamples = 4;
 template <bool kBatch>
-__global__ void __launch_bounds__(kVertexThreads) dmc_vertex_point_kernel(CellSpace space, const uint16_t* cellof,
+__global__ void __launch_bounds__(kVertexThreads, 8) dmc_vertex_point_kernel(CellSpace space, const uint16_t* cellof,
                                                                           const uint8_t* ccase, const uint32_t* rec,
                                                                           const uint8_t* vrank, const uint32_t* vwork,
                                                                           int64_t nv, float4* vp, uint32_t* list,
@@ -1145,9 +1145,12 @@ __global__ void __launch_bounds__(kVertexThreads) dmc_vertex_search_kernel(CellS
   if (tid == 0 && open) atomicAdd(stats + 7, 3ull * open);
 }
 
-// Positions, normals and local coordinates of the projected vertices.
+// Positions, normals and local coordinates of the projected vertices.  At most 72 registers (seven blocks per
+// SM): the gradients' loads are what it waits for, and at the compiler's 109 only four blocks were there to
+// cover them (47 M vertices of the saddle field 2.86 -> 2.26 ms, 16.6 M with pair normals 1.09 -> 0.91 ms; 8
+// blocks spill more than they cover).
 template <bool kBatch, bool kFF>
-__global__ void __launch_bounds__(kVertexThreads) dmc_vertex_finish_kernel(CellSpace space, const uint16_t* cellof,
+__global__ void __launch_bounds__(kVertexThreads, 7) dmc_vertex_finish_kernel(CellSpace space, const uint16_t* cellof,
                                                                          const uint32_t* vwork,
                                                                          int64_t nv, const float4* vp,
                                                                          DmcVertexOut out, int flip_all,
