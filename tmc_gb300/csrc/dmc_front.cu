@@ -23,6 +23,7 @@
 //   dmc_vertex_warp_kernel  the reference's 26x26 retry (and short lists whole), one warp per vertex
 //   dmc_quad_kernel      each cell emits the quads of its crossed interior edges 0, 3, 8 by
 //                        looking up the cells around them
+//   dmc_twin_kernel      halfedge twins and vertex degrees of a single volume's quads
 #include <cstdio>
 
 #include "common.cuh"
@@ -182,7 +183,7 @@ __global__ void __launch_bounds__(128) dmc_amb_kernel(CellSpace space, const uin
 // Launched before the host knows the counts, with room for vcap vertices, so that it runs while the host
 // wakes, reads them and makes room for the results (70 to 90 us that the GPU waited); with more vertices it
 // does nothing and is launched again.
-// The entries per vertex, written by the lanes that scan the cells, took three quarters of the pass on dense
+// The entries per vertex, written by the lanes that scan the cells, took half of the pass on dense
 // fields (stores to 32 sectors at once); gathered and written in order: 47 M vertices 440 -> 211 us, 16.6 M
 // 158 -> 138 us.
 __global__ void __launch_bounds__(32 * kOffsetWarps, 4) dmc_offsets_kernel(const CellMask* mask, const uint32_t* rec,

@@ -7,7 +7,7 @@
 //    faces whose inherited colour is 4).  Inherited colour = 3*parity(lower grid point) + axis,
 //    and two faces sharing an edge come from two grid edges of one grid face, so they never share
 //    an inherited colour: inside one class no face reads another face's new colour.  One launch
-//    per class.
+//    per class, or per group of classes that never meet on a front-end mesh (color_class).
 //  * mergeVertices3X3Y (:916-1094): a merge reads valence >= 5 vertices and writes valence-3
 //    vertices, so reads never see writes.  Several faces writing the same vertex resolve to the
 //    highest face index (the reference's last write), via atomicMax claims.

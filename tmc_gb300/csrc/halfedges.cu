@@ -18,7 +18,7 @@
 // (valence ~4) and spatially coherent, so the pairing pass reads mostly from L2.  Sorting the few
 // ids of an edge restores the reference's insertion order.  After a simplification pass the
 // structure is repaired in place around the vertices the pass touched (repair_halfedges) instead
-// of built again.
+// of built again.  (A single volume's DMC mesh takes its twins from the cells: dmc_twin_kernel.)
 #include <climits>
 
 #include "halfedges.h"

@@ -15,7 +15,9 @@
 //   tmc_classify_kernel  per-cell record: owned crossed edges, table triangle counts; ambiguous
 //                        cells listed
 //   tmc_amb_key/cursor/sort_kernel  the ambiguous list sorted by MC case
-//   tmc_amb_count_kernel the ambiguous cells' p_slice (float64), once: counts into the cell records,
+//   tmc_amb_decide_kernel, tmc_amb_count_kernel
+//                        the ambiguous cells' p_slice once (float pairs; float64 for those left in
+//                        doubt): counts into the cell records,
 //                        triangles (local codes) and inner-vertex parameters into AmbRec records
 //   tmc_offsets_kernel   in-tile scan -> per-cell vertex / triangle offsets
 //   tmc_emit_kernel      edge vertices and table triangles
