@@ -801,6 +801,7 @@ __global__ void __launch_bounds__(kSplitThreads) triangles_kernel(const int32_t*
     }
     __syncthreads();
     const unsigned n = n_open;
+    __syncthreads();  // n_open is read before the next round's quads add to it
     if (n >= kSplitThreads || base + step >= nl) {  // block-uniform: a full round, or the last
       for (unsigned x = threadIdx.x; x < n; x += kSplitThreads) {
         const int64_t i = open[x];
