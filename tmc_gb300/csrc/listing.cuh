@@ -20,8 +20,9 @@ static_assert(kScanTile == 1 << kTileShift, "listed-cell slots assume 2048-cell 
 // the ambiguous list's counter instead of one per tile: 0.28 ms).
 // kGen: the field is generated (Grid::gen): every point is evaluated once and written to
 // Grid::gen_out for the passes that follow.
-// One launch covers planes z0 .. z1 of a single volume, or the volumes of a batch (blockIdx.y).
+// One launch covers planes z0 .. z1 of a single volume, or volumes of a batch (blockIdx.y).
 constexpr int kBitThreads = 256;
+constexpr int kMaxGridRows = 65535;  // largest gridDim.y
 template <bool kGen>
 __global__ void __launch_bounds__(kBitThreads) point_bits_kernel(Grid one, const Grid* grids, int z0, int z1) {
   pdl_begin();
@@ -88,7 +89,8 @@ __global__ void __launch_bounds__(kBitThreads) point_bits_kernel(Grid one, const
   }
 }
 
-// Launches the pass over planes z0 .. z1 of a single volume, or over all planes of a batch's volumes.
+// Launches the pass over planes z0 .. z1 of a single volume, or over all planes of a batch's volumes: a grid row
+// per volume, as many volumes to a launch as a grid has rows.
 inline int launch_point_bits(const CellSpace& space, int z0, int z1, int sms, cudaStream_t st) {
   static const int res = resident_blocks(point_bits_kernel<false>, kBitThreads);
   const bool batch = space.grids != nullptr;
@@ -96,10 +98,18 @@ inline int launch_point_bits(const CellSpace& space, int z0, int z1, int sms, cu
   const int64_t need = ceil_div(ceil_div(words, 32) + 1, kBitThreads / 32);
   // two waves; a batch shares them among its volumes (at least a block each)
   const int64_t cap = std::max<int64_t>(1, (int64_t)res * sms * 2 / space.n_volumes);
-  const dim3 grid((unsigned)std::min(need, cap), batch ? (unsigned)space.n_volumes : 1u);
-  if (space.one.gen && !batch) point_bits_kernel<true><<<grid, kBitThreads, 0, st>>>(space.one, nullptr, z0, z1);
-  else point_bits_kernel<false><<<grid, kBitThreads, 0, st>>>(space.one, space.grids, z0, z1);
-  return 1;
+  const unsigned blocks = (unsigned)std::min(need, cap);
+  if (!batch) {
+    if (space.one.gen) point_bits_kernel<true><<<blocks, kBitThreads, 0, st>>>(space.one, nullptr, z0, z1);
+    else point_bits_kernel<false><<<blocks, kBitThreads, 0, st>>>(space.one, nullptr, z0, z1);
+    return 1;
+  }
+  int k = 0;
+  for (int v = 0; v < space.n_volumes; v += kMaxGridRows, k++) {
+    const dim3 grid(blocks, (unsigned)std::min(kMaxGridRows, space.n_volumes - v));
+    point_bits_kernel<false><<<grid, kBitThreads, 0, st>>>(space.one, space.grids + v, z0, z1);
+  }
+  return k;
 }
 
 // Bits x .. x + 31 of a row (lo) and x + 1 .. x + 32 (hi); x within the row.  Reads the word after

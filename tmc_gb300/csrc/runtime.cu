@@ -739,6 +739,7 @@ tmc_status dmc_extract(tmc_ctx* ctx, const tmc_volume* vol, double iso, uint32_t
   TMC_CUDA(ctx, cudaMemcpyAsync(h, sc.totals, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
   const cudaEvent_t counted = tmc::host_mark(st);
   ctx->launches += tmc::dmc_front_offsets(space, sc, st, &ctx->prof);
+  TMC_CUDA(ctx, cudaGetLastError());  // a launch that failed: the counts are not to be used
   TMC_CUDA(ctx, tmc::host_wait_mark(counted, st));
   const int64_t nv = (int64_t)(h[0] >> 32), nq = (int64_t)(h[0] & 0xffffffffull);
 
@@ -916,6 +917,7 @@ tmc_status tmc_extract(tmc_ctx* ctx, const tmc_volume* vol, double iso, uint32_t
     TMC_CUDA(ctx, cudaMemcpyAsync(h, sc.totals, 3 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
     const cudaEvent_t counted = tmc::host_mark(st);
     ctx->launches += tmc::tmc_offsets(space, sc, st, &ctx->prof);
+    TMC_CUDA(ctx, cudaGetLastError());
     TMC_CUDA(ctx, tmc::host_wait_mark(counted, st));
     n_amb = (int64_t)(uint32_t)h[kStatAmb - kStatTotals];
     if (n_amb <= sc.amb_cap) break;
@@ -1139,6 +1141,7 @@ tmc_status batch_run(tmc_ctx* ctx, const std::vector<int>& idx, const tmc_reques
     TMC_CUDA(ctx, cudaMemcpyAsync(toff, d_voff, (nb + 3) * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
     const cudaEvent_t counted = tmc::host_mark(st);
     ctx->launches += dmc ? tmc::dmc_front_offsets(space, dsc, st, &ctx->prof) : tmc::tmc_offsets(space, tsc, st, &ctx->prof);
+    TMC_CUDA(ctx, cudaGetLastError());
     TMC_CUDA(ctx, tmc::host_wait_mark(counted, st));
     if (dmc) break;
     n_amb_rec = (int64_t)(uint32_t)toff[nb + (kStatAmb - kStatTotals)];
