@@ -449,8 +449,9 @@ __device__ __forceinline__ void vertex_outputs(const Grid& g, int i, int j, int 
     if (!p64 && !out.v64) {
       const ffx::ff t = ffx::ff_mul(ffx::two_sum((float)c, p[d]), ffx::ff{g.sp_hi[d], g.sp_lo[d]});
       const ffx::ff x = ffx::ff_add_abs(ffx::ff{g.org_hi[d], g.org_lo[d]}, t);
-      out.v[o + d] = ffx::ff_certain(x, (fabsf(g.org_hi[d]) + fabsf(t.hi)) * 0x1p-43f) ? x.hi
-                                                                                       : (float)(og + (c + (double)p[d]) * sp);
+      // below 2^-80 the pairs' low parts run into the end of the float range
+      const float mag = fabsf(g.org_hi[d]) + fabsf(t.hi);
+      out.v[o + d] = mag > 0x1p-80f && ffx::ff_certain(x, mag * 0x1p-43f) ? x.hi : (float)(og + (c + (double)p[d]) * sp);
     } else {
       const double x = og + (c + (p64 ? p64[d] : (double)p[d])) * sp;
       if (!keep64) out.v[o + d] = (float)x;
