@@ -1181,8 +1181,9 @@ __device__ __noinline__ Float3 edge_normal_precise(const Grid& g, const EdgeSten
 }
 
 // The vertex on local edge e of cell (i, j, k), written at index idx.
-// kF64: positions as t_mc (mc/MarchingCubes.cpp:241-254) in float64.  Otherwise positions within an
-// ulp (the grid coordinate i + l formed exactly as a float pair), and normals in float32, whose
+// kF64: positions as t_mc (mc/MarchingCubes.cpp:241-254) in float64.  Otherwise the edge parameter l is a
+// float32 quotient (within 2^-22) and the position within an ulp of what it gives (the grid coordinate
+// i + l formed exactly as a float pair), and normals in float32, whose
 // interpolation errs by a few ulps of its inputs' size: where the gradients cancel to below 1/16 of
 // that it would exceed ~4e-6 of the unit normal, and the float pairs take over.
 template <bool kF64>
@@ -1209,7 +1210,8 @@ __device__ __forceinline__ void edge_vertex(const Grid& g, int i, int j, int k, 
     for (int d = 0; d < 3; d++) out.n[base + d] = n.x[d];
     return;
   }
-  const float l = (g.iso_f - S.f0) / (S.f1 - S.f0);
+  // the isovalue with its remainder: near 1000 a float is 3e-5 off, a good part of a small difference
+  const float l = ((g.iso_f - S.f0) + g.iso_lo) / (S.f1 - S.f0);
 #pragma unroll
   for (int d = 0; d < 3; d++) {
     // origin + (index + l) * spacing, with index + l exact as a float pair
