@@ -1119,14 +1119,13 @@ __device__ __forceinline__ void load_stencil(const Grid& g, const int p0[3], int
   }
 }
 
-// A unit normal from the interpolated gradient in float-float: within 2^-30 of the float64 one where
-// the gradients cancel to no less than 2^-10 of their size; false below that.
-// kEach: every component within 2^-27 of itself (none cancels to below 2^-14 of its inputs), so that
-// its float32 rounding is the float64 normal's but for midpoints; else false.
-template <bool kEach>
-__device__ __forceinline__ bool edge_normal_ff(const Grid& g, const EdgeStencil& S, ffx::ff l, float out[3]) {
-  ffx::ff in[3];
-  float scale = 0;
+// The float32 normal from the gradient at edge parameter l in float pairs; false where its rounding may not be the
+// float64 normal's.  el: bound of l's error.  A component before its scaling errs by 2^-42 of its inputs' size (two
+// pair sums and a product) and by their difference times el.
+__device__ __forceinline__ bool edge_normal_ff(const Grid& g, const EdgeStencil& S, ffx::ff l, float el, float out[3]) {
+  ffx::ff in[3], n[3];
+  float e[3];
+  bool ok = true;
 #pragma unroll
   for (int d = 0; d < 3; d++) {
     const ffx::ff s{g.inv2_hi[d], g.inv2_lo[d]};
@@ -1135,21 +1134,14 @@ __device__ __forceinline__ bool edge_normal_ff(const Grid& g, const EdgeStencil&
     const ffx::ff a = ffx::two_sum(S.hi[0][d], -S.lo[0][d]), b = ffx::two_sum(S.hi[1][d], -S.lo[1][d]);
     const ffx::ff a2{a.hi * m0, a.lo * m0}, b2{b.hi * m1, b.lo * m1};
     in[d] = ffx::ff_mul(ffx::ff_add(a2, ffx::ff_mul(l, ffx::ff_sub(b2, a2))), s);
-    const float size = fmaxf(fabsf(a2.hi), fabsf(b2.hi)) * s.hi;
-    if (kEach && !(fabsf(in[d].hi) >= 0x1p-14f * size)) return false;
-    scale = fmaxf(scale, size);
+    const float size = fmaxf(fabsf(a2.hi), fabsf(b2.hi));
+    ok = ok && pair_range(size) && s.hi > 0x1p-90f;
+    e[d] = size * s.hi * (0x1p-42f + 2 * el);
   }
-  const ffx::ff dot =
-      ffx::ff_add(ffx::ff_add(ffx::ff_mul(in[0], in[0]), ffx::ff_mul(in[1], in[1])), ffx::ff_mul(in[2], in[2]));
-  // out of range (or not finite), or cancelled: float64
-  if (!(dot.hi > 0x1p-80f && dot.hi < 0x1p80f) || !(scale <= 0x1p10f * sqrtf(dot.hi))) return false;
-  // 1/sqrt(dot): float estimate and one Newton step in float-float
-  const float r0 = rsqrtf(dot.hi);
-  const ffx::ff h = ffx::ff_mul_f(ffx::ff_mul_f(dot, r0), r0);
-  const ffx::ff r = ffx::ff_mul_f(ffx::ff_sub(ffx::ff_from(1.5f), ffx::ff_mul_f(h, 0.5f)), r0);
+  ok = unit_certain(in, e, n) && ok;
 #pragma unroll
-  for (int d = 0; d < 3; d++) out[d] = ffx::ff_mul(in[d], r).hi;
-  return true;
+  for (int d = 0; d < 3; d++) out[d] = n[d].hi;
+  return ok;
 }
 
 struct Float3 {
@@ -1170,13 +1162,14 @@ __device__ __noinline__ Float3 edge_normal_f64(const Grid& g, const EdgeStencil 
   for (int d = 0; d < 3; d++) r.x[d] = (float)(in[d] / nl);
   return r;
 }
-// the same from float pairs where they serve
-template <bool kEach>
+// the same from float pairs where they decide its rounding
 __device__ __noinline__ Float3 edge_normal_precise(const Grid& g, const EdgeStencil S) {
-  const ffx::ff num = ffx::ff_sub(ffx::ff{g.iso_f, g.iso_lo}, ffx::ff_from(S.f0));
-  const ffx::ff l = ffx::ff_div(num, ffx::two_sum(S.f1, -S.f0));
+  const ffx::ff num = ffx::ff_sub(ffx::ff{g.iso_f, g.iso_lo}, ffx::ff_from(S.f0)), den = ffx::two_sum(S.f1, -S.f0);
+  const ffx::ff l = ffx::ff_div(num, den);
+  // the quotient's own error, and the isovalue's as a pair (2^-48 of it)
+  const float el = 0x1p-43f + fabsf(g.iso_f) * 0x1p-47f * fabsf(ffx::rcp_est(den.hi));
   Float3 r;
-  if (edge_normal_ff<kEach>(g, S, l, r.x)) return r;
+  if (fabsf(den.hi) > 0x1p-90f && edge_normal_ff(g, S, l, el, r.x)) return r;
   return edge_normal_f64(g, S);
 }
 
@@ -1205,7 +1198,7 @@ __device__ __forceinline__ void edge_vertex(const Grid& g, int i, int j, int k, 
       out.v[base + d] = (float)x;
       out.v64[base + d] = x;
     }
-    const Float3 n = edge_normal_precise<true>(g, S);
+    const Float3 n = edge_normal_precise(g, S);
 #pragma unroll
     for (int d = 0; d < 3; d++) out.n[base + d] = n.x[d];
     return;
@@ -1235,7 +1228,7 @@ __device__ __forceinline__ void edge_vertex(const Grid& g, int i, int j, int k, 
     for (int d = 0; d < 3; d++) out.n[base + d] = in[d] * rn;
     return;
   }
-  const Float3 n = edge_normal_precise<false>(g, S);
+  const Float3 n = edge_normal_precise(g, S);
 #pragma unroll
   for (int d = 0; d < 3; d++) out.n[base + d] = n.x[d];
 }
