@@ -552,8 +552,20 @@ __device__ __noinline__ void inner_vertex_f64(const Grid& g, int i, int j, int k
   }
 }
 
-// The same for float32 outputs in float-float (within 2^-44 of the position's size; the normal within
-// 2^-30 of the float64 one), except where the gradients cancel to below 2^-10 of their size.
+// A coordinate of an inner vertex, o + (c + t) h, in float pairs; false where its float32 rounding may not be the
+// float64 position's.  e: bound of t's error.  The pairs err by 2^-43 of the sum's terms; below 2^-80 their low
+// parts leave the float range.
+__device__ __forceinline__ bool inner_position_ff(const Grid& g, int d, int c, ffx::ff t, float e, float& out) {
+  const ffx::ff h{g.sp_hi[d], g.sp_lo[d]}, o{g.org_hi[d], g.org_lo[d]};
+  const ffx::ff y = ffx::ff_mul(ffx::ff_add(ffx::ff_from((float)c), t), h), x = ffx::ff_add(o, y);
+  const float mag = fabsf(o.hi) + fabsf(y.hi);
+  out = x.hi;
+  return mag > 0x1p-80f && ffx::ff_certain(x, mag * 0x1p-43f + e * h.hi);
+}
+
+// The same for float32 outputs in float-float: positions as float64 rounds them, normals within 2^-30 of the
+// float64 ones; in float64 where a position's rounding is left open or the gradients cancel to below 2^-10 of
+// their size.
 __device__ __noinline__ void inner_vertex_ff(const Grid& g, int i, int j, int k, ffx::ff U, ffx::ff V, ffx::ff W,
                                              const TmcVertexOut out, int64_t at) {
   auto lerp = [](ffx::ff a, ffx::ff b, ffx::ff t) {
@@ -577,23 +589,21 @@ __device__ __noinline__ void inner_vertex_ff(const Grid& g, int i, int j, int k,
                            lerp(lerp(N[4], N[5], U), lerp(N[6], N[7], U), V), W);
     in[d] = ffx::ff_mul(t, ffx::ff{g.inv2_hi[d], g.inv2_lo[d]});
   }
-  const ffx::ff dot =
-      ffx::ff_add(ffx::ff_add(ffx::ff_mul(in[0], in[0]), ffx::ff_mul(in[1], in[1])), ffx::ff_mul(in[2], in[2]));
-  if (!(dot.hi > 0x1p-80f && dot.hi < 0x1p80f) || !(scale <= 0x1p10f * sqrtf(dot.hi))) {
+  ffx::ff n[3];
+  float dot, r0, x[3];
+  unit_ff(in, n, dot, r0);
+  bool ok = dot > 0x1p-80f && dot < 0x1p80f && scale <= 0x1p10f * sqrtf(dot);
+#pragma unroll
+  for (int d = 0; d < 3; d++)
+    ok = inner_position_ff(g, d, d == 0 ? i : (d == 1 ? j : k), d == 0 ? U : (d == 1 ? V : W), 0.0f, x[d]) && ok;
+  if (!ok) {
     inner_vertex_f64(g, i, j, k, ffx::ff_to_double(U), ffx::ff_to_double(V), ffx::ff_to_double(W), out, at);
     return;
   }
-  // 1/sqrt(dot): float estimate and one Newton step in float-float
-  const float r0 = rsqrtf(dot.hi);
-  const ffx::ff h = ffx::ff_mul_f(ffx::ff_mul_f(dot, r0), r0);
-  const ffx::ff r = ffx::ff_mul_f(ffx::ff_sub(ffx::ff_from(1.5f), ffx::ff_mul_f(h, 0.5f)), r0);
 #pragma unroll
   for (int d = 0; d < 3; d++) {
-    const int c0 = d == 0 ? i : (d == 1 ? j : k);
-    const ffx::ff t = ffx::ff_add(ffx::ff_from((float)c0), d == 0 ? U : (d == 1 ? V : W));
-    const ffx::ff x = ffx::ff_add(ffx::ff{g.org_hi[d], g.org_lo[d]}, ffx::ff_mul(t, ffx::ff{g.sp_hi[d], g.sp_lo[d]}));
-    out.v[3 * at + d] = x.hi;
-    out.n[3 * at + d] = ffx::ff_mul(in[d], r).hi;
+    out.v[3 * at + d] = x[d];
+    out.n[3 * at + d] = n[d].hi;
   }
 }
 
@@ -888,15 +898,16 @@ struct IdentityVid {  // local codes: edges 0..11
 };
 
 // The inner vertex of a cell with saddle points (mc/MarchingCubes.cpp:1178-1261), from the certain
-// roots; false when a parameter is not known to 2^-28 (its bound; the value itself is some 2^-10 of that off).
+// roots, and the bound e of its parameters' errors (the values themselves are some 2^-10 of that off); false when
+// the bound is above 2^-28.
 __device__ __forceinline__ bool slice_center(unsigned q_sol, const Root u[2], const Root v[2], const Root w[2],
-                                             ffx::ff out[3]) {
+                                             ffx::ff out[3], float& e) {
   using namespace ffx;
   const unsigned f00 = q_sol & 1, f01 = (q_sol >> 1) & 1, f10 = (q_sol >> 2) & 1, f11 = (q_sol >> 3) & 1,
                  f20 = (q_sol >> 4) & 1, f21 = (q_sol >> 5) & 1;
   const unsigned fc1 = f00 * f10 + f01 * f11, fc2 = f00 * f20 + f01 * f21, fc3 = f10 * f21 + f11 * f20;
   const unsigned faces = fc1 + fc2 + fc3;
-  float e = 0;
+  e = 0;
   // s0 x0 + s1 x1
   auto pick = [&e](unsigned s0, const Root& x0, unsigned s1, const Root& x1) {
     e = fmaxf(e, (s0 ? x0.e : 0.0f) + (s1 ? x1.e : 0.0f));
@@ -977,7 +988,11 @@ __global__ void __launch_bounds__(128) tmc_amb_decide_kernel(CellSpace space, co
         slice_contours(c, cnt, IdentityVid{}, ts);
       } else {
         ffx::ff x[3];
-        ok = !pos64 && slice_center(q_sol, u, v, w, x);
+        float e, at;
+        ok = !pos64 && slice_center(q_sol, u, v, w, x, e);
+        // the emission's float32 position, from these parameters, has to be the float64 one's rounding
+#pragma unroll
+        for (int d = 0; d < 3; d++) ok = ok && inner_position_ff(g, d, d == 0 ? i : (d == 1 ? j : k), x[d], e, at);
         if (ok && slice_fans(c, cnt, IdentityVid{}, 12, ts)) {
           inner = 1;
           float2* prm = reinterpret_cast<float2*>(R.prm);
