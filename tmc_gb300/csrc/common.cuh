@@ -336,7 +336,7 @@ __device__ __forceinline__ uint64_t dmc_polygon(unsigned cs, const float u[8], d
 // unit vectors in float pairs
 // ------------------------------------------------------------------------------------------
 #ifdef __CUDACC__
-// v / |v| in float pairs: 1/sqrt from the float estimate (within 2^-22) and one Newton step, 2^-43.
+// v / |v| in float pairs: 1/sqrt from the float estimate (within 2^-22) and one Newton step; 2^-42 in all.
 __device__ __forceinline__ void unit_ff(const ffx::ff v[3], ffx::ff out[3], float& dot_hi, float& r0) {
   const ffx::ff dot =
       ffx::ff_add(ffx::ff_add(ffx::ff_mul(v[0], v[0]), ffx::ff_mul(v[1], v[1])), ffx::ff_mul(v[2], v[2]));
@@ -348,24 +348,25 @@ __device__ __forceinline__ void unit_ff(const ffx::ff v[3], ffx::ff out[3], floa
   for (int d = 0; d < 3; d++) out[d] = ffx::ff_mul(v[d], r);
 }
 // The same, and whether the results' float32 roundings are those of the exact unit vector, and so of its float64
-// evaluation: v's components are within e[d] of their exact values (e[d] = 0 only for an exact zero), which moves
-// a component of the unit vector by at most e[d] / |v| along itself and its own size times |e| / |v| with the
-// length.  Not so for lengths or components near the ends of the float range, where low parts are lost.
-__device__ __forceinline__ bool unit_certain(const ffx::ff v[3], const float e[3], ffx::ff out[3]) {
+// evaluation: v's components are within e of their exact values, which moves a component of the unit vector by at
+// most e / |v| along itself and 1.74 e / |v| times its own size with the length.  Not so for lengths or components
+// near the ends of the float range, where low parts are lost.
+__device__ __forceinline__ bool unit_certain(const ffx::ff v[3], float e, ffx::ff out[3]) {
   float dot, r0;
   unit_ff(v, out, dot, r0);
   bool ok = dot > 0x1p-80f && dot < 0x1p80f;
-  const float all = e[0] + e[1] + e[2];
+  const float er = e * r0 * 1.01f;
 #pragma unroll
   for (int d = 0; d < 3; d++) {
     const float size = fabsf(out[d].hi);
-    ok = ok && ffx::ff_certain(out[d], (e[d] + size * all) * r0 * 1.01f + size * 0x1p-42f) &&
-         (size > 0x1p-50f || (size == 0.0f && e[d] == 0.0f));
+    ok = ok && size > 0x1p-50f && ffx::ff_certain(out[d], er + size * (2 * er + 0x1p-42f));
   }
   return ok;
 }
-// differences of field values whose pair products keep their low parts
-__device__ __forceinline__ bool pair_range(float size) { return size == 0.0f || (size > 0x1p-90f && size < 0x1p90f); }
+// Pairs of differences scaled by s: whether what their low parts lose at the end of the float range is nothing beside 2^-42 of the largest scaled one, `scale`.
+__device__ __forceinline__ bool pairs_hold(float scale, const float s[3]) {
+  return scale > 0x1p-100f * fmaxf(s[0], fmaxf(s[1], s[2])) && fminf(s[0], fminf(s[1], s[2])) > 0x1p-100f;
+}
 #endif
 
 // ------------------------------------------------------------------------------------------

@@ -262,7 +262,7 @@ struct Normal64 {
 // vertices whose gradients cancel so much that the float-float result would lose its margin.
 __device__ __noinline__ Normal64 normal_f64(const Grid& g, int i, int j, int k, double pu, double pv, double pw,
                                             int flip) {
-  const double inv2d[3] = {1.0 / (2 * g.dx), 1.0 / (2 * g.dy), 1.0 / (2 * g.dz)};
+  const double* inv2d = g.inv2;
   double G[8][3];
   for (int q = 0; q < 8; q++) {
     const int a = i + (q & 1), b = j + ((q >> 1) & 1), c = k + ((q >> 2) & 1);
@@ -317,11 +317,13 @@ __device__ __forceinline__ void corner_pair(const float c[8], const AxisLines& S
   lo = up ? c[q & ~(1 << d)] : S.lo[line];
 }
 
-// The normal at local coordinates p from the corner differences, as float pairs normalised (within
-// 2^-30 of the reference's float64 normal); false where the gradients cancel to below 2^-10 of their
-// size (float64 there).
+// The normal at local coordinates p from the corner differences, as float pairs normalised; false where float64
+// has to decide.  kept: the pairs themselves are kept (within 2^-30 of the reference's float64 normal; false where
+// the gradients cancel to below 2^-10 of their size).  Otherwise their float32 roundings are wanted: false where
+// these may not be the float64 normal's.  A component errs by 42 2^-48 of its differences' size: 13 2^-48 by each of
+// three interpolations (a pair sum 3, a product 2, of the difference of up to twice the size; a sum 3), the scaling.
 __device__ __forceinline__ bool normal_ff(const Grid& g, int i, int j, int k, const float c[8], const float p[3],
-                                          int flip, ffx::ff out[3]) {
+                                          int flip, bool kept, ffx::ff out[3]) {
   ffx::ff nv3[3];
   float scale = 0;  // largest |difference| * 1/(2 spacing): the size of the interpolation's inputs
 #pragma unroll
@@ -344,15 +346,10 @@ __device__ __forceinline__ bool normal_ff(const Grid& g, int i, int j, int k, co
     const ffx::ff t = ffx::ff_mul(ff_lerp(b0, b1, p[2]), ffx::ff{g.inv2_hi[d], g.inv2_lo[d]});
     nv3[d] = flip ? ffx::ff_neg(t) : t;
   }
-  const ffx::ff dot =
-      ffx::ff_add(ffx::ff_add(ffx::ff_mul(nv3[0], nv3[0]), ffx::ff_mul(nv3[1], nv3[1])), ffx::ff_mul(nv3[2], nv3[2]));
-  // 1/sqrt(dot): float estimate and one Newton step in float-float
-  const float r0 = rsqrtf(dot.hi);
-  const ffx::ff h = ffx::ff_mul_f(ffx::ff_mul_f(dot, r0), r0);
-  const ffx::ff r = ffx::ff_mul_f(ffx::ff_sub(ffx::ff_from(1.5f), ffx::ff_mul_f(h, 0.5f)), r0);
-#pragma unroll
-  for (int d = 0; d < 3; d++) out[d] = ffx::ff_mul(nv3[d], r);
-  return dot.hi > 0x1p-80f && dot.hi < 0x1p80f && scale <= 0x1p10f * sqrtf(dot.hi);
+  if (!kept) return unit_certain(nv3, scale * 0x1.5p-43f, out) && pairs_hold(scale, g.inv2_hi);
+  float dot, r0;
+  unit_ff(nv3, out, dot, r0);
+  return dot > 0x1p-80f && dot < 0x1p80f && scale <= 0x1p10f * sqrtf(dot);
 }
 
 constexpr int kVertexThreads = 128;
@@ -425,21 +422,22 @@ __device__ __forceinline__ bool vertex_contour(const Grid& g, int i, int j, int 
 // Position, normal and local coordinates of vertex vidx at local coordinates p of cell (i, j, k).
 // p64: the float64 local coordinates when they are not the floats p (the reference's unrounded mean
 // point, for contours without any valid projection sample), else null.
-// kFF: some volume keeps normals as float pairs (simplification); the float32 normals alone otherwise
+// kFF: some volume keeps normals as float pairs (simplification), kAllKept: every one does; the float32 normals
+// alone otherwise
 // Float64 (1/57 of the float32 rate) is kept to what it must decide: positions that are float64
-// outputs, float32 positions whose rounding the float pair does not certify, normals whose gradients
-// cancel to below 2^-10 of their size.  The gradients take 32 field loads (48 point by point), one
-// axis after another (109 registers).  16.6 M vertices with float64 positions and pair normals: 1.40
+// outputs, float32 positions and normals whose rounding the float pair does not certify, kept pair
+// normals whose gradients cancel to below 2^-10 of their size.  The gradients take 32 field loads (48
+// point by point), one axis after another.  16.6 M vertices with float64 positions and pair normals: 1.40
 // -> 1.09 ms; 7.6 M with float32 outputs: 0.49 -> 0.30 ms; 47 M of the saddle field, where many
 // gradients cancel to below 1/16 (float64 normals before): 15.4 -> 2.74 ms.
-template <bool kFF = true>
+template <bool kFF = true, bool kAllKept = false>
 __device__ __forceinline__ void vertex_outputs(const Grid& g, int i, int j, int k, int64_t cell,
                                                const float p[3], const double* p64, int64_t vidx,
                                                const DmcVertexOut& out, int flip, repr::Stats& st) {
   const int64_t o = 3 * vidx;
   // a simplified volume: its float32 positions and normals are written after the passes, from the
   // float64 positions and the float-pair normals kept here
-  const bool keep64 = out.n64 && (g.flags & kGridNormal64);
+  const bool keep64 = kAllKept || (out.n64 && (g.flags & kGridNormal64));
   float2* n2 = reinterpret_cast<float2*>(out.n64);
   // position: UniformGrid::position (cpp_dmc/UniformGrid.h:300-305)
 #pragma unroll
@@ -498,7 +496,7 @@ __device__ __forceinline__ void vertex_outputs(const Grid& g, int i, int j, int 
         pairs = true;
       }
     }
-    if (!pairs) pairs = normal_ff(g, i, j, k, c, p, flip, nf);
+    if (!pairs) pairs = normal_ff(g, i, j, k, c, p, flip, kFF && keep64, nf);
   }
   if (!pairs) {
     const Normal64 n = normal_f64(g, i, j, k, p64 ? p64[0] : (double)p[0], p64 ? p64[1] : (double)p[1],
@@ -1183,7 +1181,7 @@ __global__ void __launch_bounds__(kVertexThreads, 7) dmc_vertex_finish_kernel(Ce
     int i, j, k;
     cell_ijk(g, cell, i, j, k);
     const float p[3] = {q.x, q.y, q.z};
-    vertex_outputs<kFF>(g, i, j, k, cell, p, nullptr, vidx, out, flip_all | (g.flags & kGridFlip), st);
+    vertex_outputs<kFF, kFF && !kBatch>(g, i, j, k, cell, p, nullptr, vidx, out, flip_all | (g.flags & kGridFlip), st);
   }
   flush_stats(st, stats);
 }

@@ -1135,12 +1135,11 @@ __device__ __forceinline__ void load_stencil(const Grid& g, const int p0[3], int
 }
 
 // The float32 normal from the gradient at edge parameter l in float pairs; false where its rounding may not be the
-// float64 normal's.  el: bound of l's error.  A component before its scaling errs by 2^-42 of its inputs' size (two
-// pair sums and a product) and by their difference times el.
+// float64 normal's.  el: bound of l's error.  A component errs by less than 32 2^-48 of its inputs' size (two pair
+// sums of 3 2^-48, a product of 4, the difference up to twice the size; the scaling) and by their difference times el.
 __device__ __forceinline__ bool edge_normal_ff(const Grid& g, const EdgeStencil& S, ffx::ff l, float el, float out[3]) {
   ffx::ff in[3], n[3];
-  float e[3];
-  bool ok = true;
+  float scale = 0;
 #pragma unroll
   for (int d = 0; d < 3; d++) {
     const ffx::ff s{g.inv2_hi[d], g.inv2_lo[d]};
@@ -1149,11 +1148,9 @@ __device__ __forceinline__ bool edge_normal_ff(const Grid& g, const EdgeStencil&
     const ffx::ff a = ffx::two_sum(S.hi[0][d], -S.lo[0][d]), b = ffx::two_sum(S.hi[1][d], -S.lo[1][d]);
     const ffx::ff a2{a.hi * m0, a.lo * m0}, b2{b.hi * m1, b.lo * m1};
     in[d] = ffx::ff_mul(ffx::ff_add(a2, ffx::ff_mul(l, ffx::ff_sub(b2, a2))), s);
-    const float size = fmaxf(fabsf(a2.hi), fabsf(b2.hi));
-    ok = ok && pair_range(size) && s.hi > 0x1p-90f;
-    e[d] = size * s.hi * (0x1p-42f + 2 * el);
+    scale = fmaxf(scale, fmaxf(fabsf(a2.hi), fabsf(b2.hi)) * s.hi);
   }
-  ok = unit_certain(in, e, n) && ok;
+  const bool ok = unit_certain(in, scale * (0x1p-43f + 2 * el), n) && pairs_hold(scale, g.inv2_hi);
 #pragma unroll
   for (int d = 0; d < 3; d++) out[d] = n[d].hi;
   return ok;
