@@ -50,4 +50,7 @@ tmc_status ctx_fail(tmc_ctx* ctx, tmc_status s, const char* msg);
 void ctx_count_launches(tmc_ctx* ctx, int64_t n);
 // ctx takes over from's pinned block pool (both must live on the same device)
 void ctx_share_pinned(tmc_ctx* ctx, tmc_ctx* from);
+// Device bytes a request takes at its peak: the field's copy when it is in host memory, scratch and results, from
+// the plans that the extractions allocate by, at 0.3 vertices per cell.
+int64_t request_bytes(const tmc_request& r);
 }  // namespace tmc

@@ -1041,6 +1041,12 @@ DmcPostStatus dmc_color_valence(const int32_t* quads, int64_t nq, int64_t nv, ui
   return s;
 }
 
+// what its buffers add up to, per face and per vertex
+size_t dmc_postprocess_bytes(uint32_t flags, int64_t nv, int64_t nq) {
+  const bool passes = (flags & (TMC_DMC_P3X3Y_COLOR | TMC_DMC_P3X3Y_ISOLATED | TMC_DMC_P3333)) && nq > 0;
+  return (passes ? 144 : 74) * (size_t)std::max<int64_t>(nq, 1) + (passes ? 56 : 24) * (size_t)std::max<int64_t>(nv, 1) + 64 * 256;
+}
+
 DmcPostStatus dmc_postprocess(const DmcMesh& in, uint32_t flags, int sms, cudaStream_t st, DmcPostOut* out,
                               unsigned long long* h_cnt, Prof* prof, bool borrowed, const ReadyFn* ready,
                               const TwinsFn* twins) {
@@ -1056,9 +1062,7 @@ DmcPostStatus dmc_postprocess(const DmcMesh& in, uint32_t flags, int sms, cudaSt
   }
   Pool pool(st);
   const int64_t NV = std::max<int64_t>(in.nv, 1), NQ = std::max<int64_t>(in.nq, 1);
-  // what the buffers below add up to, per face and per vertex
-  const bool passes = (c3x3y || i3x3y || p3333) && in.nq > 0;
-  pool.reserve((passes ? 144 : 74) * (size_t)NQ + (passes ? 56 : 24) * (size_t)NV + 64 * 256);
+  pool.reserve(dmc_postprocess_bytes(flags, in.nv, in.nq));
 
   DmcMesh cur = in;
   HeBufs hw = halfedge_buffers(pool, NV, NQ);

@@ -55,6 +55,9 @@ DmcPostStatus dmc_postprocess(const DmcMesh& in, uint32_t flags, int sms, cudaSt
                               unsigned long long* h_staging, Prof* prof = nullptr, bool borrowed = false,
                               const ReadyFn* ready = nullptr, const TwinsFn* twins = nullptr);
 
+// Scratch of dmc_postprocess for a mesh of nv vertices and nq quads (its results come on top).
+size_t dmc_postprocess_bytes(uint32_t flags, int64_t nv, int64_t nq);
+
 // The face colouring and vertex valence stage alone (colorFaces + vertexValence,
 // cpp_dmc/DualMarchingCubes.cpp:714-871): colors holds the inherited colours on entry and the reduced
 // ones on return; valence receives one count per vertex.  Device arrays, stream-ordered on `st`.

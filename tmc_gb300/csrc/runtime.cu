@@ -98,6 +98,20 @@ tmc_status fail(tmc_ctx* ctx, tmc_status s, const char* fmt, ...) {
     }                                                                                           \
   } while (0)
 
+// what an array of `count` elements takes in a block of several
+template <typename T>
+size_t planned_bytes(int64_t count) {
+  return ((size_t)std::max<int64_t>(count, 1) * sizeof(T) + 255) & ~(size_t)255;
+}
+// A plan (see Allocs) that only adds up its arrays' bytes.
+struct PlanBytes {
+  int64_t bytes = 0;
+  template <typename T>
+  void plan(T**, int64_t count) {
+    bytes += (int64_t)planned_bytes<T>(count);
+  }
+};
+
 // Stream-ordered allocation from the device's pool; tracked for release.
 struct Allocs {
   tmc_ctx* ctx;
@@ -120,17 +134,17 @@ struct Allocs {
   std::vector<std::pair<void**, size_t>> planned;
   template <typename T>
   void plan(T** out, int64_t count) {
-    planned.emplace_back(reinterpret_cast<void**>(out), (size_t)std::max<int64_t>(count, 1) * sizeof(T));
+    planned.emplace_back(reinterpret_cast<void**>(out), planned_bytes<T>(count));
   }
   cudaError_t commit() {
     size_t total = 0;
-    for (auto& a : planned) total += (a.second + 255) & ~(size_t)255;
+    for (auto& a : planned) total += a.second;
     char* base = nullptr;
     const cudaError_t e = get(&base, total);
     if (e == cudaSuccess)
       for (auto& a : planned) {
         *a.first = base;
-        base += (a.second + 255) & ~(size_t)255;
+        base += a.second;
       }
     planned.clear();
     return e;
@@ -147,7 +161,8 @@ struct Allocs {
 };
 
 // The records of TMC's ambiguous cells, for `cap` of them.
-void plan_tmc_ambiguous(Allocs& al, tmc::TmcScratch& sc, int64_t cap) {
+template <typename Plan>
+void plan_tmc_ambiguous(Plan& al, tmc::TmcScratch& sc, int64_t cap) {
   al.plan(&sc.amb_rec, cap * tmc::kTmcAmbRecWords);
   al.plan(&sc.amb_sorted, cap);
   al.plan(&sc.amb_key, cap);
@@ -309,7 +324,8 @@ void mesh_reset(tmc_mesh* m) { std::memset(m, 0, sizeof(*m)); }
 // per-vertex scratch of the vertex kernels
 // Scratch per vertex.  vwork and vrank come with the cells', with room for a vertex per cell, because the
 // offsets pass runs before the host knows nv; it is launched again with these when there are more.
-bool plan_dmc_vertices(Allocs& al, tmc::DmcScratch& sc, int64_t nv) {
+template <typename Plan>
+bool plan_dmc_vertices(Plan& al, tmc::DmcScratch& sc, int64_t nv) {
   const bool more = nv > sc.vcap;
   if (more) {
     al.plan(&sc.vwork, nv);
@@ -324,8 +340,9 @@ bool plan_dmc_vertices(Allocs& al, tmc::DmcScratch& sc, int64_t nv) {
   return more;
 }
 
-// per-cell scratch of the DMC / TMC front ends, and their counters (zeroed by start_counters)
-void plan_dmc_cells(tmc_ctx* ctx, Allocs& al, tmc::DmcScratch& sc, int64_t ncell, int64_t tiles) {
+// per-cell scratch of the DMC / TMC front ends
+template <typename Plan>
+void plan_dmc_cells(Plan& al, tmc::DmcScratch& sc, int64_t ncell, int64_t tiles) {
   al.plan(&sc.rec, ncell);
   al.plan(&sc.rv, ncell);
   al.plan(&sc.qoff, ncell);
@@ -337,12 +354,9 @@ void plan_dmc_cells(tmc_ctx* ctx, Allocs& al, tmc::DmcScratch& sc, int64_t ncell
   al.plan(&sc.vwork, ncell);
   al.plan(&sc.vrank, ncell);
   sc.vcap = ncell;
-  sc.stats = ctx->d_stats;
-  sc.totals = ctx->d_stats + kStatTotals;
-  sc.amb_n = reinterpret_cast<unsigned*>(ctx->d_stats + kStatAmb);
-  sc.fb_count = reinterpret_cast<unsigned*>(ctx->d_stats + kStatFallback);
 }
-void plan_tmc_cells(tmc_ctx* ctx, Allocs& al, tmc::TmcScratch& sc, int64_t ncell, int64_t tiles) {
+template <typename Plan>
+void plan_tmc_cells(Plan& al, tmc::TmcScratch& sc, int64_t ncell, int64_t tiles) {
   al.plan(&sc.rec, ncell);
   al.plan(&sc.rv, ncell);
   al.plan(&sc.toff, ncell);
@@ -352,6 +366,15 @@ void plan_tmc_cells(tmc_ctx* ctx, Allocs& al, tmc::TmcScratch& sc, int64_t ncell
   al.plan(&sc.mask, tiles * (tmc::kScanTile / 32));
   al.plan(&sc.tile_sums, tiles);
   plan_tmc_ambiguous(al, sc, tmc_ambiguous_cap(ncell));
+}
+// their counters (zeroed by start_counters)
+void counters(tmc_ctx* ctx, tmc::DmcScratch& sc) {
+  sc.stats = ctx->d_stats;
+  sc.totals = ctx->d_stats + kStatTotals;
+  sc.amb_n = reinterpret_cast<unsigned*>(ctx->d_stats + kStatAmb);
+  sc.fb_count = reinterpret_cast<unsigned*>(ctx->d_stats + kStatFallback);
+}
+void counters(tmc_ctx* ctx, tmc::TmcScratch& sc) {
   sc.stats = ctx->d_stats;
   sc.totals = ctx->d_stats + kStatTotals;
   sc.amb_n = reinterpret_cast<unsigned*>(ctx->d_stats + kStatAmb);
@@ -730,7 +753,8 @@ tmc_status dmc_extract(tmc_ctx* ctx, const tmc_volume* vol, double iso, uint32_t
   const int64_t ncell = g.ncells();
   tmc::DmcScratch sc{};
   al.plan(&g.bits, g.bit_words() + 4);
-  plan_dmc_cells(ctx, al, sc, ncell, tmc::ceil_div(ncell, tmc::kScanTile));
+  plan_dmc_cells(al, sc, ncell, tmc::ceil_div(ncell, tmc::kScanTile));
+  counters(ctx, sc);
   TMC_CUDA(ctx, al.commit());
   const tmc::CellSpace space = tmc::single_space(g);
   TMC_CUDA(ctx, start_counters(ctx));
@@ -866,7 +890,8 @@ tmc_status dmc_extract(tmc_ctx* ctx, const tmc_volume* vol, double iso, uint32_t
 }
 
 // scratch of a TMC mesh's halfedge build (nv vertices, nh halfedges)
-void plan_tmc_halfedges(Allocs& al, tmc::HeWork& w, int32_t*& twin, uint8_t*& flag, int64_t nv, int64_t nh) {
+template <typename Plan>
+void plan_tmc_halfedges(Plan& al, tmc::HeWork& w, int32_t*& twin, uint8_t*& flag, int64_t nv, int64_t nh) {
   al.plan(&w.deg, nv);
   al.plan(&w.off, nv);
   al.plan(&w.rank, nh);
@@ -904,7 +929,8 @@ tmc_status tmc_extract(tmc_ctx* ctx, const tmc_volume* vol, double iso, uint32_t
   const int64_t ncell = g.ncells();
   tmc::TmcScratch sc{};
   al.plan(&g.bits, g.bit_words() + 4);
-  plan_tmc_cells(ctx, al, sc, ncell, tmc::ceil_div(ncell, tmc::kScanTile));
+  plan_tmc_cells(al, sc, ncell, tmc::ceil_div(ncell, tmc::kScanTile));
+  counters(ctx, sc);
   TMC_CUDA(ctx, al.commit());
   const tmc::CellSpace space = tmc::single_space(g);
   TMC_CUDA(ctx, start_counters(ctx));
@@ -1091,8 +1117,10 @@ tmc_status batch_run(tmc_ctx* ctx, const std::vector<int>& idx, const tmc_reques
   al.plan(&d_tile0, nb + 1);
   al.plan(&d_voff, nb + 3);
   al.plan(&d_tile_vol, tiles);
-  if (dmc) plan_dmc_cells(ctx, al, dsc, ncell, tiles);
-  else plan_tmc_cells(ctx, al, tsc, ncell, tiles);
+  if (dmc) plan_dmc_cells(al, dsc, ncell, tiles);
+  else plan_tmc_cells(al, tsc, ncell, tiles);
+  counters(ctx, dsc);
+  counters(ctx, tsc);
   TMC_CUDA(ctx, al.commit());
   for (tmc::Grid& g : grids) {
     g.bits = bits;
@@ -1444,4 +1472,43 @@ cudaStream_t ctx_stream(const tmc_ctx* ctx) { return ctx->stream; }
 tmc_status ctx_fail(tmc_ctx* ctx, tmc_status s, const char* msg) { return fail(ctx, s, "%s", msg); }
 void ctx_count_launches(tmc_ctx* ctx, int64_t n) { ctx->launches += n; }
 void ctx_share_pinned(tmc_ctx* ctx, tmc_ctx* from) { ctx->pinned = from->pinned; }
+int64_t request_bytes(const tmc_request& r) {
+  const int64_t voxels = (int64_t)r.vol.nx * r.vol.ny * r.vol.nz;
+  const int64_t cells = (int64_t)(r.vol.nx - 1) * (r.vol.ny - 1) * (r.vol.nz - 1);
+  const int64_t tiles = ceil_div(cells, kScanTile), nv = cells * 3 / 10;
+  uint32_t f = r.flags;
+  if (f & TMC_DMC_SIMPLIFY) f |= TMC_DMC_P3X3Y_COLOR | TMC_DMC_P3X3Y_ISOLATED | TMC_DMC_P3333;
+  const bool simplify = f & (TMC_DMC_P3X3Y_COLOR | TMC_DMC_P3X3Y_ISOLATED | TMC_DMC_P3333);
+  const bool halfedges = f & TMC_OUT_HALFEDGES, f64 = f & TMC_OUT_POS_F64, triangles = f & TMC_OUT_TRIANGLES;
+  PlanBytes p;
+  uint32_t* bits = nullptr;
+  p.plan(&bits, (int64_t)r.vol.nz * r.vol.ny * ((r.vol.nx + 31) / 32) + 4);
+  int64_t b = (r.vol.on_device ? 0 : 4 * voxels) + 24 * nv;  // the field, positions and normals
+  if (r.algo == TMC_ALGO_DMC) {
+    const int64_t nq = nv;
+    DmcScratch sc{};
+    uint8_t* colors = nullptr;
+    plan_dmc_cells(p, sc, tiles * kScanTile, tiles);
+    plan_dmc_vertices(p, sc, nv);
+    p.plan(&colors, nq);
+    b += 16 * nq + (f & TMC_OUT_LOCAL ? 20 * nv : 0) + (f64 || triangles || simplify ? 24 * nv : 0);
+    if (simplify) b += (24 + 24 + (f64 ? 24 : 0)) * nv + 16 * nq;  // pair normals, and what is made anew
+    if (simplify || halfedges || triangles) b += (int64_t)dmc_postprocess_bytes(f, nv, nq);
+    if (halfedges) b += (64 + 4) * nq + 4 * nv;
+    if (triangles) b += 24 * nq;
+  } else {
+    const int64_t nt = 2 * nv, nh = 3 * nt;
+    TmcScratch sc{};
+    plan_tmc_cells(p, sc, tiles * kScanTile, tiles);
+    b += 12 * nt + (f64 ? 24 * nv : 0);
+    if (halfedges) {
+      HeWork w{};
+      int32_t* twin = nullptr;
+      uint8_t* flag = nullptr;
+      plan_tmc_halfedges(p, w, twin, flag, nv, nh);
+      b += 16 * nh + 4 * nv + 4 * nt;
+    }
+  }
+  return b + p.bytes;
+}
 }  // namespace tmc

@@ -7,9 +7,7 @@
 // admitted into the next as soon as a worker and enough of the budget are free, and their device
 // work overlaps with the running batch.
 //
-// Admission is by an estimate of each request's device footprint (field copy when the field is in
-// host memory, per-cell scratch, per-vertex scratch and outputs at a conservative surface density);
-// a request larger than the whole budget runs alone when nothing else is admitted.
+// Admission is by an estimate of each request's device footprint (tmc::request_bytes); a request larger than the whole budget runs alone when nothing else is admitted.
 //
 // The request's field must stay valid until its ticket completes.  Meshes come back through
 // tmc_server_wait and are released with tmc_server_release (they belong to a worker's context).
@@ -47,21 +45,6 @@ struct Worker {
   std::mutex lock;  // guards ctx (extraction, mesh release)
   std::thread thread;
 };
-
-// bytes per cell of device footprint at a conservative surface density (0.3 vertices per cell)
-int64_t estimate_bytes(const tmc_request& r) {
-  const int64_t voxels = (int64_t)r.vol.nx * r.vol.ny * r.vol.nz;
-  const int64_t cells = (int64_t)(r.vol.nx - 1) * (r.vol.ny - 1) * (r.vol.nz - 1);
-  int64_t b = r.vol.on_device ? 0 : 4 * voxels;
-  b += 16 * cells;                      // records, offsets, tile sums
-  const int64_t verts = cells * 3 / 10;
-  const bool dmc = r.algo == TMC_ALGO_DMC;
-  b += verts * (dmc ? 24 + 16 + 200 : 24 + 24);  // positions/normals, quads or triangles, vertex scratch
-  if (r.flags & (TMC_OUT_HALFEDGES | TMC_DMC_SIMPLIFY | TMC_DMC_P3X3Y_COLOR | TMC_DMC_P3X3Y_ISOLATED | TMC_DMC_P3333))
-    b += verts * 160;                   // halfedge build and simplification buffers
-  if (r.flags & (TMC_OUT_POS_F64 | TMC_OUT_TRIANGLES)) b += verts * 24;
-  return b;
-}
 
 // The argument checks of the extraction entry points, made at submission so that a malformed
 // request fails alone instead of failing the batch it would join.
@@ -252,7 +235,7 @@ tmc_status tmc_server_submit(tmc_server* s, const tmc_request* req, int64_t* tic
     const int64_t id = s->next_ticket++;
     Ticket& t = s->tickets[id];
     t.req = *req;
-    t.est = estimate_bytes(*req);
+    t.est = tmc::request_bytes(*req);
     t.cells = (int64_t)(req->vol.nx - 1) * (req->vol.ny - 1) * (req->vol.nz - 1);
     s->pending.push_back(id);
     s->n_submitted++;
