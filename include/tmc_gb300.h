@@ -264,7 +264,10 @@ typedef struct tmc_request {
   uint32_t algo;  /* TMC_ALGO_DMC or TMC_ALGO_TMC */
   uint32_t flags;
 } tmc_request;
-/* Extract n independent requests in one batched pipeline (device-resident fields). */
+/* Extract n independent requests in one batched pipeline (device-resident fields).  With device results
+ * (no TMC_OUT_HOST) the call returns once the meshes' sizes are known, and work queued on the context's
+ * stream writes their arrays: read them on that stream or after tmc_ctx_synchronize, and keep the fields
+ * until then or until the first of the meshes is freed (tmc_mesh_free waits for the batch). */
 tmc_status tmc_batch_extract(tmc_ctx* ctx, int32_t n, const tmc_request* reqs, tmc_mesh* outs);
 /* Autotuner (no reference counterpart): times `rounds` batched extractions of the given requests
  * for each candidate launch shape (coordinate descent over the TMC_TUNE_* keys) and keeps the

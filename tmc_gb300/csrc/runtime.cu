@@ -68,6 +68,7 @@ constexpr size_t kPinnedTables = 8192;
 struct SharedBlock {
   std::vector<void*> dev;
   cudaStream_t stream = nullptr;
+  bool in_flight = true;  // the batch's last kernels may still run, and read the caller's fields
   ~SharedBlock() {
     for (void* p : dev) cudaFreeAsync(p, stream);
   }
@@ -684,8 +685,12 @@ tmc_status tmc_mesh_free(tmc_ctx* ctx, tmc_mesh* mesh) {
   if (mp) {
     cudaSetDevice(ctx->device);
     for (void* p : mp->dev) cudaFreeAsync(p, ctx->stream);
+    // the next call may reuse these pinned blocks; a batch with device results returned before its kernels were done,
+    // and a caller who has freed its mesh may free or rewrite the field
+    const bool wait = !mp->host.empty() || (mp->shared && mp->shared->in_flight);
+    if (mp->shared) mp->shared->in_flight = false;
     mp->shared.reset();
-    if (!mp->host.empty()) tmc::host_wait(ctx->stream);  // the next call may reuse these pinned blocks
+    if (wait) tmc::host_wait(ctx->stream);
     for (void* p : mp->host) ctx->pinned_put(p);
     delete mp;
   }

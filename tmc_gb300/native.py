@@ -361,7 +361,8 @@ class Context:
         return col.cpu().numpy().astype(np.int32), val[:int(nr_v)].cpu().numpy()
 
     def batch_raw(self, volumes: list, isos: list, algos: list, flags: list) -> list:
-        """tmc_batch_extract over prepared tmc_volume structs; returns the meshes (caller frees)."""
+        """tmc_batch_extract over prepared tmc_volume structs; returns the meshes (caller frees).  Device
+        results are complete after synchronize(), or for work on the context's stream."""
         n = len(volumes)
         reqs = (Request * n)()
         for q in range(n):
