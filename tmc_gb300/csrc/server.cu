@@ -143,6 +143,19 @@ struct tmc_server {
           sts[0] = st;
           msgs[0] = tmc_last_error(W->ctx);
         }
+        // a batch with device results returns before its last kernels are done; a ticket that is done says that
+        // they are: its mesh can be read and its field given up, and its bytes are free for others
+        bool on_device = false;
+        for (const tmc_request& r : reqs) on_device = on_device || !(r.flags & TMC_OUT_HOST);
+        if (on_device && batch.size() > 1) {
+          const tmc_status done = tmc_ctx_synchronize(W->ctx);
+          for (size_t q = 0; done && q < batch.size(); q++) {
+            if (sts[q]) continue;
+            sts[q] = done;
+            msgs[q] = tmc_last_error(W->ctx);
+            tmc_mesh_free(W->ctx, &outs[q]);
+          }
+        }
       }
       {
         std::lock_guard<std::mutex> lk(m);
