@@ -139,8 +139,8 @@ __device__ __forceinline__ uint32_t tile_listed(const CellMask* mask, int64_t ti
   return a.y + __popc(a.x);
 }
 // Chunk q of 32 slots when the chunks of all tiles are walked without a list of the non-empty ones (the
-// kernels take them from the chunk list, scan.cuh).  Every tile's listed cells sit in its front slots,
-// so the chunks run over the tiles first (chunk r of a run covers slots 32 * (r / W) .. + 31 of the
+// kernels take the chunk list, scan.cuh; a CPU check holds this order).  Every tile's listed cells sit in its
+// front slots, so the chunks run over the tiles first (chunk r of a run covers slots 32 * (r / W) .. + 31 of the
 // run's tile r % W): consecutive warps take the front slots of consecutive tiles.  The runs are windows
 // of kChunkWindow consecutive tiles (a few z-planes of a volume), taken in order, so that the cells
 // processed at any moment, and the field around them, stay within a narrow band that the L2 holds.

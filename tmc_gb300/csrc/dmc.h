@@ -46,7 +46,6 @@ struct DmcScratch {
 // Each launcher returns the number of kernels it launched.  The counters (stats, totals, amb_n,
 // fb_count) are zero when a call starts.
 // Per-cell scratch is indexed in the cell space (space.n cells, padding included).
-int64_t dmc_tiles(const CellSpace& space);  // scan tiles of the space
 // gates: classify the tiles of each gate once its event has completed (a host field arriving in
 // slabs); none: the whole field is on the device
 int dmc_front_count(const CellSpace& space, DmcScratch& s, int sms, cudaStream_t st, Prof* prof = nullptr,

@@ -243,9 +243,10 @@ __global__ void __launch_bounds__(32 * kOffsetWarps, 4) dmc_offsets_kernel(const
 }
 
 // ------------------------------------------------------------------------------------------
-// vertices: one thread per output vertex (work list from the offsets kernel).  The representative
-// comes from representative_fast (dmc_repr.cuh): float32 search with certified float-float
-// rounding, bit-identical to the reference's float/double arithmetic.
+// vertices (work list from the offsets kernel): the representatives of dmc_repr.cuh, a float32 search with
+// certified float-float rounding, bit-identical to the reference's float/double arithmetic.  Its one-step
+// form makes the points of nearly all (dmc_vertex_point_kernel, dmc_vertex_search_kernel), the contours it
+// leaves take representative_7x7 and the 26x26 retry (dmc_vertex_kernel, dmc_vertex_warp_kernel).
 // ------------------------------------------------------------------------------------------
 // estimateGradient at a grid point (cpp_dmc/UniformGrid.cpp:512-540): central differences with
 // the reference's border indexing ((i<0) ? 0 : (i>=max) ? max-i : i).
@@ -429,7 +430,8 @@ __device__ __forceinline__ bool vertex_contour(const Grid& g, int i, int j, int 
 // normals whose gradients cancel to below 2^-10 of their size.  The gradients take 32 field loads (48
 // point by point), one axis after another.  16.6 M vertices with float64 positions and pair normals: 1.40
 // -> 1.09 ms; 7.6 M with float32 outputs: 0.49 -> 0.30 ms; 47 M of the saddle field, where many
-// gradients cancel to below 1/16 (float64 normals before): 15.4 -> 2.74 ms.
+// gradients cancel to below 1/16 (float64 normals before): 15.4 -> 2.49 ms with 72 registers, 10,000
+// of them in float64.
 template <bool kFF = true, bool kAllKept = false>
 __device__ __forceinline__ void vertex_outputs(const Grid& g, int i, int j, int k, int64_t cell,
                                                const float p[3], const double* p64, int64_t vidx,
@@ -1161,8 +1163,8 @@ __global__ void __launch_bounds__(kVertexThreads) dmc_vertex_search_kernel(CellS
 
 // Positions, normals and local coordinates of the projected vertices.  At most 72 registers (seven blocks per
 // SM): the gradients' loads are what it waits for, and at the compiler's 109 only four blocks were there to
-// cover them (47 M vertices of the saddle field 2.86 -> 2.26 ms, 16.6 M with pair normals 1.09 -> 0.91 ms; 8
-// blocks spill more than they cover).
+// cover them (47 M vertices of the saddle field 2.86 -> 2.26 ms, 2.49 since uncertain normals are told apart;
+// 16.6 M with pair normals 1.09 -> 0.91 ms; 8 blocks spill more than they cover).
 template <bool kBatch, bool kFF>
 __global__ void __launch_bounds__(kVertexThreads, 7) dmc_vertex_finish_kernel(CellSpace space, const uint16_t* cellof,
                                                                          const uint32_t* vwork,
@@ -1495,8 +1497,6 @@ int dmc_front_count(const CellSpace& space, DmcScratch& s, int sms, cudaStream_t
   scan_tile_sums(s.tile_sums, tiles, s.totals, st);
   return k + 1;
 }
-
-int64_t dmc_tiles(const CellSpace& space) { return ceil_div(space.n, kScanTile); }
 
 int dmc_front_offsets(const CellSpace& space, DmcScratch& s, cudaStream_t st, Prof* prof) {
   Stage t(prof, "dmc_scan", st);

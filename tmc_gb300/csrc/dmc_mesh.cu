@@ -317,7 +317,7 @@ __device__ __forceinline__ void mark(uint8_t* marks, int v, unsigned m) {
 }
 
 // Marks the removed vertices and lists the midpoint merges (destination, two sources); the
-// float64 midpoints run densely in midpoint_kernel (a few merging faces per warp would otherwise
+// midpoints run densely in midpoint_kernel (a few merging faces per warp would otherwise
 // pay the float64 pipe for the whole warp).  Each destination has one owner, and the sources are
 // never destinations (valence >= 5 vs valence 3), so the merges are independent.
 // marks: the valence-3 corners of the removed faces (merge targets and removed vertices) are touched, the

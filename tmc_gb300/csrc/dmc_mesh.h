@@ -15,7 +15,7 @@ struct DmcMesh {
   float* v = nullptr;  // null on entry to a simplification: made from v64 and n64 after the passes
   float* n = nullptr;
   double* v64 = nullptr;
-  double* n64 = nullptr;  // normals while simplifying, float pairs (hi, lo) per 8-byte slot (merges average them in float64)
+  double* n64 = nullptr;  // normals while simplifying, float pairs (hi, lo) per 8-byte slot (merges average the pairs)
   int32_t* quads = nullptr;
   uint8_t* colors = nullptr;
 };

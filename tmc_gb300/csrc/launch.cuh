@@ -12,7 +12,9 @@ namespace tmc {
 // 131x117x140 DMC with all outputs (87 kernels): 885 -> 721 us; 57x48x71 TMC with halfedges (18) 244 -> 208;
 // 64^3 DMC (12) 150 -> 134; no difference on calls of milliseconds.
 // Work that is not a kernel (copies, fills, event waits) still separates what is before it from what is
-// after; a kernel behind an event wait is launched plainly.
+// after.  A wait in the stream holds back the launch itself, early or not: an event's, or one that the memory
+// pool puts there when an allocation takes over what another stream freed (and nothing is touched before
+// pdl_begin()).  Kernels behind the code's own event waits are launched plainly all the same.
 __device__ __forceinline__ void pdl_begin() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -1306,7 +1306,8 @@ __device__ __forceinline__ void interior_vertex_ids(int64_t vcell, int cx, int64
 // search in the running counts).  Cells whose triangles overflow their records are left out
 // (tmc_ambiguous_again_kernel).  Float32 outputs take positions and normals from float pairs, one
 // axis after another (96 registers; 254 with float64 positions and all 24 gradients of a cell held
-// at once).  512^3 noise: 0.81 -> 0.41 ms; 1024x1024x64 saddles, 11 M ambiguous cells: 10.3 -> 3.2 ms.
+// at once).  512^3 noise: 0.81 -> 0.41 ms; 1024x1024x64 saddles, 11 M ambiguous cells: 10.3 -> 3.3 ms (3.2
+// before the positions' roundings were looked at).
 constexpr int kAmbThreads = 128;
 __device__ __forceinline__ int owner_of(const int32_t* upto, int t) {  // first cell with upto[cell] > t
   int o = 0;
