@@ -303,10 +303,11 @@ inline __host__ __device__ __noinline__ bool decider_ge(float f0, float f1, floa
   const ff a = two_prod(f0, f3), b = two_prod(f1, f2);
   const ff num = ff_sub(a, b);
   const ff den = ff_sub(ff_sub(ff_add(ff_from(f0), ff_from(f3)), ff_from(f1)), ff_from(f2));
-  if (den.hi != 0.0f) {
+  const float mag = fabsf(a.hi) + fabsf(b.hi);
+  // products whose low parts leave the float range (values of 1e-15 and less, of 1e18 and more) are not bounded so
+  if (den.hi != 0.0f && mag > 0x1p-95f && mag < 0x1p120f) {
     const ff q = ff_div(num, den);
     const ff d = ff_sub(q, iso_ff);
-    const float mag = fabsf(a.hi) + fabsf(b.hi);
     const float err = mag * 0x1p-44f / fabsf(den.hi) + fabsf(q.hi) * 0x1p-44f + fabsf(iso_ff.hi) * 0x1p-46f +
                       (fabsf(f0) + fabsf(f1) + fabsf(f2) + fabsf(f3)) * 0x1p-44f * fabsf(q.hi) / fabsf(den.hi);
     if (d.hi > err) return true;
