@@ -490,8 +490,8 @@ __device__ __forceinline__ void vertex_outputs(const Grid& g, int i, int j, int 
       const float dot = nv3[0] * nv3[0] + nv3[1] * nv3[1] + nv3[2] * nv3[2];
       // The float32 interpolation errs by a few ulps of `scale`; where the gradients cancel to below
       // 1/16 of it (strongly uneven spacing, near critical points) that would exceed ~4e-6 of the
-      // unit normal: float pairs instead.
-      if (scale <= 16.0f * sqrtf(dot)) {
+      // unit normal: float pairs instead, as where the squares leave the float range.
+      if (dot > 0x1p-100f && dot < 0x1p100f && scale <= 16.0f * sqrtf(dot)) {
         const float rn = rsqrtf(dot);
 #pragma unroll
         for (int d = 0; d < 3; d++) nf[d] = ffx::ff_from(nv3[d] * rn);

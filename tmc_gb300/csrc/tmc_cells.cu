@@ -1234,7 +1234,7 @@ __device__ __forceinline__ void edge_vertex(const Grid& g, int i, int j, int k, 
     scale = fmaxf(scale, fmaxf(fabsf(n0), fabsf(n1)));
   }
   const float dot = in[0] * in[0] + in[1] * in[1] + in[2] * in[2];
-  if (scale <= 16.0f * sqrtf(dot)) {
+  if (dot > 0x1p-100f && dot < 0x1p100f && scale <= 16.0f * sqrtf(dot)) {
     const float rn = rsqrtf(dot);
 #pragma unroll
     for (int d = 0; d < 3; d++) out.n[base + d] = in[d] * rn;
