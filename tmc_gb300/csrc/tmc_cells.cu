@@ -22,6 +22,8 @@
 //   tmc_offsets_kernel   in-tile scan -> per-cell vertex / triangle offsets
 //   tmc_emit_kernel      edge vertices and table triangles
 //   tmc_ambiguous_kernel the ambiguous cells' triangles and inner vertices from their records
+//   tmc_inner_again_kernel, tmc_ambiguous_again_kernel
+//                        the inner vertices and cells that need p_slice a second time
 #include "ffloat.cuh"
 #include "listing.cuh"
 #include "scan.cuh"
@@ -157,7 +159,8 @@ struct TriSink {
 //   w[0]     slot of the cell
 //   w[1]     bits 0-7 MC case, 8-13 triangles, 14-16 inner vertices, 17 triangles beyond the record
 //            (emission runs p_slice again), 18 a singular face the reference cannot triangulate,
-//            19 the parameters are float pairs (hi, lo) in the float64 slots
+//            19 the parameters are float pairs (hi, lo) in the first three float64 slots, the bound of
+//            their errors the first float of the fourth
 //   w[2..13] six float64 parameters of the inner vertices: (u, v, w) of the single inner vertex, or
 //            (u0, u1, v0, v1, w0, w1) of the six hexagon corners
 //   w[14..31] kAmbRecTris triangles as packed local codes (TriSink)
@@ -564,9 +567,13 @@ __device__ __forceinline__ bool inner_position_ff(const Grid& g, int d, int c, f
 }
 
 // The same for float32 outputs in float-float: positions as float64 rounds them, normals within 2^-30 of the
-// float64 ones; in float64 where a position's rounding is left open or the gradients cancel to below 2^-10 of
-// their size.
-__device__ __noinline__ void inner_vertex_ff(const Grid& g, int i, int j, int k, ffx::ff U, ffx::ff V, ffx::ff W,
+// float64 ones.  Writes nothing where float64 has to decide: kArithmetic, a position's rounding is left open or the
+// gradients cancel to below 2^-10 of their size.  e: bound of the parameters' errors (0: none to speak of).  Each moves a gradient component by at
+// most twice its inputs' size, so the normal by 10.4 e times their ratio to the gradient; kParameters where that may
+// be more than 2^-20 (some 2^-30 in fact; steep fields, whose parameters have to come from float64).  At 2^-24 a
+// quarter of the saddle field's are made again, 3.3 -> 4.3 ms instead of 3.45.
+enum { kDone = 0, kArithmetic = 1, kParameters = 2 };
+__device__ __noinline__ int inner_vertex_ff(const Grid& g, int i, int j, int k, ffx::ff U, ffx::ff V, ffx::ff W, float e,
                                              const TmcVertexOut out, int64_t at) {
   auto lerp = [](ffx::ff a, ffx::ff b, ffx::ff t) {
     return ffx::ff_add_abs(a, ffx::ff_mul(ffx::ff_add_abs(b, ffx::ff_neg(a)), t));
@@ -592,19 +599,18 @@ __device__ __noinline__ void inner_vertex_ff(const Grid& g, int i, int j, int k,
   ffx::ff n[3];
   float dot, r0, x[3];
   unit_ff(in, n, dot, r0);
+  if (e > 0.0f && !(10.5f * e * scale * r0 <= 0x1p-20f)) return kParameters;
   bool ok = dot > 0x1p-80f && dot < 0x1p80f && scale <= 0x1p10f * sqrtf(dot);
 #pragma unroll
   for (int d = 0; d < 3; d++)
     ok = inner_position_ff(g, d, d == 0 ? i : (d == 1 ? j : k), d == 0 ? U : (d == 1 ? V : W), 0.0f, x[d]) && ok;
-  if (!ok) {
-    inner_vertex_f64(g, i, j, k, ffx::ff_to_double(U), ffx::ff_to_double(V), ffx::ff_to_double(W), out, at);
-    return;
-  }
+  if (!ok) return kArithmetic;
 #pragma unroll
   for (int d = 0; d < 3; d++) {
     out.v[3 * at + d] = x[d];
     out.n[3 * at + d] = n[d].hi;
   }
+  return kDone;
 }
 
 __device__ void load_amb_cell(const Grid& g, int i, int j, int k, const float u[8], AmbCell& a, bool geometry) {
@@ -988,7 +994,7 @@ __global__ void __launch_bounds__(128) tmc_amb_decide_kernel(CellSpace space, co
         slice_contours(c, cnt, IdentityVid{}, ts);
       } else {
         ffx::ff x[3];
-        float e, at;
+        float e = 0, at;
         ok = !pos64 && slice_center(q_sol, u, v, w, x, e);
         // the emission's float32 position, from these parameters, has to be the float64 one's rounding
 #pragma unroll
@@ -998,6 +1004,7 @@ __global__ void __launch_bounds__(128) tmc_amb_decide_kernel(CellSpace space, co
           float2* prm = reinterpret_cast<float2*>(R.prm);
 #pragma unroll
           for (int d = 0; d < 3; d++) prm[d] = make_float2(x[d].hi, x[d].lo);
+          prm[3] = make_float2(e, 0.0f);
         }
       }
       if (ok) {
@@ -1321,7 +1328,8 @@ __global__ void __launch_bounds__(kAmbThreads) tmc_ambiguous_kernel(CellSpace sp
                                                                     const int32_t* toff,
                                                                     const unsigned long long* tile_off,
                                                                     TmcVertexOut out, int32_t* tris,
-                                                                    const AmbRec* recs, const unsigned* count) {
+                                                                    const AmbRec* recs, const unsigned* count,
+                                                                    uint32_t* open, unsigned* nopen) {
   pdl_begin();
   constexpr int kWarps = kAmbThreads / 32;
   constexpr unsigned kAll = 0xffffffffu;
@@ -1394,8 +1402,19 @@ __global__ void __launch_bounds__(kAmbThreads) tmc_ambiguous_kernel(CellSpace sp
       if ((recs[a0 + o].info >> 19) & 1) {  // float pairs: one inner vertex, float32 outputs
         const float2* x = reinterpret_cast<const float2*>(prm);
         const ffx::ff U{x[0].x, x[0].y}, V{x[1].x, x[1].y}, W{x[2].x, x[2].y};
-        inner_vertex_ff(g, c.x, c.y, c.z, U, V, W, out,
-                        (int64_t)vid[32 * 12 + o] + (int32_t)(ld(tile_off + g.vbase / kScanTile) >> 32));
+        const int64_t at = (int64_t)vid[32 * 12 + o] + (int32_t)(ld(tile_off + g.vbase / kScanTile) >> 32);
+        const int what = inner_vertex_ff(g, c.x, c.y, c.z, U, V, W, x[3].x, out, at);
+        if (what == kArithmetic)
+          inner_vertex_f64(g, c.x, c.y, c.z, ffx::ff_to_double(U), ffx::ff_to_double(V), ffx::ff_to_double(W), out, at);
+        const bool again = what == kParameters;
+        const unsigned am = __activemask(), bal = __ballot_sync(am, again);
+        if (bal) {  // for tmc_inner_again_kernel
+          const int leader = __ffs(bal) - 1;
+          unsigned base = 0;
+          if (lane == leader) base = atomicAdd(nopen, (unsigned)__popc(bal));
+          base = __shfl_sync(am, base, leader);
+          if (again) open[base + __popc(bal & ((1u << lane) - 1u))] = a0 + o;
+        }
         continue;
       }
       double u = prm[0], v = prm[1], w = prm[2];
@@ -1407,10 +1426,39 @@ __global__ void __launch_bounds__(kAmbThreads) tmc_ambiguous_kernel(CellSpace sp
       // vertices are numbered within the volume; the outputs start at its first one
       const int64_t at = (int64_t)vid[32 * (12 + q) + o] + (int32_t)(ld(tile_off + g.vbase / kScanTile) >> 32);
       // float64 outputs requested for this volume: the reference's float64 arithmetic
-      if (g.flags & kGridPos64) inner_vertex_f64(g, c.x, c.y, c.z, u, v, w, out, at);
-      else inner_vertex_ff(g, c.x, c.y, c.z, ffx::ff_from_double(u), ffx::ff_from_double(v), ffx::ff_from_double(w), out, at);
+      if ((g.flags & kGridPos64) || inner_vertex_ff(g, c.x, c.y, c.z, ffx::ff_from_double(u), ffx::ff_from_double(v),
+                                                    ffx::ff_from_double(w), 0.0f, out, at) != kDone)
+        inner_vertex_f64(g, c.x, c.y, c.z, u, v, w, out, at);
     }
     __syncwarp();  // the columns are read
+  }
+}
+
+// The inner vertices whose normals need the reference's float64 parameters (listed by tmc_ambiguous_kernel): p_slice
+// again for them, one thread per vertex.
+__global__ void __launch_bounds__(128) tmc_inner_again_kernel(CellSpace space, const uint16_t* cellof, const uint2* rv,
+                                                              TmcVertexOut out, const AmbRec* recs,
+                                                              const uint32_t* open, const unsigned* nopen) {
+  pdl_begin();
+  const unsigned n = *nopen;
+  for (unsigned x = blockIdx.x * blockDim.x + threadIdx.x; x < n; x += gridDim.x * blockDim.x) {
+    const AmbRec& R = recs[open[x]];
+    const uint32_t slot = R.slot;
+    const int64_t vcell = slot_cell(cellof, slot);
+    const uint2 r = rv[slot];
+    const Grid& g = space.grids ? space.grids[ld(space.tile_vol + vcell / kScanTile)] : space.one;
+    int i, j, k;
+    tcell_ijk(g, vcell - g.vbase, i, j, k);
+    float u[8];
+    tload_corners(g, i, j, k, u);
+    AmbCell amb;
+    load_amb_cell(g, i, j, k, u, amb, false);
+    int32_t vid[12];
+    for (int e = 0; e < 12; e++) vid[e] = e;
+    double prm[6] = {0, 0, 0, 0, 0, 0};
+    TriSink ts{nullptr, nullptr, 0};
+    p_slice_dev(R.info & 0xFF, amb.F, g.iso, vid, 12, ts, amb.P, amb.N, nullptr, prm);
+    inner_vertex_f64(g, i, j, k, prm[0], prm[1], prm[2], out, (int64_t)(int32_t)r.y + __popc(trec_owned(r.x)));
   }
 }
 
@@ -1666,11 +1714,18 @@ int tmc_emit(const CellSpace& space, TmcScratch& s, int64_t n_amb, int64_t n_ove
   static const int r_amb = resident_blocks(tmc_ambiguous_kernel, kAmbThreads);
   launch(tmc_ambiguous_kernel, (unsigned)wave_grid(r_amb, sms, 8, n_amb, kAmbThreads), kAmbThreads, st, 
       space, s.mask, s.cellof, s.rv, s.toff, s.tile_sums, vo, tris, reinterpret_cast<const AmbRec*>(s.amb_rec),
-      s.amb_n);
-  if (n_overflow == 0) return 2;
+      s.amb_n, s.amb_doubt, s.amb_hist + 513);
+  int launched = 2;
+  if (space.grids || !vo.v64) {  // float64 outputs take no parameters as pairs
+    static const int r_again = resident_blocks(tmc_inner_again_kernel, 128);
+    launch(tmc_inner_again_kernel, (unsigned)wave_grid(r_again, sms, 4, n_amb, 128), 128, st, space, s.cellof, s.rv, vo,
+           reinterpret_cast<const AmbRec*>(s.amb_rec), s.amb_doubt, s.amb_hist + 513);
+    launched++;
+  }
+  if (n_overflow == 0) return launched;
   launch(tmc_ambiguous_again_kernel, (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n_amb, 128), (int64_t)sms * 2)), 128, st, space, s.mask, s.cellof, s.rv, s.toff, s.tile_sums, vo, tris,
                                              reinterpret_cast<const AmbRec*>(s.amb_rec), s.amb_n);
-  return 3;
+  return launched + 1;
 }
 
 }  // namespace tmc

@@ -28,8 +28,9 @@ struct TmcScratch {
                         // its p_slice for the emission pass (tmc_cells.cu, AmbRec)
   uint32_t* amb_sorted; // the ambiguous cells' slots sorted by MC case (one per ambiguous cell)
   uint8_t* amb_key;     // their cases, in list order (one per ambiguous cell)
-  uint32_t* amb_doubt;  // places in amb_sorted that float pairs could not decide (one per ambiguous cell)
-  unsigned* amb_hist;   // 513: per-case counts, scatter cursors, cells in doubt
+  uint32_t* amb_doubt;  // places in amb_sorted that float pairs could not decide, then records whose inner vertex needs
+                        // float64 parameters (one per ambiguous cell)
+  unsigned* amb_hist;   // 514: per-case counts, scatter cursors, cells in doubt, inner vertices to be made again
   // listed cells (common.cuh): rec, rv and toff hold one entry per listed cell at its slot, the
   // ambiguous-cell list holds slots
   CellMask* mask;       // per 32 cells of the space
