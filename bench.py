@@ -130,10 +130,10 @@ class ClockSampler:
 # 131.1 MB field), scaled to the full launch by the units it processes (traffic grows with the
 # vertex / cell count).
 ROOFLINE_GROUPS = {
-    "dmc_vertex": (("dmc_vertex_point", "dmc_vertex_finish", "dmc_vertex"), 742.7 / 131.6),
+    "dmc_vertex": (("dmc_vertex_point", "dmc_vertex_finish", "dmc_vertex"), 746.7 / 131.6),
     "dmc_halfedges": (("dmc_halfedges",), None),
-    "tmc_emit": (("tmc_emit",), 786.4 / 267.7),
-    "dmc_classify": (("dmc_classify",), 197.1 / 131.1),
+    "tmc_emit": (("tmc_emit",), 780.5 / 267.7),
+    "dmc_classify": (("dmc_classify",), 197.3 / 131.1),
     "tmc_classify": (("tmc_classify",), None),
     "dmc_quad": (("dmc_quad",), None),
     "dmc_triangles": (("dmc_triangles",), None),
